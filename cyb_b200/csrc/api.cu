@@ -21,6 +21,56 @@ static const size_t kStatusBytes = 256 + 8 * (8 + 30000 * 8);
 static const size_t kStatusBytes = 256;
 #endif
 
+static void free_scratch(qeng_scratch* sc) {
+  for (qeng_buf* b : {&sc->planes, &sc->part})
+    if (b->ptr) cudaFree(b->ptr);
+  delete sc;
+}
+
+static bool capturing(cudaStream_t stream) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(stream, &st) == cudaSuccess && st != cudaStreamCaptureStatusNone;
+}
+
+qeng_scratch* qeng_scratch_for(qeng_ctx* ctx, cudaStream_t stream) {
+  auto& v = ctx->scratch;  // most recently used last
+  for (size_t i = v.size(); i-- > 0;)
+    if (v[i]->stream == stream) {
+      if (i + 1 != v.size()) {
+        qeng_scratch* sc = v[i];
+        v.erase(v.begin() + i);
+        v.push_back(sc);
+      }
+      return v.back();
+    }
+  // A captured stream is usually one of its own: the calls before the capture, on another stream, made the buffers.
+  if (capturing(stream)) return v.empty() ? nullptr : v.back();
+  if (v.size() >= (size_t)kMaxScratch) {
+    cudaDeviceSynchronize();  // its stream may still be running
+    free_scratch(v.front());
+    v.erase(v.begin());
+    ctx->scratch_gen++;
+  }
+  v.push_back(new qeng_scratch());
+  v.back()->stream = stream;
+  return v.back();
+}
+
+// Grows outside the steady state only; a growing call drains the device first.
+int32_t qeng_scratch_grow(qeng_ctx* ctx, qeng_buf* b, size_t bytes, cudaStream_t stream) {
+  if (bytes <= b->bytes) return QENG_OK;
+  if (capturing(stream))
+    return qeng_fail(ctx, QENG_ERR_STATE, "scratch of %zu bytes needed inside a stream capture: make one call of the shape before capturing", bytes);
+  QENG_CUDA(ctx, cudaDeviceSynchronize());
+  if (b->ptr) cudaFree(b->ptr);
+  b->ptr = nullptr;
+  b->bytes = 0;
+  ctx->scratch_gen++;
+  QENG_CUDA(ctx, cudaMalloc(&b->ptr, bytes));
+  b->bytes = bytes;
+  return QENG_OK;
+}
+
 extern "C" {
 
 int32_t qeng_version(void) { return 100; }
@@ -81,7 +131,7 @@ int32_t qeng_destroy(qeng_ctx* ctx) {
   qeng_tp_release(ctx);
   if (ctx->attn_scratch) cudaFree(ctx->attn_scratch);
   if (ctx->status) cudaFree(ctx->status);
-  if (ctx->xbf16) cudaFree(ctx->xbf16);
+  for (qeng_scratch* sc : ctx->scratch) free_scratch(sc);
   if (ctx->ximage) cudaFree(ctx->ximage);
   if (ctx->tail_val) cudaFree(ctx->tail_val);
   if (ctx->tail_idx) cudaFree(ctx->tail_idx);

@@ -334,7 +334,7 @@ int32_t run_layer_prefill(qeng_ctx* ctx, qeng_decoder* d, int l, int64_t rows, c
   const bool tp = d->cfg.tp_world > 1;
   __half* pool = d->pool + (size_t)l * d->pages * d->Hkv * 2 * kPage * kHD;
   int32_t rc = qeng_rmsnorm(ctx, d->x, L.norm1, rows, dm, d->cfg.rms_eps, d->xnr, st);
-  if (rc == QENG_OK) rc = qeng_gemm_q4_prefill(ctx, L.wqkv, d->xnr, QENG_F32, rows, dm, d->qkv, d->nqkv, 0, st);
+  if (rc == QENG_OK) rc = qeng_gemm_many_rows(ctx, L.wqkv, d->xnr, QENG_F32, rows, dm, d->qkv, d->nqkv, 0, 1, st);
   if (rc != QENG_OK) return rc;
   rope_append_kernel<<<(unsigned)rows, 256, 0, st>>>(d->qkv, d->rope_cs, d->pos, table, d->max_pages, (int)d->pages,
                                                      d->Hq, d->Hkv, d->cfg.max_seq, d->q16, pool, ctx->status, L.qnorm, L.knorm, d->cfg.rms_eps);
@@ -349,8 +349,8 @@ int32_t run_layer_prefill(qeng_ctx* ctx, qeng_decoder* d, int l, int64_t rows, c
   }
   const int64_t n = rows * dm;
   auto row_split_tc = [&](const qeng_weight* w, const float* in, int64_t ldin) -> int32_t {
-    if (!tp) return qeng_gemm_q4_prefill(ctx, w, in, QENG_F32, rows, ldin, d->x, dm, 1, st);
-    int32_t r = qeng_gemm_q4_prefill(ctx, w, in, QENG_F32, rows, ldin, d->part, dm, 0, st);
+    if (!tp) return qeng_gemm_many_rows(ctx, w, in, QENG_F32, rows, ldin, d->x, dm, 1, 1, st);
+    int32_t r = qeng_gemm_many_rows(ctx, w, in, QENG_F32, rows, ldin, d->part, dm, 0, 1, st);
     if (r == QENG_OK) r = qeng_tp_all_reduce_internal(ctx, d->part, n, st);
     if (r != QENG_OK) return r;
     add_inplace_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(d->x, d->part, n);
@@ -358,7 +358,7 @@ int32_t run_layer_prefill(qeng_ctx* ctx, qeng_decoder* d, int l, int64_t rows, c
   };
   rc = row_split_tc(L.wo, d->att, nq);
   if (rc == QENG_OK) rc = qeng_rmsnorm(ctx, d->x, L.norm2, rows, dm, d->cfg.rms_eps, d->xnr, st);
-  if (rc == QENG_OK) rc = qeng_gemm_q4_prefill(ctx, L.wgu, d->xnr, QENG_F32, rows, dm, d->gu, 2 * d->F, 0, st);
+  if (rc == QENG_OK) rc = qeng_gemm_many_rows(ctx, L.wgu, d->xnr, QENG_F32, rows, dm, d->gu, 2 * d->F, 0, 1, st);
   if (rc != QENG_OK) return rc;
   const int64_t na = rows * d->F;
   swiglu_interleaved_kernel<<<(unsigned)((na + 255) / 256), 256, 0, st>>>(d->gu, rows, d->F, d->act);

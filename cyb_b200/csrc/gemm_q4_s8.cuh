@@ -111,8 +111,8 @@ __device__ __forceinline__ void imma(int (&d)[4], uint32_t a0, uint32_t a1, uint
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 // one 32-block of 16 weight rows: lane (g, t) holds w0 = codes of row g, w1 = codes of row g+8, each
-// the 8 codes of k = 8t + j in nibble j.  The even nibbles (j = 0,2,4,6) land in the MMA's k slots
-// 4t..4t+3, the odd ones in 16+4t..16+4t+3; the staged activation bytes use the same order.
+// the 8 codes of k = 8t + j in nibble qeng_nib(j).  The even nibbles (j = 0,4,1,5) land in the MMA's k
+// slots 4t..4t+3, the odd ones (j = 2,6,3,7) in 16+4t..16+4t+3; the staged activation bytes use the same order.
 __device__ __forceinline__ void block_mma(int (&d)[4], uint32_t w0, uint32_t w1, uint32_t b0, uint32_t b1) {
   const uint32_t m = 0x0f0f0f0fu;
   imma(d, w0 & m, w1 & m, (w0 >> 4) & m, (w1 >> 4) & m, b0, b1);
@@ -126,7 +126,7 @@ __device__ __forceinline__ void imma_s8(int (&d)[4], uint32_t a0, uint32_t a1, u
 }
 // Weight format of a matmul: Q4 = 4-bit codes (two 32-blocks per uint4 and lane, 512 B per 64-wide
 // chunk of a row tile); Q8 = signed bytes (one 32-block per uint4 and lane: the bytes of row g at
-// k = 8t + 0,2,4,6, of row g+8 likewise, then k = 8t + 1,3,5,7 of both rows, i.e. the A registers of
+// k = 8t + 0,4,1,5, of row g+8 likewise, then k = 8t + 2,6,3,7 of both rows, i.e. the A registers of
 // the MMA in the k order the staged activations use; 1024 B per chunk).  Both carry the same scale
 // plane.  `WBlocks` holds the two blocks of one chunk for this lane.
 template <bool Q8>
@@ -195,7 +195,7 @@ __device__ __forceinline__ float act_f32(const void* x, int dtype, long long i) 
 
 // Shared-memory geometry of the staged activations of one K slice (bytes, relative to `base`).
 //   xq   : [cols][col_stride]  s8 bytes; column c = 2 * row + limb; inside a column the 32 bytes of
-//          block b start at 32 b: [t 0..3][k = 8t + 0,2,4,6,1,3,5,7]
+//          block b start at 32 b: [t 0..3][k = 8t + 0,4,1,5,2,6,3,7]
 //   zero : col_stride bytes of zeros (only when several blocks share a fragment)
 //   zin  : [cols][nblk] int32   kBias - 8 * (sum of the column's bytes in the block)
 //   fex  : [cols][nblk] float   2^e (x 128 for the hi limb), 0 for blocks beyond K
@@ -274,7 +274,7 @@ __device__ __forceinline__ void quantise_group(const float (&v)[8], bool valid, 
   int q[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) q[i] = min(__float_as_int(fmaf(v[i], inv, kBiasF)) - (int)kBias, kMaxQ);
-  uint32_t w0[LIMBS], w1[LIMBS];  // bytes of k = 0,2,4,6 and of k = 1,3,5,7, per limb
+  uint32_t w0[LIMBS], w1[LIMBS];  // bytes of k = 0,4,1,5 and of k = 2,6,3,7 (even and odd nibbles), per limb
   int sum[LIMBS];
 #pragma unroll
   for (int l = 0; l < LIMBS; ++l) {
@@ -282,8 +282,8 @@ __device__ __forceinline__ void quantise_group(const float (&v)[8], bool valid, 
     uint32_t d[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) d[i] = l == 0 ? (uint32_t)(q[i] >> sh) : (uint32_t)((q[i] >> sh) & 127);
-    w0[l] = __byte_perm(__byte_perm(d[0], d[2], 0x0040), __byte_perm(d[4], d[6], 0x0040), 0x5410);
-    w1[l] = __byte_perm(__byte_perm(d[1], d[3], 0x0040), __byte_perm(d[5], d[7], 0x0040), 0x5410);
+    w0[l] = __byte_perm(__byte_perm(d[0], d[4], 0x0040), __byte_perm(d[1], d[5], 0x0040), 0x5410);
+    w1[l] = __byte_perm(__byte_perm(d[2], d[6], 0x0040), __byte_perm(d[3], d[7], 0x0040), 0x5410);
     sum[l] = __dp4a((int)w0[l], 0x01010101, __dp4a((int)w1[l], 0x01010101, 0));
   }
   // sums over the quad: the most significant limb is signed and (with three limbs) travels alone; the

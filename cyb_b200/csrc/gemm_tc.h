@@ -1,0 +1,30 @@
+// Tensor-core matmul of many activation rows (gemm_tc.cu) and the per-stream scratch it works in.
+#pragma once
+#include <cuda_bf16.h>
+
+#include "qeng_internal.h"
+
+// What happens to the finished sums of a tile.
+struct qeng_tc_epi {
+  int kind = QENG_EPI_STORE;  // STORE, ACCUM (y += ...), SWIGLU (N/2 columns out), QKV (rotary, q16 and KV pages)
+  float* y = nullptr;
+  long long ldy = 0;
+  // SWIGLU only: the result as one or two bf16 planes (the operand of the next matmul) instead of f32
+  __nv_bfloat16* yb = nullptr;
+  long long ldyb = 0, yb_plane = 0;
+  int yb_planes = 1;
+  qeng_qkv_epi qkv = {};
+};
+
+// Activations as bf16 planes: value = plane 0 (+ plane 1), rows `ld` apart, planes `plane` elements apart.
+struct qeng_tc_x {
+  const void* data = nullptr;
+  long long ld = 0, plane = 0;
+  int planes = 1;
+};
+
+// wp = 1: weights rounded to bf16 (4-bit blocks only); wp = 2: weights as two bf16 terms
+int32_t qeng_gemm_tc(qeng_ctx* ctx, const qeng_weight* w, const qeng_tc_x& x, int64_t M, int wp, const qeng_tc_epi& epi, cudaStream_t stream);
+// rows of x (any type), RMS-normalised if gamma is given -> `planes` bf16 planes [M][K]
+int32_t qeng_tc_prep(qeng_ctx* ctx, const void* x, int32_t dtype, int64_t M, int64_t K, int64_t ldx, const float* gamma, float eps,
+                     int planes, void* out, cudaStream_t stream);

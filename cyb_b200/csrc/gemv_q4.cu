@@ -70,14 +70,6 @@ __device__ __forceinline__ float load_act(const void* x, int dtype, long long i)
   return __uint_as_float(u);
 }
 
-// position of k (relative to the slice start) inside the staged f16 row: the
-// eight values of one (block, t) group are stored in the order 0,4,1,5,2,6,3,7
-// so that one 128-bit shared load yields the four B registers of both MMAs.
-__device__ __forceinline__ int stage_pos(int kk) {
-  int j = kk & 7;
-  return (kk & ~7) + ((j & 3) << 1) + (j >> 2);
-}
-
 template <int NT, int U>
 __global__ void __launch_bounds__(kThreads) gemv_q4_kernel(const GemvParams p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -151,14 +143,13 @@ __global__ void __launch_bounds__(kThreads) gemv_q4_kernel(const GemvParams p) {
             v = load_act(p.x, p.x_dtype, (long long)m * p.ldx + k);
             if (p.gamma != nullptr) v = v * rinv[m] * p.gamma[k];
           }
-          int pos = stage_pos(kk);
           if (p.split) {
             __half hi = __float2half_rn(v);
             __half lo = __float2half_rn(v - __half2float(hi));
-            xs_h[(size_t)(2 * m) * CS + pos] = hi;
-            xs_h[(size_t)(2 * m + 1) * CS + pos] = lo;
+            xs_h[(size_t)(2 * m) * CS + kk] = hi;
+            xs_h[(size_t)(2 * m + 1) * CS + kk] = lo;
           } else {
-            xs_h[(size_t)m * CS + pos] = __float2half_rn(v);
+            xs_h[(size_t)m * CS + kk] = __float2half_rn(v);
           }
         }
         __syncthreads();
@@ -349,8 +340,12 @@ int32_t qeng_gemm_q4(qeng_ctx* ctx, const qeng_weight* w, const void* x, int32_t
   if (M < 1) return qeng_fail(ctx, QENG_ERR_SHAPE, "gemm_q4: M=%lld", (long long)M);
   if (ldx < w->K || ldy < w->N) return qeng_fail(ctx, QENG_ERR_SHAPE, "gemm_q4: leading dimension smaller than the row");
   QENG_ENTER(ctx);
-  if (M >= kPrefillRows && w->fmt == QENG_FMT_Q4)  // dense contraction: dequantise to bf16 in shared memory, tcgen05 MMA
-    return qeng_gemm_q4_prefill(ctx, w, x, x_dtype, M, ldx, y, ldy, (flags & QENG_GEMM_ACCUMULATE) ? 1 : 0, (cudaStream_t)stream);
+  if (M >= kManyRows) {  // dense contraction: dequantise to bf16 in shared memory, tcgen05 MMA
+    const bool prompt = M >= kPrefillRows && w->fmt == QENG_FMT_Q4;
+    if (prompt && x_dtype == QENG_F16)
+      return qeng_fail(ctx, QENG_ERR_SHAPE, "gemm_q4 (prefill): f16 activations are not supported, use f32 or bf16");
+    return qeng_gemm_many_rows(ctx, w, x, x_dtype, M, ldx, y, ldy, (flags & QENG_GEMM_ACCUMULATE) ? 1 : 0, prompt ? 1 : 2, (cudaStream_t)stream);
+  }
   qeng_gemm_fuse fuse;
   fuse.epilogue = (flags & QENG_GEMM_ACCUMULATE) ? QENG_EPI_ACCUM : QENG_EPI_STORE;
   fuse.two_limbs = (flags & QENG_GEMM_FAST_F16) != 0;

@@ -43,7 +43,7 @@ inline float half_bits_to_float(uint16_t h) {
 
 inline uint32_t pack8(const uint8_t* p) {
   uint32_t w = 0;
-  for (int j = 0; j < 8; j++) w |= (uint32_t)(p[j] & 15u) << (4 * j);
+  for (int j = 0; j < 8; j++) w |= (uint32_t)(p[j] & 15u) << (4 * qeng_nib(j));
   return w;
 }
 
@@ -61,7 +61,7 @@ __global__ void unpack_k4_kernel(const uint4* __restrict__ qs, const float* __re
   const uint32_t w = lane[b1 * 2 + hi];
   uint8_t* dst = q + n * K + wk * 8;
 #pragma unroll
-  for (int j = 0; j < 8; j++) dst[j] = (uint8_t)((w >> (4 * j)) & 15u);
+  for (int j = 0; j < 8; j++) dst[j] = (uint8_t)((w >> (4 * qeng_nib(j))) & 15u);
   if (t == 0) {
     const float* sp = sc + ((tile * nchunks + chunk) * 8 + g) * 8;
     dm[(n * (K / 32) + blk) * 2] = sp[b1 * 2 + hi];
@@ -85,7 +85,7 @@ __global__ void dequant_k4_kernel(const uint4* __restrict__ qs, const float* __r
   const float D = sp[b1 * 2 + hi], M = sp[4 + b1 * 2 + hi];
   float* dst = out + n * K + wk * 8;
 #pragma unroll
-  for (int j = 0; j < 8; j++) dst[j] = __fsub_rn(__fmul_rn(D, (float)((w >> (4 * j)) & 15u)), M);
+  for (int j = 0; j < 8; j++) dst[j] = __fsub_rn(__fmul_rn(D, (float)((w >> (4 * qeng_nib(j))) & 15u)), M);
 }
 
 }  // namespace

@@ -11,10 +11,10 @@
 
 namespace {
 
-// one 32-bit word = codes of k0..k0+7 of one row, nibble j = code[k0+j]
+// one 32-bit word = codes of k0..k0+7 of one row, code[k0+j] in nibble qeng_nib(j)
 inline uint32_t pack8(const uint8_t* p) {
   uint32_t w = 0;
-  for (int j = 0; j < 8; j++) w |= (uint32_t)(p[j] & 15u) << (4 * j);
+  for (int j = 0; j < 8; j++) w |= (uint32_t)(p[j] & 15u) << (4 * qeng_nib(j));
   return w;
 }
 
@@ -34,7 +34,7 @@ __global__ void unpack_q4_kernel(const uint4* __restrict__ qs, const uint2* __re
   uint32_t w = lane[b1 * 2 + hi];
   uint8_t* dst = q + n * K + wk * 8;
 #pragma unroll
-  for (int j = 0; j < 8; j++) dst[j] = (uint8_t)((w >> (4 * j)) & 15u);
+  for (int j = 0; j < 8; j++) dst[j] = (uint8_t)((w >> (4 * qeng_nib(j))) & 15u);
   if (t == 0) {
     const uint16_t* sp = reinterpret_cast<const uint16_t*>(sc + (tile * nchunks + chunk) * 8 + g);
     s[n * (K / 32) + blk] = sp[b1 * 2 + hi];
@@ -57,7 +57,7 @@ __global__ void dequant_q4_kernel(const uint4* __restrict__ qs, const uint2* __r
   float scale = __half2float(sp[b1 * 2 + hi]);
   float* dst = out + n * K + wk * 8;
 #pragma unroll
-  for (int j = 0; j < 8; j++) dst[j] = (float)((int)((w >> (4 * j)) & 15u) - 8) * scale;
+  for (int j = 0; j < 8; j++) dst[j] = (float)((int)((w >> (4 * qeng_nib(j))) & 15u) - 8) * scale;
 }
 
 // Import-time quantiser: one warp per (row tile, 64-wide chunk) writes its 512 bytes of the nibble
@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(256) quantize_q4_kernel(const void* __restrict
     for (int j = 0; j < 8; ++j) {
       int q = (int)__fadd_rn(__fmul_rn(v[j], inv), 8.5f);
       q = q > 15 ? 15 : (q < 0 ? 0 : q);
-      w |= (uint32_t)q << (4 * j);
+      w |= (uint32_t)q << (4 * qeng_nib(j));
     }
     words[idx] = w;
     sbits[idx] = (uint32_t)__half_as_ushort(__float2half_rn(d));

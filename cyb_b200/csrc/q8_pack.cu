@@ -27,8 +27,8 @@ __host__ __device__ inline size_t q8_pos(int64_t n, int64_t k, int64_t nchunks) 
   const int64_t tile = n / 16, r = n % 16, g = r % 8, hi = r / 8;
   const int64_t blk = k / 32, kk = k % 32, t = kk / 8, j = kk % 8;
   const int64_t chunk = blk / 2, b1 = blk % 2;
-  const int64_t word = (j & 1) * 2 + hi;  // x, y: even k; z, w: odd k
-  return (size_t)(((tile * nchunks + chunk) * 2 + b1) * 32 + g * 4 + t) * 16 + (size_t)word * 4 + (size_t)(j >> 1);
+  const int64_t nib = qeng_nib((int)j), word = (nib & 1) * 2 + hi;  // the byte order of the unpacked 4-bit codes
+  return (size_t)(((tile * nchunks + chunk) * 2 + b1) * 32 + g * 4 + t) * 16 + (size_t)word * 4 + (size_t)(nib >> 1);
 }
 
 __global__ void unpack_q8_kernel(const unsigned char* __restrict__ qs, const uint2* __restrict__ sc, int64_t N, int64_t K,

@@ -17,13 +17,17 @@
 //    g = lane/4, t = lane%4 the four words are
 //       .x = row g   , block 2c      .y = row g+8 , block 2c
 //       .z = row g   , block 2c+1    .w = row g+8 , block 2c+1
-//    and each word holds the codes of k = 32*block + 8*t + j in nibble j
-//    (bits 4j..4j+3).  One warp-wide 128-bit load therefore fetches 512
+//    and each word holds the codes of k = 32*block + 8*t + j in nibble
+//    qeng_nib(j): the pairs (0,1), (2,3), (4,5), (6,7) sit 16 bits apart, so
+//    that one AND leaves two consecutive k in the halves of a register, the
+//    order a 16-bit MMA operand is stored in.  One warp-wide 128-bit load fetches 512
 //    contiguous bytes and every lane receives exactly the A-fragment words of
 //    an m16n8k16 MMA over that chunk;
 //  * scale plane: [tile][chunk][g 0..7] one uint2 = four f16:
 //       (row g, blk 2c), (row g+8, blk 2c), (row g, blk 2c+1), (row g+8, blk 2c+1).
 enum { QENG_FMT_Q4 = 0, QENG_FMT_Q8 = 1, QENG_FMT_K4 = 2 };
+
+__host__ __device__ inline int qeng_nib(int j) { return (j >> 1) + 4 * (j & 1); }
 
 struct qeng_weight {
   int fmt = QENG_FMT_Q4;  // Q4: 4-bit codes, w = (c - 8) s; Q8: signed bytes, w = q s (both: one f16 s per 32-block);
@@ -34,12 +38,27 @@ struct qeng_weight {
   uint4* qs;           // weight plane: Q4 ntiles*nchunks*32 uint4 (nibbles), Q8 ntiles*nchunks*64 uint4 (bytes)
   uint2* sc;           // scale plane,  ntiles*nchunks*8 uint2 (K4: ntiles*nchunks*256 bytes)
   int64_t bytes;       // device bytes held
+  // tensor maps of both planes for the tensor-core matmul (gemm_tc.cu), encoded on first use: [1 or 2 chunks per box][codes, scales]
+  mutable bool tc_maps_ready = false;
+  alignas(64) mutable unsigned char tc_maps[2][2][128];
   const qeng_weight* next = nullptr;  // matrix the caller multiplies by after this one (L2 prefetch hint)
 };
 
 struct qeng_kv_pool {
   int64_t pages, kv_heads, hd;
   __half* data;        // [pages][kv_heads][2][16][hd]
+};
+
+// Device buffer that only ever grows.
+struct qeng_buf {
+  void* ptr = nullptr;
+  size_t bytes = 0;
+};
+// Working memory of one stream's calls: calls on different streams of a context do not share it.
+struct qeng_scratch {
+  cudaStream_t stream = nullptr;
+  qeng_buf planes;    // activations as bf16 planes
+  qeng_buf part;      // partial sums of tiles cut along K
 };
 
 struct qeng_ctx {
@@ -50,9 +69,8 @@ struct qeng_ctx {
   float* attn_scratch = nullptr;
   size_t attn_scratch_bytes = 0;
   int32_t* status = nullptr;  // device status word (0 = ok)
-  // bf16 copy of f32 activations for the tensor-core prefill matmul
-  void* xbf16 = nullptr;
-  size_t xbf16_bytes = 0;
+  // working memory of the tensor-core matmul, one set per stream that calls it (qeng_scratch_for)
+  std::vector<qeng_scratch*> scratch;
   // activations quantised once per decode-batch matmul (more than 4 rows), one image per K slice
   void* ximage = nullptr;
   size_t ximage_bytes = 0;
@@ -220,10 +238,18 @@ const unsigned* qeng_tp_fuse_seq(const qeng_ctx* ctx);
 int32_t qeng_tp_fuse_gather(qeng_ctx* ctx, float* x, int64_t rows, int64_t dm, int kind, int layer, int layers, cudaStream_t stream);
 int32_t qeng_tp_fuse_advance(qeng_ctx* ctx, cudaStream_t stream);
 
-// gemm_q4_tc.cu: tcgen05 prefill matmul (bf16 operands, f32 accumulation in tensor memory)
-int32_t qeng_gemm_q4_prefill(qeng_ctx* ctx, const qeng_weight* w, const void* x, int32_t x_dtype, int64_t M, int64_t ldx,
-                             float* y, int64_t ldy, int accumulate, cudaStream_t stream);
-constexpr int64_t kPrefillRows = 256;  // from this many rows on, matmuls take the tensor-core path
+// api.cu: the scratch of a stream (made on first use, at most kMaxScratch sets per context, the least recently
+// used one given back); null inside a stream capture when the context has none yet.
+constexpr int kMaxScratch = 8;
+qeng_scratch* qeng_scratch_for(qeng_ctx* ctx, cudaStream_t stream);
+int32_t qeng_scratch_grow(qeng_ctx* ctx, qeng_buf* b, size_t bytes, cudaStream_t stream);
+
+// gemm_tc.cu: tcgen05 matmul of many rows.  wp = 1: bf16 operands; wp = 2: two bf16 terms per weight and per
+// f32 / f16 activation
+int32_t qeng_gemm_many_rows(qeng_ctx* ctx, const qeng_weight* w, const void* x, int32_t x_dtype, int64_t M, int64_t ldx,
+                            float* y, int64_t ldy, int accumulate, int wp, cudaStream_t stream);
+constexpr int64_t kPrefillRows = 256;  // from this many rows on, 4-bit matmuls run on operands rounded to bf16
+constexpr int64_t kManyRows = 17;      // from this many rows on, matmuls take the tensor-core path
 
 void qeng_weight_dequant_q8(const qeng_weight* w, float* out, cudaStream_t stream);
 void qeng_weight_dequant_k4(const qeng_weight* w, float* out, cudaStream_t stream);

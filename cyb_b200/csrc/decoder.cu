@@ -14,7 +14,8 @@
 
 #include <vector>
 
-#include "qeng_internal.h"
+#include "attn_prefill.h"
+#include "gemm_tc.h"
 
 namespace {
 
@@ -38,6 +39,7 @@ struct Layer {
   float* norm2 = nullptr;
   float *qnorm = nullptr, *knorm = nullptr;  // optional per-head gains [128] (QK-norm)
   HostMat pend[7];  // host shards waiting for their fusion partners
+  alignas(64) unsigned char kv_map[128];  // tensor map of this layer's KV pages
 };
 
 // rows of q|k|v (f32, straight from the QKV matmul) -> rotated q as f16, rotated k and v
@@ -46,7 +48,7 @@ struct Layer {
 // head is RMS-normalised over its 128 dims before the rotation.
 __global__ void __launch_bounds__(256) rope_append_kernel(const float* __restrict__ qkv, const float* __restrict__ cs,
                                                           const int32_t* __restrict__ pos,
-                                                          const int32_t* __restrict__ table, int max_pages, int pages,
+                                                          const int32_t* __restrict__ table, int rows_per_seq, int max_pages, int pages,
                                                           int Hq, int Hkv, int max_seq, __half* __restrict__ q16,
                                                           __half* __restrict__ pool, int32_t* status,
                                                           const float* __restrict__ qg, const float* __restrict__ kg,
@@ -57,7 +59,7 @@ __global__ void __launch_bounds__(256) rope_append_kernel(const float* __restric
     if (threadIdx.x == 0) atomicExch(status, 2);
     return;
   }
-  const int pid = table[(size_t)row * max_pages + (ps >> 4)];
+  const int pid = table[(size_t)(row / rows_per_seq) * max_pages + (ps >> 4)];
   if ((unsigned)pid >= (unsigned)pages) {
     if (threadIdx.x == 0) atomicExch(status, 1);
     return;
@@ -111,6 +113,40 @@ __global__ void __launch_bounds__(256) rope_append_kernel(const float* __restric
     pool[((size_t)pid * Hkv + h) * (2 * kPage * kHD) + kPage * kHD + (ps & 15) * kHD + i] =
         __float2half_rn(src[nq + nkv + h * kHD + pi]);
   }
+}
+
+// Start of a prompt call: rows of sequence b at positions base[b], base[b] + 1, ..., their embeddings.  D % 8 == 0.
+struct PromptBase {
+  int len[16];
+};
+__global__ void __launch_bounds__(256) prompt_rows_kernel(const uint16_t* __restrict__ table, const int32_t* __restrict__ tokens, int D, int V,
+                                                          int T, const PromptBase base, float* __restrict__ x, int32_t* __restrict__ pos,
+                                                          int32_t* __restrict__ lens, int32_t* status) {
+  const int row = blockIdx.x;
+  int tok = tokens[row];
+  if ((unsigned)tok >= (unsigned)V) {
+    if (threadIdx.x == 0) atomicExch(status, 3);
+    tok = 0;
+  }
+  if (threadIdx.x == 0) {
+    const int p = base.len[row / T] + row % T;
+    pos[row] = p;
+    lens[row] = p + 1;
+  }
+  const uint4* src = reinterpret_cast<const uint4*>(table + (size_t)tok * D);
+  float4* dst = reinterpret_cast<float4*>(x + (size_t)row * D);
+  for (int i = threadIdx.x; i < D / 8; i += 256) {
+    const uint4 w = src[i];
+    dst[2 * i] = make_float4(__uint_as_float(w.x << 16), __uint_as_float(w.x & 0xffff0000u), __uint_as_float(w.y << 16), __uint_as_float(w.y & 0xffff0000u));
+    dst[2 * i + 1] = make_float4(__uint_as_float(w.z << 16), __uint_as_float(w.z & 0xffff0000u), __uint_as_float(w.w << 16), __uint_as_float(w.w & 0xffff0000u));
+  }
+}
+
+// End of a prompt call: the hidden state of every sequence's last row, for the LM head
+__global__ void __launch_bounds__(256) last_rows_kernel(const float* __restrict__ x, int T, int D, float* __restrict__ out) {
+  const float4* src = reinterpret_cast<const float4*>(x + ((size_t)blockIdx.x * T + T - 1) * D);
+  float4* dst = reinterpret_cast<float4*>(out + (size_t)blockIdx.x * D);
+  for (int i = threadIdx.x; i < D / 4; i += 256) dst[i] = src[i];
 }
 
 // Unfused end of a decode step (batches the fused LM head does not take): record the sampled
@@ -185,7 +221,8 @@ struct qeng_decoder {
   int64_t rows_cap = 0;
   float *x = nullptr, *qkv = nullptr, *att = nullptr, *act = nullptr, *part = nullptr;
   float* xalt = nullptr;  // second residual buffer: a fused tensor-parallel gather reads one and writes the other
-  float *xnr = nullptr, *gu = nullptr;  // prefill only: normalised rows, gate|up before SwiGLU
+  float* xnr = nullptr;  // many rows only: the normalised rows.  There xnr, att and act each hold two bf16 planes instead of f32
+  int32_t* h_tok = nullptr;  // pinned: the tokens of a prompt call
   __half* q16 = nullptr;
   int32_t *pos = nullptr, *lens = nullptr, *table = nullptr, *tok = nullptr;  // per row
   // decode state
@@ -218,10 +255,6 @@ struct qeng_decoder {
 
 namespace {
 
-// Prompt rows go through the decode attention kernel one "sequence" per row, at most this many
-// per launch (bounds its grid, its arrival counters and its split scratch).
-constexpr int64_t kAttnRowsPerCall = 2048;
-
 // Grow the per-row buffers.  A captured decode step holds their addresses, so it is dropped here
 // and captured again by the next decode call.
 int32_t ensure_rows(qeng_ctx* ctx, qeng_decoder* d, int64_t rows) {
@@ -229,13 +262,14 @@ int32_t ensure_rows(qeng_ctx* ctx, qeng_decoder* d, int64_t rows) {
   QENG_CUDA(ctx, cudaDeviceSynchronize());
   if (d->graph) { cudaGraphExecDestroy(d->graph); d->graph = nullptr; }
   qeng_step_free(d->fused); d->fused = nullptr; d->step_planned = false;
-  float** fb[] = {&d->x, &d->xalt, &d->qkv, &d->att, &d->act, &d->part, &d->xnr, &d->gu};
+  float** fb[] = {&d->x, &d->xalt, &d->qkv, &d->att, &d->act, &d->part, &d->xnr};
   for (auto p : fb)
     if (*p) { cudaFree(*p); *p = nullptr; }
   if (d->q16) { cudaFree(d->q16); d->q16 = nullptr; }
   int32_t** ib[] = {&d->pos, &d->lens, &d->table, &d->tok};
   for (auto p : ib)
     if (*p) { cudaFree(*p); *p = nullptr; }
+  if (d->h_tok) { cudaFreeHost(d->h_tok); d->h_tok = nullptr; }
   d->rows_cap = 0;
   const int64_t dm = d->cfg.d_model;
   QENG_CUDA(ctx, cudaMalloc(&d->x, rows * dm * 4));
@@ -244,17 +278,16 @@ int32_t ensure_rows(qeng_ctx* ctx, qeng_decoder* d, int64_t rows) {
   QENG_CUDA(ctx, cudaMalloc(&d->att, rows * d->Hq * kHD * 4));
   QENG_CUDA(ctx, cudaMalloc(&d->act, rows * d->F * 4));
   QENG_CUDA(ctx, cudaMalloc(&d->part, rows * dm * 4));
-  if (rows >= kPrefillRows) {
-    QENG_CUDA(ctx, cudaMalloc(&d->xnr, rows * dm * 4));
-    QENG_CUDA(ctx, cudaMalloc(&d->gu, rows * 2 * d->F * 4));
-  }
+  if (rows >= kManyRows) QENG_CUDA(ctx, cudaMalloc(&d->xnr, rows * dm * 4));
   QENG_CUDA(ctx, cudaMalloc(&d->q16, rows * d->Hq * kHD * 2));
   QENG_CUDA(ctx, cudaMalloc(&d->pos, rows * 4));
   QENG_CUDA(ctx, cudaMalloc(&d->lens, rows * 4));
-  QENG_CUDA(ctx, cudaMalloc(&d->table, rows * d->max_pages * 4));
+  const int64_t few = rows < kManyRows ? rows : kManyRows - 1;  // larger prompts use the sequences' own page tables
+  QENG_CUDA(ctx, cudaMalloc(&d->table, few * d->max_pages * 4));
+  QENG_CUDA(ctx, cudaMallocHost(&d->h_tok, rows * 4));
   QENG_CUDA(ctx, cudaMalloc(&d->tok, rows * 4));
   d->rows_cap = rows;
-  return qeng_attn_reserve(ctx, rows < kAttnRowsPerCall ? rows : kAttnRowsPerCall, d->Hq, d->Hkv, d->max_pages);
+  return qeng_attn_reserve(ctx, few, d->Hq, d->Hkv, d->max_pages);
 }
 
 // matmul over `rows` activation rows in chunks the decode kernels accept: the largest row count
@@ -291,6 +324,8 @@ __global__ void add_inplace_kernel(float* __restrict__ x, const float* __restric
   if (i < n) x[i] += p[i];
 }
 
+int32_t reduce_part(qeng_ctx* ctx, qeng_decoder* d, int64_t rows, cudaStream_t st);
+
 int32_t row_split(qeng_ctx* ctx, qeng_decoder* d, const qeng_weight* w, const float* in, int64_t ldin, int64_t rows,
                   cudaStream_t st) {
   const int64_t dm = d->cfg.d_model;
@@ -302,13 +337,28 @@ int32_t row_split(qeng_ctx* ctx, qeng_decoder* d, const qeng_weight* w, const fl
   }
   f.epilogue = QENG_EPI_STORE;
   int32_t rc = mm(ctx, d, w, in, ldin, rows, d->part, dm, f, st);
-  if (rc != QENG_OK) return rc;
-  const int64_t n = rows * dm;
+  return rc == QENG_OK ? reduce_part(ctx, d, rows, st) : rc;
+}
+
+// the same projection of many rows given as bf16 planes, on the tensor cores
+int32_t row_split_many(qeng_ctx* ctx, qeng_decoder* d, const qeng_weight* w, const qeng_tc_x& in, int64_t rows, int wp, cudaStream_t st) {
+  const bool one = d->cfg.tp_world == 1;
+  qeng_tc_epi e;
+  e.kind = one ? QENG_EPI_ACCUM : QENG_EPI_STORE;
+  e.y = one ? d->x : d->part;
+  e.ldy = d->cfg.d_model;
+  int32_t rc = qeng_gemm_tc(ctx, w, in, rows, wp, e, st);
+  return rc == QENG_OK && !one ? reduce_part(ctx, d, rows, st) : rc;
+}
+
+// x += d->part summed over the ranks
+int32_t reduce_part(qeng_ctx* ctx, qeng_decoder* d, int64_t rows, cudaStream_t st) {
+  const int64_t n = rows * d->cfg.d_model;
   if (qeng_tp_p2p_ready(ctx, n)) {  // push, wait, sum and residual add in one kernel
     d->launches += 1;
     return qeng_tp_allreduce_add(ctx, d->x, d->part, n, st);
   }
-  rc = qeng_tp_all_reduce_internal(ctx, d->part, n, st);
+  int32_t rc = qeng_tp_all_reduce_internal(ctx, d->part, n, st);
   if (rc != QENG_OK) return rc;
   add_inplace_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(d->x, d->part, n);
   QENG_LAUNCH_CHECK(ctx);
@@ -316,54 +366,53 @@ int32_t row_split(qeng_ctx* ctx, qeng_decoder* d, const qeng_weight* w, const fl
   return QENG_OK;
 }
 
-// gate|up rows are interleaved 8/8 per 16-row tile: act[m][8j + r] = silu(gu[m][16j + r]) * gu[m][16j + r + 8]
-__global__ void swiglu_interleaved_kernel(const float* __restrict__ gu, int64_t rows, int F, float* __restrict__ act) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= rows * F) return;
-  const int64_t m = i / F;
-  const int c = (int)(i - m * F);
-  const float* src = gu + m * 2 * F + (c >> 3) * 16 + (c & 7);
-  const float g = src[0];
-  act[i] = g / (1.0f + __expf(-g)) * src[8];
-}
-
-// The same layer for many rows (prompt phase): unfused small operators around the tensor-core matmul.
-int32_t run_layer_prefill(qeng_ctx* ctx, qeng_decoder* d, int l, int64_t rows, const int32_t* table, cudaStream_t st) {
+// One layer over many rows (prompt phase), T per sequence: every matmul on the tensor cores, the operators between
+// them in their epilogues (rotary embedding, KV append, SwiGLU, residual add).  Between the kernels the activations
+// travel as bf16 planes: one where the matmul rounds its operands to bf16 anyway (256 rows of 4-bit blocks and more),
+// two (17 bits) where it does not.
+int32_t run_layer_many(qeng_ctx* ctx, qeng_decoder* d, int l, int64_t rows, int64_t T, cudaStream_t st) {
   Layer& L = d->layers[l];
   const int64_t dm = d->cfg.d_model, nq = (int64_t)d->Hq * kHD;
-  const bool tp = d->cfg.tp_world > 1;
+  const bool all_q4 = L.wqkv->fmt == QENG_FMT_Q4 && L.wo->fmt == QENG_FMT_Q4 && L.wgu->fmt == QENG_FMT_Q4 && L.wdown->fmt == QENG_FMT_Q4;
+  const int planes = rows >= kPrefillRows && all_q4 ? 1 : 2;
   __half* pool = d->pool + (size_t)l * d->pages * d->Hkv * 2 * kPage * kHD;
-  int32_t rc = qeng_rmsnorm(ctx, d->x, L.norm1, rows, dm, d->cfg.rms_eps, d->xnr, st);
-  if (rc == QENG_OK) rc = qeng_gemm_many_rows(ctx, L.wqkv, d->xnr, QENG_F32, rows, dm, d->qkv, d->nqkv, 0, 1, st);
-  if (rc != QENG_OK) return rc;
-  rope_append_kernel<<<(unsigned)rows, 256, 0, st>>>(d->qkv, d->rope_cs, d->pos, table, d->max_pages, (int)d->pages,
-                                                     d->Hq, d->Hkv, d->cfg.max_seq, d->q16, pool, ctx->status, L.qnorm, L.knorm, d->cfg.rms_eps);
-  QENG_LAUNCH_CHECK(ctx);
-  d->view.pages = d->pages; d->view.kv_heads = d->Hkv; d->view.hd = kHD; d->view.data = pool;
-  for (int64_t r0 = 0; r0 < rows; r0 += kAttnRowsPerCall) {
-    const int64_t nr = rows - r0 < kAttnRowsPerCall ? rows - r0 : kAttnRowsPerCall;
-    rc = qeng_attn_decode_ex(ctx, &d->view, reinterpret_cast<const uint16_t*>(d->q16 + r0 * nq), table + r0 * d->max_pages,
-                             d->max_pages, d->lens + r0, nr, d->Hq, 1.0f / sqrtf((float)kHD), d->cfg.attn_softcap,
-                             d->cfg.sliding_window, d->att + r0 * nq, st);
-    if (rc != QENG_OK) return rc;
-  }
-  const int64_t n = rows * dm;
-  auto row_split_tc = [&](const qeng_weight* w, const float* in, int64_t ldin) -> int32_t {
-    if (!tp) return qeng_gemm_many_rows(ctx, w, in, QENG_F32, rows, ldin, d->x, dm, 1, 1, st);
-    int32_t r = qeng_gemm_many_rows(ctx, w, in, QENG_F32, rows, ldin, d->part, dm, 0, 1, st);
-    if (r == QENG_OK) r = qeng_tp_all_reduce_internal(ctx, d->part, n, st);
-    if (r != QENG_OK) return r;
-    add_inplace_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(d->x, d->part, n);
-    return QENG_OK;
+  auto operand = [&](float* buf, int64_t ld) {
+    qeng_tc_x x;
+    x.data = buf; x.ld = ld; x.plane = rows * ld; x.planes = planes;
+    return x;
   };
-  rc = row_split_tc(L.wo, d->att, nq);
-  if (rc == QENG_OK) rc = qeng_rmsnorm(ctx, d->x, L.norm2, rows, dm, d->cfg.rms_eps, d->xnr, st);
-  if (rc == QENG_OK) rc = qeng_gemm_many_rows(ctx, L.wgu, d->xnr, QENG_F32, rows, dm, d->gu, 2 * d->F, 0, 1, st);
+  int32_t rc = qeng_tc_prep(ctx, d->x, QENG_F32, rows, dm, dm, L.norm1, d->cfg.rms_eps, planes, d->xnr, st);
   if (rc != QENG_OK) return rc;
-  const int64_t na = rows * d->F;
-  swiglu_interleaved_kernel<<<(unsigned)((na + 255) / 256), 256, 0, st>>>(d->gu, rows, d->F, d->act);
-  QENG_LAUNCH_CHECK(ctx);
-  return row_split_tc(L.wdown, d->act, d->F);
+  qeng_tc_epi e;
+  if (L.qnorm == nullptr) {
+    e.kind = QENG_EPI_QKV;
+    e.qkv.pos = d->pos; e.qkv.table = d->dec_table; e.qkv.rows_per_seq = (int)T; e.qkv.cs = d->rope_cs; e.qkv.q16 = d->q16; e.qkv.pool = pool;
+    e.qkv.max_pages = d->max_pages; e.qkv.pages = (int)d->pages; e.qkv.Hq = d->Hq; e.qkv.Hkv = d->Hkv; e.qkv.max_seq = d->cfg.max_seq;
+  } else {
+    e.kind = QENG_EPI_STORE; e.y = d->qkv; e.ldy = d->nqkv;
+  }
+  rc = qeng_gemm_tc(ctx, L.wqkv, operand(d->xnr, dm), rows, planes, e, st);
+  if (rc != QENG_OK) return rc;
+  if (L.qnorm != nullptr) {
+    rope_append_kernel<<<(unsigned)rows, 256, 0, st>>>(d->qkv, d->rope_cs, d->pos, d->dec_table, (int)T, d->max_pages, (int)d->pages,
+                                                       d->Hq, d->Hkv, d->cfg.max_seq, d->q16, pool, ctx->status, L.qnorm, L.knorm, d->cfg.rms_eps);
+    QENG_LAUNCH_CHECK(ctx);
+  }
+  qeng_prefill_attn a;
+  a.q16 = d->q16; a.table = d->dec_table; a.lens = d->lens;
+  a.out = reinterpret_cast<__nv_bfloat16*>(d->att); a.ldo = nq; a.plane = rows * nq; a.planes = planes;
+  a.B = (int)(rows / T); a.T = (int)T; a.Hq = d->Hq; a.Hkv = d->Hkv; a.max_pages = d->max_pages; a.pages = (int)d->pages;
+  a.scale = 1.0f / sqrtf((float)kHD); a.softcap = d->cfg.attn_softcap; a.window = d->cfg.sliding_window; a.status = ctx->status;
+  rc = qeng_attn_prefill(ctx, a, L.kv_map, st);
+  if (rc == QENG_OK) rc = row_split_many(ctx, d, L.wo, operand(d->att, nq), rows, planes, st);
+  if (rc == QENG_OK) rc = qeng_tc_prep(ctx, d->x, QENG_F32, rows, dm, dm, L.norm2, d->cfg.rms_eps, planes, d->xnr, st);
+  if (rc != QENG_OK) return rc;
+  qeng_tc_epi eg;
+  eg.kind = QENG_EPI_SWIGLU;
+  eg.yb = reinterpret_cast<__nv_bfloat16*>(d->act); eg.ldyb = d->F; eg.yb_plane = rows * d->F; eg.yb_planes = planes;
+  rc = qeng_gemm_tc(ctx, L.wgu, operand(d->xnr, dm), rows, planes, eg, st);
+  if (rc == QENG_OK) rc = row_split_many(ctx, d, L.wdown, operand(d->act, d->F), rows, planes, st);
+  return rc;
 }
 
 // One layer over `rows` rows whose positions / lengths / page-table rows are on the device.
@@ -371,14 +420,14 @@ int32_t run_layer_prefill(qeng_ctx* ctx, qeng_decoder* d, int l, int64_t rows, c
 // down send their partial sums from the epilogue to every rank's inbox, the next matmul's staging
 // adds the parts onto the residual rows of *px and leaves the result in the other residual buffer,
 // to which *px then points.  No collective kernel runs.
-int32_t run_layer(qeng_ctx* ctx, qeng_decoder* d, int l, int64_t rows, const int32_t* table, cudaStream_t st, float** px = nullptr) {
+// T = rows per sequence (1 in decode steps).
+int32_t run_layer(qeng_ctx* ctx, qeng_decoder* d, int l, int64_t rows, int64_t T, const int32_t* table, cudaStream_t st, float** px = nullptr) {
   Layer& L = d->layers[l];
   if (!L.wqkv || !L.wo || !L.wgu || !L.wdown || !L.norm1 || !L.norm2)
     return qeng_fail(ctx, QENG_ERR_STATE, "decoder: layer %d is not fully loaded", l);
-  // the tensor-core prompt path dequantises 4-bit blocks; a layer with 8-bit blocks takes its prompt rows
-  // through the decode kernels in passes of 16
-  const bool all_q4 = L.wqkv->fmt == QENG_FMT_Q4 && L.wo->fmt == QENG_FMT_Q4 && L.wgu->fmt == QENG_FMT_Q4 && L.wdown->fmt == QENG_FMT_Q4;
-  if (rows >= kPrefillRows && all_q4) return run_layer_prefill(ctx, d, l, rows, table, st);
+  if ((L.qnorm == nullptr) != (L.knorm == nullptr))
+    return qeng_fail(ctx, QENG_ERR_STATE, "decoder: layer %d has only one of the q / k head gains", l);
+  if (rows >= kManyRows) return run_layer_many(ctx, d, l, rows, T, st);
   const int64_t dm = d->cfg.d_model;
   const bool fused = px != nullptr;
   float* x = fused ? *px : d->x;
@@ -391,8 +440,6 @@ int32_t run_layer(qeng_ctx* ctx, qeng_decoder* d, int l, int64_t rows, const int
     f.tp_gather_kind = 1; f.tp_gather_layer = l - 1; f.tp_writeback = other(x);
   }
   int32_t rc;
-  if ((L.qnorm == nullptr) != (L.knorm == nullptr))
-    return qeng_fail(ctx, QENG_ERR_STATE, "decoder: layer %d has only one of the q / k head gains", l);
   if (L.qnorm == nullptr && qeng_gemm_q4_stream_fits(ctx, L.wqkv, 1)) {
     // q|k|v projection with rotary embedding, f16 rounding and KV append in its epilogue
     qeng_qkv_epi E;
@@ -404,7 +451,7 @@ int32_t run_layer(qeng_ctx* ctx, qeng_decoder* d, int l, int64_t rows, const int
   } else {
     rc = mm(ctx, d, L.wqkv, x, dm, rows, d->qkv, d->nqkv, f, st);
     if (rc != QENG_OK) return rc;
-    rope_append_kernel<<<(unsigned)rows, 256, 0, st>>>(d->qkv, d->rope_cs, d->pos, table, d->max_pages, (int)d->pages,
+    rope_append_kernel<<<(unsigned)rows, 256, 0, st>>>(d->qkv, d->rope_cs, d->pos, table, 1, d->max_pages, (int)d->pages,
                                                        d->Hq, d->Hkv, d->cfg.max_seq, d->q16, pool, ctx->status, L.qnorm, L.knorm, d->cfg.rms_eps);
     QENG_LAUNCH_CHECK(ctx);
     d->launches++;
@@ -549,7 +596,7 @@ int32_t decode_step(qeng_ctx* ctx, qeng_decoder* d, cudaStream_t st) {
   }
   float* x = d->x;
   for (int l = 0; l < d->cfg.layers; ++l) {
-    int32_t rc = run_layer(ctx, d, l, B, d->dec_table, st, fused ? &x : nullptr);
+    int32_t rc = run_layer(ctx, d, l, B, 1, d->dec_table, st, fused ? &x : nullptr);
     if (rc != QENG_OK) return rc;
   }
   if (fused) {
@@ -654,7 +701,10 @@ int32_t qeng_decoder_create(qeng_ctx* ctx, const qeng_model_cfg* cfg, qeng_decod
     qeng_decoder_free(ctx, d);
     return qeng_fail(ctx, QENG_ERR_CUDA, "decoder_create: %s", cudaGetErrorString(e));
   }
-  int32_t rc = ensure_rows(ctx, d, cfg->max_batch);
+  int32_t rc = QENG_OK;
+  for (int l = 0; rc == QENG_OK && l < cfg->layers; ++l)
+    rc = qeng_kv_map(ctx, d->pool + (size_t)l * d->pages * d->Hkv * 2 * kPage * kHD, d->pages * d->Hkv * 2 * kPage, d->layers[l].kv_map);
+  if (rc == QENG_OK) rc = ensure_rows(ctx, d, cfg->max_batch);
   if (rc != QENG_OK) {
     qeng_decoder_free(ctx, d);
     return rc;
@@ -676,12 +726,13 @@ int32_t qeng_decoder_free(qeng_ctx* ctx, qeng_decoder* d) {
     if (L.qnorm) cudaFree(L.qnorm);
     if (L.knorm) cudaFree(L.knorm);
   }
-  void* bufs[] = {d->emb, d->lm_head, d->final_norm, d->rope_cs, d->pool, d->x, d->xalt, d->qkv, d->att, d->act, d->part, d->xnr, d->gu, d->q16,
+  void* bufs[] = {d->emb, d->lm_head, d->final_norm, d->rope_cs, d->pool, d->x, d->xalt, d->qkv, d->att, d->act, d->part, d->xnr, d->q16,
                   d->pos, d->lens, d->table, d->tok, d->xn, d->xlast, d->logits, d->next, d->out_tokens, d->step, d->dec_table, d->tp_pairs, d->tp_gath};
   for (void* p : bufs)
     if (p) cudaFree(p);
   if (d->own_stream) cudaStreamDestroy(d->own_stream);
   if (d->h_out) cudaFreeHost(d->h_out);
+  if (d->h_tok) cudaFreeHost(d->h_tok);
   delete d;
   return QENG_OK;
 }
@@ -883,26 +934,23 @@ int32_t qeng_decoder_prefill(qeng_ctx* ctx, qeng_decoder* d, const int32_t* toke
   int32_t rc = ensure_rows(ctx, d, rows);
   if (rc != QENG_OK) return rc;
   cudaStream_t st = d->stream;
-  std::vector<int32_t> pos(rows), lens(rows), table((size_t)rows * d->max_pages);
-  for (int b = 0; b < batch; ++b)
-    for (int tt = 0; tt < T; ++tt) {
-      const int64_t r = (int64_t)b * T + tt;
-      pos[r] = d->len[b] + tt;
-      lens[r] = pos[r] + 1;
-      for (int p = 0; p < d->max_pages; ++p) table[(size_t)r * d->max_pages + p] = p * d->cfg.max_batch + b;
-    }
-  int32_t* dtok = d->tok;
-  cudaMemcpyAsync(dtok, tokens, rows * 4, cudaMemcpyHostToDevice, st);
-  cudaMemcpyAsync(d->pos, pos.data(), rows * 4, cudaMemcpyHostToDevice, st);
-  cudaMemcpyAsync(d->lens, lens.data(), rows * 4, cudaMemcpyHostToDevice, st);
-  cudaMemcpyAsync(d->table, table.data(), table.size() * 4, cudaMemcpyHostToDevice, st);
-  rc = qeng_embed(ctx, d->emb, dtok, rows, d->cfg.d_model, d->cfg.vocab, d->x, st);
-  for (int l = 0; rc == QENG_OK && l < d->cfg.layers; ++l) rc = run_layer(ctx, d, l, rows, d->table, st);
+  memcpy(d->h_tok, tokens, (size_t)rows * 4);
+  QENG_CUDA(ctx, cudaMemcpyAsync(d->tok, d->h_tok, rows * 4, cudaMemcpyHostToDevice, st));
+  std::vector<int32_t> table;
+  if (rows < kManyRows) {  // the decode kernels take one page table per row
+    table.resize((size_t)rows * d->max_pages);
+    for (int64_t r = 0; r < rows; ++r)
+      for (int p = 0; p < d->max_pages; ++p) table[(size_t)r * d->max_pages + p] = p * d->cfg.max_batch + (int32_t)(r / T);
+    QENG_CUDA(ctx, cudaMemcpyAsync(d->table, table.data(), table.size() * 4, cudaMemcpyHostToDevice, st));
+  }
+  PromptBase base = {};
+  for (int b = 0; b < batch; ++b) base.len[b] = d->len[b];
+  prompt_rows_kernel<<<(unsigned)rows, 256, 0, st>>>(d->emb, d->tok, d->cfg.d_model, d->cfg.vocab, T, base, d->x, d->pos, d->lens, ctx->status);
+  QENG_LAUNCH_CHECK(ctx);
+  for (int l = 0; rc == QENG_OK && l < d->cfg.layers; ++l) rc = run_layer(ctx, d, l, rows, T, d->table, st);
   if (rc == QENG_OK) {
-    // hidden state of the last prompt position of every sequence, gathered for the LM head
-    for (int b = 0; b < batch; ++b)
-      cudaMemcpyAsync(d->xlast + (size_t)b * d->cfg.d_model, d->x + ((size_t)b * T + T - 1) * d->cfg.d_model,
-                      (size_t)d->cfg.d_model * 4, cudaMemcpyDeviceToDevice, st);
+    last_rows_kernel<<<(unsigned)batch, 256, 0, st>>>(d->x, T, d->cfg.d_model, d->xlast);
+    QENG_LAUNCH_CHECK(ctx);
     rc = tail(ctx, d, d->xlast, batch, false, st);
   }
   cudaError_t e = cudaStreamSynchronize(st);
@@ -1031,18 +1079,19 @@ int32_t qeng_decoder_layer(qeng_ctx* ctx, qeng_decoder* d, int32_t layer, const 
   if (rc != QENG_OK) return rc;
   cudaStream_t st = (cudaStream_t)stream;
   // all rows belong to sequence 0 (a prompt chunk or a single step)
-  std::vector<int32_t> lens(rows), table((size_t)rows * d->max_pages);
+  const bool few = rows < kManyRows;
+  std::vector<int32_t> lens(rows), table(few ? (size_t)rows * d->max_pages : 0);
   for (int r = 0; r < rows; ++r) {
     if (pos[r] < 0 || pos[r] >= d->cfg.max_seq) return qeng_fail(ctx, QENG_ERR_ARG, "decoder_layer: position outside the cache");
     lens[r] = pos[r] + 1;
-    for (int p = 0; p < d->max_pages; ++p) table[(size_t)r * d->max_pages + p] = p * d->cfg.max_batch;
+    for (int p = 0; few && p < d->max_pages; ++p) table[(size_t)r * d->max_pages + p] = p * d->cfg.max_batch;
   }
   QENG_CUDA(ctx, cudaMemcpyAsync(d->pos, pos, rows * 4, cudaMemcpyHostToDevice, st));
   QENG_CUDA(ctx, cudaMemcpyAsync(d->lens, lens.data(), rows * 4, cudaMemcpyHostToDevice, st));
-  QENG_CUDA(ctx, cudaMemcpyAsync(d->table, table.data(), table.size() * 4, cudaMemcpyHostToDevice, st));
+  if (few) QENG_CUDA(ctx, cudaMemcpyAsync(d->table, table.data(), table.size() * 4, cudaMemcpyHostToDevice, st));
   d->next_ready = false;  // the activation buffer is reused
   QENG_CUDA(ctx, cudaMemcpyAsync(d->x, x_in, (size_t)rows * d->cfg.d_model * 4, cudaMemcpyDeviceToDevice, st));
-  rc = run_layer(ctx, d, layer, rows, d->table, st);
+  rc = run_layer(ctx, d, layer, rows, rows, d->table, st);
   if (rc != QENG_OK) return rc;
   QENG_CUDA(ctx, cudaMemcpyAsync(x_out, d->x, (size_t)rows * d->cfg.d_model * 4, cudaMemcpyDeviceToDevice, st));
   QENG_CUDA(ctx, cudaStreamSynchronize(st));  // host staging buffers go out of scope

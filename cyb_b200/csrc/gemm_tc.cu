@@ -374,7 +374,7 @@ __device__ __forceinline__ void finish16(const TcParams& p, int n, int m0, int c
       if (head < q.Hq) {
         dst = q.q16 + ((size_t)m * q.Hq + head) * 128 + d;
       } else {
-        const int pid = q.table[(size_t)m * q.max_pages + (ps >> 4)];
+        const int pid = q.table[(size_t)(m / q.rows_per_seq) * q.max_pages + (ps >> 4)];
         if ((unsigned)pid >= (unsigned)q.pages) {
           atomicExch(p.status, 1);
           continue;
@@ -817,6 +817,8 @@ int32_t launch(qeng_ctx* ctx, const qeng_weight* w, const TcParams& p, const Pla
 }
 
 }  // namespace
+
+void* qeng_tensor_map_encoder() { return reinterpret_cast<void*>(encode_fn()); }
 
 int32_t qeng_tc_prep(qeng_ctx* ctx, const void* x, int32_t dtype, int64_t M, int64_t K, int64_t ldx, const float* gamma, float eps,
                      int planes, void* out, cudaStream_t stream) {

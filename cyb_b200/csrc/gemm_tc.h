@@ -25,6 +25,8 @@ struct qeng_tc_x {
 
 // wp = 1: weights rounded to bf16 (4-bit blocks only); wp = 2: weights as two bf16 terms
 int32_t qeng_gemm_tc(qeng_ctx* ctx, const qeng_weight* w, const qeng_tc_x& x, int64_t M, int wp, const qeng_tc_epi& epi, cudaStream_t stream);
+// the driver's cuTensorMapEncodeTiled, or null
+void* qeng_tensor_map_encoder();
 // rows of x (any type), RMS-normalised if gamma is given -> `planes` bf16 planes [M][K]
 int32_t qeng_tc_prep(qeng_ctx* ctx, const void* x, int32_t dtype, int64_t M, int64_t K, int64_t ldx, const float* gamma, float eps,
                      int planes, void* out, cudaStream_t stream);

@@ -133,6 +133,7 @@ struct qeng_qkv_epi {
   __half* q16;             // [M][Hq][128]
   __half* pool;            // [pages][Hkv][2][16][128]
   int max_pages, pages, Hq, Hkv, max_seq;
+  int rows_per_seq = 1;    // tensor-core matmul only: rows that share a page table
 };
 
 struct qeng_gemm_fuse {

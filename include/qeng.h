@@ -282,12 +282,11 @@ int32_t qeng_decoder_free(qeng_ctx* ctx, qeng_decoder* dec);
 int32_t qeng_decoder_load_matrix(qeng_ctx* ctx, qeng_decoder* dec, int32_t layer, int32_t which,
                                  const uint8_t* q, const uint16_t* s, int64_t N, int64_t K);
 /* The same for 8-bit blocks (q: one signed byte per weight).  The matrices that the executor fuses
- * (q, k, v of a layer; gate, up of a layer) must come in one format; prompts of layers with 8-bit
- * blocks run through the decode kernels in passes of 16 rows. */
+ * (q, k, v of a layer; gate, up of a layer) must come in one format. */
 int32_t qeng_decoder_load_matrix_q8(qeng_ctx* ctx, qeng_decoder* dec, int32_t layer, int32_t which,
                                     const int8_t* q, const uint16_t* s, int64_t N, int64_t K);
 /* The same for Q4_K super-blocks (see qeng_weight_pack_q4k); decode steps of up to 4 sequences take
- * such layers in one pass, larger batches and prompts in passes of 4 rows. */
+ * such layers in one pass, batches of 5 to 16 in passes of 4 rows. */
 int32_t qeng_decoder_load_matrix_q4k(qeng_ctx* ctx, qeng_decoder* dec, int32_t layer, int32_t which,
                                      const uint8_t* blocks, int64_t N, int64_t K);
 /* RMSNorm gains of a layer (which = 0: before attention, 1: before FFN), HOST f32[d_model].
@@ -324,9 +323,8 @@ int32_t qeng_decoder_load_file(qeng_ctx* ctx, qeng_decoder* dec, const char* pat
 int32_t qeng_decoder_reset(qeng_ctx* ctx, qeng_decoder* dec, int32_t batch);
 /* Prompt phase: tokens HOST int32 [batch, T]; fills the KV cache and leaves the
  * logits of the last prompt position.  Synchronous.  batch * T rows are processed at once (buffers
- * grow to that size on first use: about 150 KB per row at the 7B shape); from 256 rows on, layers of
- * 4-bit blocks take the tensor-core matmul.  Attention runs the decode kernel over the prompt rows in
- * launches of 2048 rows, so its KV traffic grows with T^2; feed long prompts in chunks (successive
+ * grow to that size on first use: about 130 KB per row at the 7B shape); from 17 rows on they take the
+ * tensor-core matmul and the causal prompt attention.  Long prompts may be fed in chunks (successive
  * calls append) to bound memory and to report progress. */
 int32_t qeng_decoder_prefill(qeng_ctx* ctx, qeng_decoder* dec, const int32_t* tokens, int32_t batch, int32_t T);
 /* Greedy decode: runs `steps` steps; each step samples from the current logits,

@@ -142,12 +142,15 @@ def _np_ptr(a):
 
 
 def _dev_ptr(t):
-    return _vp(t.data_ptr())
+    return t.data_ptr()  # the argument types convert a plain integer; an object of our own costs another microsecond
 
 
 def _cur_stream():
+    """The calling thread's current CUDA stream on its current device."""
     import torch
-    return _vp(torch.cuda.current_stream().cuda_stream)
+    if not torch.cuda.is_initialized():
+        torch.cuda.init()
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 class Context:
@@ -281,17 +284,20 @@ class Context:
         assert x.is_cuda and x.dim() == 2 and x.stride(1) == 1
         m = x.shape[0]
         if out is None:
-            out = torch.empty((m, w.rows), dtype=torch.float32, device=x.device)
-        self.check(_lib.qeng_gemm_q4(self.h, w.h, _dev_ptr(x), dt, m, x.stride(0), _dev_ptr(out), out.stride(0), flags,
-                                     _cur_stream()))
+            out = x.new_empty((m, w.rows), dtype=torch.float32)
+        rc = _lib.qeng_gemm_q4(self.h, w.h, x.data_ptr(), dt, m, x.stride(0), out.data_ptr(), out.stride(0), flags, _cur_stream())
+        if rc:
+            self.check(rc)
         return out
 
     def gemv_q4(self, w, x, out=None):
         import torch
         assert x.is_cuda and x.dtype == torch.float32 and x.is_contiguous()
         if out is None:
-            out = torch.empty((w.rows,), dtype=torch.float32, device=x.device)
-        self.check(_lib.qeng_gemv_q4(self.h, w.h, _dev_ptr(x), _dev_ptr(out), _cur_stream()))
+            out = x.new_empty((w.rows,))
+        rc = _lib.qeng_gemv_q4(self.h, w.h, x.data_ptr(), out.data_ptr(), _cur_stream())
+        if rc:
+            self.check(rc)
         return out
 
     def rmsnorm(self, x, gamma, eps):
@@ -357,7 +363,7 @@ class Context:
         b, hq, hd = q.shape
         assert q.dtype == torch.float16 and q.is_contiguous()
         if out is None:
-            out = torch.empty((b, hq, hd), dtype=torch.float32, device=q.device)
+            out = q.new_empty((b, hq, hd), dtype=torch.float32)
         scale = float(hd) ** -0.5 if scale is None else scale
         if softcap or window:
             self.check(_lib.qeng_attn_decode_ex(self.h, pool.h, _dev_ptr(q), _dev_ptr(table), table.shape[1], _dev_ptr(lens),

@@ -34,7 +34,7 @@ def sources():
 
 def _deps():
     inc = os.path.join(HERE, "..", "include", "qeng.h")
-    return sources() + [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith(".h")] + [inc]
+    return sources() + [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".h", ".cuh"))] + [inc]
 
 
 def up_to_date():

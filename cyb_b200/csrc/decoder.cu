@@ -381,7 +381,7 @@ int32_t run_layer_many(qeng_ctx* ctx, qeng_decoder* d, int l, int64_t rows, int6
     x.data = buf; x.ld = ld; x.plane = rows * ld; x.planes = planes;
     return x;
   };
-  int32_t rc = qeng_tc_prep(ctx, d->x, QENG_F32, rows, dm, dm, L.norm1, d->cfg.rms_eps, planes, d->xnr, st);
+  int32_t rc = qeng_tc_prep(ctx, d->x, QENG_F32, rows, dm, dm, L.norm1, d->cfg.rms_eps, planes, d->xnr, nullptr, st);
   if (rc != QENG_OK) return rc;
   qeng_tc_epi e;
   if (L.qnorm == nullptr) {
@@ -405,7 +405,7 @@ int32_t run_layer_many(qeng_ctx* ctx, qeng_decoder* d, int l, int64_t rows, int6
   a.scale = 1.0f / sqrtf((float)kHD); a.softcap = d->cfg.attn_softcap; a.window = d->cfg.sliding_window; a.status = ctx->status;
   rc = qeng_attn_prefill(ctx, a, L.kv_map, st);
   if (rc == QENG_OK) rc = row_split_many(ctx, d, L.wo, operand(d->att, nq), rows, planes, st);
-  if (rc == QENG_OK) rc = qeng_tc_prep(ctx, d->x, QENG_F32, rows, dm, dm, L.norm2, d->cfg.rms_eps, planes, d->xnr, st);
+  if (rc == QENG_OK) rc = qeng_tc_prep(ctx, d->x, QENG_F32, rows, dm, dm, L.norm2, d->cfg.rms_eps, planes, d->xnr, nullptr, st);
   if (rc != QENG_OK) return rc;
   qeng_tc_epi eg;
   eg.kind = QENG_EPI_SWIGLU;
@@ -413,6 +413,60 @@ int32_t run_layer_many(qeng_ctx* ctx, qeng_decoder* d, int l, int64_t rows, int6
   rc = qeng_gemm_tc(ctx, L.wgu, operand(d->xnr, dm), rows, planes, eg, st);
   if (rc == QENG_OK) rc = row_split_many(ctx, d, L.wdown, operand(d->act, d->F), rows, planes, st);
   return rc;
+}
+
+// Whether a layer's decode batch (or short prompt) of this many rows takes run_layer_batch: one rank (the fused
+// tensor-parallel exchange lives in the streaming matmul), rows that the kernel takes for every matrix.
+bool batch_fits(const qeng_ctx* ctx, const qeng_decoder* d, const Layer& L, int64_t rows) {
+  if (d->cfg.tp_world != 1 || rows >= kManyRows) return false;
+  for (const qeng_weight* w : {L.wqkv, L.wo, L.wgu, L.wdown})
+    if (!qeng_gemm_rows_fits(ctx, w, rows, 2)) return false;
+  return true;
+}
+
+// One layer over a decode batch (5 to 16 rows): the activations of a matmul become two bf16 planes in a small kernel
+// (with the norm, where there is one), the matmul's second kernel runs the epilogue.
+int32_t run_layer_batch(qeng_ctx* ctx, qeng_decoder* d, int l, int64_t rows, const int32_t* table, cudaStream_t st) {
+  Layer& L = d->layers[l];
+  const int64_t dm = d->cfg.d_model, nq = (int64_t)d->Hq * kHD;
+  __half* pool = d->pool + (size_t)l * d->pages * d->Hkv * 2 * kPage * kHD;
+  qeng_tc_epi e;
+  if (L.qnorm == nullptr) {
+    e.kind = QENG_EPI_QKV;
+    e.qkv.pos = d->pos; e.qkv.table = table; e.qkv.cs = d->rope_cs; e.qkv.q16 = d->q16; e.qkv.pool = pool;
+    e.qkv.max_pages = d->max_pages; e.qkv.pages = (int)d->pages; e.qkv.Hq = d->Hq; e.qkv.Hkv = d->Hkv; e.qkv.max_seq = d->cfg.max_seq;
+  } else {
+    e.y = d->qkv; e.ldy = d->nqkv;
+  }
+  int32_t rc = qeng_gemm_rows_prep(ctx, L.wqkv, d->x, QENG_F32, rows, dm, L.norm1, d->cfg.rms_eps, e, st);
+  if (rc != QENG_OK) return rc;
+  if (L.qnorm != nullptr) {
+    rope_append_kernel<<<(unsigned)rows, 256, 0, st>>>(d->qkv, d->rope_cs, d->pos, table, 1, d->max_pages, (int)d->pages,
+                                                       d->Hq, d->Hkv, d->cfg.max_seq, d->q16, pool, ctx->status, L.qnorm, L.knorm, d->cfg.rms_eps);
+    QENG_LAUNCH_CHECK(ctx);
+  }
+  d->view.pages = d->pages; d->view.kv_heads = d->Hkv; d->view.hd = kHD; d->view.data = pool;
+  rc = qeng_attn_decode_ex(ctx, &d->view, reinterpret_cast<const uint16_t*>(d->q16), table, d->max_pages, d->lens, rows,
+                           d->Hq, 1.0f / sqrtf((float)kHD), d->cfg.attn_softcap, d->cfg.sliding_window, d->att, st);
+  if (rc != QENG_OK) return rc;
+  qeng_tc_epi er;
+  er.kind = QENG_EPI_ACCUM; er.y = d->x; er.ldy = dm;
+  rc = qeng_gemm_rows_prep(ctx, L.wo, d->att, QENG_F32, rows, nq, nullptr, 0.f, er, st);
+  if (rc != QENG_OK) return rc;
+  qeng_tc_epi eg;
+  eg.kind = QENG_EPI_SWIGLU;
+  if (L.wdown->fmt == QENG_FMT_K4) {  // its matmul needs block sums of the planes: they are made from f32 rows
+    eg.y = d->act; eg.ldy = d->F;
+  } else {
+    eg.yb = reinterpret_cast<__nv_bfloat16*>(d->act); eg.ldyb = d->F; eg.yb_plane = rows * d->F; eg.yb_planes = 2;
+  }
+  rc = qeng_gemm_rows_prep(ctx, L.wgu, d->x, QENG_F32, rows, dm, L.norm2, d->cfg.rms_eps, eg, st);
+  if (rc != QENG_OK) return rc;
+  d->launches += 12;
+  if (L.wdown->fmt == QENG_FMT_K4) return qeng_gemm_rows_prep(ctx, L.wdown, d->act, QENG_F32, rows, d->F, nullptr, 0.f, er, st);
+  qeng_tc_x x;
+  x.data = d->act; x.ld = d->F; x.plane = rows * d->F; x.planes = 2;
+  return qeng_gemm_rows(ctx, L.wdown, x, nullptr, rows, er, st);
 }
 
 // One layer over `rows` rows whose positions / lengths / page-table rows are on the device.
@@ -428,6 +482,7 @@ int32_t run_layer(qeng_ctx* ctx, qeng_decoder* d, int l, int64_t rows, int64_t T
   if ((L.qnorm == nullptr) != (L.knorm == nullptr))
     return qeng_fail(ctx, QENG_ERR_STATE, "decoder: layer %d has only one of the q / k head gains", l);
   if (rows >= kManyRows) return run_layer_many(ctx, d, l, rows, T, st);
+  if (px == nullptr && batch_fits(ctx, d, L, rows)) return run_layer_batch(ctx, d, l, rows, table, st);
   const int64_t dm = d->cfg.d_model;
   const bool fused = px != nullptr;
   float* x = fused ? *px : d->x;
@@ -977,6 +1032,9 @@ int32_t qeng_decoder_decode(qeng_ctx* ctx, qeng_decoder* d, int32_t steps, int32
     const qeng_weight* ws[4] = {L0.wqkv, L0.wo, L0.wgu, L0.wdown};
     for (int i = 0; rc == QENG_OK && i < 4; ++i)
       if (ws[i]) rc = qeng_gemm_q4_stream_reserve(ctx, ws[i], B < 16 ? B : 16);
+    for (const Layer& L : d->layers)
+      for (const qeng_weight* w : {L.wqkv, L.wo, L.wgu, L.wdown})
+        if (rc == QENG_OK && w && qeng_gemm_rows_fits(ctx, w, B, 2)) rc = qeng_gemm_rows_reserve(ctx, w, B, 2, st);
     if (rc != QENG_OK) return rc;
   }
   std::vector<int32_t> pos(B), lens(B);

@@ -1,0 +1,303 @@
+// Building blocks of the matmuls of many rows: barriers, TMA, tcgen05, the work split over CTA pairs
+// (gemm_tc.cu), and the epilogues (also gemm_rows.cu).
+#pragma once
+#include <cuda.h>
+#include <cuda_bf16.h>
+
+#include "gemm_tc.h"
+
+namespace qeng_tc {
+
+constexpr int kBK = 64;                  // k per chunk: one 128-byte swizzled row of bf16
+constexpr int kAPlane = 128 * kBK * 2;   // 16 KB: this CTA's 128 weight rows of a chunk
+constexpr int kMaxStages = 8, kMaxSlots = 12;
+constexpr size_t kSmemBudget = 226 * 1024;
+
+template <int FMT> struct Fmt;
+template <> struct Fmt<QENG_FMT_Q4> { static constexpr int kW = 512, kS = 64; };
+template <> struct Fmt<QENG_FMT_Q8> { static constexpr int kW = 1024, kS = 64; };
+template <> struct Fmt<QENG_FMT_K4> { static constexpr int kW = 512, kS = 256; };
+inline int chunk_w(int fmt) { return fmt == QENG_FMT_Q8 ? 1024 : 512; }
+inline int chunk_s(int fmt) { return fmt == QENG_FMT_K4 ? 256 : 64; }
+inline int slot_bytes_of(int fmt, int kst) { return kst * 8 * (chunk_w(fmt) + chunk_s(fmt)); }
+
+struct TcParams {
+  int nk;                    // stages of KST chunks along K
+  int M, N;
+  int bn, m_tiles, n_tiles;  // tokens per tile, token tiles, 256-row weight tiles
+  int dp_tiles, sk_tiles;    // whole tiles (round-robin), tiles cut along K
+  int nstages, nslots;       // rings: operand tiles, packed weights
+  qeng_tc_epi e;
+  int npairs;
+  float* ws;                 // stream-K partials: [pair][2][CTA of the pair][bn][128]
+  int32_t* status;
+};
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ uint32_t map_leader(uint32_t addr) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;\n" : "=r"(r) : "r"(addr));
+  return r;
+}
+__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bar), "r"(count));
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
+}
+// arrive on a barrier of either CTA of the pair (address from map_leader)
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];\n" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// Bounded wait: gives up (false) two seconds after the first failed attempt; a healthy wait ends
+// in microseconds.  The clock is read once per 64 attempts.
+__device__ __forceinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity) {
+  unsigned long long t0;
+  asm volatile("mov.u64 %0, %globaltimer;\n" : "=l"(t0));
+  for (;;) {
+    for (int i = 0; i < 64; ++i)
+      if (mbar_try_wait(bar, parity)) return true;
+    unsigned long long t1;
+    asm volatile("mov.u64 %0, %globaltimer;\n" : "=l"(t1));
+    if (t1 - t0 > 2000000000ull) return false;
+  }
+}
+// After a wait that ran out: copies this warp issued are given a tenth of a millisecond to land before the CTA leaves.
+__device__ __forceinline__ void grace() {
+  unsigned long long t0, t1;
+  asm volatile("mov.u64 %0, %globaltimer;\n" : "=l"(t0));
+  do asm volatile("mov.u64 %0, %globaltimer;\n" : "=l"(t1));
+  while (t1 - t0 < 100000ull);
+}
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
+  return mbar_try_wait(bar, parity) || mbar_wait_slow(bar, parity);
+}
+// one box of a packed plane: `box` chunks x 8 row tiles (beyond the matrix: zeros)
+__device__ __forceinline__ void tma_w(uint32_t dst, const CUtensorMap* map, int chunk, int tile, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];\n" ::"r"(dst),
+      "l"(map), "r"(0), "r"(chunk), "r"(tile), "r"(bar)
+      : "memory");
+}
+// one box of the activation planes into this CTA's shared memory; the bytes are counted on the leader's barrier
+__device__ __forceinline__ void tma_x(uint32_t dst, const CUtensorMap* map, int k, int m, int plane, uint32_t leader_bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];\n" ::"r"(dst),
+      "l"(map), "r"(k), "r"(m), "r"(plane), "r"(leader_bar)
+      : "memory");
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+
+// 64-bit shared-memory matrix descriptor: K-major, 128-byte swizzle, 8-row groups 1024 B apart.
+__device__ __forceinline__ uint64_t make_desc(uint32_t saddr) {
+  uint64_t d = 0;
+  d |= (uint64_t)((saddr & 0x3ffff) >> 4);  // start address
+  d |= (uint64_t)1 << 16;                   // leading byte offset (unused for swizzled K-major)
+  d |= (uint64_t)(1024 >> 4) << 32;         // stride byte offset
+  d |= (uint64_t)1 << 46;                   // descriptor version of this architecture
+  d |= (uint64_t)2 << 61;                   // 128-byte swizzle
+  return d;
+}
+__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc)
+      : "memory");
+}
+// arrives at the barrier at this offset in both CTAs once the MMAs issued so far have finished
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n" ::"r"(bar),
+               "h"((uint16_t)3)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+      "tcgen05.wait::ld.sync.aligned;\n"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+      : "r"(taddr)
+      : "memory");
+}
+// one lane of a converged warp: lets the operands of the instructions it issues stay warp-uniform
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n selp.u32 %0, 1, 0, q;\n}\n" : "=r"(p));
+  return p != 0;
+}
+__device__ __forceinline__ uint4 lds128(uint32_t a) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint32_t lds32(uint32_t a) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1];\n" : "=r"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint2 lds64(uint32_t a) {
+  uint2 v;
+  asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];\n" : "=r"(v.x), "=r"(v.y) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void sts128(uint32_t a, const uint32_t (&o)[4]) {
+  asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};\n" ::"r"(a), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
+}
+
+// ---- the sequence of (tile, K range) segments of one CTA pair; every role walks the same one ----------
+struct Seg {
+  int tile, k0, k1;
+};
+struct Segments {
+  int next_dp, npairs, u, u1;
+  __device__ Segments(const TcParams& p, int pair) : next_dp(pair), npairs(p.npairs) {
+    const long long U = (long long)p.sk_tiles * p.nk;
+    u = (int)(U * pair / npairs);
+    u1 = (int)(U * (pair + 1) / npairs);
+  }
+  __device__ bool next(const TcParams& p, Seg& s) {
+    if (next_dp < p.dp_tiles) {
+      s.tile = next_dp;
+      s.k0 = 0;
+      s.k1 = p.nk;
+      next_dp += npairs;
+      return true;
+    }
+    if (u >= u1) return false;
+    const int r = u / p.nk;
+    s.tile = p.dp_tiles + r;
+    s.k0 = u - r * p.nk;
+    s.k1 = min(p.nk, s.k0 + (u1 - u));
+    u += s.k1 - s.k0;
+    return true;
+  }
+};
+// Tiles in groups of 8 token tiles, weight tiles inside a group: a wave of pairs then works on few distinct
+// activation tiles and few weight tiles at once, and both are read from HBM once per wave.
+__device__ __forceinline__ void tile_pos(const TcParams& p, int tile, int& mt, int& nt) {
+  const int grp = 8 * p.n_tiles, gi = tile / grp, first = gi * 8, rows = min(8, p.m_tiles - first);
+  const int r = tile - gi * grp;
+  mt = first + r % rows;
+  nt = r / rows;
+}
+// the pair whose share holds unit u
+__device__ __forceinline__ int pair_of_unit(long long U, int np, int u) {
+  int q = (int)((long long)u * np / U);
+  while (q + 1 < np && (int)(U * (q + 1) / np) <= u) ++q;
+  while (q > 0 && (int)(U * q / np) > u) --q;
+  return q;
+}
+
+// this lane's column (weight row `row` of its CTA) of pair q's partial of split tile r
+__device__ __forceinline__ float* partial(const TcParams& p, int q, int r, uint32_t rank, int row) {
+  const long long U = (long long)p.sk_tiles * p.nk;
+  const int slot = (int)(U * q / p.npairs) / p.nk == r ? 0 : 1;  // the first tile of the pair's share, or a later one
+  return p.ws + ((size_t)(q * 2 + slot) * 2 + rank) * p.bn * 128 + row;
+}
+
+__device__ __forceinline__ __nv_bfloat162 bf2(uint32_t v) { return *reinterpret_cast<__nv_bfloat162*>(&v); }
+__device__ __forceinline__ uint32_t u32(__nv_bfloat162 v) { return *reinterpret_cast<uint32_t*>(&v); }
+
+
+// ---- epilogue of up to NT (8 or 16) tokens of this lane's weight row -------------------------------------------------
+// n = weight row of this lane (rows of a warp are 32 consecutive ones, so whole 16-row tiles); v[i] = sum of token m0 + i
+__device__ __forceinline__ void st_planes(const qeng_tc_epi& e, size_t at, float f) {
+  const __nv_bfloat16 h = __float2bfloat16_rn(f);
+  e.yb[at] = h;
+  if (e.yb_planes == 2) e.yb[at + e.yb_plane] = __float2bfloat16_rn(f - __bfloat162float(h));
+}
+template <int NT>
+__device__ __forceinline__ void finish(const qeng_tc_epi& e, int N, int32_t* status, int n, int m0, int cnt, const float (&v)[NT], int lane) {
+  if (e.kind == QENG_EPI_STORE || e.kind == QENG_EPI_ACCUM) {
+    if (n >= N) return;
+    float* dst = e.y + (size_t)m0 * e.ldy + n;
+    if (cnt >= NT) {
+      if (e.kind == QENG_EPI_ACCUM) {
+        float old[NT];
+#pragma unroll
+        for (int i = 0; i < NT; ++i) old[i] = dst[(size_t)i * e.ldy];
+#pragma unroll
+        for (int i = 0; i < NT; ++i) dst[(size_t)i * e.ldy] = old[i] + v[i];
+      } else {
+#pragma unroll
+        for (int i = 0; i < NT; ++i) dst[(size_t)i * e.ldy] = v[i];
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < NT; ++i)
+        if (i < cnt) dst[(size_t)i * e.ldy] = e.kind == QENG_EPI_ACCUM ? dst[(size_t)i * e.ldy] + v[i] : v[i];
+    }
+    return;
+  }
+  // SWIGLU and QKV combine rows r and r + 8 of a 16-row tile: lanes with bit 3 clear take the even tokens, the others
+  // the odd ones, so one exchange per token pair keeps every lane busy
+  const int odd = (lane >> 3) & 1, r = lane & 7, tile = n >> 4;
+#pragma unroll
+  for (int i = 0; i < NT; i += 2) {
+    const float got = __shfl_xor_sync(0xffffffffu, odd ? v[i] : v[i + 1], 8);
+    const float a = odd ? got : v[i], b = odd ? v[i + 1] : got;  // rows r and r + 8
+    const int t = i + odd, m = m0 + t;
+    if (t >= cnt || n >= N) continue;
+    if (e.kind == QENG_EPI_SWIGLU) {
+      const float f = a / (1.0f + __expf(-a)) * b;
+      if (e.yb != nullptr) st_planes(e, (size_t)m * e.ldyb + (size_t)tile * 8 + r, f);
+      else e.y[(size_t)m * e.ldy + (size_t)tile * 8 + r] = f;
+    } else {
+      const qeng_qkv_epi& q = e.qkv;
+      const int head = tile >> 3, d = ((tile & 7) << 3) + r, ps = q.pos[m];
+      if (ps < 0 || ps >= q.max_seq || (ps >> 4) >= q.max_pages) {
+        atomicExch(status, 2);
+        continue;
+      }
+      float lo = a, hi = b;
+      if (head < q.Hq + q.Hkv) {
+        const float c = q.cs[(size_t)ps * 128 + d], sn = q.cs[(size_t)ps * 128 + 64 + d];
+        lo = a * c - b * sn;
+        hi = b * c + a * sn;
+      }
+      __half* dst;
+      if (head < q.Hq) {
+        dst = q.q16 + ((size_t)m * q.Hq + head) * 128 + d;
+      } else {
+        const int pid = q.table[(size_t)(m / q.rows_per_seq) * q.max_pages + (ps >> 4)];
+        if ((unsigned)pid >= (unsigned)q.pages) {
+          atomicExch(status, 1);
+          continue;
+        }
+        const int kh = head - q.Hq, isv = kh >= q.Hkv ? 1 : 0;
+        dst = q.pool + (((size_t)pid * q.Hkv + (kh - isv * q.Hkv)) * 2 + isv) * (16 * 128) + (ps & 15) * 128 + d;
+      }
+      dst[0] = __float2half_rn(lo);
+      dst[64] = __float2half_rn(hi);
+    }
+  }
+}
+
+struct Plan {
+  int kst, nk, bn, m_tiles, n_tiles, dp_tiles, sk_tiles, npairs, nstages, nslots;
+  int box_rows;  // rows of an activation box
+  size_t smem, ws_floats;
+};
+// gemm_tc.cu: kernel parameters and the tensor map of the activations for a plan; QENG_ERR_STATE when the plan cuts
+// tiles along K and no workspace can be had (inside a stream capture)
+int32_t prepare(qeng_ctx* ctx, const qeng_weight* w, const qeng_tc_x& x, int64_t M, const qeng_tc_epi& epi, cudaStream_t stream,
+                const Plan* pl, TcParams* p, CUtensorMap* map);
+// sums the partials of the tiles cut along K
+int32_t reduce(qeng_ctx* ctx, const TcParams& p, cudaStream_t stream);
+
+}  // namespace qeng_tc

@@ -17,7 +17,7 @@
 //  * the f16 block scale is applied in f32 to the block result.
 #include <mma.h>
 
-#include "qeng_internal.h"
+#include "gemm_tc.h"
 
 namespace {
 
@@ -340,7 +340,7 @@ int32_t qeng_gemm_q4(qeng_ctx* ctx, const qeng_weight* w, const void* x, int32_t
   if (M < 1) return qeng_fail(ctx, QENG_ERR_SHAPE, "gemm_q4: M=%lld", (long long)M);
   if (ldx < w->K || ldy < w->N) return qeng_fail(ctx, QENG_ERR_SHAPE, "gemm_q4: leading dimension smaller than the row");
   QENG_ENTER(ctx);
-  if (M >= kManyRows) {  // dense contraction: dequantise to bf16 in shared memory, tcgen05 MMA
+  if (M >= kManyRows || qeng_gemm_rows_fits(ctx, w, M, x_dtype == QENG_BF16 ? 1 : 2)) {  // dense contraction: dequantise to bf16 in shared memory, tcgen05 MMA
     const bool prompt = M >= kPrefillRows && w->fmt == QENG_FMT_Q4;
     if (prompt && x_dtype == QENG_F16)
       return qeng_fail(ctx, QENG_ERR_SHAPE, "gemm_q4 (prefill): f16 activations are not supported, use f32 or bf16");

@@ -41,6 +41,8 @@ struct qeng_weight {
   // tensor maps of both planes for the tensor-core matmul (gemm_tc.cu), encoded on first use: [1 or 2 chunks per box][codes, scales]
   mutable bool tc_maps_ready = false;
   alignas(64) mutable unsigned char tc_maps[2][2][128];
+  mutable int rows_plan[4][10] = {};  // gemm_rows.cu: plans of the last few row counts
+  mutable int rows_plan_next = 0;
   const qeng_weight* next = nullptr;  // matrix the caller multiplies by after this one (L2 prefetch hint)
 };
 
@@ -250,7 +252,7 @@ int32_t qeng_scratch_grow(qeng_ctx* ctx, qeng_buf* b, size_t bytes, cudaStream_t
 int32_t qeng_gemm_many_rows(qeng_ctx* ctx, const qeng_weight* w, const void* x, int32_t x_dtype, int64_t M, int64_t ldx,
                             float* y, int64_t ldy, int accumulate, int wp, cudaStream_t stream);
 constexpr int64_t kPrefillRows = 256;  // from this many rows on, 4-bit matmuls run on operands rounded to bf16
-constexpr int64_t kManyRows = 17;      // from this many rows on, matmuls take the tensor-core path
+constexpr int64_t kManyRows = 17;      // from this many rows on, prompt layers take the tensor-core path
 
 void qeng_weight_dequant_q8(const qeng_weight* w, float* out, cudaStream_t stream);
 void qeng_weight_dequant_k4(const qeng_weight* w, float* out, cudaStream_t stream);

@@ -1,0 +1,86 @@
+"""Matmuls of several rows (bf16 operands in two terms, tensor-memory and mma.sync kernels) and the prompt path at the
+edges of their tiles, against float64 arithmetic."""
+import numpy as np
+import pytest
+
+from oracle import ref
+
+pytestmark = pytest.mark.gpu
+DT = ("float32", "bfloat16", "float16")
+
+
+def _weight(ctx, fmt, n, k):
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(7)
+    if fmt == "q4k":
+        _, _, blocks = ref.make_q4k(ref.rng_of(7), n, k)
+        return ctx.pack_q4k(blocks, n, k)
+    w = torch.randn(n, k, device="cuda", generator=g) * 0.05
+    return ctx.quantize_q4(w) if fmt == "q4" else ctx.quantize_q8(w)
+
+
+# Rows: the smallest and largest of the mma.sync kernel's column tiles, of the tensor-memory kernel's token tiles (16 to
+# 256) and of its two- and one-chunk stages.  N: one row tile, a remainder of 256; K: one block, an odd block count, one
+# that cuts tiles along K.
+# Bound: an operand in two bf16 terms is off by 2^-17 of itself at most, bf16 operands by nothing; f32 sums of K products
+# in chains of up to K / 16 tensor-core steps that truncate add K / 16 * 2^-24 of the running sum: 3e-5 covers both at
+# these K (the random errors measured are ten times smaller).
+@pytest.mark.parametrize("fmt", ["q4", "q8", "q4k"])
+@pytest.mark.parametrize("m", [3, 5, 8, 9, 16, 17, 32, 33, 64, 65, 112, 113, 129, 255])
+def test_rows_and_widths(ctx, fmt, m):
+    import torch
+    shapes = [(16, 256), (272, 768)] if fmt == "q4k" else [(16, 32), (272, 736), (1040, 992)]
+    for i, (n, k) in enumerate(shapes):
+        w = _weight(ctx, fmt, n, k)
+        wd = w.dequant().double()
+        for dt in DT:
+            if dt != "bfloat16" and m < 5:
+                continue  # those rows take the integer kernel (tests of its own)
+            x = torch.randn(m, k, device="cuda").to(getattr(torch, dt))
+            y = torch.full((m, n + 8), 0.25, device="cuda")[:, :n]
+            acc = (m + i) % 2
+            ctx.gemm_q4(w, x, out=y, flags=acc)
+            want = x.double() @ wd.T + (0.25 if acc else 0.0)
+            err = float((y.double() - want).abs().max() / want.abs().max())
+            assert err < 3e-5, (fmt, m, n, k, dt, err)
+    ctx.device_status()
+
+
+def test_results_do_not_depend_on_the_call_before(ctx):
+    """Back-to-back calls of several shapes share workspaces and overlap at their ends."""
+    import torch
+    ws = [_weight(ctx, f, n, k) for f, n, k in (("q4", 4096, 4096), ("q8", 1040, 992), ("q4", 272, 736))]
+    calls = [(w, torch.randn(m, w.cols, device="cuda").to(d)) for w in ws for m, d in
+             ((8, torch.bfloat16), (16, torch.float32), (101, torch.float32), (300, torch.bfloat16))]
+    want = []
+    for w, x in calls:
+        want.append(ctx.gemm_q4(w, x).clone())
+        torch.cuda.synchronize()
+    for _ in range(3):
+        got = [ctx.gemm_q4(w, x) for w, x in calls]
+        for a, b in zip(got, want):
+            assert torch.equal(a, b)
+    ctx.device_status()
+
+
+# Prompt attention tiles hold 64 (token, head) rows and 32 keys: prompts one short of, at and one beyond a tile, continued
+# from an odd length, with a window that ends inside a tile, two sequences of unequal history are not possible (one length
+# per call), so two equal ones.
+@pytest.mark.parametrize("softcap,window", [(0.0, 0), (20.0, 0), (0.0, 21)])
+@pytest.mark.parametrize("lens", [(31, 1), (32, 33), (65, 18), (17, 40)])
+def test_prompt_in_two_calls_matches_the_teacher(ctx, lens, softcap, window):
+    from cyb_b200 import qeng
+    cfg = ref.DecoderConfig(layers=2, d=256, ffn=512, heads=4, kv_heads=2, vocab=320, attn_softcap=softcap, sliding_window=window)
+    W = ref.make_decoder_weights(cfg, seed=5)
+    dec = ctx.decoder(layers=2, d_model=256, ffn=512, heads=4, kv_heads=2, vocab=320, max_batch=2, max_seq=128,
+                      attn_softcap=softcap, sliding_window=window)
+    qeng.load_decoder_weights(dec, W, cfg)
+    prompt = ref.rng_of(sum(lens)).integers(0, 320, (2, sum(lens))).astype(np.int32)
+    dec.reset(2)
+    dec.prefill(prompt[:, :lens[0]])
+    dec.prefill(prompt[:, lens[0]:])
+    want, logs = ref.Decoder(cfg, W).generate(prompt, 3)
+    assert ref.err_inf(dec.logits(), logs[0]) < 2e-3
+    assert np.array_equal(dec.decode(3), want)
+    dec.free()

@@ -149,21 +149,6 @@ __global__ void __launch_bounds__(256) last_rows_kernel(const float* __restrict_
   for (int i = threadIdx.x; i < D / 4; i += 256) dst[i] = src[i];
 }
 
-// Unfused end of a decode step (batches the fused LM head does not take): record the sampled
-// tokens as entry step+1, move every sequence one token on.
-__global__ void advance_kernel(const int32_t* __restrict__ next, int32_t* pos, int32_t* lens, int32_t* out_tokens,
-                               int32_t* step, int B) {
-  const int b = threadIdx.x;
-  const int st = *step;
-  __syncthreads();
-  if (b < B) {
-    out_tokens[(size_t)(st + 1) * B + b] = next[b];
-    pos[b] += 1;
-    lens[b] += 1;
-  }
-  if (b == 0) *step = st + 1;
-}
-
 // Start of a decode call: the token sampled from the logits already present is entry 0.
 __global__ void record_first_kernel(const int32_t* __restrict__ next, int32_t* out_tokens, int B) {
   if ((int)threadIdx.x < B) out_tokens[threadIdx.x] = next[threadIdx.x];
@@ -226,7 +211,7 @@ struct qeng_decoder {
   __half* q16 = nullptr;
   int32_t *pos = nullptr, *lens = nullptr, *table = nullptr, *tok = nullptr;  // per row
   // decode state
-  float *xn = nullptr, *xlast = nullptr, *logits = nullptr;
+  float *xlast = nullptr, *logits = nullptr;
   int32_t *next = nullptr, *out_tokens = nullptr, *step = nullptr, *dec_table = nullptr;
   int max_steps = 0;
   int32_t* h_out = nullptr;  // pinned: the tokens of a decode call, then the status word (one synchronisation per call)
@@ -542,27 +527,24 @@ int32_t run_layer(qeng_ctx* ctx, qeng_decoder* d, int l, int64_t rows, int64_t T
   return rc;
 }
 
-// sharded LM head: every rank fills its vocabulary columns of the logits, in chunks of up to 4 rows
+// sharded LM head: every rank fills its vocabulary columns of the logits
 int32_t tail_sharded(qeng_ctx* ctx, qeng_decoder* d, const float* x_last, int B, bool finalize, cudaStream_t st) {
   const int dm = d->cfg.d_model, V = d->cfg.vocab, W = d->cfg.tp_world, R = d->cfg.tp_rank;
   if (!finalize)  // the other ranks' columns must be zero for the sum below
     QENG_CUDA(ctx, cudaMemsetAsync(d->logits, 0, (size_t)B * V * 4, st));
-  for (int m0 = 0; m0 < B; m0 += 4) {
-    qeng_lm_tail t;
-    t.table = d->lm_head; t.x = x_last + (size_t)m0 * dm; t.M = B - m0 < 4 ? B - m0 : 4; t.D = dm; t.V = d->vloc;
-    t.logits = d->logits + (size_t)m0 * V; t.v0 = d->v0; t.Vtot = V; t.ldl = V;
-    t.gamma = d->final_norm; t.eps = d->cfg.rms_eps; t.softcap = d->cfg.final_softcap;
-    if (finalize) { t.pairs = d->tp_pairs; t.pair_slot = R * B + m0; }
-    d->launches += 1;
-    int32_t rc = qeng_lm_head_fused(ctx, t, st);
-    if (rc != QENG_OK) return rc;
-  }
+  qeng_lm_tail t;
+  t.table = d->lm_head; t.x = x_last; t.M = B; t.D = dm; t.V = d->vloc;
+  t.logits = d->logits; t.v0 = d->v0; t.Vtot = V; t.ldl = V;
+  t.gamma = d->final_norm; t.eps = d->cfg.rms_eps; t.softcap = d->cfg.final_softcap;
+  if (finalize) { t.pairs = d->tp_pairs; t.pair_slot = R * B; }
+  d->launches += 1;
+  int32_t rc = qeng_lm_head_fused(ctx, t, st);
+  if (rc != QENG_OK) return rc;
   if (!finalize) {  // prompt end: every rank needs the full logits (zero + x = x, so the sum is exact)
     d->logits_partial = false;
     return qeng_tp_all_reduce_internal(ctx, d->logits, (int64_t)B * V, st);
   }
   const int64_t n = (int64_t)2 * W * B;  // a multiple of 4: W is even
-  int32_t rc;
   if (qeng_tp_p2p_ready(ctx, n)) {
     rc = qeng_tp_allreduce_add(ctx, d->tp_gath, d->tp_pairs, n, st);  // tp_gath is zero on entry
   } else {
@@ -581,36 +563,15 @@ int32_t tail_sharded(qeng_ctx* ctx, qeng_decoder* d, const float* x_last, int B,
 // final norm + LM head (+ greedy finalisation: sample, record, advance, embed the next token)
 int32_t tail(qeng_ctx* ctx, qeng_decoder* d, const float* x_last, int B, bool finalize, cudaStream_t st) {
   if (d->vsplit) return tail_sharded(ctx, d, x_last, B, finalize, st);
-  if (B <= 4) {
-    qeng_lm_tail t;
-    t.table = d->lm_head; t.x = x_last; t.M = B; t.D = d->cfg.d_model; t.V = d->cfg.vocab; t.logits = d->logits;
-    t.gamma = d->final_norm; t.eps = d->cfg.rms_eps; t.softcap = d->cfg.final_softcap;
-    if (finalize) {
-      t.next = d->next; t.emb = d->emb; t.xout = d->x; t.pos = d->pos; t.lens = d->lens;
-      t.out_tokens = d->out_tokens; t.step = d->step;
-    }
-    d->launches += 1;
-    return qeng_lm_head_fused(ctx, t, st);
+  qeng_lm_tail t;
+  t.table = d->lm_head; t.x = x_last; t.M = B; t.D = d->cfg.d_model; t.V = d->cfg.vocab; t.logits = d->logits;
+  t.gamma = d->final_norm; t.eps = d->cfg.rms_eps; t.softcap = d->cfg.final_softcap;
+  if (finalize) {
+    t.next = d->next; t.emb = d->emb; t.xout = d->x; t.pos = d->pos; t.lens = d->lens;
+    t.out_tokens = d->out_tokens; t.step = d->step;
   }
-  int32_t rc = qeng_rmsnorm(ctx, x_last, d->final_norm, B, d->cfg.d_model, d->cfg.rms_eps, d->xn, st);
-  if (rc != QENG_OK) return rc;
-  for (int m0 = 0; m0 < B; m0 += 4) {  // the LM head takes 4 rows per launch
-    qeng_lm_tail t;
-    t.table = d->lm_head; t.x = d->xn + (size_t)m0 * d->cfg.d_model; t.M = B - m0 < 4 ? B - m0 : 4;
-    t.D = d->cfg.d_model; t.V = d->cfg.vocab; t.logits = d->logits + (size_t)m0 * d->cfg.vocab;
-    t.softcap = d->cfg.final_softcap;
-    rc = qeng_lm_head_fused(ctx, t, st);
-    if (rc != QENG_OK) return rc;
-  }
-  d->launches += 1 + (B + 3) / 4;
-  if (!finalize) return QENG_OK;
-  rc = qeng_argmax(ctx, d->logits, B, d->cfg.vocab, d->next, st);
-  if (rc != QENG_OK) return rc;
-  advance_kernel<<<1, 32 * ((B + 31) / 32), 0, st>>>(d->next, d->pos, d->lens, d->out_tokens, d->step, B);
-  QENG_LAUNCH_CHECK(ctx);
-  rc = qeng_embed(ctx, d->emb, d->next, B, d->cfg.d_model, d->cfg.vocab, d->x, st);
-  d->launches += 3;
-  return rc;
+  d->launches += 1;
+  return qeng_lm_head_fused(ctx, t, st);
 }
 
 // Plan the fused step kernel for this decoder (once per set of weights and buffers).  Leaves
@@ -716,7 +677,6 @@ int32_t qeng_decoder_create(qeng_ctx* ctx, const qeng_model_cfg* cfg, qeng_decod
   cudaError_t e = cudaMalloc(&d->pool, pool_bytes);
   if (e == cudaSuccess) e = cudaMemset(d->pool, 0, pool_bytes);
   if (e == cudaSuccess) e = cudaMalloc(&d->rope_cs, (size_t)cfg->max_seq * kHD * 4);
-  if (e == cudaSuccess) e = cudaMalloc(&d->xn, (size_t)cfg->max_batch * dm * 4);
   if (e == cudaSuccess) e = cudaMalloc(&d->xlast, (size_t)cfg->max_batch * dm * 4);
   if (e == cudaSuccess) e = cudaMalloc(&d->logits, (size_t)cfg->max_batch * cfg->vocab * 4);
   if (e == cudaSuccess) e = cudaMalloc(&d->next, 64 * 4);
@@ -782,7 +742,7 @@ int32_t qeng_decoder_free(qeng_ctx* ctx, qeng_decoder* d) {
     if (L.knorm) cudaFree(L.knorm);
   }
   void* bufs[] = {d->emb, d->lm_head, d->final_norm, d->rope_cs, d->pool, d->x, d->xalt, d->qkv, d->att, d->act, d->part, d->xnr, d->q16,
-                  d->pos, d->lens, d->table, d->tok, d->xn, d->xlast, d->logits, d->next, d->out_tokens, d->step, d->dec_table, d->tp_pairs, d->tp_gath};
+                  d->pos, d->lens, d->table, d->tok, d->xlast, d->logits, d->next, d->out_tokens, d->step, d->dec_table, d->tp_pairs, d->tp_gath};
   for (void* p : bufs)
     if (p) cudaFree(p);
   if (d->own_stream) cudaStreamDestroy(d->own_stream);

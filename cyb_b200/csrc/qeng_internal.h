@@ -176,8 +176,8 @@ int32_t qeng_gemm_q4_stream(qeng_ctx* ctx, const qeng_weight* w, const void* x, 
 bool qeng_gemm_q4_stream_fits(const qeng_ctx* ctx, const qeng_weight* w, int64_t M);
 int32_t qeng_gemm_q4_stream_reserve(qeng_ctx* ctx, const qeng_weight* w, int64_t M);
 
-// ops.cu: LM head with optional fused RMSNorm and optional greedy finalisation (argmax over the
-// vocabulary, record the token, advance the sequences, gather the next embedding) in one launch.
+// lm_head.cu: LM head with optional RMSNorm and optional greedy finalisation (argmax over the vocabulary,
+// record the token, advance the sequences, gather the next embedding).
 struct qeng_lm_tail {
   const uint16_t* table = nullptr;  // bf16 [V][D]
   const float* x = nullptr;         // [M][D]
@@ -201,6 +201,7 @@ struct qeng_lm_tail {
                                     // sampling compares the raw values (the map is monotonic)
 };
 int32_t qeng_lm_head_fused(qeng_ctx* ctx, const qeng_lm_tail& t, cudaStream_t stream);
+constexpr int64_t kHeadRows = 16;  // rows per launch
 
 // decode_step.cu: all layers of one decode step (1 or 2 rows) in one persistent cooperative kernel
 struct qeng_step;

@@ -84,3 +84,18 @@ def test_prompt_in_two_calls_matches_the_teacher(ctx, lens, softcap, window):
     assert ref.err_inf(dec.logits(), logs[0]) < 2e-3
     assert np.array_equal(dec.decode(3), want)
     dec.free()
+
+
+# Rows: one, a full launch and one over; V: less than one 8-row tile, a ragged last tile, and more than one round of CTAs;
+# D: one chunk of 64, a cut one, many.  Bound: the activations are exact, a chunk of 64 products truncates at 4
+# tensor-core steps (4 * 2^-24 of its partial sums) and the chunks are added with compensation: 2^-21 of the largest sum.
+@pytest.mark.parametrize("v,d", [(5, 64), (1000, 200), (40001, 1032), (320, 4096)])
+def test_lm_head_edges(ctx, v, d):
+    import torch
+    tb = (torch.randn(v, d, device="cuda") * 0.05).bfloat16()
+    for m in (1, 5, 16, 17):
+        x = torch.randn(m * d + 1, device="cuda")[1 if m == 5 else 0:][:m * d].view(m, d)
+        y = ctx.lm_head(tb.view(torch.int16), x)
+        want = x.double() @ tb.double().T
+        assert float((y.double() - want).abs().max() / want.abs().max()) < 2.0 ** -21, (v, d, m)
+    ctx.device_status()

@@ -2,37 +2,38 @@
 //
 // Pool layout: f16 [page][kv head][K|V][16 tokens][128], so the K tile and the
 // V tile of one (page, kv head) are 8 KB contiguous.  One CTA serves one
-// (sequence, kv head, split).  A producer warp looks up the page ids and brings
-// the CTA's page tiles into a ring of 8 KB shared-memory slots with bulk
-// asynchronous copies (cp.async.bulk, completion counted on an mbarrier), so the
-// bytes in flight per SM (two CTAs x 80 KB) do not depend on registers.  Four
-// consumer warps take the slots round-robin, read the K and V tiles into MMA
-// fragments with 128-bit shared loads (the contraction index of an MMA may be
-// permuted freely as long as both operands agree, which lets every lane read
-// contiguous 16-byte pieces), and keep an online softmax (max, sum, out) per
-// query head of the group.  Warps are merged in shared memory.  Splits: the eight CTAs of a thread-block cluster take the pages of a
+// (sequence, kv head, split).  Each warp looks after the pages it will read: it
+// keeps two in flight in shared-memory slots of its own (TMA, 128-byte swizzle,
+// completion on an mbarrier) and refills a slot when it has consumed it.  The query heads
+// of the group are the eight columns of every MMA, S^T = K Q^T and O^T = V^T P^T,
+// so that K and V are the 16-row operands, read with ldmatrix without bank
+// conflicts, and no MMA row is wasted on absent heads; P changes its layout with
+// movmatrix.  Online softmax (max, sum, out) per query head; warps are merged in shared memory.
+// Splits: the CTAs of a thread-block cluster (up to 16) take the pages of a
 // sequence round-robin and merge through distributed shared memory (no scratch,
-// no atomics); caches beyond 16K tokens fall back to fixed page ranges merged
+// no atomics); many (sequence, kv head) pairs take fixed page ranges merged
 // through a scratch buffer by the CTA that arrives last.
 //
-// HBM-bound: algorithmic bytes = sum_b len_b * kv_heads * 2 * 128 * 2.
+// HBM-bound: algorithmic bytes = sum_b len_b * kv_heads * 2 * 128 * 2.  With one producer warp for all slots, clusters of
+// eight and Q as the (mostly empty) 16-row operand: 1 x 15001 tokens, 8 kv heads 36 us, now 16 us (floor 9.5); 16 ragged
+// sequences of 512 to 4096 tokens 39 us, now 32 us (24.5); 16 of 4096: 74 us, now 48 us (42).
+#include <cuda.h>
 #include <math.h>
-#include <stdlib.h>
+#include <string.h>
 
+#include "attn_prefill.h"
 #include "qeng_internal.h"
 
 namespace {
 
-constexpr int kAW = 4;  // consumer warps per CTA (one more warp produces)
-constexpr int kAT = (kAW + 1) * 32;  // threads per CTA
-constexpr int kRing = 8;             // ring slots of one page tile (K and V of 16 tokens: 8 KB)
-// A slot must always be consumed by the same warp (page i goes to warp i % kAW and slot i % kRing):
-// a warp that consumed round r of a slot cannot then wait for round r + 2 before round r + 1 has
-// landed, which a parity wait could not tell from round r + 2 being there.
-static_assert(kRing % kAW == 0, "every ring slot belongs to one consumer warp");
 constexpr int kSlotBytes = 2 * 16 * 128 * 2;
 constexpr int kHD = 128;
-constexpr int kCS = 8;  // largest cluster: CTAs (splits) per sequence and kv head; the launch picks 1, 2, 4 or 8
+constexpr int kHDP = kHD + 4;  // row stride of the warps' outputs in shared memory: no bank conflicts
+constexpr int kCS = 16;  // largest cluster: CTAs (splits) per sequence and kv head
+constexpr int kAW = 4;      // warps per CTA of the fixed splits, three CTAs per SM
+constexpr int kAT = kAW * 32;
+constexpr int kDepth = 2;  // pages in flight per warp
+constexpr int ring_bytes(int warps, int depth) { return warps * depth * kSlotBytes + 1024; }  // and its alignment
 
 __device__ __forceinline__ uint32_t cluster_map(const void* smem_ptr, uint32_t cta_rank) {
   uint32_t r;
@@ -60,7 +61,6 @@ struct AttnParams {
   int32_t* status;
   int* counters;   // [B][Hkv] arrivals per (sequence, kv head); null = merge in a second kernel
   int pages, Hkv, Hq, grp, max_pages, pps, S;
-  float scale_log2;
   float scale, softcap;  // softcap > 0: logits = softcap * tanh(q.k * scale / softcap) (Gemma family)
   int window;            // > 0: only the last `window` tokens of a sequence are attended (sliding window)
 };
@@ -78,9 +78,9 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n selp.u32 %0, 1, 0, p;\n}\n"
+      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
       : "=r"(ok)
-      : "r"(bar), "r"(parity), "r"(1000u)
+      : "r"(bar), "r"(parity)
       : "memory");
   return ok != 0;
 }
@@ -97,27 +97,29 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
     if (t1 - t0 > 2000000000ull) return false;
   }
 }
-__device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(dst),
-               "l"(src), "r"(bytes), "r"(bar)
+// K and V tile of one (page, kv head): 32 rows as two halves of 64 dims, 128-byte swizzled
+__device__ __forceinline__ void page_g2s(uint32_t dst, const CUtensorMap* map, int row, uint32_t bar) {
+  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];\n" ::"r"(dst), "l"(map),
+               "r"(0), "r"(row), "r"(0), "r"(bar)
                : "memory");
 }
-__device__ __forceinline__ uint4 lds128(uint32_t addr) {
-  return *reinterpret_cast<const uint4*>(__cvta_shared_to_generic((size_t)addr));
+__device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldsm4_t(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ uint32_t transpose8x8(uint32_t a) {
+  uint32_t d;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;\n" : "=r"(d) : "r"(a));
+  return d;
 }
 
-__device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                         uint32_t b0, uint32_t b1) {
+__device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   asm volatile(
       "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
-__device__ __forceinline__ uint4 ldg_nc(const uint4* p) {
-  uint4 v;
-  asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
-  return v;
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
 __device__ __forceinline__ uint32_t pack_h2(float a, float b) {
@@ -125,30 +127,28 @@ __device__ __forceinline__ uint32_t pack_h2(float a, float b) {
   return *reinterpret_cast<uint32_t*>(&h);
 }
 
-template <bool kCl>
-__device__ __forceinline__ void attn_decode_body(const AttnParams& p) {
+template <bool kCl, int kW, int kD>
+__device__ __forceinline__ void attn_decode_body(const AttnParams& p, const CUtensorMap* kvmap) {
+  constexpr int kRing = kD * kW;
   // the output projection that follows may start streaming its weights as CTAs of this kernel retire
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
-  extern __shared__ __align__(128) unsigned char ring[];  // kRing slots of one page tile (K then V)
-  __shared__ __align__(8) uint64_t full[kRing], empty[kRing];
-  __shared__ int slot_ok[kRing];
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* ring = smem_raw + (1024u - (smem_u32(smem_raw) & 1023u)) % 1024u;  // kRing slots of one page tile
+  __shared__ __align__(8) uint64_t full[kRing];
   const int s = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  // Without a window the first 32 page-table entries of this CTA do not depend on the sequence
-  // length: the producer asks for them together with the length instead of after it (one memory
+  if (tid == 0) {
+    for (int i = 0; i < kRing; ++i) mbar_init(smem_u32(full + i), 1);
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  // Without a window the warp's first 32 page-table entries do not depend on the sequence
+  // length: they are asked for together with the length instead of after it (one memory
   // round trip less on the way to the first page).  Entries past the sequence are read (the table
   // row is max_pages long) and never used.
-  int pid_spec = -1;
-  if (warp == kAW && p.window == 0) {
-    const int idx = kCl ? s + lane * p.S : s * p.pps + lane;
-    if (idx < p.max_pages && (kCl || lane < p.pps)) pid_spec = p.table[(size_t)b * p.max_pages + idx];
-  }
-  if (tid == 0) {
-    for (int i = 0; i < kRing; ++i) {
-      mbar_init(smem_u32(full + i), 1);
-      mbar_init(smem_u32(empty + i), 1);
-    }
-    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  int pid_cur = -1;
+  if (p.window == 0) {
+    const int i = warp + kW * lane, idx = kCl ? s + i * p.S : s * p.pps + i;
+    if (idx < p.max_pages && (kCl || i < p.pps)) pid_cur = p.table[(size_t)b * p.max_pages + idx];
   }
   __syncthreads();
   // Pages of this CTA, in order: in a cluster the CTAs interleave the pages of the sequence (page =
@@ -170,170 +170,176 @@ __device__ __forceinline__ void attn_decode_body(const AttnParams& p) {
   }
 
   // merge buffers: they live in the ring, which is free once every page of this CTA is consumed
-  float (*sm_o)[8][kHD] = reinterpret_cast<float (*)[8][kHD]>(ring);                                   // [kAW][8][kHD]
-  float (*c_o)[kHD] = reinterpret_cast<float (*)[kHD]>(ring + sizeof(float) * kAW * 8 * kHD);           // [8][kHD]
-  float (*sm_m)[8] = reinterpret_cast<float (*)[8]>(ring + sizeof(float) * (kAW + 1) * 8 * kHD);        // [kAW][8]
-  float (*sm_l)[8] = sm_m + kAW;                                                                        // [kAW][8]
-  float* c_m = &sm_l[kAW][0];                                                                           // [8]
+  float (*sm_o)[8][kHDP] = reinterpret_cast<float (*)[8][kHDP]>(ring);                                   // [kW][8][kHDP]
+  float (*c_o)[kHD] = reinterpret_cast<float (*)[kHD]>(ring + sizeof(float) * kW * 8 * kHDP);           // [8][kHD]
+  float (*sm_m)[8] = reinterpret_cast<float (*)[8]>(ring + sizeof(float) * (kW * 8 * kHDP + 8 * kHD));        // [kW][8]
+  float (*sm_l)[8] = sm_m + kW;                                                                        // [kW][8]
+  float* c_m = &sm_l[kW][0];                                                                           // [8]
   float* c_l = c_m + 8;                                                                                 // [8]
 
-  float m_run = -INFINITY, l_run = 0.f;
-  float o[16][4];
+  // per lane: query heads 2t and 2t + 1 of the group
+  float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
+  float o[8][4];  // O^T: tile j, rows d = 16 j + g and + 8, columns = the lane's two heads
 #pragma unroll
-  for (int j = 0; j < 16; ++j)
+  for (int j = 0; j < 8; ++j)
 #pragma unroll
     for (int i = 0; i < 4; ++i) o[j][i] = 0.f;
 
-  if (warp == kAW) {
-    // ===== producer: page ids 32 at a time, one 8 KB bulk copy per page ==========================
-    bool failed = false;
-    for (int base = 0; base < n_mine; base += 32) {
-      const int i = base + lane;
-      int pid = -1;
-      if (i < n_mine) pid = (base == 0 && p.window == 0) ? pid_spec : p.table[(size_t)b * p.max_pages + first + i * pstep];
-      const int cnt = min(32, n_mine - base);
-      for (int j = 0; j < cnt; ++j) {
-        const int pj = __shfl_sync(0xffffffffu, pid, j);
-        if (lane == 0) {
-          const int it = base + j, slot = it % kRing;
-          if (!failed && !mbar_wait(smem_u32(empty + slot), ((uint32_t)(it / kRing) & 1u) ^ 1u)) failed = true;
-          const uint32_t bar = smem_u32(full + slot);
-          if ((unsigned)pj >= (unsigned)p.pages) {  // malformed page table: record, hand over an empty slot
-            atomicExch(p.status, 1);
-            slot_ok[slot] = 0;
-            mbar_arrive(bar);
-          } else {
-            slot_ok[slot] = 1;
-            mbar_expect_tx(bar, kSlotBytes);
-            bulk_g2s(smem_u32(ring) + (uint32_t)slot * kSlotBytes, p.pool + ((size_t)pj * p.Hkv + h) * (2 * 16 * kHD), kSlotBytes, bar);
-          }
-        }
+  // Pages warp, warp + kW, ... of the CTA's are this warp's.  It keeps kD of them in flight in slots of its own and refills
+  // a slot as soon as it has consumed it: no other warp is involved (one producer warp that looked after every slot of the
+  // CTA took 240 ns for each page).  32 page ids at a time, the next 32 asked for one block ahead.
+  const int nw = n_mine > warp ? (n_mine - warp + kW - 1) / kW : 0;
+  auto page_id = [&](int n) { return n < nw ? p.table[(size_t)b * p.max_pages + first + (warp + kW * n) * pstep] : -1; };
+  if (p.window != 0) pid_cur = page_id(lane);
+  int pid_next = page_id(32 + lane);
+  const uint32_t slots = smem_u32(ring) + (uint32_t)(warp * kD) * kSlotBytes, bars = smem_u32(full + warp * kD);
+  auto fetch = [&](int n, int base, int slot) {  // page n of the warp; base: the first page that pid_cur holds
+    const int pj = __shfl_sync(0xffffffffu, n - base < 32 ? pid_cur : pid_next, n & 31);
+    if (lane == 0) {
+      if ((unsigned)pj >= (unsigned)p.pages) {  // malformed page table: record, hand over an empty slot
+        atomicExch(p.status, 1);
+        mbar_arrive(bars + 8u * slot);
+      } else {
+        mbar_expect_tx(bars + 8u * slot, kSlotBytes);
+        page_g2s(slots + (uint32_t)slot * kSlotBytes, kvmap, (pj * p.Hkv + h) * 32, bars + 8u * slot);
       }
     }
-    if (failed && lane == 0) atomicExch(p.status, 4);
-  } else {
-    // ===== consumers =================================================================================
-    // Q fragments: row g of the A operand = query head h*grp+g (rows >= grp are zero)
-    uint4 qa[4];
+  };
+  for (int n = 0; n < kD && n < nw; ++n) fetch(n, 0, n);
+  {
+    // The group's heads are the 8 columns of every MMA: S^T = K Q^T (rows = 16 tokens), O^T = V^T P^T (rows = 16 dims).
+    uint32_t qb[8][2];  // column g = query head h * grp + g (zero columns from grp on)
 #pragma unroll
-    for (int i = 0; i < 4; ++i) qa[i] = make_uint4(0u, 0u, 0u, 0u);
+    for (int j = 0; j < 8; ++j) qb[j][0] = qb[j][1] = 0u;
     if (g < p.grp) {
-      const uint4* qp = reinterpret_cast<const uint4*>(p.q + ((size_t)b * p.Hq + (size_t)h * p.grp + g) * kHD);
+      const uint32_t* qp = reinterpret_cast<const uint32_t*>(p.q + ((size_t)b * p.Hq + (size_t)h * p.grp + g) * kHD);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) qa[i] = qp[i * 4 + t];
-    }
-    auto compute_tile = [&](int pg, uint32_t kt, uint32_t vt) {
-      // K rows of tokens g and g+8: the 16 bytes at d = 32i + 8t .. +7.  V is fetched only after the
-      // scores are done, so that the K and V fragments never hold registers at the same time.
-      uint4 kq[2][4];
-#pragma unroll
-      for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) kq[nt][i] = lds128(kt + (uint32_t)(((nt * 8 + g) * 16 + i * 4 + t) * 16));
-      // S = Q K^T for 16 tokens: two n-tiles of 8 tokens
-      float sacc[2][4];
-#pragma unroll
-      for (int nt = 0; nt < 2; ++nt) {
-        sacc[nt][0] = sacc[nt][1] = sacc[nt][2] = sacc[nt][3] = 0.f;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          mma16816(sacc[nt], qa[i].x, 0u, qa[i].y, 0u, kq[nt][i].x, kq[nt][i].y);
-          mma16816(sacc[nt], qa[i].z, 0u, qa[i].w, 0u, kq[nt][i].z, kq[nt][i].w);
-        }
+      for (int j = 0; j < 8; ++j) {
+        qb[j][0] = qp[8 * j + t];
+        qb[j][1] = qp[8 * j + 4 + t];
       }
-      // scale (optionally soft-capped), log2 domain, mask the tail of the last page and what lies before the window
+    }
+    // ldmatrix rows of this lane: K tokens lane % 16, dims + 8 from lane 16 on; V (transposed) tokens + 8 from lane 16
+    // on, dims + 8 in lanes 8-15 and 24-31
+    const int krow = lane & 15, kc = lane >> 4, vrow = 16 + (lane & 7) + (lane >> 4) * 8, vc = (lane >> 3) & 1;
+    const float sc = p.scale * 1.4426950408889634f;
+    auto chunk_at = [](int r, int c) { return (uint32_t)((c >> 3) * 4096 + r * 128 + (((c & 7) ^ (r & 7)) << 4)); };
+    auto compute_tile = [&](int pg, uint32_t kv) {
+      float sa[2][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) sa[0][i] = sa[1][i] = 0.f;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        uint32_t ka[4];
+        ldsm4(kv + chunk_at(krow, 2 * j + kc), ka);
+        mma16816(sa[j & 1], ka, qb[j][0], qb[j][1]);
+      }
+      // scale (optionally soft-capped), log2 domain; lane: tokens g (i < 2) and g + 8, heads 2t and 2t + 1
       const int tok0 = pg * 16;
+      const bool edge = tok0 + 16 > len || tok0 < win0;
       float sv[4];
 #pragma unroll
-      for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          const int tok = tok0 + nt * 8 + 2 * t + c;
-          float x = sacc[nt][c] * p.scale;
-          if (p.softcap > 0.f) x = p.softcap * tanhf(x / p.softcap);
-          sv[nt * 2 + c] = (tok < len && tok >= win0) ? x * 1.4426950408889634f : -INFINITY;
+      for (int i = 0; i < 4; ++i) {
+        float x = sa[0][i] + sa[1][i];
+        if (p.softcap > 0.f) x = p.softcap * tanhf(x * p.scale / p.softcap) * 1.4426950408889634f;
+        else x *= sc;
+        if (edge) {
+          const int tok = tok0 + g + (i >> 1) * 8;
+          if (tok >= len || tok < win0) x = -INFINITY;
         }
-      float tmax = fmaxf(fmaxf(sv[0], sv[1]), fmaxf(sv[2], sv[3]));
-      tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, 1));
-      tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, 2));
-      const float m_new = fmaxf(m_run, tmax);  // finite: a listed page holds at least one attended token
-      const float alpha = exp2f(m_run - m_new);
-      float pr[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) pr[i] = exp2f(sv[i] - m_new);
-      l_run = l_run * alpha + (pr[0] + pr[1] + pr[2] + pr[3]);
-      m_run = m_new;
-      if (__any_sync(0xffffffffu, alpha != 1.0f)) {
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          o[j][0] *= alpha;
-          o[j][1] *= alpha;
-        }
+        sv[i] = x;
       }
-      // P as A operand, split into two f16 terms so no probability precision is lost
-      const uint32_t ph0 = pack_h2(pr[0], pr[1]), ph1 = pack_h2(pr[2], pr[3]);
-      const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&ph0));
-      const float2 f1 = __half22float2(*reinterpret_cast<const __half2*>(&ph1));
-      const uint32_t pl0 = pack_h2(pr[0] - f0.x, pr[1] - f0.y), pl1 = pack_h2(pr[2] - f1.x, pr[3] - f1.y);
-      // V rows of tokens 2t, 2t+1, 2t+8, 2t+9: d = 8g..8g+7 and 64+8g..64+8g+7
-      uint4 vv[4][2];
+      float mx[2] = {fmaxf(sv[0], sv[2]), fmaxf(sv[1], sv[3])}, alpha[2];
 #pragma unroll
-      for (int x = 0; x < 4; ++x) {
-        const int tk = 2 * t + (x & 1) + ((x >> 1) << 3);
-#pragma unroll
-        for (int r = 0; r < 2; ++r) vv[x][r] = lds128(vt + (uint32_t)((tk * 16 + r * 8 + g) * 16));
+      for (int o2 = 4; o2 <= 16; o2 <<= 1) {
+        mx[0] = fmaxf(mx[0], __shfl_xor_sync(0xffffffffu, mx[0], o2));
+        mx[1] = fmaxf(mx[1], __shfl_xor_sync(0xffffffffu, mx[1], o2));
       }
-      // zero V rows that are not attended (their probability is 0, but 0 * garbage may be NaN)
-      if (tok0 + 16 > len || tok0 < win0) {
 #pragma unroll
-        for (int x = 0; x < 4; ++x) {
-          const int tok = tok0 + 2 * t + (x & 1) + ((x >> 1) << 3);
-          if (tok >= len || tok < win0) vv[x][0] = vv[x][1] = make_uint4(0u, 0u, 0u, 0u);
+      for (int i = 0; i < 2; ++i) {
+        const float m_new = fmaxf(m_run[i], mx[i]);  // finite: a listed page holds at least one attended token
+        alpha[i] = exp2f(m_run[i] - m_new);
+        m_run[i] = m_new;
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) sv[i] = exp2f(sv[i] - m_run[i & 1]);
+      l_run[0] = l_run[0] * alpha[0] + (sv[0] + sv[2]);
+      l_run[1] = l_run[1] * alpha[1] + (sv[1] + sv[3]);
+      if (__any_sync(0xffffffffu, alpha[0] != 1.0f || alpha[1] != 1.0f)) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          o[j][0] *= alpha[0]; o[j][1] *= alpha[1];
+          o[j][2] *= alpha[0]; o[j][3] *= alpha[1];
         }
       }
-      // O += P V : n-tile j covers d = 8n + (j&7) + 64*(j>>3), n = column of the tile
+      // P as B operand (tokens x heads transposed within the warp), in two f16 terms so no probability precision is lost
+      uint32_t hi[2], lo[2];
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const int r = j >> 3, jj = j & 7;
-        const uint32_t* va = reinterpret_cast<const uint32_t*>(&vv[0][r]);
-        const uint32_t* vb = reinterpret_cast<const uint32_t*>(&vv[1][r]);
-        const uint32_t* vc = reinterpret_cast<const uint32_t*>(&vv[2][r]);
-        const uint32_t* vd = reinterpret_cast<const uint32_t*>(&vv[3][r]);
-        const uint32_t sel = (jj & 1) ? 0x7632u : 0x5410u;
-        const uint32_t b0 = __byte_perm(va[jj >> 1], vb[jj >> 1], sel);
-        const uint32_t b1 = __byte_perm(vc[jj >> 1], vd[jj >> 1], sel);
-        mma16816(o[j], ph0, 0u, ph1, 0u, b0, b1);
-        mma16816(o[j], pl0, 0u, pl1, 0u, b0, b1);
+      for (int i = 0; i < 2; ++i) {
+        hi[i] = pack_h2(sv[2 * i], sv[2 * i + 1]);
+        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hi[i]));
+        lo[i] = transpose8x8(pack_h2(sv[2 * i] - f.x, sv[2 * i + 1] - f.y));
+        hi[i] = transpose8x8(hi[i]);
+      }
+      // V rows that are not attended are zeroed (their probability is 0, but 0 * garbage may be NaN)
+      uint32_t keep[2] = {0xffffffffu, 0xffffffffu};
+      if (edge) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int tok = tok0 + 8 * i + 2 * t;
+          keep[i] = (tok < len && tok >= win0 ? 0xffffu : 0u) | (tok + 1 < len && tok + 1 >= win0 ? 0xffff0000u : 0u);
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        uint32_t va[4];
+        ldsm4_t(kv + chunk_at(vrow, 2 * j + vc), va);
+        if (edge) {
+          va[0] &= keep[0]; va[1] &= keep[0];
+          va[2] &= keep[1]; va[3] &= keep[1];
+        }
+        mma16816(o[j], va, hi[0], hi[1]);
+        mma16816(o[j], va, lo[0], lo[1]);
       }
     };
     bool failed = false;
-    for (int it = warp; it < n_mine; it += kAW) {
-      const int slot = it % kRing;
-      if (!failed && !mbar_wait(smem_u32(full + slot), (uint32_t)(it / kRing) & 1u)) failed = true;
-      if (slot_ok[slot]) {
-        const uint32_t kt = smem_u32(ring) + (uint32_t)slot * kSlotBytes, vt = kt + 16 * kHD * 2;
-        compute_tile(first + it * pstep, kt, vt);
+    int slot = 0;
+    uint32_t ph = 0;
+    for (int n = 0; n < nw; ++n) {
+      if ((n & 31) == 0 && n > 0) {
+        pid_cur = pid_next;
+        pid_next = page_id(n + 32 + lane);
       }
+      if (!failed && !mbar_wait(bars + 8u * slot, ph)) failed = true;
       __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(empty + slot));  // the slot may be refilled
+      if ((unsigned)__shfl_sync(0xffffffffu, pid_cur, n & 31) < (unsigned)p.pages)
+        compute_tile(first + (warp + kW * n) * pstep, slots + (uint32_t)slot * kSlotBytes);
+      __syncwarp();
+      if (n + kD < nw) fetch(n + kD, n & ~31, slot);
+      if (++slot == kD) { slot = 0; ph ^= 1u; }
     }
     if (failed && lane == 0) atomicExch(p.status, 4);
   }
 
   // ---- merge the warps of this CTA ------------------------------------------
   __syncthreads();  // every warp is done with the ring: it becomes the merge buffers
-  l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);
-  l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
-  if (warp < kAW && g < p.grp) {
-    if (t == 0) {
-      sm_m[warp][g] = m_run;
-      sm_l[warp][g] = l_run;
-    }
+  {
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      const int dbase = (j & 7) + 64 * (j >> 3);
-      sm_o[warp][g][8 * (2 * t) + dbase] = o[j][0];
-      sm_o[warp][g][8 * (2 * t + 1) + dbase] = o[j][1];
+    for (int i = 0; i < 2; ++i) {
+#pragma unroll
+      for (int o2 = 4; o2 <= 16; o2 <<= 1) l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], o2);
+      const int hh = 2 * t + i;
+      if (hh < p.grp) {
+        if (g == 0) {
+          sm_m[warp][hh] = m_run[i];
+          sm_l[warp][hh] = l_run[i];
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          sm_o[warp][hh][16 * j + g] = o[j][i];
+          sm_o[warp][hh][16 * j + 8 + g] = o[j][2 + i];
+        }
+      }
     }
   }
   __syncthreads();
@@ -342,10 +348,10 @@ __device__ __forceinline__ void attn_decode_body(const AttnParams& p) {
   for (int hh = 0; hh < p.grp && tid < kHD; ++hh) {
     float M = -INFINITY;
 #pragma unroll
-    for (int w = 0; w < kAW; ++w) M = fmaxf(M, sm_m[w][hh]);
+    for (int w = 0; w < kW; ++w) M = fmaxf(M, sm_m[w][hh]);
     float L = 0.f, O = 0.f;
 #pragma unroll
-    for (int w = 0; w < kAW; ++w) {
+    for (int w = 0; w < kW; ++w) {
       const float f = sm_m[w][hh] == -INFINITY ? 0.f : exp2f(sm_m[w][hh] - M);  // a warp without pages
       L += sm_l[w][hh] * f;
       O += sm_o[w][hh][tid] * f;
@@ -373,7 +379,7 @@ __device__ __forceinline__ void attn_decode_body(const AttnParams& p) {
     if (cs > 1) cluster_sync();
     else __syncthreads();
     const int dper = kHD / cs;
-    for (int e = tid; e < p.grp * dper; e += kAT) {
+    for (int e = tid; e < p.grp * dper; e += kW * 32) {
       const int hh = e / dper, d = s * dper + e % dper;
       float mr[kCS], lr[kCS], orr[kCS];
 #pragma unroll
@@ -412,7 +418,7 @@ __device__ __forceinline__ void attn_decode_body(const AttnParams& p) {
   __threadfence();
   // one warp per query head; lanes first share the (max, sum) pairs of the splits, then each lane
   // merges 4 of the 128 output dims with independent (pipelined) loads
-  for (int hh = warp; hh < p.grp && warp < kAW; hh += kAW) {
+  for (int hh = warp; hh < p.grp; hh += kW) {
     const size_t row0 = ((size_t)b * p.Hq + (size_t)h * p.grp + hh) * p.S;
     float M = -INFINITY;
     for (int s2 = lane; s2 < ns; s2 += 32) M = fmaxf(M, __ldcg(p.part_ml + (row0 + s2) * 2));
@@ -441,15 +447,18 @@ __device__ __forceinline__ void attn_decode_body(const AttnParams& p) {
 }
 
 // three CTAs per SM (<= 136 registers): this path is chosen when there are many pages per SM to cover
-__global__ void __launch_bounds__(kAT, 3) attn_decode_kernel(const AttnParams p) { attn_decode_body<false>(p); }
+__global__ void __launch_bounds__(kAT, 3) attn_decode_kernel(const AttnParams p, const __grid_constant__ CUtensorMap kvmap) {
+  attn_decode_body<false, kAW, kDepth>(p, &kvmap);
+}
 
 // launched with a cluster dimension of (p.S, 1, 1) = (gridDim.x, 1, 1)
-__global__ void __launch_bounds__(kAT) attn_decode_cluster_kernel(const AttnParams p) {
+template <int kW, int kD>
+__global__ void __launch_bounds__(kW * 32, 1) attn_decode_cluster_kernel(const AttnParams p, const __grid_constant__ CUtensorMap kvmap) {
 #ifdef QENG_TRACE
   unsigned long long* rec = nullptr;
   if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0) rec = qeng_trace_open(p.status, 2);
 #endif
-  attn_decode_body<true>(p);
+  attn_decode_body<true, kW, kD>(p, &kvmap);
 #ifdef QENG_TRACE
   if (rec) rec[4] = qeng_trace_now();
 #endif
@@ -494,6 +503,31 @@ __global__ void kv_append_kernel(__half* pool, const float* k, const float* v, c
 
 }  // namespace
 
+static int g_clusters16[64][2];  // per device: clusters of 16 CTAs of 6 and of 4 warps that fit at a time
+
+// opt-in sizes of the cluster kernel with W warps, and how many clusters of 16 the device holds at a time
+template <int W>
+static int32_t cluster_configure(qeng_ctx* ctx, int* clusters16) {
+  auto* fn = attn_decode_cluster_kernel<W, kDepth>;
+  QENG_CUDA(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, ring_bytes(W, kDepth)));
+  QENG_CUDA(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(16, 1, 64);
+  cfg.blockDim = dim3(W * 32);
+  cfg.dynamicSmemBytes = ring_bytes(W, kDepth);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 16;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (cudaOccupancyMaxActiveClusters(clusters16, fn, &cfg) != cudaSuccess) {
+    *clusters16 = 0;  // no such clusters here: the launches stay at eight
+    (void)cudaGetLastError();
+  }
+  return QENG_OK;
+}
+
 // ---- scratch for the entry point that allocates nothing ---------------------------------
 // Some hosts may not allocate device memory once they are running: a runtime that hands the
 // engine a fixed memory budget at start-up, or a caller inside a region where the CUDA
@@ -514,8 +548,9 @@ constexpr int kMaxAttnCounters = 1 << 16;  // (sequence, kv head) pairs per call
 static int pages_per_split(const qeng_ctx* ctx, int64_t B, int64_t Hkv, int64_t max_pages) {
   // the fixed-split kernel keeps three CTAs per SM resident: one full wave of them is the target
   int64_t target = (int64_t)ctx->sm_count * (ctx->attn_ctas_per_sm > 0 ? ctx->attn_ctas_per_sm : 3);
-  // splits per (sequence, kv head) that fill the wave, then equal page ranges for the longest sequence
-  int64_t S = (target + B * Hkv - 1) / (B * Hkv);
+  // splits per (sequence, kv head) that fill the wave without going over it, then equal page ranges for the longest
+  // sequence.  (16 sequences of 4096 tokens, 8 kv heads: 3 splits 48 us; 4 splits, a wave and a bit, 55 us.)
+  int64_t S = target / (B * Hkv);
   if (S < 1) S = 1;
   int64_t pps = (max_pages + S - 1) / S;
   pps = (pps + kAW - 1) / kAW * kAW;
@@ -564,6 +599,13 @@ int32_t qeng_kv_pool_create(qeng_ctx* ctx, int64_t pages, int64_t kv_heads, int6
     delete p;
     return qeng_fail(ctx, QENG_ERR_CUDA, "kv_pool_create: %s", cudaGetErrorString(e));
   }
+  int32_t rc = qeng_kv_map(ctx, p->data, pages * kv_heads * 32, p->map);
+  if (rc != QENG_OK) {
+    cudaFree(p->data);
+    delete p;
+    return rc;
+  }
+  p->mapped = true;
   *out = p;
   return QENG_OK;
 }
@@ -593,12 +635,23 @@ int32_t qeng_kv_append(qeng_ctx* ctx, qeng_kv_pool* pool, const float* k, const 
 }
 
 // opt-in shared memory of the two attention kernels (the page-tile ring), once per device
+// tensor map of a pool: made with the pool, or here for a view of a layer's part of one
+static int32_t attn_map(qeng_ctx* ctx, const qeng_kv_pool* pool, CUtensorMap* map) {
+  if (pool->mapped) {
+    memcpy(map, pool->map, sizeof(*map));
+    return QENG_OK;
+  }
+  return qeng_kv_map(ctx, pool->data, pool->pages * pool->kv_heads * 32, map);
+}
+
 static int32_t attn_configure(qeng_ctx* ctx) {
   static bool configured_on[64] = {};
   bool& configured = configured_on[ctx->device & 63];
   if (configured) return QENG_OK;
-  QENG_CUDA(ctx, cudaFuncSetAttribute(attn_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRing * kSlotBytes));
-  QENG_CUDA(ctx, cudaFuncSetAttribute(attn_decode_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRing * kSlotBytes));
+  QENG_CUDA(ctx, cudaFuncSetAttribute(attn_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ring_bytes(kAW, kDepth)));
+  int32_t rc = cluster_configure<6>(ctx, &g_clusters16[ctx->device & 63][0]);
+  if (rc == QENG_OK) rc = cluster_configure<4>(ctx, &g_clusters16[ctx->device & 63][1]);
+  if (rc != QENG_OK) return rc;
   configured = true;
   return QENG_OK;
 }
@@ -627,21 +680,32 @@ int32_t qeng_attn_decode_ex(qeng_ctx* ctx, const qeng_kv_pool* pool, const uint1
   p.table = page_table; p.lens = lens; p.out = out; p.status = ctx->status;
   p.pages = (int)pool->pages; p.Hkv = (int)pool->kv_heads; p.Hq = (int)Hq; p.grp = (int)(Hq / pool->kv_heads);
   p.max_pages = (int)max_pages;
-  p.scale_log2 = scale * 1.4426950408889634f;
   p.scale = scale; p.softcap = softcap; p.window = window;
-  const bool no_cluster = !ctx->attn_cluster;
-  // Cluster path: 1, 2, 4 or 8 CTAs per (sequence, kv head), as many as keep the grid within about one
-  // wave (two CTAs per SM), merged through distributed shared memory; caches beyond 16K tokens and
-  // long caches at large batch (bandwidth-bound, a little faster there) take the fixed splits below.
-  int cs = kCS;
-  while (cs > 1 && B * pool->kv_heads * cs > 2 * (int64_t)ctx->sm_count) cs >>= 1;
-  if (!no_cluster && max_pages <= 1024 && B * pool->kv_heads * max_pages <= 16384) {
+  CUtensorMap map;
+  int32_t rc1 = attn_map(ctx, pool, &map);
+  if (rc1 != QENG_OK) return rc1;
+  // Cluster path: as many CTAs per (sequence, kv head) as keep the grid within two CTAs per SM, sixteen where the device
+  // holds all the clusters of sixteen at a time (of 6 warps, else of 4).  Below four CTAs per pair the fixed splits are
+  // as fast on long caches and faster on short ones (16 x 64 tokens: 4.8 against 7.0 us).
+  const int64_t pairs = B * pool->kv_heads;
+  const int* clusters16 = g_clusters16[ctx->device & 63];
+  int cs = 8, warps = 6;
+  if (pairs <= clusters16[0]) {
+    cs = 16;
+  } else if (pairs <= clusters16[1]) {
+    cs = 16;
+    warps = 4;
+  }
+  while (cs > 1 && pairs * cs > 2 * (int64_t)ctx->sm_count) cs >>= 1;
+  if (ctx->attn_cluster && cs >= 4) {
     p.pps = 0; p.S = cs; p.counters = nullptr; p.part_o = nullptr; p.part_ml = nullptr;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)cs, (unsigned)p.Hkv, (unsigned)B);
-    cfg.blockDim = dim3(kAT);
-    cfg.dynamicSmemBytes = kRing * kSlotBytes;
+    cfg.blockDim = dim3((unsigned)warps * 32);
+    cfg.dynamicSmemBytes = ring_bytes(warps, kDepth);
     cfg.stream = (cudaStream_t)stream;
+    // (launched with programmatic serialisation as well, a one-sequence decode step got 2 % slower: the CTAs that wait
+    // keep shared memory from the matmul in front)
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = (unsigned)cs;
@@ -649,7 +713,7 @@ int32_t qeng_attn_decode_ex(qeng_ctx* ctx, const qeng_kv_pool* pool, const uint1
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    QENG_CUDA(ctx, cudaLaunchKernelEx(&cfg, attn_decode_cluster_kernel, p));
+    QENG_CUDA(ctx, cudaLaunchKernelEx(&cfg, warps == 6 ? attn_decode_cluster_kernel<6, kDepth> : attn_decode_cluster_kernel<4, kDepth>, p, map));
     return QENG_OK;
   }
   p.pps = pages_per_split(ctx, B, pool->kv_heads, max_pages);
@@ -660,7 +724,7 @@ int32_t qeng_attn_decode_ex(qeng_ctx* ctx, const qeng_kv_pool* pool, const uint1
   p.part_o = ctx->attn_scratch + kMaxAttnCounters;
   p.part_ml = p.part_o + (size_t)B * Hq * p.S * kHD;
   dim3 grid((unsigned)p.S, (unsigned)p.Hkv, (unsigned)B);
-  attn_decode_kernel<<<grid, kAT, kRing * kSlotBytes, (cudaStream_t)stream>>>(p);
+  attn_decode_kernel<<<grid, kAT, ring_bytes(kAW, kDepth), (cudaStream_t)stream>>>(p, map);
   QENG_LAUNCH_CHECK(ctx);
   return QENG_OK;
 }
@@ -702,10 +766,14 @@ int32_t qeng_attn_decode_noalloc(qeng_ctx* ctx, const qeng_kv_pool* pool, const 
   p.table = page_table; p.lens = lens; p.out = out; p.status = ctx->status;
   p.pages = (int)pool->pages; p.Hkv = (int)pool->kv_heads; p.Hq = (int)Hq; p.grp = (int)(Hq / pool->kv_heads);
   p.max_pages = (int)max_pages;
-  p.scale_log2 = scale * 1.4426950408889634f;
   p.scale = scale; p.softcap = 0.f; p.window = 0;
   {
     int32_t rc0 = attn_configure(ctx);
+    if (rc0 != QENG_OK) return rc0;
+  }
+  CUtensorMap map;
+  {
+    int32_t rc0 = attn_map(ctx, pool, &map);
     if (rc0 != QENG_OK) return rc0;
   }
   // every partial that the merge reads is written by this call first: nothing has to start at zero
@@ -713,7 +781,7 @@ int32_t qeng_attn_decode_noalloc(qeng_ctx* ctx, const qeng_kv_pool* pool, const 
   p.part_o = scratch;
   p.part_ml = scratch + (size_t)B * Hq * p.S * kHD;
   dim3 grid((unsigned)p.S, (unsigned)p.Hkv, (unsigned)B);
-  attn_decode_kernel<<<grid, kAT, kRing * kSlotBytes, (cudaStream_t)stream>>>(p);
+  attn_decode_kernel<<<grid, kAT, ring_bytes(kAW, kDepth), (cudaStream_t)stream>>>(p, map);
   QENG_LAUNCH_CHECK(ctx);
   dim3 grid2((unsigned)Hq, (unsigned)B);
   attn_combine_kernel<<<grid2, kHD, 0, (cudaStream_t)stream>>>(p);

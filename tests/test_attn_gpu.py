@@ -178,3 +178,32 @@ def test_long_cache_on_the_fixed_split_path_with_a_window(ctx):
     pool.free()
     pool2.free()
     c2.close()
+
+
+# Pairs of (sequence, kv head): clusters of 16 with six and four warps, of 8, of 4, fixed splits.  Lengths: one token, the
+# edges of a page, a page for every warp in flight and one over, more than 32 pages per warp (the second block of page ids).
+# Bound: scores are f32 sums of exact products in 4 tensor-core steps of two chains (8 * 2^-24 of partial sums below 64:
+# 3e-5 absolute, times the scale 0.09: 3e-6 relative on a weight), weights hold 22 bits, outputs are averages of |v| < 6.
+@pytest.mark.parametrize("b,kv,long", [(1, 8, 3200 * 16), (2, 8, 3000), (5, 8, 8000), (9, 8, 800 * 16 + 3), (19, 4, 3000), (3, 2, 5000)])
+def test_splits_of_every_form(ctx, b, kv, long):
+    import torch
+    lens = np.array(([long, 1, 15, 16, 17, 191 * 16 + 1, 192 * 16, 193 * 16, 31] * 3)[:b], np.int32)
+    lens = np.minimum(lens, long)
+    npages = (lens + 15) // 16
+    pool = ctx.kv_pool(int(npages.sum()), kv)
+    t = pool.tensor().normal_()
+    order = ref.rng_of(b).permutation(int(npages.sum())).astype(np.int32)
+    table = np.zeros((b, int(npages.max())), np.int32)
+    for i, o in enumerate(np.cumsum(npages) - npages):
+        table[i, :npages[i]] = order[o:o + npages[i]]
+    grp = 4 if kv > 2 else 8
+    q = torch.randn(b, kv * grp, 128, device="cuda").half()
+    out = ctx.attn_decode(pool, q, torch.from_numpy(table).cuda(), torch.from_numpy(lens).cuda())
+    ctx.device_status()
+    t = t.view(-1, kv, 2, 16, 128)
+    for i in range(b):
+        kvs = t[torch.from_numpy(table[i, :npages[i]]).cuda().long()].double()          # [page][kv][2][16][128]
+        kvs = kvs.permute(2, 1, 0, 3, 4).reshape(2, kv, -1, 128)[:, :, :int(lens[i])]
+        s = torch.einsum("hgd,htd->hgt", q[i].double().view(kv, grp, 128), kvs[0]) * 128 ** -0.5
+        want = torch.einsum("hgt,htd->hgd", s.softmax(-1), kvs[1]).reshape(kv * grp, 128)
+        assert float((out[i].double() - want).abs().max()) < 2e-5, (i, int(lens[i]))

@@ -99,7 +99,7 @@ template <int FMT, int XP, int NT>
 // then waiting there when this one ends.
 __global__ void __launch_bounds__(kThreadsR + 160, 1) gemm_rows_kernel(const RowsParams p) {
   constexpr int kW = Fmt<FMT>::kW, kS = Fmt<FMT>::kS;
-  constexpr int kRows = XP == 2 ? 4 * NT : 8 * NT;  // activation rows the tiles hold
+  constexpr int kRows = 8 * NT / XP, NR = NT / XP;  // activation rows the tiles hold; accumulators (hi and lo share one)
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t full[kMaxRing], empty[kMaxRing], xbar;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
@@ -155,16 +155,16 @@ __global__ void __launch_bounds__(kThreadsR + 160, 1) gemm_rows_kernel(const Row
     const int cols = XP * p.M;
     if (lane == 0) mbar_expect_tx(smem_u32(&xbar), (uint32_t)(cols * kval * 2));
     __syncwarp();
-    for (int c = lane; c < cols; c += 32) {  // column c: row c / XP, plane c % XP
-      const int m = c / XP, pl = c % XP;
-      bulk_g2s(xs + (uint32_t)c * xstride, p.x + (size_t)pl * p.plane + (size_t)m * p.ldx + kbeg, (uint32_t)kval * 2u, smem_u32(&xbar));
+    for (int c = lane; c < cols; c += 32) {  // column of row m, plane pl: pl * kRows + m
+      const int pl = c / p.M, m = c - pl * p.M;
+      bulk_g2s(xs + (uint32_t)(pl * kRows + m) * xstride, p.x + (size_t)pl * p.plane + (size_t)m * p.ldx + kbeg, (uint32_t)kval * 2u, smem_u32(&xbar));
     }
   }
   if (FMT == QENG_FMT_K4) {
     for (int i = tid; i < XP * p.M * nc * 2; i += kWarps * 32) {
       const int c = i / (nc * 2), b = i - c * nc * 2;  // plane-major: c = plane * M + m
       const float v = p.xsum[(size_t)c * p.nchunks * 2 + c0 * 2 + b];
-      asm volatile("st.shared.f32 [%0], %1;\n" ::"r"(sums + (uint32_t)((c % p.M) * XP + c / p.M) * sstride + (uint32_t)b * 4u), "f"(v) : "memory");
+      asm volatile("st.shared.f32 [%0], %1;\n" ::"r"(sums + (uint32_t)(c / p.M * kRows + c % p.M) * sstride + (uint32_t)b * 4u), "f"(v) : "memory");
     }
   }
   asm volatile("bar.sync 1, %0;\n" ::"n"(kWarps * 32) : "memory");
@@ -180,9 +180,9 @@ __global__ void __launch_bounds__(kThreadsR + 160, 1) gemm_rows_kernel(const Row
     for (int u = u0 + gi; u < u0 + un; u += kGroups) {  // park is a multiple of the groups: unit u is always group u % 4's
       const int s = u % p.nring;
       if (!failed && !mbar_wait(smem_u32(full + s), (uint32_t)(u / p.nring) & 1u)) failed = true;
-      unsigned long long acc[NT][2];  // column tile, row g / g + 8: the lane's two columns
+      unsigned long long acc[NR][2];  // column tile, row g / g + 8: the lane's two columns
 #pragma unroll
-      for (int n = 0; n < NT; ++n) acc[n][0] = acc[n][1] = 0ull;
+      for (int n = 0; n < NR; ++n) acc[n][0] = acc[n][1] = 0ull;
       const uint32_t wb = ring + (uint32_t)s * slot + (uint32_t)lane * 16u, sb = ring + (uint32_t)s * slot + (uint32_t)p.slice * kW;
 #pragma unroll 1
       for (int c = wi; c < nc; c += kGroupWarps) {
@@ -213,25 +213,36 @@ __global__ void __launch_bounds__(kThreadsR + 160, 1) gemm_rows_kernel(const Row
             a1[0] = pair4<FMT>(u, 2, kc); a1[1] = pair4<FMT>(v, 2, kc); a1[2] = pair4<FMT>(u, 3, kc); a1[3] = pair4<FMT>(v, 3, kc);
           }
           uint4 x[NT];
-          float d[NT][4];
+          float d[NR][4];
 #pragma unroll
           for (int n = 0; n < NT; ++n) x[n] = ld128(xc + (uint32_t)(8 * n) * xstride + (uint32_t)b * 64u);
 #pragma unroll
-          for (int n = 0; n < NT; ++n) mma_bf16(d[n], a0, x[n].x, x[n].y, zero);
+          for (int n = 0; n < NR; ++n) mma_bf16(d[n], a0, x[n].x, x[n].y, zero);
 #pragma unroll
-          for (int n = 0; n < NT; ++n) mma_bf16(d[n], a1, x[n].z, x[n].w, d[n]);
+          for (int n = 0; n < NR; ++n) mma_bf16(d[n], a1, x[n].z, x[n].w, d[n]);
+          if (XP == 2) {
+#pragma unroll
+            for (int n = 0; n < NR; ++n) mma_bf16(d[n], a0, x[NT - NR + n].x, x[NT - NR + n].y, d[n]);
+#pragma unroll
+            for (int n = 0; n < NR; ++n) mma_bf16(d[n], a1, x[NT - NR + n].z, x[NT - NR + n].w, d[n]);
+          }
           const unsigned long long s0 = pack2(sg[b][0], sg[b][0]), s1 = pack2(sg[b][1], sg[b][1]);
 #pragma unroll
-          for (int n = 0; n < NT; ++n) {
+          for (int n = 0; n < NR; ++n) {
             fma2(acc[n][0], s0, pack2(d[n][0], d[n][1]));
             fma2(acc[n][1], s1, pack2(d[n][2], d[n][3]));
           }
           if (FMT == QENG_FMT_K4) {
             const unsigned long long m0 = pack2(mn[b][0], mn[b][0]), m1 = pack2(mn[b][1], mn[b][1]);
 #pragma unroll
-            for (int n = 0; n < NT; ++n) {
+            for (int n = 0; n < NR; ++n) {
               const uint32_t sa = sums + (uint32_t)(8 * n + 2 * t) * sstride + (uint32_t)(2 * c + b) * 4u;
-              const unsigned long long x2 = pack2(ldf(sa), ldf(sa + sstride));
+              float e0 = ldf(sa), e1 = ldf(sa + sstride);
+              if (XP == 2) {
+                e0 += ldf(sa + kRows * sstride);
+                e1 += ldf(sa + (kRows + 1) * sstride);
+              }
+              const unsigned long long x2 = pack2(e0, e1);
               fma2(acc[n][0], m0, x2);
               fma2(acc[n][1], m1, x2);
             }
@@ -243,16 +254,11 @@ __global__ void __launch_bounds__(kThreadsR + 160, 1) gemm_rows_kernel(const Row
       // park: [unit][warp of the group][row m][16]
       float* pk = red + (size_t)((u - u0) * kGroupWarps + wi) * (kRows * 16);
 #pragma unroll
-      for (int n = 0; n < NT; ++n) {
-        if (XP == 2) {  // the two columns are the planes of one row
-          pk[(4 * n + t) * 16 + g] = lo_of(acc[n][0]) + hi_of(acc[n][0]);
-          pk[(4 * n + t) * 16 + g + 8] = lo_of(acc[n][1]) + hi_of(acc[n][1]);
-        } else {
-          pk[(8 * n + 2 * t) * 16 + g] = lo_of(acc[n][0]);
-          pk[(8 * n + 2 * t + 1) * 16 + g] = hi_of(acc[n][0]);
-          pk[(8 * n + 2 * t) * 16 + g + 8] = lo_of(acc[n][1]);
-          pk[(8 * n + 2 * t + 1) * 16 + g + 8] = hi_of(acc[n][1]);
-        }
+      for (int n = 0; n < NR; ++n) {
+        pk[(8 * n + 2 * t) * 16 + g] = lo_of(acc[n][0]);
+        pk[(8 * n + 2 * t + 1) * 16 + g] = hi_of(acc[n][0]);
+        pk[(8 * n + 2 * t) * 16 + g + 8] = lo_of(acc[n][1]);
+        pk[(8 * n + 2 * t + 1) * 16 + g + 8] = hi_of(acc[n][1]);
       }
     }
     asm volatile("bar.sync 1, %0;\n" ::"n"(kWarps * 32) : "memory");
@@ -304,9 +310,9 @@ struct RowsPlan {
 RowsPlan find_plan(const qeng_ctx* ctx, const qeng_weight* w, int64_t M, int xp) {
   RowsPlan best = {};
   const int cols = (int)M * xp, sms = ctx->sm_count;
-  const int nt = cols <= 8 ? 1 : cols <= 16 ? 2 : 4;
+  const int nt = xp == 1 && cols <= 8 ? 1 : cols <= 16 ? 2 : 4;  // two planes: a tile of each at least
   if (cols > kMostCols) return best;
-  const int rows = xp == 2 ? 4 * nt : 8 * nt, nch = (int)w->nchunks, ntiles = (int)w->ntiles;
+  const int rows = 8 * nt / xp, nch = (int)w->nchunks, ntiles = (int)w->ntiles;
   const size_t per_chunk = (size_t)(chunk_w(w->fmt) + chunk_s(w->fmt)), unit_red = (size_t)kGroupWarps * rows * 16 * 4;
   double best_cost = 1e30;
   for (int nsl = 1; nsl <= nch && nsl <= sms; ++nsl) {
@@ -379,7 +385,7 @@ int32_t launch_rows(qeng_ctx* ctx, const RowsParams& p, const RowsPlan& pl, cons
 template <int FMT, int XP>
 int32_t launch_nt(qeng_ctx* ctx, const RowsParams& p, const RowsPlan& pl, const qeng_tc_epi& e, int N, cudaStream_t stream) {
   switch (pl.nt) {
-    case 1: return launch_rows<FMT, XP, 1>(ctx, p, pl, e, N, stream);
+    case 1: return launch_rows<FMT, 1, 1>(ctx, p, pl, e, N, stream);  // one plane only
     case 2: return launch_rows<FMT, XP, 2>(ctx, p, pl, e, N, stream);
     default: return launch_rows<FMT, XP, 4>(ctx, p, pl, e, N, stream);
   }

@@ -19,7 +19,6 @@
 // sequences of 512 to 4096 tokens 39 us, now 32 us (24.5); 16 of 4096: 74 us, now 48 us (42).
 #include <cuda.h>
 #include <math.h>
-#include <string.h>
 
 #include "attn_prefill.h"
 #include "qeng_internal.h"
@@ -599,13 +598,6 @@ int32_t qeng_kv_pool_create(qeng_ctx* ctx, int64_t pages, int64_t kv_heads, int6
     delete p;
     return qeng_fail(ctx, QENG_ERR_CUDA, "kv_pool_create: %s", cudaGetErrorString(e));
   }
-  int32_t rc = qeng_kv_map(ctx, p->data, pages * kv_heads * 32, p->map);
-  if (rc != QENG_OK) {
-    cudaFree(p->data);
-    delete p;
-    return rc;
-  }
-  p->mapped = true;
   *out = p;
   return QENG_OK;
 }
@@ -635,15 +627,6 @@ int32_t qeng_kv_append(qeng_ctx* ctx, qeng_kv_pool* pool, const float* k, const 
 }
 
 // opt-in shared memory of the two attention kernels (the page-tile ring), once per device
-// tensor map of a pool: made with the pool, or here for a view of a layer's part of one
-static int32_t attn_map(qeng_ctx* ctx, const qeng_kv_pool* pool, CUtensorMap* map) {
-  if (pool->mapped) {
-    memcpy(map, pool->map, sizeof(*map));
-    return QENG_OK;
-  }
-  return qeng_kv_map(ctx, pool->data, pool->pages * pool->kv_heads * 32, map);
-}
-
 static int32_t attn_configure(qeng_ctx* ctx) {
   static bool configured_on[64] = {};
   bool& configured = configured_on[ctx->device & 63];
@@ -682,7 +665,7 @@ int32_t qeng_attn_decode_ex(qeng_ctx* ctx, const qeng_kv_pool* pool, const uint1
   p.max_pages = (int)max_pages;
   p.scale = scale; p.softcap = softcap; p.window = window;
   CUtensorMap map;
-  int32_t rc1 = attn_map(ctx, pool, &map);
+  int32_t rc1 = qeng_kv_map(ctx, pool->data, pool->pages * pool->kv_heads * 32, &map);
   if (rc1 != QENG_OK) return rc1;
   // Cluster path: as many CTAs per (sequence, kv head) as keep the grid within two CTAs per SM, sixteen where the device
   // holds all the clusters of sixteen at a time (of 6 warps, else of 4).  Below four CTAs per pair the fixed splits are
@@ -773,7 +756,7 @@ int32_t qeng_attn_decode_noalloc(qeng_ctx* ctx, const qeng_kv_pool* pool, const 
   }
   CUtensorMap map;
   {
-    int32_t rc0 = attn_map(ctx, pool, &map);
+    int32_t rc0 = qeng_kv_map(ctx, pool->data, pool->pages * pool->kv_heads * 32, &map);
     if (rc0 != QENG_OK) return rc0;
   }
   // every partial that the merge reads is written by this call first: nothing has to start at zero

@@ -49,8 +49,6 @@ struct qeng_weight {
 struct qeng_kv_pool {
   int64_t pages, kv_heads, hd;
   __half* data;        // [pages][kv_heads][2][16][hd]
-  bool mapped = false;  // map is the pool's tensor map
-  alignas(64) unsigned char map[128];
 };
 
 // Device buffer that only ever grows.

@@ -393,6 +393,8 @@ __global__ void __launch_bounds__(kPrepThreads) tc_prep_kernel(const void* __res
                                                       float* __restrict__ sums, int sum_blocks) {
   __shared__ float sh[kPrepThreads / 32];
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  if (gamma != nullptr)  // the weights of a layer pass through L2 between two uses of its gains
+    for (int k = threadIdx.x * 8; k < K; k += 8 * kPrepThreads) asm volatile("prefetch.global.L1 [%0];\n" ::"l"(gamma + k));
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
   const int tid = threadIdx.x;
   const long long row = blockIdx.x;
@@ -413,28 +415,9 @@ __global__ void __launch_bounds__(kPrepThreads) tc_prep_kernel(const void* __res
     }
   };
   float rs = 1.f;
-  if (gamma != nullptr) {
-    float ss = 0.f;
-    for (int k = tid * 4; k < K; k += 4 * kPrepThreads) {
-      float v[4];
-      load4(k, v);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) ss = fmaf(v[i], v[i], ss);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    if ((tid & 31) == 0) sh[tid >> 5] = ss;
-    __syncthreads();
-    float tot = 0.f;
-#pragma unroll
-    for (int w = 0; w < kPrepThreads / 32; ++w) tot += sh[w];
-    rs = rsqrtf(tot / (float)K + eps);
-  }
-  for (int k = ((int)blockIdx.y * kPrepThreads + tid) * 4; (k & ~127) < K; k += 4 * kPrepThreads * (int)gridDim.y) {  // whole warps: the block sums are shuffled
+  auto emit = [&](int k, float (&v)[4]) {  // whole warps: the block sums are shuffled
     uint2 hi = make_uint2(0u, 0u), lo = make_uint2(0u, 0u);
     if (k < K) {
-      float v[4];
-      load4(k, v);
       if (gamma != nullptr) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) v[i] = v[i] * rs * gamma[k + i];
@@ -460,6 +443,51 @@ __global__ void __launch_bounds__(kPrepThreads) tc_prep_kernel(const void* __res
         if (planes == 2) sums[((long long)gridDim.x + row) * sum_blocks + blk] = sl0;
       }
     }
+  };
+  if (gamma == nullptr) {
+    for (int k = ((int)blockIdx.y * kPrepThreads + tid) * 4; (k & ~127) < K; k += 4 * kPrepThreads * (int)gridDim.y) {
+      float v[4] = {};
+      if (k < K) load4(k, v);
+      emit(k, v);
+    }
+    return;
+  }
+  // the first kKeep * 2048 values of the row stay in registers across the reduction
+  constexpr int kKeep = 4;
+  float v[kKeep][4], ss = 0.f;
+#pragma unroll
+  for (int j = 0; j < kKeep; ++j) {
+    const int k = (j * kPrepThreads + tid) * 4;
+    v[j][0] = v[j][1] = v[j][2] = v[j][3] = 0.f;
+    if (k < K) load4(k, v[j]);
+  }
+#pragma unroll
+  for (int j = 0; j < kKeep; ++j)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) ss = fmaf(v[j][i], v[j][i], ss);
+  for (int k = (kKeep * kPrepThreads + tid) * 4; k < K; k += 4 * kPrepThreads) {
+    float w[4];
+    load4(k, w);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) ss = fmaf(w[i], w[i], ss);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  if ((tid & 31) == 0) sh[tid >> 5] = ss;
+  __syncthreads();
+  float tot = 0.f;
+#pragma unroll
+  for (int w = 0; w < kPrepThreads / 32; ++w) tot += sh[w];
+  rs = rsqrtf(tot / (float)K + eps);
+#pragma unroll
+  for (int j = 0; j < kKeep; ++j) {
+    const int k = (j * kPrepThreads + tid) * 4;
+    if ((k & ~127) < K) emit(k, v[j]);
+  }
+  for (int k = (kKeep * kPrepThreads + tid) * 4; (k & ~127) < K; k += 4 * kPrepThreads) {
+    float w[4] = {};
+    if (k < K) load4(k, w);
+    emit(k, w);
   }
 }
 

@@ -3,7 +3,8 @@
 //
 // HBM-bound: V * D * 2 bytes of table, read once whatever the number of rows.  The table is the A operand of tcgen05
 // MMAs as it is; the activations are three bf16 planes, which hold a f32 exactly, as 48 columns of B.  A CTA owns `rpc`
-// consecutive vocabulary rows (up to 256: two accumulators of 128 lanes), so that one round of CTAs covers the table;
+// consecutive vocabulary rows (up to 256: two accumulators of 128 lanes), so that one round of CTAs covers a table of up
+// to 256 rows per SM (37888 on 148) and several equal rounds a larger one;
 // TMA brings 64-wide K chunks of them through a ring that keeps 200 KB in flight, filled before the kernel in front has
 // ended.  Four warps write the activations of each chunk beside it, times the RMSNorm gain, and sum the squares as they
 // go: the norm's factor is common to a row and multiplies its finished sums.  Tensor memory accumulates one chunk; the
@@ -168,6 +169,23 @@ __global__ void __launch_bounds__(kThreadsL, 1) lm_head_kernel(const HeadParams 
         if (in && m < t.M) load8(t.x + (size_t)m * t.D + k, x0[j], x1[j]);
       }
     };
+    // The sums of squares are complete with the warp's last chunk of the first tile and are handed over right there: the
+    // epilogue waits for them at the end of that tile, and until it goes on no ring stage of the second one is freed.
+    bool published = false;
+    auto publish = [&]() {
+#pragma unroll
+      for (int j = 0; j < kM / 4; ++j) {
+        float v = ss[j];
+        v += __shfl_xor_sync(0xffffffffu, v, 1);
+        v += __shfl_xor_sync(0xffffffffu, v, 2);
+        v += __shfl_xor_sync(0xffffffffu, v, 4);
+        if (c8 == 0) ssq[w][r4 + 4 * j] = v;
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&ss_ready));
+      published = true;
+    };
+    if (w >= p.nk) publish();  // no chunk of the first tile is this warp's
     fetch(w);
     for (int i = w; i < total; i += kConv) {
       const int s = i % p.nstages;
@@ -203,17 +221,9 @@ __global__ void __launch_bounds__(kThreadsL, 1) lm_head_kernel(const HeadParams 
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(full + s));
       fetch(i + kConv);
+      if (i < p.nk && i + kConv >= p.nk) publish();
     }
-#pragma unroll
-    for (int j = 0; j < kM / 4; ++j) {
-      float v = ss[j];
-      v += __shfl_xor_sync(0xffffffffu, v, 1);
-      v += __shfl_xor_sync(0xffffffffu, v, 2);
-      v += __shfl_xor_sync(0xffffffffu, v, 4);
-      if (c8 == 0) ssq[w][r4 + 4 * j] = v;
-    }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(smem_u32(&ss_ready));
+    if (!published) publish();
     if (failed && lane == 0) atomicExch(p.status, 4);
   } else {
     // ===== epilogue: lane = vocabulary row =======================================================================

@@ -327,3 +327,31 @@ def test_softcap_and_sliding_window_decoder(ctx):
     assert not np.array_equal(plain, want)  # the switches change the continuation on this input
     ctx.device_status()
     dec.free()
+
+
+@pytest.mark.parametrize("batch", [1, 16])
+def test_vocabulary_of_several_head_rounds(ctx, batch):
+    """More vocabulary rows than one round of the LM head's CTAs covers (256 per SM), and more 64-wide chunks of the hidden
+    width than its ring and accumulators hold: the RMSNorm factor of the first round must not wait for the second one.
+    Prompt logits and greedy tokens against the float64 teacher."""
+    from cyb_b200 import qeng
+    cfg = ref.DecoderConfig(layers=1, d=1024, ffn=512, heads=8, kv_heads=2, vocab=256 * ctx.sm_count + 2128)
+    W = ref.make_decoder_weights(cfg, seed=6)
+    dec = ctx.decoder(layers=1, d_model=1024, ffn=512, heads=8, kv_heads=2, vocab=cfg.vocab, max_batch=batch, max_seq=16)
+    qeng.load_decoder_weights(dec, W, cfg)
+    prompt = ref.rng_of(600 + batch).integers(0, cfg.vocab, (batch, 3)).astype(np.int32)
+    want, logs = ref.Decoder(cfg, W).generate(prompt, 3)
+    dec.reset(batch)
+    dec.prefill(prompt)
+    ctx.device_status()
+    assert ref.err_inf(dec.logits(), logs[0]) < 2e-3
+    toks = dec.decode(3)
+    ctx.device_status()
+    for b in range(batch):  # a token may only differ where the teacher's two best logits are closer than the gate
+        for s in range(3):
+            if toks[b, s] != want[b, s]:
+                top = np.sort(logs[s][b])[-2:]
+                assert top[1] - top[0] < 2e-3 * np.abs(logs[s][b]).max(), (b, s)
+                break
+    assert (toks == want).mean() > 0.9
+    dec.free()

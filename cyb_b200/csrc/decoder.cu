@@ -968,9 +968,20 @@ int32_t qeng_decoder_prefill(qeng_ctx* ctx, qeng_decoder* d, const int32_t* toke
     QENG_LAUNCH_CHECK(ctx);
     rc = tail(ctx, d, d->xlast, batch, false, st);
   }
-  cudaError_t e = cudaStreamSynchronize(st);
+  int32_t* h_status = d->h_out + (size_t)d->max_steps * d->cfg.max_batch;
+  cudaError_t e = cudaMemcpyAsync(h_status, ctx->status, 4, cudaMemcpyDeviceToHost, st);
+  const cudaError_t es = cudaStreamSynchronize(st);
+  if (e == cudaSuccess) e = es;
   if (rc != QENG_OK) return rc;
   if (e != cudaSuccess) return qeng_fail(ctx, QENG_ERR_CUDA, "decoder_prefill: %s", cudaGetErrorString(e));
+  // A wait that ran out leaves results unwritten: there are no logits to go on from.  (A malformed input, status 1 to 3,
+  // stays for the decode call or qeng_device_status to report.)
+  if (*h_status >= 4) {
+    d->have_logits = d->next_ready = false;
+    const int32_t status = *h_status;
+    cudaMemset(ctx->status, 0, 4);
+    return qeng_fail(ctx, QENG_ERR_DEVICE_STATUS, "decoder_prefill: a kernel reported status %d (4 = a bounded wait on a copy or MMA ran out, 5 = a peer never delivered its part of an all-reduce)", status);
+  }
   for (int b = 0; b < batch; ++b) d->len[b] += T;
   d->have_logits = true;
   d->next_ready = false;
@@ -1059,7 +1070,7 @@ int32_t qeng_decoder_decode(qeng_ctx* ctx, qeng_decoder* d, int32_t steps, int32
   d->next_ready = status == 0;
   if (status != 0) {
     cudaMemset(ctx->status, 0, 4);
-    return qeng_fail(ctx, QENG_ERR_DEVICE_STATUS, "decoder_decode: a kernel reported status %d (1 = page id outside the pool, 2 = position outside the cache, 3 = token id outside the vocabulary)", status);
+    return qeng_fail(ctx, QENG_ERR_DEVICE_STATUS, "decoder_decode: a kernel reported status %d (1 = page id outside the pool, 2 = position outside the cache, 3 = token id outside the vocabulary, 4 = a bounded wait on a copy or MMA ran out, 5 = a peer never delivered its part of an all-reduce)", status);
   }
   // device order is [step][batch]; the caller gets [batch][steps]
   for (int s = 0; s < steps; ++s)

@@ -325,7 +325,9 @@ int32_t qeng_decoder_reset(qeng_ctx* ctx, qeng_decoder* dec, int32_t batch);
  * logits of the last prompt position.  Synchronous.  batch * T rows are processed at once (buffers
  * grow to that size on first use: about 130 KB per row at the 7B shape); from 17 rows on they take the
  * tensor-core matmul and the causal prompt attention.  Long prompts may be fed in chunks (successive
- * calls append) to bound memory and to report progress. */
+ * calls append) to bound memory and to report progress.  A device-side wait that ran out is reported here
+ * (QENG_ERR_DEVICE_STATUS, the prompt does not count as read); a token outside the vocabulary by the next
+ * decode call or qeng_device_status. */
 int32_t qeng_decoder_prefill(qeng_ctx* ctx, qeng_decoder* dec, const int32_t* tokens, int32_t batch, int32_t T);
 /* Greedy decode: runs `steps` steps; each step samples from the current logits,
  * feeds the sampled token and computes the next logits.  Writes the sampled

@@ -75,6 +75,20 @@ def test_state_errors(ctx):
     dec.free()
 
 
+def test_malformed_prompt_token_is_reported_by_the_decode_call(ctx):
+    """The prompt call reads the status word but leaves a malformed input there; the decode call reports it, once."""
+    from cyb_b200 import qeng
+    cfg, W, dec = _make(ctx, max_batch=1, max_seq=32)
+    dec.reset(1)
+    dec.prefill(np.array([[1, cfg.vocab, 2]], np.int32))
+    with pytest.raises(qeng.QengError) as e:
+        dec.decode(1)
+    assert e.value.code == -7 and "status 3" in str(e.value)
+    dec.decode(1)
+    ctx.device_status()
+    dec.free()
+
+
 def test_teacher_forced_layer_on_the_tensor_core_path(ctx):
     """256 rows or more take the tcgen05 matmul (bf16 operands): gate 5e-3 per layer against the
     unrounded float64 teacher; the decode step on top of that cache is back on the exact path."""

@@ -21,21 +21,65 @@ static const size_t kStatusBytes = 256 + 8 * (8 + 30000 * 8);
 static const size_t kStatusBytes = 256;
 #endif
 
+// Allocations are no part of any graph: they are made outside the thread's capture mode, so that a call inside a capture,
+// or beside one on another stream, may make its working memory.
+struct OutsideCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  OutsideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~OutsideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 static void free_scratch(qeng_scratch* sc) {
+  OutsideCapture outside;
+  for (void* p : sc->kept) cudaFree(p);
   for (qeng_buf* b : {&sc->planes, &sc->part})
     if (b->ptr) cudaFree(b->ptr);
   delete sc;
 }
 
-static bool capturing(cudaStream_t stream) {
-  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-  return cudaStreamIsCapturing(stream, &st) == cudaSuccess && st != cudaStreamCaptureStatusNone;
+// gives back the sets of captures whose graphs are gone
+static void free_retired(qeng_ctx* ctx) {
+  auto& v = ctx->scratch;
+  for (size_t i = v.size(); i-- > 0;)
+    if (v[i]->capture != 0 && v[i]->done->load()) {
+      free_scratch(v[i]);
+      v.erase(v.begin() + i);
+    }
+}
+
+// Ties the set to the graph being captured: `done` is raised when the graph and its executables no longer exist.
+// Without the tie (a failing call) the set stays until the context is destroyed.
+static void tie_to_graph(qeng_scratch* sc, cudaGraph_t graph) {
+  using Flag = std::shared_ptr<std::atomic<bool>>;
+  sc->done = std::make_shared<std::atomic<bool>>(false);
+  Flag* flag = new Flag(sc->done);
+  cudaUserObject_t obj;
+  const auto raise = [](void* p) {
+    (*reinterpret_cast<Flag*>(p))->store(true);
+    delete reinterpret_cast<Flag*>(p);
+  };
+  if (cudaUserObjectCreate(&obj, flag, raise, 1, cudaUserObjectNoDestructorSync) != cudaSuccess) {
+    delete flag;
+    (void)cudaGetLastError();
+  } else if (cudaGraphRetainUserObject(graph, obj, 1, cudaGraphUserObjectMove) != cudaSuccess) {
+    sc->done = std::make_shared<std::atomic<bool>>(false);
+    cudaUserObjectRelease(obj, 1);
+    (void)cudaGetLastError();
+  }
 }
 
 qeng_scratch* qeng_scratch_for(qeng_ctx* ctx, cudaStream_t stream) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  cudaGraph_t graph = nullptr;
+  if (cudaStreamGetCaptureInfo(stream, &st, &id, &graph) != cudaSuccess) {
+    (void)cudaGetLastError();  // the default stream, while another one is captured
+    st = cudaStreamCaptureStatusNone;
+  }
+  if (st != cudaStreamCaptureStatusActive) id = 0;
   auto& v = ctx->scratch;  // most recently used last
   for (size_t i = v.size(); i-- > 0;)
-    if (v[i]->stream == stream) {
+    if (v[i]->stream == stream && v[i]->capture == id) {
       if (i + 1 != v.size()) {
         qeng_scratch* sc = v[i];
         v.erase(v.begin() + i);
@@ -43,30 +87,55 @@ qeng_scratch* qeng_scratch_for(qeng_ctx* ctx, cudaStream_t stream) {
       }
       return v.back();
     }
-  // A captured stream is usually one of its own: the calls before the capture, on another stream, made the buffers.
-  if (capturing(stream)) return v.empty() ? nullptr : v.back();
-  if (v.size() >= (size_t)kMaxScratch) {
-    cudaDeviceSynchronize();  // its stream may still be running
-    free_scratch(v.front());
-    v.erase(v.begin());
-    ctx->scratch_gen++;
+  qeng_scratch* sc = nullptr;
+  if (id != 0) {
+    for (size_t i = 0; i < v.size() && !sc; ++i)
+      if (v[i]->capture != 0 && v[i]->done->load()) {
+        sc = v[i];
+        v.erase(v.begin() + i);
+      }
+    if (!sc) sc = new qeng_scratch();
+    sc->capture = id;
+    tie_to_graph(sc, graph);
+  } else {
+    free_retired(ctx);
+    size_t streams = 0, oldest = v.size();
+    for (size_t i = v.size(); i-- > 0;)
+      if (v[i]->capture == 0) {
+        ++streams;
+        oldest = i;
+      }
+    if (streams >= (size_t)kMaxScratch) {
+      cudaDeviceSynchronize();  // its stream may still be running
+      free_scratch(v[oldest]);
+      v.erase(v.begin() + oldest);
+    }
+    sc = new qeng_scratch();
   }
-  v.push_back(new qeng_scratch());
-  v.back()->stream = stream;
-  return v.back();
+  sc->stream = stream;
+  v.push_back(sc);
+  return sc;
 }
 
-// Grows outside the steady state only; a growing call drains the device first.
-int32_t qeng_scratch_grow(qeng_ctx* ctx, qeng_buf* b, size_t bytes, cudaStream_t stream) {
+// Grows outside the steady state only; outside captures a growing call drains the device first.
+int32_t qeng_scratch_grow(qeng_ctx* ctx, qeng_scratch* sc, qeng_buf* b, size_t bytes) {
   if (bytes <= b->bytes) return QENG_OK;
-  if (capturing(stream))
-    return qeng_fail(ctx, QENG_ERR_STATE, "scratch of %zu bytes needed inside a stream capture: make one call of the shape before capturing", bytes);
-  QENG_CUDA(ctx, cudaDeviceSynchronize());
-  if (b->ptr) cudaFree(b->ptr);
+  if (b->ptr && sc->capture != 0) {
+    sc->kept.push_back(b->ptr);
+  } else if (b->ptr) {
+    QENG_CUDA(ctx, cudaDeviceSynchronize());
+    cudaFree(b->ptr);
+    free_retired(ctx);
+  }
   b->ptr = nullptr;
   b->bytes = 0;
-  ctx->scratch_gen++;
-  QENG_CUDA(ctx, cudaMalloc(&b->ptr, bytes));
+  OutsideCapture outside;
+  const cudaError_t e = cudaMalloc(&b->ptr, bytes);
+  if (e != cudaSuccess) {
+    b->ptr = nullptr;
+    (void)cudaGetLastError();  // not the next launch's error
+    return qeng_fail(ctx, QENG_ERR_CUDA, "scratch of %zu bytes: %s", bytes, cudaGetErrorString(e));
+  }
   b->bytes = bytes;
   return QENG_OK;
 }

@@ -1003,9 +1003,6 @@ int32_t qeng_decoder_decode(qeng_ctx* ctx, qeng_decoder* d, int32_t steps, int32
     const qeng_weight* ws[4] = {L0.wqkv, L0.wo, L0.wgu, L0.wdown};
     for (int i = 0; rc == QENG_OK && i < 4; ++i)
       if (ws[i]) rc = qeng_gemm_q4_stream_reserve(ctx, ws[i], B < 16 ? B : 16);
-    for (const Layer& L : d->layers)
-      for (const qeng_weight* w : {L.wqkv, L.wo, L.wgu, L.wdown})
-        if (rc == QENG_OK && w && qeng_gemm_rows_fits(ctx, w, B, 2)) rc = qeng_gemm_rows_reserve(ctx, w, B, 2, st);
     if (rc != QENG_OK) return rc;
   }
   std::vector<int32_t> pos(B), lens(B);

@@ -439,15 +439,6 @@ bool qeng_gemm_rows_fits(const qeng_ctx* ctx, const qeng_weight* w, int64_t M, i
 
 static size_t planes_bytes(const qeng_weight* w, int64_t M, int planes) { return ((size_t)planes * M * w->K * 2 + 15) & ~(size_t)15; }
 
-int32_t qeng_gemm_rows_reserve(qeng_ctx* ctx, const qeng_weight* w, int64_t M, int planes, cudaStream_t stream) {
-  const RowsPlan pl = rows_plan(ctx, w, M, planes);
-  qeng_scratch* sc = pl.ok ? qeng_scratch_for(ctx, stream) : nullptr;
-  if (!sc) return QENG_OK;
-  const int32_t rc = qeng_scratch_grow(ctx, &sc->part, (size_t)pl.nsl * M * w->N * 4, stream);
-  if (rc != QENG_OK) return rc;
-  return qeng_scratch_grow(ctx, &sc->planes, planes_bytes(w, M, planes) + (w->fmt == QENG_FMT_K4 ? (size_t)planes * M * w->nchunks * 8 : 0), stream);
-}
-
 // rows of any type through the kernels above; with `gamma` they are RMS-normalised first
 int32_t qeng_gemm_rows_prep(qeng_ctx* ctx, const qeng_weight* w, const void* x, int32_t dtype, int64_t M, int64_t ldx, const float* gamma, float eps,
                             const qeng_tc_epi& epi, cudaStream_t stream) {
@@ -458,10 +449,10 @@ int32_t qeng_gemm_rows_prep(qeng_ctx* ctx, const qeng_weight* w, const void* x, 
     xx.ld = ldx;
     return qeng_gemm_rows(ctx, w, xx, nullptr, M, epi, stream);
   }
-  int32_t rc = qeng_gemm_rows_reserve(ctx, w, M, planes, stream);
   qeng_scratch* sc = qeng_scratch_for(ctx, stream);
+  const size_t sum_bytes = w->fmt == QENG_FMT_K4 ? (size_t)planes * M * w->nchunks * 8 : 0;
+  int32_t rc = qeng_scratch_grow(ctx, sc, &sc->planes, planes_bytes(w, M, planes) + sum_bytes);
   if (rc != QENG_OK) return rc;
-  if (!sc) return qeng_fail(ctx, QENG_ERR_STATE, "gemm_q4: no activation scratch inside this stream capture (make one call of the shape before capturing)");
   qeng_tc_x xx;
   xx.data = sc->planes.ptr;
   xx.ld = w->K;
@@ -477,8 +468,7 @@ int32_t qeng_gemm_rows(qeng_ctx* ctx, const qeng_weight* w, const qeng_tc_x& x, 
   if (!pl.ok) return qeng_fail(ctx, QENG_ERR_SHAPE, "gemm_rows: %lld rows over [%lld, %lld] do not fit", (long long)M, (long long)w->N, (long long)w->K);
   if (w->fmt == QENG_FMT_K4 && xsum == nullptr) return qeng_fail(ctx, QENG_ERR_ARG, "gemm_rows: K-quant blocks need the block sums of the activations");
   qeng_scratch* sc = qeng_scratch_for(ctx, stream);
-  if (!sc) return qeng_fail(ctx, QENG_ERR_STATE, "gemm_q4: no workspace inside this stream capture (make one call of the shape before capturing)");
-  const int32_t rc = qeng_scratch_grow(ctx, &sc->part, (size_t)pl.nsl * M * w->N * 4, stream);
+  const int32_t rc = qeng_scratch_grow(ctx, sc, &sc->part, (size_t)pl.nsl * M * w->N * 4);
   if (rc != QENG_OK) return rc;
   RowsParams p;
   p.qs = reinterpret_cast<const char*>(w->qs); p.sc = reinterpret_cast<const char*>(w->sc);

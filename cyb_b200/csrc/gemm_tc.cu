@@ -607,8 +607,7 @@ int32_t qeng_tc::prepare(qeng_ctx* ctx, const qeng_weight* w, const qeng_tc_x& x
   p->ws = nullptr;
   if (pl->sk_tiles > 0) {
     qeng_scratch* sc = qeng_scratch_for(ctx, stream);
-    const int32_t rc = sc ? qeng_scratch_grow(ctx, &sc->part, pl->ws_floats * 4, stream) : QENG_ERR_STATE;
-    if (rc != QENG_OK) return rc;
+    if (qeng_scratch_grow(ctx, sc, &sc->part, pl->ws_floats * 4) != QENG_OK) return QENG_ERR_STATE;
     p->ws = reinterpret_cast<float*>(sc->part.ptr);
   }
   EncodeFn enc = encode_fn();
@@ -668,7 +667,7 @@ int32_t qeng_gemm_tc(qeng_ctx* ctx, const qeng_weight* w, const qeng_tc_x& x, in
   TcParams p;
   CUtensorMap map;
   int32_t rc = prepare(ctx, w, x, M, epi, stream, &pl, &p, &map);
-  if (rc == QENG_ERR_STATE) {  // no workspace inside this capture: whole tiles only
+  if (rc == QENG_ERR_STATE) {  // no memory for the workspace: whole tiles only
     pl = make_plan(ctx, w, M, wp, xp, false);
     rc = prepare(ctx, w, x, M, epi, stream, &pl, &p, &map);
   }
@@ -703,8 +702,7 @@ int32_t qeng_gemm_many_rows(qeng_ctx* ctx, const qeng_weight* w, const void* x, 
     xx.ld = w->K;
     xx.plane = M * w->K;
     qeng_scratch* sc = qeng_scratch_for(ctx, stream);
-    if (!sc) return qeng_fail(ctx, QENG_ERR_STATE, "gemm_q4: no activation scratch inside this stream capture (make one call of the shape before capturing)");
-    int32_t rc = qeng_scratch_grow(ctx, &sc->planes, (size_t)planes * M * w->K * 2, stream);
+    int32_t rc = qeng_scratch_grow(ctx, sc, &sc->planes, (size_t)planes * M * w->K * 2);
     if (rc == QENG_OK) rc = qeng_tc_prep(ctx, x, x_dtype, M, w->K, ldx, nullptr, 0.f, planes, sc->planes.ptr, nullptr, stream);
     if (rc != QENG_OK) return rc;
     xx.data = sc->planes.ptr;

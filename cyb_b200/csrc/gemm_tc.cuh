@@ -294,7 +294,7 @@ struct Plan {
   size_t smem, ws_floats;
 };
 // gemm_tc.cu: kernel parameters and the tensor map of the activations for a plan; QENG_ERR_STATE when the plan cuts
-// tiles along K and no workspace can be had (inside a stream capture)
+// tiles along K and there is no memory for the workspace
 int32_t prepare(qeng_ctx* ctx, const qeng_weight* w, const qeng_tc_x& x, int64_t M, const qeng_tc_epi& epi, cudaStream_t stream,
                 const Plan* pl, TcParams* p, CUtensorMap* map);
 // sums the partials of the tiles cut along K

@@ -34,7 +34,6 @@ int32_t qeng_tc_prep(qeng_ctx* ctx, const void* x, int32_t dtype, int64_t M, int
 
 // gemm_rows.cu: a few rows (all formats) at the precision of wp = 2; planes: 1 for bf16 rows, else 2
 bool qeng_gemm_rows_fits(const qeng_ctx* ctx, const qeng_weight* w, int64_t M, int planes);
-int32_t qeng_gemm_rows_reserve(qeng_ctx* ctx, const qeng_weight* w, int64_t M, int planes, cudaStream_t stream);
 int32_t qeng_gemm_rows_prep(qeng_ctx* ctx, const qeng_weight* w, const void* x, int32_t dtype, int64_t M, int64_t ldx, const float* gamma, float eps,
                             const qeng_tc_epi& epi, cudaStream_t stream);
 int32_t qeng_gemm_rows(qeng_ctx* ctx, const qeng_weight* w, const qeng_tc_x& x, const float* xsum, int64_t M, const qeng_tc_epi& epi, cudaStream_t stream);

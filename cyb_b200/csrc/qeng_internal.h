@@ -5,6 +5,8 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include <atomic>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -56,11 +58,16 @@ struct qeng_buf {
   void* ptr = nullptr;
   size_t bytes = 0;
 };
-// Working memory of one stream's calls: calls on different streams of a context do not share it.
+// Working memory of one stream's calls: calls on different streams of a context do not share it.  Calls made while the
+// stream is captured get a set of that capture's own, which no call outside its graph touches and which keeps its
+// addresses until the graph and everything instantiated from it are gone.
 struct qeng_scratch {
   cudaStream_t stream = nullptr;
+  unsigned long long capture = 0;            // id of the capture, 0 = calls outside captures
+  std::shared_ptr<std::atomic<bool>> done;   // captures: the graph is gone
   qeng_buf planes;    // activations as bf16 planes
   qeng_buf part;      // partial sums of tiles cut along K
+  std::vector<void*> kept;  // captures: outgrown buffers that earlier nodes of the graph still use
 };
 
 struct qeng_ctx {
@@ -71,7 +78,7 @@ struct qeng_ctx {
   float* attn_scratch = nullptr;
   size_t attn_scratch_bytes = 0;
   int32_t* status = nullptr;  // device status word (0 = ok)
-  // working memory of the tensor-core matmul, one set per stream that calls it (qeng_scratch_for)
+  // working memory of the tensor-core matmul, one set per stream and per capture that calls it (qeng_scratch_for)
   std::vector<qeng_scratch*> scratch;
   // activations quantised once per decode-batch matmul (more than 4 rows), one image per K slice
   void* ximage = nullptr;
@@ -242,11 +249,12 @@ const unsigned* qeng_tp_fuse_seq(const qeng_ctx* ctx);
 int32_t qeng_tp_fuse_gather(qeng_ctx* ctx, float* x, int64_t rows, int64_t dm, int kind, int layer, int layers, cudaStream_t stream);
 int32_t qeng_tp_fuse_advance(qeng_ctx* ctx, cudaStream_t stream);
 
-// api.cu: the scratch of a stream (made on first use, at most kMaxScratch sets per context, the least recently
-// used one given back); null inside a stream capture when the context has none yet.
+// api.cu: the scratch of a stream, or of the capture it is in, made on first use.  At most kMaxScratch sets of streams
+// per context, the least recently used one given back; a capture's set is used again by a later capture, or given back
+// when a set is made or grown outside captures, once its graph is gone.
 constexpr int kMaxScratch = 8;
 qeng_scratch* qeng_scratch_for(qeng_ctx* ctx, cudaStream_t stream);
-int32_t qeng_scratch_grow(qeng_ctx* ctx, qeng_buf* b, size_t bytes, cudaStream_t stream);
+int32_t qeng_scratch_grow(qeng_ctx* ctx, qeng_scratch* sc, qeng_buf* b, size_t bytes);
 
 // gemm_tc.cu: tcgen05 matmul of many rows.  wp = 1: bf16 operands; wp = 2: two bf16 terms per weight and per
 // f32 / f16 activation

@@ -17,6 +17,10 @@
  *    packed weights, KV pools and decoders are opaque handles owned by the
  *    engine; `stream` is a cudaStream_t passed as void* (NULL = default
  *    stream); work is asynchronous on that stream unless stated otherwise;
+ *  - calls of one context on different streams may overlap, and matmuls may be captured into a
+ *    graph without a call before: the working memory of a capture is its own and stays until the
+ *    graph and everything instantiated from it are destroyed (or the context is).  Executables
+ *    of one captured graph share it, as they share their outputs: they may not run at once;
  *  - there is no CPU fallback: an unsupported shape is an error.
  */
 #ifndef QENG_H_

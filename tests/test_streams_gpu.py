@@ -1,0 +1,154 @@
+"""Calls on several streams of one context and inside stream captures: whose working memory a call uses, how long it stays."""
+import numpy as np
+import pytest
+
+from oracle import ref
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def fresh(ctx):
+    """A context that holds no working memory yet (the session's one has loaded the kernels)."""
+    from cyb_b200 import qeng
+    c = qeng.Context(0)
+    yield c
+    c.device_status()
+    c.close()
+
+
+def _weight(ctx, fmt, n, k):
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n + k)
+    if fmt == "q4k":
+        return ctx.pack_q4k(ref.make_q4k(ref.rng_of(7), n, k)[2], n, k)
+    w = torch.randn(n, k, device="cuda", generator=g) * 0.05
+    return ctx.quantize_q4(w) if fmt == "q4" else ctx.quantize_q8(w)
+
+
+# one shape of every kernel and of every buffer it needs: slices without planes, planes, block sums, tiles cut along K
+SHAPES = [("q4", 3, "bfloat16"), ("q4", 4, "bfloat16"), ("q8", 8, "float32"), ("q4k", 16, "float16"), ("q4", 101, "float32"),
+          ("q4", 300, "bfloat16"), ("q4", 300, "float32")]
+N, K = 2064, 1280
+
+
+@pytest.mark.parametrize("fmt,m,dt", SHAPES)
+def test_captured_matmul_has_a_workspace_of_its_own(ctx, fresh, fmt, m, dt):
+    """The first call of the context is captured; its graph is replayed beside calls on the stream that did not capture,
+    and after calls that outgrow and displace every stream's buffers."""
+    import torch
+    w0 = _weight(ctx, fmt, N, K)
+    w = _weight(fresh, fmt, N, K)
+    x = torch.randn(m, K, device="cuda").to(getattr(torch, dt))
+    x2 = torch.randn(m, K, device="cuda").to(getattr(torch, dt))
+    want, want2 = ctx.gemm_q4(w0, x), ctx.gemm_q4(w0, x2)  # loads the kernels, too
+    y = torch.zeros(m, N, device="cuda")
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        fresh.gemm_q4(w, x, out=y)
+    for _ in range(20):
+        g.replay()
+        y2 = fresh.gemm_q4(w, x2)
+    torch.cuda.synchronize()
+    assert torch.equal(y, want) and torch.equal(y2, want2)
+    side = torch.cuda.Stream()
+    for _ in range(20):  # side by side
+        with torch.cuda.stream(side):
+            g.replay()
+        y2 = fresh.gemm_q4(w, x2)
+    torch.cuda.synchronize()
+    assert torch.equal(y, want) and torch.equal(y2, want2)
+    big = torch.randn(4 * m, K, device="cuda").to(getattr(torch, dt))
+    for s in [torch.cuda.Stream() for _ in range(10)]:
+        with torch.cuda.stream(s):
+            fresh.gemm_q4(w, big)
+    fresh.gemm_q4(w, big)
+    torch.cuda.synchronize()
+    y.zero_()
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, want)
+
+
+def test_two_streams_of_one_capture(ctx):
+    """Branches of one graph run side by side: they may not share a workspace either, nor may a second call outgrow what the
+    first one of the capture uses."""
+    import torch
+    w = _weight(ctx, "q4", N, K)
+    xs = [torch.randn(m, K, device="cuda") for m in (40, 40, 101)]
+    want = [ctx.gemm_q4(w, x) for x in xs]
+    ys = [torch.zeros_like(t) for t in want]
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        side.wait_stream(torch.cuda.current_stream())
+        ctx.gemm_q4(w, xs[0], out=ys[0])
+        ctx.gemm_q4(w, xs[2], out=ys[2])
+        with torch.cuda.stream(side):
+            ctx.gemm_q4(w, xs[1], out=ys[1])
+        torch.cuda.current_stream().wait_stream(side)
+    for _ in range(10):
+        for t in ys:
+            t.zero_()
+        g.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(ys, want))
+    ctx.device_status()
+
+
+def test_working_memory_of_dropped_graphs_is_used_again(fresh):
+    import torch
+    w = _weight(fresh, "q4", 4096, 4096)
+    x, y = torch.randn(2048, 4096, device="cuda"), torch.zeros(2048, 4096, device="cuda")
+    fresh.gemm_q4(w, x, out=y)
+
+    def once():
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            fresh.gemm_q4(w, x, out=y)  # 16 MB of bf16 rows
+        g.replay()
+        torch.cuda.synchronize()
+        del g
+
+    once()
+    before = torch.cuda.mem_get_info()[0]
+    for _ in range(16):
+        once()
+    assert before - torch.cuda.mem_get_info()[0] < 64 << 20
+
+
+def test_decoder_moved_to_another_stream(ctx):
+    """The captured decode step keeps working memory of its own when the decoder changes streams: matmuls still running on
+    the stream it left do not disturb it."""
+    import torch
+    from cyb_b200 import qeng
+    cfg = ref.DecoderConfig(layers=2, d=256, ffn=512, heads=4, kv_heads=2, vocab=320)
+    W = ref.make_decoder_weights(cfg, seed=5)
+    dec = ctx.decoder(layers=2, d_model=256, ffn=512, heads=4, kv_heads=2, vocab=320, max_batch=8, max_seq=96)
+    qeng.load_decoder_weights(dec, W, cfg)
+    prompt = ref.rng_of(8).integers(0, 320, (8, 5)).astype(np.int32)
+    want, _ = ref.Decoder(cfg, W).generate(prompt, 24)
+    w = _weight(ctx, "q4", 4096, 4096)
+    x = torch.randn(16, 4096, device="cuda")
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    with torch.cuda.stream(b):
+        ctx.gemm_q4(w, x)
+    with torch.cuda.stream(a):
+        dec.use_current_stream()
+    dec.reset(8)
+    dec.prefill(prompt)
+    got = [dec.decode(4)]
+    with torch.cuda.stream(b):
+        dec.use_current_stream()
+    for _ in range(5):
+        with torch.cuda.stream(a):
+            for _ in range(200):
+                ctx.gemm_q4(w, x)
+        got.append(dec.decode(4))
+    torch.cuda.synchronize()
+    assert np.array_equal(np.concatenate(got, 1), want)
+    ctx.device_status()
+    dec.free()

@@ -32,7 +32,7 @@ struct OutsideCapture {
 static void free_scratch(qeng_scratch* sc) {
   OutsideCapture outside;
   for (void* p : sc->kept) cudaFree(p);
-  for (qeng_buf* b : {&sc->planes, &sc->part})
+  for (qeng_buf* b : {&sc->planes, &sc->part, &sc->attn})
     if (b->ptr) cudaFree(b->ptr);
   delete sc;
 }
@@ -118,7 +118,7 @@ qeng_scratch* qeng_scratch_for(qeng_ctx* ctx, cudaStream_t stream) {
 }
 
 // Grows outside the steady state only; outside captures a growing call drains the device first.
-int32_t qeng_scratch_grow(qeng_ctx* ctx, qeng_scratch* sc, qeng_buf* b, size_t bytes) {
+int32_t qeng_scratch_grow(qeng_ctx* ctx, qeng_scratch* sc, qeng_buf* b, size_t bytes, bool zeroed) {
   if (bytes <= b->bytes) return QENG_OK;
   if (b->ptr && sc->capture != 0) {
     sc->kept.push_back(b->ptr);
@@ -130,7 +130,18 @@ int32_t qeng_scratch_grow(qeng_ctx* ctx, qeng_scratch* sc, qeng_buf* b, size_t b
   b->ptr = nullptr;
   b->bytes = 0;
   OutsideCapture outside;
-  const cudaError_t e = cudaMalloc(&b->ptr, bytes);
+  cudaError_t e = cudaMalloc(&b->ptr, bytes);
+  if (e == cudaSuccess && zeroed) {  // on a stream of its own: in a capture the zeros are no node of the graph either
+    cudaStream_t s;
+    e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+    if (e == cudaSuccess) {
+      e = cudaMemsetAsync(b->ptr, 0, bytes, s);
+      const cudaError_t es = cudaStreamSynchronize(s);
+      if (e == cudaSuccess) e = es;
+      cudaStreamDestroy(s);
+    }
+    if (e != cudaSuccess) cudaFree(b->ptr);
+  }
   if (e != cudaSuccess) {
     b->ptr = nullptr;
     (void)cudaGetLastError();  // not the next launch's error
@@ -198,7 +209,6 @@ int32_t qeng_destroy(qeng_ctx* ctx) {
   if (!ctx) return QENG_ERR_ARG;
   cudaSetDevice(ctx->device);
   qeng_tp_release(ctx);
-  if (ctx->attn_scratch) cudaFree(ctx->attn_scratch);
   if (ctx->status) cudaFree(ctx->status);
   for (qeng_scratch* sc : ctx->scratch) free_scratch(sc);
   if (ctx->ximage) cudaFree(ctx->ximage);

@@ -12,7 +12,7 @@
 // Splits: the CTAs of a thread-block cluster (up to 16) take the pages of a
 // sequence round-robin and merge through distributed shared memory (no scratch,
 // no atomics); many (sequence, kv head) pairs take fixed page ranges merged
-// through a scratch buffer by the CTA that arrives last.
+// through a scratch buffer (one per stream, one per capture) by the CTA that arrives last.
 //
 // HBM-bound: algorithmic bytes = sum_b len_b * kv_heads * 2 * 128 * 2.  With one producer warp for all slots, clusters of
 // eight and Q as the (mostly empty) 16-row operand: 1 x 15001 tokens, 8 kv heads 36 us, now 16 us (floor 9.5); 16 ragged
@@ -558,28 +558,6 @@ static int pages_per_split(const qeng_ctx* ctx, int64_t B, int64_t Hkv, int64_t 
   return (int)pps;
 }
 
-// Grow the split scratch of the context to what a call of this shape needs.
-// The steady state never allocates; a growing call drains the device first.
-int32_t qeng_attn_reserve(qeng_ctx* ctx, int64_t B, int64_t Hq, int64_t Hkv, int64_t max_pages) {
-  const int pps = pages_per_split(ctx, B, Hkv, max_pages);
-  const int64_t S = (max_pages + pps - 1) / pps;
-  if (B * Hkv > kMaxAttnCounters)
-    return qeng_fail(ctx, QENG_ERR_SHAPE, "attn: B * kv_heads = %lld exceeds %d", (long long)(B * Hkv), kMaxAttnCounters);
-  // arrival counters first (fixed place for every shape), partials behind them
-  size_t need = (size_t)kMaxAttnCounters * sizeof(int) + (size_t)B * Hq * S * (kHD + 2) * sizeof(float);
-  if (need <= ctx->attn_scratch_bytes) return QENG_OK;
-  QENG_CUDA(ctx, cudaSetDevice(ctx->device));
-  QENG_CUDA(ctx, cudaDeviceSynchronize());
-  if (ctx->attn_scratch) cudaFree(ctx->attn_scratch);
-  ctx->attn_scratch = nullptr;
-  ctx->attn_scratch_bytes = 0;
-  ctx->scratch_gen++;
-  QENG_CUDA(ctx, cudaMalloc(&ctx->attn_scratch, need));
-  QENG_CUDA(ctx, cudaMemset(ctx->attn_scratch, 0, need));  // the arrival counters start at zero and return to it
-  ctx->attn_scratch_bytes = need;
-  return QENG_OK;
-}
-
 extern "C" {
 
 int32_t qeng_kv_pool_create(qeng_ctx* ctx, int64_t pages, int64_t kv_heads, int64_t hd, qeng_kv_pool** out) {
@@ -680,7 +658,21 @@ int32_t qeng_attn_decode_ex(qeng_ctx* ctx, const qeng_kv_pool* pool, const uint1
     warps = 4;
   }
   while (cs > 1 && pairs * cs > 2 * (int64_t)ctx->sm_count) cs >>= 1;
-  if (ctx->attn_cluster && cs >= 4) {
+  bool cluster = ctx->attn_cluster && cs >= 4;
+  qeng_scratch* sc = nullptr;
+  if (!cluster) {
+    p.pps = pages_per_split(ctx, B, pool->kv_heads, max_pages);
+    p.S = (int)((max_pages + p.pps - 1) / p.pps);
+    if (pairs > kMaxAttnCounters)
+      return qeng_fail(ctx, QENG_ERR_SHAPE, "attn: B * kv_heads = %lld exceeds %d", (long long)pairs, kMaxAttnCounters);
+    // arrival counters first (fixed place for every shape; they start at zero and return to it), partials behind them
+    sc = qeng_scratch_for(ctx, (cudaStream_t)stream);
+    const size_t need = (size_t)kMaxAttnCounters * sizeof(int) + (size_t)B * Hq * p.S * (kHD + 2) * sizeof(float);
+    const int32_t rc = qeng_scratch_grow(ctx, sc, &sc->attn, need, true);
+    if (rc != QENG_OK && !ctx->attn_cluster) return rc;
+    cluster = rc != QENG_OK;  // no memory for the partials: clusters need none
+  }
+  if (cluster) {
     p.pps = 0; p.S = cs; p.counters = nullptr; p.part_o = nullptr; p.part_ml = nullptr;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)cs, (unsigned)p.Hkv, (unsigned)B);
@@ -699,12 +691,8 @@ int32_t qeng_attn_decode_ex(qeng_ctx* ctx, const qeng_kv_pool* pool, const uint1
     QENG_CUDA(ctx, cudaLaunchKernelEx(&cfg, warps == 6 ? attn_decode_cluster_kernel<6, kDepth> : attn_decode_cluster_kernel<4, kDepth>, p, map));
     return QENG_OK;
   }
-  p.pps = pages_per_split(ctx, B, pool->kv_heads, max_pages);
-  p.S = (int)((max_pages + p.pps - 1) / p.pps);
-  int32_t rc = qeng_attn_reserve(ctx, B, Hq, pool->kv_heads, max_pages);
-  if (rc != QENG_OK) return rc;
-  p.counters = reinterpret_cast<int*>(ctx->attn_scratch);
-  p.part_o = ctx->attn_scratch + kMaxAttnCounters;
+  p.counters = reinterpret_cast<int*>(sc->attn.ptr);
+  p.part_o = reinterpret_cast<float*>(sc->attn.ptr) + kMaxAttnCounters;
   p.part_ml = p.part_o + (size_t)B * Hq * p.S * kHD;
   dim3 grid((unsigned)p.S, (unsigned)p.Hkv, (unsigned)B);
   attn_decode_kernel<<<grid, kAT, ring_bytes(kAW, kDepth), (cudaStream_t)stream>>>(p, map);

@@ -272,7 +272,7 @@ int32_t ensure_rows(qeng_ctx* ctx, qeng_decoder* d, int64_t rows) {
   QENG_CUDA(ctx, cudaMallocHost(&d->h_tok, rows * 4));
   QENG_CUDA(ctx, cudaMalloc(&d->tok, rows * 4));
   d->rows_cap = rows;
-  return qeng_attn_reserve(ctx, few, d->Hq, d->Hkv, d->max_pages);
+  return QENG_OK;
 }
 
 // matmul over `rows` activation rows in chunks the decode kernels accept: the largest row count
@@ -998,7 +998,7 @@ int32_t qeng_decoder_decode(qeng_ctx* ctx, qeng_decoder* d, int32_t steps, int32
   QENG_CUDA(ctx, cudaSetDevice(ctx->device));
   cudaStream_t st = d->stream;
   {
-    int32_t rc = qeng_attn_reserve(ctx, B, d->Hq, d->Hkv, d->max_pages);  // never allocate inside the capture
+    int32_t rc = QENG_OK;  // the activation images are not allocated inside the capture
     const Layer& L0 = d->layers[0];
     const qeng_weight* ws[4] = {L0.wqkv, L0.wo, L0.wgu, L0.wdown};
     for (int i = 0; rc == QENG_OK && i < 4; ++i)

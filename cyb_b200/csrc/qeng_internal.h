@@ -67,6 +67,7 @@ struct qeng_scratch {
   std::shared_ptr<std::atomic<bool>> done;   // captures: the graph is gone
   qeng_buf planes;    // activations as bf16 planes
   qeng_buf part;      // partial sums of tiles cut along K
+  qeng_buf attn;      // decode attention: arrival counters (zero between calls), then the partials of the splits
   std::vector<void*> kept;  // captures: outgrown buffers that earlier nodes of the graph still use
 };
 
@@ -74,11 +75,8 @@ struct qeng_ctx {
   int device = 0;
   int sm_count = 0;
   std::string err;
-  // scratch for split-KV attention partials and device status words
-  float* attn_scratch = nullptr;
-  size_t attn_scratch_bytes = 0;
   int32_t* status = nullptr;  // device status word (0 = ok)
-  // working memory of the tensor-core matmul, one set per stream and per capture that calls it (qeng_scratch_for)
+  // working memory of matmuls and attention, one set per stream and per capture that needs it (qeng_scratch_for)
   std::vector<qeng_scratch*> scratch;
   // activations quantised once per decode-batch matmul (more than 4 rows), one image per K slice
   void* ximage = nullptr;
@@ -97,7 +95,7 @@ struct qeng_ctx {
   // remaining switches of qeng_options
   bool p2p_allowed = true, attn_cluster = true, step_kernel = false;
   int attn_ctas_per_sm = 3, stream_groups = 0, stream_stage_chunks = 0;
-  // bumped whenever attn_scratch moves: a captured graph that holds the old address is stale
+  // bumped whenever ximage moves: a captured graph that holds the old address is stale
   uint64_t scratch_gen = 0;
   // per-CTA argmax partials and the arrival counter of the fused LM head
   float* tail_val = nullptr;
@@ -171,9 +169,6 @@ enum { QENG_EPI_STORE = 0, QENG_EPI_ACCUM = 1, QENG_EPI_RESID = 2, QENG_EPI_SWIG
 int32_t qeng_gemm_q4_decode(qeng_ctx* ctx, const qeng_weight* w, const void* x, int32_t x_dtype,
                             int64_t M, int64_t ldx, float* y, int64_t ldy, bool split_f32,
                             const qeng_gemm_fuse& fuse, cudaStream_t stream);
-
-// attn_decode.cu: size the context's split scratch for a shape (may allocate; never call while capturing)
-int32_t qeng_attn_reserve(qeng_ctx* ctx, int64_t B, int64_t Hq, int64_t Hkv, int64_t max_pages);
 
 // gemv_q4_stream.cu: the persistent bulk-copy kernel; *handled = false when the shape does not fit it
 int32_t qeng_gemm_q4_stream(qeng_ctx* ctx, const qeng_weight* w, const void* x, int32_t x_dtype, int64_t M,
@@ -254,7 +249,8 @@ int32_t qeng_tp_fuse_advance(qeng_ctx* ctx, cudaStream_t stream);
 // when a set is made or grown outside captures, once its graph is gone.
 constexpr int kMaxScratch = 8;
 qeng_scratch* qeng_scratch_for(qeng_ctx* ctx, cudaStream_t stream);
-int32_t qeng_scratch_grow(qeng_ctx* ctx, qeng_scratch* sc, qeng_buf* b, size_t bytes);
+// `zeroed`: a new buffer starts as zeros
+int32_t qeng_scratch_grow(qeng_ctx* ctx, qeng_scratch* sc, qeng_buf* b, size_t bytes, bool zeroed = false);
 
 // gemm_tc.cu: tcgen05 matmul of many rows.  wp = 1: bf16 operands; wp = 2: two bf16 terms per weight and per
 // f32 / f16 activation

@@ -17,7 +17,7 @@
  *    packed weights, KV pools and decoders are opaque handles owned by the
  *    engine; `stream` is a cudaStream_t passed as void* (NULL = default
  *    stream); work is asynchronous on that stream unless stated otherwise;
- *  - calls of one context on different streams may overlap, and matmuls may be captured into a
+ *  - calls of one context on different streams may overlap, and calls may be captured into a
  *    graph without a call before: the working memory of a capture is its own and stays until the
  *    graph and everything instantiated from it are destroyed (or the context is).  Executables
  *    of one captured graph share it, as they share their outputs: they may not run at once;
@@ -227,7 +227,8 @@ int32_t qeng_kv_append(qeng_ctx* ctx, qeng_kv_pool* pool, const float* k, const 
                        void* stream);
 /* out[B,Hq,hd] f32 = softmax(q K^T * scale) V per sequence over its first
  * lens[b] cached tokens; q f16 [B,Hq,hd]; split over the KV length with a
- * merge of the partial (max, sum, out) triples.  Uses scratch owned by ctx. */
+ * merge of the partial (max, sum, out) triples.  Many sequences use scratch owned by ctx, one per
+ * stream and per capture. */
 int32_t qeng_attn_decode(qeng_ctx* ctx, const qeng_kv_pool* pool, const uint16_t* q_f16,
                          const int32_t* page_table, int64_t max_pages, const int32_t* lens,
                          int64_t B, int64_t Hq, float scale, float* out, void* stream);

@@ -32,7 +32,7 @@ struct OutsideCapture {
 static void free_scratch(qeng_scratch* sc) {
   OutsideCapture outside;
   for (void* p : sc->kept) cudaFree(p);
-  for (qeng_buf* b : {&sc->planes, &sc->part, &sc->attn})
+  for (qeng_buf* b : {&sc->planes, &sc->part, &sc->image, &sc->attn})
     if (b->ptr) cudaFree(b->ptr);
   delete sc;
 }
@@ -211,7 +211,6 @@ int32_t qeng_destroy(qeng_ctx* ctx) {
   qeng_tp_release(ctx);
   if (ctx->status) cudaFree(ctx->status);
   for (qeng_scratch* sc : ctx->scratch) free_scratch(sc);
-  if (ctx->ximage) cudaFree(ctx->ximage);
   if (ctx->tail_val) cudaFree(ctx->tail_val);
   if (ctx->tail_idx) cudaFree(ctx->tail_idx);
   if (ctx->tail_cnt) cudaFree(ctx->tail_cnt);

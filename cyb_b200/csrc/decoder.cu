@@ -230,7 +230,6 @@ struct qeng_decoder {
   cudaStream_t own_stream = nullptr;
   cudaGraphExec_t graph = nullptr;
   int graph_batch = 0;
-  uint64_t graph_scratch_gen = 0;  // ctx->scratch_gen at capture time
   // the fused decode step (all layers in one persistent kernel), planned lazily; dropped whenever a
   // buffer or weight it points at is replaced
   qeng_step* fused = nullptr;
@@ -997,14 +996,6 @@ int32_t qeng_decoder_decode(qeng_ctx* ctx, qeng_decoder* d, int32_t steps, int32
     if (d->len[b] + steps > d->cfg.max_seq) return qeng_fail(ctx, QENG_ERR_SHAPE, "decoder_decode: would exceed max_seq");
   QENG_CUDA(ctx, cudaSetDevice(ctx->device));
   cudaStream_t st = d->stream;
-  {
-    int32_t rc = QENG_OK;  // the activation images are not allocated inside the capture
-    const Layer& L0 = d->layers[0];
-    const qeng_weight* ws[4] = {L0.wqkv, L0.wo, L0.wgu, L0.wdown};
-    for (int i = 0; rc == QENG_OK && i < 4; ++i)
-      if (ws[i]) rc = qeng_gemm_q4_stream_reserve(ctx, ws[i], B < 16 ? B : 16);
-    if (rc != QENG_OK) return rc;
-  }
   std::vector<int32_t> pos(B), lens(B);
   for (int b = 0; b < B; ++b) { pos[b] = d->len[b]; lens[b] = d->len[b] + 1; }
   if (!d->next_ready) {  // right after a decode step the device copies are already one token on
@@ -1037,7 +1028,7 @@ int32_t qeng_decoder_decode(qeng_ctx* ctx, qeng_decoder* d, int32_t steps, int32
       if (rc != QENG_OK) return rc;
     }
   } else {
-    if (!d->graph || d->graph_batch != B || d->graph_scratch_gen != ctx->scratch_gen) {
+    if (!d->graph || d->graph_batch != B) {
       QENG_CUDA(ctx, cudaStreamSynchronize(st));
       if (d->graph) { cudaGraphExecDestroy(d->graph); d->graph = nullptr; }
       cudaGraph_t g = nullptr;
@@ -1051,7 +1042,6 @@ int32_t qeng_decoder_decode(qeng_ctx* ctx, qeng_decoder* d, int32_t steps, int32
       cudaGraphDestroy(g);
       if (e != cudaSuccess) return qeng_fail(ctx, QENG_ERR_CUDA, "decoder_decode: instantiate failed: %s", cudaGetErrorString(e));
       d->graph_batch = B;
-      d->graph_scratch_gen = ctx->scratch_gen;
     }
     for (int s = 0; s < steps; ++s) QENG_CUDA(ctx, cudaGraphLaunch(d->graph, st));
   }

@@ -785,24 +785,6 @@ StreamFit stream_fit(const qeng_ctx* ctx, const qeng_weight* w, int64_t M, bool 
 
 bool qeng_gemm_q4_stream_fits(const qeng_ctx* ctx, const qeng_weight* w, int64_t M) { return stream_fit(ctx, w, M, false).ok; }
 
-// Grow the context's activation-image scratch to what a matmul of M rows over `w` needs (never
-// inside a stream capture: the decoder calls this before it captures a step).
-int32_t qeng_gemm_q4_stream_reserve(qeng_ctx* ctx, const qeng_weight* w, int64_t M) {
-  const StreamFit f = stream_fit(ctx, w, M, false);
-  if (!f.ok || !f.imaged) return QENG_OK;
-  const size_t need = (size_t)f.nslices * f.image_slice_bytes;
-  if (need <= ctx->ximage_bytes) return QENG_OK;
-  QENG_CUDA(ctx, cudaSetDevice(ctx->device));
-  QENG_CUDA(ctx, cudaDeviceSynchronize());
-  if (ctx->ximage) cudaFree(ctx->ximage);
-  ctx->ximage = nullptr;
-  ctx->ximage_bytes = 0;
-  QENG_CUDA(ctx, cudaMalloc(&ctx->ximage, need));
-  ctx->ximage_bytes = need;
-  ctx->scratch_gen++;
-  return QENG_OK;
-}
-
 // *handled = false when the shape does not fit this kernel; the caller then uses the
 // register-streaming kernel.
 int32_t qeng_gemm_q4_stream(qeng_ctx* ctx, const qeng_weight* w, const void* x, int32_t x_dtype, int64_t M,
@@ -854,7 +836,8 @@ int32_t qeng_gemm_q4_stream(qeng_ctx* ctx, const qeng_weight* w, const void* x, 
   }
   p.ximage = nullptr; p.ximage_slice_bytes = f.image_slice_bytes;
   if (f.imaged) {
-    int32_t rr = qeng_gemm_q4_stream_reserve(ctx, w, M);  // grows outside the steady state only
+    qeng_scratch* sc = qeng_scratch_for(ctx, stream);
+    const int32_t rr = qeng_scratch_grow(ctx, sc, &sc->image, (size_t)f.nslices * f.image_slice_bytes);
     if (rr != QENG_OK) return rr;
     const XLayout L = x_layout(f.cols, f.slice_chunks, false);
     const size_t qsmem = 2 * (size_t)L.col_stride + 4 * (size_t)L.zs + (p.gather_world > 0 ? (size_t)w->K * 4 : 0);
@@ -875,12 +858,12 @@ int32_t qeng_gemm_q4_stream(qeng_ctx* ctx, const qeng_weight* w, const void* x, 
     qc.attrs = qa;
     qc.numAttrs = ctx->pdl ? 1 : 0;
     QENG_CUDA(ctx, cudaLaunchKernelEx(&qc, quantise_rows_kernel, x, (int)x_dtype, (long long)ldx, (int)M, (int)w->K, fuse.norm_gamma,
-                                      fuse.norm_eps, f.slice_chunks, reinterpret_cast<unsigned char*>(ctx->ximage), f.image_slice_bytes,
+                                      fuse.norm_eps, f.slice_chunks, reinterpret_cast<unsigned char*>(sc->image.ptr), f.image_slice_bytes,
                                       p.gather_inbox, p.gather_world, p.tp_seq, p.tp_tags_per_step, p.gather_tag_off, p.x_writeback,
                                       ctx->status));
     // the main kernel then sees completed activations: its own staging gathers nothing
     p.gather_world = 0;
-    p.ximage = reinterpret_cast<const unsigned char*>(ctx->ximage);
+    p.ximage = reinterpret_cast<const unsigned char*>(sc->image.ptr);
   }
   *handled = true;
   // Tile groups: more groups hide more of the per-tile reduction, but a group with no tile idles,

@@ -67,6 +67,7 @@ struct qeng_scratch {
   std::shared_ptr<std::atomic<bool>> done;   // captures: the graph is gone
   qeng_buf planes;    // activations as bf16 planes
   qeng_buf part;      // partial sums of tiles cut along K
+  qeng_buf image;     // streaming matmul of more than 4 rows: activations quantised once, one image per K slice
   qeng_buf attn;      // decode attention: arrival counters (zero between calls), then the partials of the splits
   std::vector<void*> kept;  // captures: outgrown buffers that earlier nodes of the graph still use
 };
@@ -78,9 +79,6 @@ struct qeng_ctx {
   int32_t* status = nullptr;  // device status word (0 = ok)
   // working memory of matmuls and attention, one set per stream and per capture that needs it (qeng_scratch_for)
   std::vector<qeng_scratch*> scratch;
-  // activations quantised once per decode-batch matmul (more than 4 rows), one image per K slice
-  void* ximage = nullptr;
-  size_t ximage_bytes = 0;
   // tensor parallelism (tp.cu)
   void* nccl_comm = nullptr;
   int tp_rank = 0, tp_world = 1;
@@ -95,8 +93,6 @@ struct qeng_ctx {
   // remaining switches of qeng_options
   bool p2p_allowed = true, attn_cluster = true, step_kernel = false;
   int attn_ctas_per_sm = 3, stream_groups = 0, stream_stage_chunks = 0;
-  // bumped whenever ximage moves: a captured graph that holds the old address is stale
-  uint64_t scratch_gen = 0;
   // per-CTA argmax partials and the arrival counter of the fused LM head
   float* tail_val = nullptr;
   int32_t* tail_idx = nullptr;
@@ -176,7 +172,6 @@ int32_t qeng_gemm_q4_stream(qeng_ctx* ctx, const qeng_weight* w, const void* x, 
                             bool* handled);
 // true when the streaming kernel takes this shape (its fused-only epilogues may then be used)
 bool qeng_gemm_q4_stream_fits(const qeng_ctx* ctx, const qeng_weight* w, int64_t M);
-int32_t qeng_gemm_q4_stream_reserve(qeng_ctx* ctx, const qeng_weight* w, int64_t M);
 
 // lm_head.cu: LM head with optional RMSNorm and optional greedy finalisation (argmax over the vocabulary,
 // record the token, advance the sequences, gather the next embedding).

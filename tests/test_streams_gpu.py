@@ -72,6 +72,35 @@ def test_captured_matmul_has_a_workspace_of_its_own(ctx, fresh, fmt, m, dt):
     assert torch.equal(y, want)
 
 
+def test_row_count_that_only_the_streaming_matmul_takes(ctx, fresh):
+    """8 rows over a K too wide for the batch kernel's slices: quantised activation images, on two streams and in a graph."""
+    import torch
+    n, k = 64, 10 ** 6 + 32
+    w = _weight(fresh, "q4", n, k)
+    xs = [torch.randn(8, k, device="cuda") for _ in range(3)]
+    want = [ctx.gemm_q4(w, x) for x in xs]
+    exact = w.dequant().double()
+    for x, y in zip(xs, want):  # activations in 15 bits per block
+        assert float((y.double() - x.double() @ exact.T).norm() / y.double().norm()) < 3e-4
+    y = torch.zeros_like(want[0])
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        fresh.gemm_q4(w, xs[0], out=y)
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    outs = [[], []]
+    for _ in range(20):
+        with torch.cuda.stream(streams[0]):
+            g.replay()
+        for i in (0, 1):
+            with torch.cuda.stream(streams[1 + i]):
+                outs[i].append(fresh.gemm_q4(w, xs[1 + i]))
+    torch.cuda.synchronize()
+    assert torch.equal(y, want[0])
+    for i in (0, 1):
+        assert all(torch.equal(o, want[1 + i]) for o in outs[i])
+
+
 def test_two_streams_of_one_capture(ctx):
     """Branches of one graph run side by side: they may not share a workspace either, nor may a second call outgrow what the
     first one of the capture uses."""

@@ -379,6 +379,7 @@ RowsPlan find_plan(const qeng_ctx* ctx, const qeng_weight* w, int64_t M, int xp)
 
 // The search takes a few microseconds of the host: a weight keeps the plans of the last four (rows, planes) it met.
 RowsPlan rows_plan(const qeng_ctx* ctx, const qeng_weight* w, int64_t M, int xp) {
+  std::lock_guard<std::mutex> hold(w->lock);
   for (const auto& e : w->rows_plan)
     if (e[0] == M && e[1] == xp && e[2] == ctx->sm_count) {
       RowsPlan r = {e[3] != 0, e[4], e[5], e[6], e[7], e[8] & 0xff, e[8] >> 8, (size_t)e[9]};

@@ -556,6 +556,7 @@ Plan make_plan(const qeng_ctx* ctx, const qeng_weight* w, int64_t M, int wp, int
 
 // tensor maps of the packed planes, boxes of kst chunks x 8 row tiles of 64-bit words; kept with the weight
 bool weight_maps(const qeng_weight* w) {
+  std::lock_guard<std::mutex> hold(w->lock);
   if (w->tc_maps_ready) return true;
   EncodeFn enc = encode_fn();
   for (int kst = 1; kst <= 2; ++kst)

@@ -7,6 +7,7 @@
 
 #include <atomic>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -40,7 +41,9 @@ struct qeng_weight {
   uint4* qs;           // weight plane: Q4 ntiles*nchunks*32 uint4 (nibbles), Q8 ntiles*nchunks*64 uint4 (bytes)
   uint2* sc;           // scale plane,  ntiles*nchunks*8 uint2 (K4: ntiles*nchunks*256 bytes)
   int64_t bytes;       // device bytes held
-  // tensor maps of both planes for the tensor-core matmul (gemm_tc.cu), encoded on first use: [1 or 2 chunks per box][codes, scales]
+  // What the matmuls work out on first use.  The lock guards it: contexts in several threads may share a weight.
+  mutable std::mutex lock;
+  // tensor maps of both planes for the tensor-core matmul (gemm_tc.cu), unchanged once encoded: [1 or 2 chunks per box][codes, scales]
   mutable bool tc_maps_ready = false;
   alignas(64) mutable unsigned char tc_maps[2][2][128];
   mutable int rows_plan[4][10] = {};  // gemm_rows.cu: plans of the last few row counts

@@ -12,7 +12,8 @@
  *    never throws or aborts; qeng_last_error() gives the text of the last
  *    failure on that context;
  *  - a context is bound to one CUDA device and is used by one host thread at a
- *    time; one context per GPU for tensor parallelism;
+ *    time; one context per GPU for tensor parallelism.  Contexts of one device may
+ *    share weights and multiply by them from several threads at once;
  *  - activation / output pointers are DEVICE pointers owned by the caller;
  *    packed weights, KV pools and decoders are opaque handles owned by the
  *    engine; `stream` is a cudaStream_t passed as void* (NULL = default

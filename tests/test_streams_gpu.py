@@ -101,6 +101,38 @@ def test_row_count_that_only_the_streaming_matmul_takes(ctx, fresh):
         assert all(torch.equal(o, want[1 + i]) for o in outs[i])
 
 
+def test_weight_shared_by_contexts_of_two_threads(ctx, fresh):
+    """Two threads, each with its context and stream, over one weight: every call works out or looks up what the weight keeps
+    per row count (more row counts than it keeps)."""
+    import threading
+    import torch
+    w = _weight(ctx, "q4", N, K)
+    rows = (5, 6, 8, 9, 12, 16, 24, 32)
+    xs = [torch.randn(m, K, device="cuda").to(torch.bfloat16) for m in rows]
+    want = [ctx.gemm_q4(w, x) for x in xs]
+    torch.cuda.synchronize()
+    bad = []
+
+    def work(c, order):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for i in order * 40:
+                    y = c.gemm_q4(w, xs[i])
+                    torch.cuda.current_stream().synchronize()
+                    if not torch.equal(y, want[i]):
+                        bad.append(rows[i])
+        except Exception as e:  # noqa: BLE001  reported by the assertion
+            bad.append(e)
+
+    n = len(rows)
+    threads = [threading.Thread(target=work, args=a) for a in ((ctx, list(range(n))), (fresh, [(3 * i) % n for i in range(n)]))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad, bad
+
+
 def test_two_streams_of_one_capture(ctx):
     """Branches of one graph run side by side: they may not share a workspace either, nor may a second call outgrow what the
     first one of the capture uses."""

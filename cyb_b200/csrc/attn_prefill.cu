@@ -14,6 +14,8 @@
 #include <cuda_bf16.h>
 #include <math.h>
 
+#include <type_traits>
+
 #include "attn_prefill.h"
 
 namespace {
@@ -81,6 +83,29 @@ __device__ __forceinline__ uint32_t pack_h2(float a, float b) {
 // byte offset of 16-byte chunk c (0..15) of row r in a tile of [2 halves][rows][128 B], 128-byte swizzled
 __device__ __forceinline__ uint32_t chunk_at(int rows, int r, int c) {
   return (uint32_t)((c >> 3) * rows * 128 + r * 128 + (((c & 7) ^ (r & 7)) << 4));
+}
+
+__device__ __forceinline__ __half2 ldh2(uint32_t a) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1];\n" : "=r"(v) : "r"(a) : "memory");
+  return *reinterpret_cast<__half2*>(&v);
+}
+// whether the values of a tile's keys up to kv1 hold an infinity or a NaN (asked by whole warps)
+__device__ __forceinline__ bool tile_not_finite(uint32_t kv, int key0, int kv1, int lane) {
+  uint32_t worst = 0;  // largest magnitude bits of the halves: an exponent of all ones has 0x7c00 and more
+  if (key0 + lane < kv1) {  // lane = key
+    const uint32_t row = kv + (uint32_t)(lane >> 4) * kPageBytes;
+#pragma unroll
+    for (int c = 0; c < 16; ++c) {
+      uint4 v;
+      asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];\n"
+                   : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                   : "r"(row + chunk_at(32, 16 + (lane & 15), c))
+                   : "memory");
+      worst = __vmaxu2(worst, __vmaxu2(__vmaxu2(v.x & 0x7fff7fffu, v.y & 0x7fff7fffu), __vmaxu2(v.z & 0x7fff7fffu, v.w & 0x7fff7fffu)));
+    }
+  }
+  return __any_sync(0xffffffffu, (worst & 0xffffu) >= 0x7c00u || (worst >> 16) >= 0x7c00u);
 }
 
 __global__ void __launch_bounds__(kThreads, 3) attn_prefill_kernel(const qeng_prefill_attn p, const __grid_constant__ CUtensorMap kvmap) {
@@ -163,13 +188,7 @@ __global__ void __launch_bounds__(kThreads, 3) attn_prefill_kernel(const qeng_pr
   }
 
   // ===== consumers: rows warp * 16 + g and + 8 =========================================================
-  int len[2], win[2], tok[2];
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    tok[i] = (warp * 16 + g + 8 * i) / grp;
-    len[i] = tok[i] < ntok ? min(lens[tok[i]], p.max_pages * 16) : 0;
-    win[i] = p.window > 0 ? max(0, len[i] - p.window) : 0;
-  }
+  auto token_of = [&](int i) { return (warp * 16 + g + 8 * i) / grp; };  // worked out where needed: registers are short
   const float sc = p.scale * 1.4426950408889634f;
   float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
   float o[16][4];
@@ -180,11 +199,17 @@ __global__ void __launch_bounds__(kThreads, 3) attn_prefill_kernel(const qeng_pr
 
   // ldmatrix row of this lane: A (queries): rows 0..15, chunk lane/16; K: row lane%8, chunk lane/8; V: row lane%16, chunk lane/16
   const int qrow = warp * 16 + (lane & 15), qc = lane >> 4, krow = lane & 7, kc = lane >> 3, vrow = 16 + (lane & 15), vc = lane >> 4;
-  int s = 0;
-  uint32_t ph = 0;
-  for (int kt = t0; kt < t1; ++kt) {
-    if (!failed && !mbar_wait(smem_u32(full + s), ph)) failed = true;
-    const uint32_t kv = ring + (uint32_t)s * kStageBytes;
+  // one tile of 32 keys; kEdge: not every row attends every key of it
+  auto tile = [&](int kt, uint32_t kv, auto edge_tile) {
+    constexpr bool kEdge = decltype(edge_tile)::value;
+    int len[2], win[2];  // the keys that the lane's two rows attend: [win, len)
+    if (kEdge) {
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        len[i] = token_of(i) < ntok ? min(lens[token_of(i)], p.max_pages * 16) : 0;
+        win[i] = p.window > 0 ? max(0, len[i] - p.window) : 0;
+      }
+    }
     float sa[4][4];
 #pragma unroll
     for (int n = 0; n < 4; ++n) sa[n][0] = sa[n][1] = sa[n][2] = sa[n][3] = 0.f;
@@ -202,7 +227,6 @@ __global__ void __launch_bounds__(kThreads, 3) attn_prefill_kernel(const qeng_pr
       }
     }
     // scale (optionally soft-capped), log2 domain, mask
-    const bool edge = (kt + 1) * kTile > len_min || kt * kTile < win_max || ntok < tpt;
     float mx[2] = {-INFINITY, -INFINITY};
 #pragma unroll
     for (int n = 0; n < 4; ++n)
@@ -211,7 +235,7 @@ __global__ void __launch_bounds__(kThreads, 3) attn_prefill_kernel(const qeng_pr
         float x = sa[n][c];
         if (p.softcap > 0.f) x = p.softcap * tanhf(x * p.scale / p.softcap) * 1.4426950408889634f;
         else x *= sc;
-        if (edge) {
+        if (kEdge) {
           const int key = kt * kTile + n * 8 + 2 * t + (c & 1), i = c >> 1;
           if (key >= len[i] || key < win[i]) x = -INFINITY;
         }
@@ -244,40 +268,73 @@ __global__ void __launch_bounds__(kThreads, 3) attn_prefill_kernel(const qeng_pr
         o[j][2] *= alpha[1]; o[j][3] *= alpha[1];
       }
     }
-    const bool tail = (kt + 1) * kTile > kv1;
+    // Where the rows attend different keys, a value that is not finite would reach rows that do not attend it (their weight
+    // is zero, but zero times infinity is NaN): such a tile, which real caches do not hold, goes key by key.
+    if (kEdge && tile_not_finite(kv, kt * kTile, kv1, lane)) {
+#pragma unroll 1
+      for (int k = 0; k < kTile; ++k) {
+        const int n = k >> 3, c = k & 1, src = (lane & ~3) | ((k & 7) >> 1), key = kt * kTile + k;
+        float w[2];  // weights of the lane's two rows for this key, from the lane of the quad that holds them
 #pragma unroll
-    for (int pg = 0; pg < 2; ++pg) {
-      uint32_t hi[4], lo[4];
+        for (int i = 0; i < 2; ++i) {
+          float x = 0.f;
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {  // a0: keys 2t row g, a1: row g+8, a2 / a3: keys 2t + 8
-        const float x = sa[2 * pg + (q >> 1)][2 * (q & 1)], y = sa[2 * pg + (q >> 1)][2 * (q & 1) + 1];
-        hi[q] = pack_h2(x, y);
-        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hi[q]));
-        lo[q] = pack_h2(x - f.x, y - f.y);
-      }
-      // keys past the context: their weight is zero, but zero times whatever the page holds there may be NaN
-      uint32_t keep[2] = {0xffffffffu, 0xffffffffu};
-      if (tail) {
+          for (int m = 0; m < 4; ++m)
+            if (m == n) x = c ? sa[m][2 * i + 1] : sa[m][2 * i];
+          w[i] = __shfl_sync(0xffffffffu, x, src);
+        }
+        const bool on0 = key < len[0] && key >= win[0], on1 = key < len[1] && key >= win[1];
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          const int key = kt * kTile + pg * 16 + q * 8 + 2 * t;
-          keep[q] = (key < kv1 ? 0xffffu : 0u) | (key + 1 < kv1 ? 0xffff0000u : 0u);
+        for (int j = 0; j < 16; ++j) {
+          const float2 v = __half22float2(ldh2(kv + (uint32_t)(k >> 4) * kPageBytes + chunk_at(32, 16 + (k & 15), j) + (uint32_t)t * 4u));
+          if (on0) { o[j][0] = fmaf(w[0], v.x, o[j][0]); o[j][1] = fmaf(w[0], v.y, o[j][1]); }
+          if (on1) { o[j][2] = fmaf(w[1], v.x, o[j][2]); o[j][3] = fmaf(w[1], v.y, o[j][3]); }
         }
       }
+    } else {
+      const bool tail = kEdge && (kt + 1) * kTile > kv1;
 #pragma unroll
-      for (int c = 0; c < 16; c += 2) {
-        uint32_t vb[4];
-        ldsm4_t(kv + (uint32_t)pg * kPageBytes + chunk_at(32, vrow, c + vc), vb);
+      for (int pg = 0; pg < 2; ++pg) {
+        uint32_t hi[4], lo[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {  // a0: keys 2t row g, a1: row g+8, a2 / a3: keys 2t + 8
+          const float x = sa[2 * pg + (q >> 1)][2 * (q & 1)], y = sa[2 * pg + (q >> 1)][2 * (q & 1) + 1];
+          hi[q] = pack_h2(x, y);
+          const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hi[q]));
+          lo[q] = pack_h2(x - f.x, y - f.y);
+        }
+        // keys past the context: their weight is zero, but zero times whatever the page holds there may be NaN
+        uint32_t keep[2] = {0xffffffffu, 0xffffffffu};
         if (tail) {
-          vb[0] &= keep[0]; vb[1] &= keep[1];
-          vb[2] &= keep[0]; vb[3] &= keep[1];
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            const int key = kt * kTile + pg * 16 + q * 8 + 2 * t;
+            keep[q] = (key < kv1 ? 0xffffu : 0u) | (key + 1 < kv1 ? 0xffff0000u : 0u);
+          }
         }
-        mma16816(o[c], hi, vb[0], vb[1]);
-        mma16816(o[c + 1], hi, vb[2], vb[3]);
-        mma16816(o[c], lo, vb[0], vb[1]);
-        mma16816(o[c + 1], lo, vb[2], vb[3]);
+#pragma unroll
+        for (int c = 0; c < 16; c += 2) {
+          uint32_t vb[4];
+          ldsm4_t(kv + (uint32_t)pg * kPageBytes + chunk_at(32, vrow, c + vc), vb);
+          if (tail) {
+            vb[0] &= keep[0]; vb[1] &= keep[1];
+            vb[2] &= keep[0]; vb[3] &= keep[1];
+          }
+          mma16816(o[c], hi, vb[0], vb[1]);
+          mma16816(o[c + 1], hi, vb[2], vb[3]);
+          mma16816(o[c], lo, vb[0], vb[1]);
+          mma16816(o[c + 1], lo, vb[2], vb[3]);
+        }
       }
     }
+  };
+  int s = 0;
+  uint32_t ph = 0;
+  for (int kt = t0; kt < t1; ++kt) {
+    if (!failed && !mbar_wait(smem_u32(full + s), ph)) failed = true;
+    const uint32_t kv = ring + (uint32_t)s * kStageBytes;
+    if ((kt + 1) * kTile > len_min || kt * kTile < win_max || ntok < tpt) tile(kt, kv, std::true_type());
+    else tile(kt, kv, std::false_type());
     __syncwarp();
     if (lane == 0) mbar_arrive(smem_u32(empty + s));
     if (++s == kStages) { s = 0; ph ^= 1u; }
@@ -287,10 +344,11 @@ __global__ void __launch_bounds__(kThreads, 3) attn_prefill_kernel(const qeng_pr
   for (int i = 0; i < 2; ++i) {
     l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], 1);
     l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], 2);
-    if (tok[i] >= ntok) continue;
+    const int tok = token_of(i);
+    if (tok >= ntok) continue;
     const float inv = l_run[i] > 0.f ? 1.f / l_run[i] : 0.f;
-    const int head = h * grp + (warp * 16 + g + 8 * i) - tok[i] * grp;
-    const size_t at = ((size_t)b * p.T + tt0 + tok[i]) * p.ldo + (size_t)head * kHD + 2 * t;
+    const int head = h * grp + (warp * 16 + g + 8 * i) - tok * grp;
+    const size_t at = ((size_t)b * p.T + tt0 + tok) * p.ldo + (size_t)head * kHD + 2 * t;
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
       const float x = o[j][2 * i] * inv, y = o[j][2 * i + 1] * inv;

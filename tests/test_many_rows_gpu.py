@@ -99,3 +99,34 @@ def test_lm_head_edges(ctx, v, d):
         want = x.double() @ tb.double().T
         assert float((y.double() - want).abs().max() / want.abs().max()) < 2.0 ** -21, (v, d, m)
     ctx.device_status()
+
+
+# A 64-row tile of the prompt attention holds tokens that attend different keys.  Token 20's values overflow f16: the rows
+# that do not attend it (before it, and with a window of 8 those from 28 on) give what they give without it.
+@pytest.mark.parametrize("window", [0, 8])
+def test_prompt_rows_do_not_see_infinite_values_they_do_not_attend(ctx, window):
+    import torch
+    from cyb_b200 import qeng
+    cfg = ref.DecoderConfig(layers=1, d=256, ffn=512, heads=4, kv_heads=2, vocab=320, sliding_window=window)
+    W = ref.make_decoder_weights(cfg, seed=5)
+    q, s = W["layers"][0]["wv"]
+    q, s = q.copy(), s.copy()
+    q[:, :32], s[:, 0] = 8, 60000.0  # the first block only acts through column 0
+    q[:, 0] = 15
+    W["layers"][0]["wv"] = (q, s)
+    dec = ctx.decoder(layers=1, d_model=256, ffn=512, heads=4, kv_heads=2, vocab=320, max_batch=1, max_seq=64, sliding_window=window)
+    qeng.load_decoder_weights(dec, W, cfg)
+    x = torch.randn(40, 256, device="cuda", generator=torch.Generator(device="cuda").manual_seed(3))
+    x[:, 0] = 0.0
+    plain = dec.layer(0, x, np.arange(40))
+    assert bool(torch.isfinite(plain).all())
+    x[20, 0] = 8.0
+    got = dec.layer(0, x, np.arange(40))
+    attends = range(20, 28 if window else 40)
+    assert not bool(torch.isfinite(got[20]).any())
+    rest = [r for r in range(40) if r not in attends]
+    assert bool(torch.isfinite(got[rest]).all())
+    # weights of one tile are summed in another order there: a few units of the two-term operands' 2^-17
+    assert float((got[rest] - plain[rest]).abs().max() / plain.abs().max()) < 1e-4
+    ctx.device_status()
+    dec.free()

@@ -119,6 +119,7 @@ qeng_scratch* qeng_scratch_for(qeng_ctx* ctx, cudaStream_t stream) {
 
 // Grows outside the steady state only; outside captures a growing call drains the device first.
 int32_t qeng_scratch_grow(qeng_ctx* ctx, qeng_scratch* sc, qeng_buf* b, size_t bytes, bool zeroed) {
+  ctx->no_memory = false;
   if (bytes <= b->bytes) return QENG_OK;
   if (b->ptr && sc->capture != 0) {
     sc->kept.push_back(b->ptr);
@@ -144,6 +145,7 @@ int32_t qeng_scratch_grow(qeng_ctx* ctx, qeng_scratch* sc, qeng_buf* b, size_t b
   }
   if (e != cudaSuccess) {
     b->ptr = nullptr;
+    ctx->no_memory = e == cudaErrorMemoryAllocation;
     (void)cudaGetLastError();  // not the next launch's error
     return qeng_fail(ctx, QENG_ERR_CUDA, "scratch of %zu bytes: %s", bytes, cudaGetErrorString(e));
   }

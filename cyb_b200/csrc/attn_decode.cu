@@ -669,7 +669,7 @@ int32_t qeng_attn_decode_ex(qeng_ctx* ctx, const qeng_kv_pool* pool, const uint1
     sc = qeng_scratch_for(ctx, (cudaStream_t)stream);
     const size_t need = (size_t)kMaxAttnCounters * sizeof(int) + (size_t)B * Hq * p.S * (kHD + 2) * sizeof(float);
     const int32_t rc = qeng_scratch_grow(ctx, sc, &sc->attn, need, true);
-    if (rc != QENG_OK && !ctx->attn_cluster) return rc;
+    if (rc != QENG_OK && (!ctx->attn_cluster || !ctx->no_memory)) return rc;
     cluster = rc != QENG_OK;  // no memory for the partials: clusters need none
   }
   if (cluster) {

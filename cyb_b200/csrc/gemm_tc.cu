@@ -35,7 +35,7 @@
 //
 // Every wait is bounded; on expiry the kernel records status 4, stops waiting and still frees its
 // tensor memory before it returns.
-#include <vector>
+#include <algorithm>
 
 #include "gemm_tc.cuh"
 
@@ -608,7 +608,8 @@ int32_t qeng_tc::prepare(qeng_ctx* ctx, const qeng_weight* w, const qeng_tc_x& x
   p->ws = nullptr;
   if (pl->sk_tiles > 0) {
     qeng_scratch* sc = qeng_scratch_for(ctx, stream);
-    if (qeng_scratch_grow(ctx, sc, &sc->part, pl->ws_floats * 4) != QENG_OK) return QENG_ERR_STATE;
+    const int32_t rc = qeng_scratch_grow(ctx, sc, &sc->part, pl->ws_floats * 4);
+    if (rc != QENG_OK) return ctx->no_memory ? QENG_ERR_STATE : rc;
     p->ws = reinterpret_cast<float*>(sc->part.ptr);
   }
   EncodeFn enc = encode_fn();
@@ -694,19 +695,23 @@ int32_t qeng_gemm_many_rows(qeng_ctx* ctx, const qeng_weight* w, const void* x, 
   const int planes = wp == 1 || x_dtype == QENG_BF16 ? 1 : 2;
   if (wp == 2 && qeng_gemm_rows_fits(ctx, w, M, planes)) return qeng_gemm_rows_prep(ctx, w, x, x_dtype, M, ldx, nullptr, 0.f, e, stream);
   qeng_tc_x xx;
-  const bool direct = x_dtype == QENG_BF16 && ((reinterpret_cast<uintptr_t>(x) | (uintptr_t)(ldx * 2)) & 15) == 0;
-  if (direct) {
+  if (x_dtype == QENG_BF16 && ((reinterpret_cast<uintptr_t>(x) | (uintptr_t)(ldx * 2)) & 15) == 0) {
     xx.data = x;
     xx.ld = ldx;
-  } else {
-    xx.planes = planes;
-    xx.ld = w->K;
-    xx.plane = M * w->K;
-    qeng_scratch* sc = qeng_scratch_for(ctx, stream);
-    int32_t rc = qeng_scratch_grow(ctx, sc, &sc->planes, (size_t)planes * M * w->K * 2);
-    if (rc == QENG_OK) rc = qeng_tc_prep(ctx, x, x_dtype, M, w->K, ldx, nullptr, 0.f, planes, sc->planes.ptr, nullptr, stream);
-    if (rc != QENG_OK) return rc;
-    xx.data = sc->planes.ptr;
+    return qeng_gemm_tc(ctx, w, xx, M, wp, e, stream);
   }
-  return qeng_gemm_tc(ctx, w, xx, M, wp, e, stream);
+  // the planes of one pass take a gigabyte at most (or those of 256 rows, if that is more)
+  const int64_t row_bytes = (int64_t)planes * w->K * 2, most = std::max<int64_t>(256, ((int64_t)1 << 30) / row_bytes);
+  const int64_t passes = (M + most - 1) / most, step = (M + passes - 1) / passes;
+  qeng_scratch* sc = qeng_scratch_for(ctx, stream);
+  int32_t rc = qeng_scratch_grow(ctx, sc, &sc->planes, (size_t)(step * row_bytes));
+  for (int64_t m0 = 0; rc == QENG_OK && m0 < M; m0 += step) {
+    const int64_t rows = std::min(step, M - m0);
+    const char* src = reinterpret_cast<const char*>(x) + m0 * ldx * (x_dtype == QENG_F32 ? 4 : 2);
+    rc = qeng_tc_prep(ctx, src, x_dtype, rows, w->K, ldx, nullptr, 0.f, planes, sc->planes.ptr, nullptr, stream);
+    xx.data = sc->planes.ptr; xx.planes = planes; xx.ld = w->K; xx.plane = rows * w->K;
+    e.y = y + m0 * ldy;
+    if (rc == QENG_OK) rc = qeng_gemm_tc(ctx, w, xx, rows, wp, e, stream);
+  }
+  return rc;
 }

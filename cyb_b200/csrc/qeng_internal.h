@@ -82,6 +82,7 @@ struct qeng_ctx {
   int32_t* status = nullptr;  // device status word (0 = ok)
   // working memory of matmuls and attention, one set per stream and per capture that needs it (qeng_scratch_for)
   std::vector<qeng_scratch*> scratch;
+  bool no_memory = false;     // whether the last qeng_scratch_grow failed for want of device memory
   // tensor parallelism (tp.cu)
   void* nccl_comm = nullptr;
   int tp_rank = 0, tp_world = 1;

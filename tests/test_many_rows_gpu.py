@@ -47,6 +47,22 @@ def test_rows_and_widths(ctx, fmt, m):
     ctx.device_status()
 
 
+def test_rows_of_more_than_one_pass(ctx):
+    """The bf16 planes of f32 rows beyond a gigabyte: two passes, of an odd total, added onto y."""
+    import torch
+    n, k, m = 272, 32768, 8203
+    w = _weight(ctx, "q8", n, k)
+    wd = w.dequant().double()
+    x = torch.randn(m, k, device="cuda")
+    y = torch.full((m, n + 8), 0.25, device="cuda")[:, :n]
+    ctx.gemm_q4(w, x, out=y, flags=1)
+    for r in (slice(0, 200), slice(4000, 4300), slice(m - 200, m)):
+        want = x[r].double() @ wd.T + 0.25
+        # K / 16 truncating tensor-core steps of 2^-24 of the running sum, as above: 1.3e-4 at the most
+        assert float((y[r].double() - want).abs().max() / want.abs().max()) < 1.3e-4
+    ctx.device_status()
+
+
 def test_results_do_not_depend_on_the_call_before(ctx):
     """Back-to-back calls of several shapes share workspaces and overlap at their ends."""
     import torch

@@ -254,3 +254,37 @@ def test_attention_of_many_sequences_on_two_streams(ctx, fresh):
         assert all(torch.equal(o, got[0]) for o in got)
     for args, _ in cases:
         args[0].free()
+
+
+def test_calls_that_find_no_memory_for_their_workspace(ctx, fresh):
+    """8-bit, K-quant and short 4-bit matmuls and the attention of many sequences need none in passes or clusters: a full
+    device makes them slower, not fail, and the failed allocation is not reported by the next launch."""
+    import torch
+    n = 1040
+    cases = []
+    for fmt, m, k in (("q8", 4096, 8192), ("q4k", 2048, 8192), ("q4", 255, 65536)):  # planes of 64 MB and more
+        w = _weight(fresh, fmt, n, k)
+        x = torch.randn(m, k, device="cuda")
+        cases.append((w, x, ctx.gemm_q4(w, x), torch.empty(m, n, device="cuda")))
+        for r in (1, 4, 15, 16):  # loads the kernels of the passes
+            ctx.gemm_q4(w, x[:r])
+    args, want = _attn_case(fresh, 4)
+    held = ctx.attn_decode(*args)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    hog = []
+    for part in (1 << 30, 1 << 26, 1 << 24):  # down to 32..48 MB, which kernels still to be loaded may need
+        while torch.cuda.mem_get_info()[0] > part + (32 << 20):
+            hog.append(torch.empty(part, dtype=torch.uint8, device="cuda"))
+    assert torch.cuda.mem_get_info()[0] < 56 << 20
+    for w, x, y, out in cases:
+        fresh.gemm_q4(w, x, out=out)
+    fresh.attn_decode(*args, out=held)
+    torch.cuda.synchronize()
+    hog.clear()
+    torch.cuda.empty_cache()
+    for w, x, y, out in cases:
+        # activations in 15 bits per block against bf16 pairs
+        assert float((out - y).norm() / y.norm()) < 3e-4, w.fmt
+    assert ref.err_inf(held.cpu().numpy(), want) < 1e-4
+    args[0].free()

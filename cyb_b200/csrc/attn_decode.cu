@@ -317,7 +317,10 @@ __device__ __forceinline__ void attn_decode_body(const AttnParams& p, const CUte
       if (n + kD < nw) fetch(n + kD, n & ~31, slot);
       if (++slot == kD) { slot = 0; ph ^= 1u; }
     }
-    if (failed && lane == 0) atomicExch(p.status, 4);
+    if (failed) {
+      if (lane == 0) atomicExch(p.status, 4);
+      grace();
+    }
   }
 
   // ---- merge the warps of this CTA ------------------------------------------

@@ -113,6 +113,7 @@ __global__ void __launch_bounds__(kThreads, 3) attn_prefill_kernel(const qeng_pr
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t ring = base + kQBytes;
   __shared__ __align__(8) uint64_t full[kStages], empty[kStages];
+  __shared__ volatile int gave_up;  // a consumer stopped waiting: nobody waits for the producer's copies any more
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int grp = p.Hq / p.Hkv, tpt = kRows / grp;             // tokens per tile
   const int b = blockIdx.z, h = blockIdx.y, tt0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * tpt;  // long tiles first
@@ -124,6 +125,7 @@ __global__ void __launch_bounds__(kThreads, 3) attn_prefill_kernel(const qeng_pr
       mbar_init(smem_u32(full + s), 1);
       mbar_init(smem_u32(empty + s), kNW);
     }
+    gave_up = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
@@ -184,6 +186,7 @@ __global__ void __launch_bounds__(kThreads, 3) attn_prefill_kernel(const qeng_pr
       if (++s == kStages) { s = 0; ph ^= 1u; }
     }
     if (failed && lane == 0) atomicExch(p.status, 4);
+    if (failed || gave_up) grace();
     return;
   }
 
@@ -339,7 +342,11 @@ __global__ void __launch_bounds__(kThreads, 3) attn_prefill_kernel(const qeng_pr
     if (lane == 0) mbar_arrive(smem_u32(empty + s));
     if (++s == kStages) { s = 0; ph ^= 1u; }
   }
-  if (failed && lane == 0) atomicExch(p.status, 4);
+  if (failed) {
+    gave_up = 1;
+    if (lane == 0) atomicExch(p.status, 4);
+    grace();
+  }
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
     l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], 1);

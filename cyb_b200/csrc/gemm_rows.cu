@@ -105,6 +105,7 @@ __global__ void __launch_bounds__(kThreadsR + 160, 1) gemm_rows_kernel(const Row
   constexpr int kRows = 8 * NT / XP, NR = NT / XP;  // activation rows the tiles hold; accumulators (hi and lo share one)
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t full[kMaxRing], empty[kMaxRing], xbar;
+  __shared__ volatile int gave_up;  // a consumer stopped waiting: nobody waits for the producer's copies any more
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int sl = blockIdx.x / p.cps, r0 = blockIdx.x - sl * p.cps;
   const int c0 = sl * p.slice, nc = min(p.slice, p.nchunks - c0);
@@ -123,6 +124,7 @@ __global__ void __launch_bounds__(kThreadsR + 160, 1) gemm_rows_kernel(const Row
       mbar_init(smem_u32(empty + s), kGroupWarps);
     }
     mbar_init(smem_u32(&xbar), 1);
+    gave_up = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   __syncthreads();
@@ -140,10 +142,8 @@ __global__ void __launch_bounds__(kThreadsR + 160, 1) gemm_rows_kernel(const Row
         bulk_g2s(dst, p.qs + at * kW, (uint32_t)nc * kW, bar);
         bulk_g2s(dst + (uint32_t)p.slice * kW, p.sc + at * kS, (uint32_t)nc * kS, bar);
       }
-      if (failed) {
-        atomicExch(p.status, 4);
-        grace();
-      }
+      if (failed) atomicExch(p.status, 4);
+      if (failed || gave_up) grace();
     }
     return;
   }
@@ -280,7 +280,11 @@ __global__ void __launch_bounds__(kThreadsR + 160, 1) gemm_rows_kernel(const Row
     }
     if (u0 + p.park < units) asm volatile("bar.sync 1, %0;\n" ::"n"(kWarps * 32) : "memory");
   }
-  if (failed && lane == 0) atomicExch(p.status, 4);
+  if (failed) {
+    gave_up = 1;
+    if (lane == 0) atomicExch(p.status, 4);
+    grace();
+  }
 }
 
 // Sums of the slices and the epilogue.  A warp = 32 weight rows (whole 16-row tiles) x 4 activation rows; up to four

@@ -353,9 +353,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     }
     if (failed && lane == 0) atomicExch(p.status, 4);
   }
-  if (failed) grace();
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-  __syncthreads();
+  if (__syncthreads_or(failed)) grace();
   cluster_sync();  // no CTA leaves while its peer may still signal it or read its shared memory
   if (warp == 3) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;\n" ::"r"(tmem));
 }

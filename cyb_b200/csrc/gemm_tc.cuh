@@ -74,13 +74,6 @@ __device__ __forceinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity) {
     if (t1 - t0 > 2000000000ull) return false;
   }
 }
-// After a wait that ran out: copies this warp issued are given a tenth of a millisecond to land before the CTA leaves.
-__device__ __forceinline__ void grace() {
-  unsigned long long t0, t1;
-  asm volatile("mov.u64 %0, %globaltimer;\n" : "=l"(t0));
-  do asm volatile("mov.u64 %0, %globaltimer;\n" : "=l"(t1));
-  while (t1 - t0 < 100000ull);
-}
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
   return mbar_try_wait(bar, parity) || mbar_wait_slow(bar, parity);
 }

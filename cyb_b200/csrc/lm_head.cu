@@ -97,10 +97,7 @@ __global__ void __launch_bounds__(kThreadsL, 1) lm_head_kernel(const HeadParams 
         mbar_expect_tx(smem_u32(full + s), a_bytes);
         tma_2d(smem + (uint32_t)s * stage, &wmap, (i % p.nk) * kBK, ((int)blockIdx.x + i / p.nk * (int)gridDim.x) * p.rpc, smem_u32(full + s));
       }
-      if (failed) {
-        atomicExch(p.status, 4);
-        grace();
-      }
+      if (failed) atomicExch(p.status, 4);
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -367,7 +364,7 @@ __global__ void __launch_bounds__(kThreadsL, 1) lm_head_kernel(const HeadParams 
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-  __syncthreads();
+  if (__syncthreads_or(failed)) grace();
   if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;\n" ::"r"(tmem));
 }
 

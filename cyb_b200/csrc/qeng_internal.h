@@ -265,6 +265,17 @@ void qeng_weight_dequant_k4(const qeng_weight* w, float* out, cudaStream_t strea
 int32_t qeng_weight_pack_k4(qeng_ctx* ctx, const uint8_t* q, const float* dm, int64_t N, int64_t K, qeng_weight** out);
 int32_t qeng_q4k_expand(qeng_ctx* ctx, const uint8_t* blocks, int64_t N, int64_t K, std::vector<uint8_t>* q, std::vector<float>* dm);
 
+#ifdef __CUDACC__
+// After a wait that ran out: copies on their way into this CTA are given a tenth of a millisecond to land before it leaves
+// or uses their place for something else.
+__device__ __forceinline__ void grace() {
+  unsigned long long t0, t1;
+  asm volatile("mov.u64 %0, %globaltimer;\n" : "=l"(t0));
+  do asm volatile("mov.u64 %0, %globaltimer;\n" : "=l"(t1));
+  while (t1 - t0 < 100000ull);
+}
+#endif
+
 #if defined(QENG_TRACE) && defined(__CUDACC__)
 // tuning builds only: a launch log behind the status word (status + 256 bytes: a counter, then records
 // of 8 u64: kind, then %globaltimer stamps)

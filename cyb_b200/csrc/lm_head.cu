@@ -204,8 +204,9 @@ __global__ void __launch_bounds__(kThreadsL, 1) lm_head_kernel(const HeadParams 
           for (int pl = 0; pl < 3; ++pl) {
             const __nv_bfloat162 h = __floats2bfloat162_rn(a0, a1);
             o[pl][e] = *reinterpret_cast<const uint32_t*>(&h);
-            a0 -= __uint_as_float(o[pl][e] << 16);
-            a1 -= __uint_as_float(o[pl][e] & 0xffff0000u);
+            const float h0 = __uint_as_float(o[pl][e] << 16), h1 = __uint_as_float(o[pl][e] & 0xffff0000u);
+            a0 = isinf(h0) ? 0.f : a0 - h0;  // an infinity is whole in the first plane
+            a1 = isinf(h1) ? 0.f : a1 - h1;
           }
         }
 #pragma unroll
@@ -264,7 +265,7 @@ __global__ void __launch_bounds__(kThreadsL, 1) lm_head_kernel(const HeadParams 
         if (lane == 0) mbar_arrive(smem_u32(acc_empty + buf));
       }
 #pragma unroll
-      for (int m = 0; m < kM; ++m) acc[m] += low[m];
+      for (int m = 0; m < kM; ++m) acc[m] = isinf(acc[m]) ? acc[m] : acc[m] + low[m];  // an infinite sum has no remainder
       if (t.gamma != nullptr) {
         if (!failed && !mbar_wait(smem_u32(&ss_ready), 0)) failed = true;
 #pragma unroll

@@ -146,3 +146,18 @@ def test_prompt_rows_do_not_see_infinite_values_they_do_not_attend(ctx, window):
     assert float((got[rest] - plain[rest]).abs().max() / plain.abs().max()) < 1e-4
     ctx.device_status()
     dec.free()
+
+
+def test_lm_head_of_infinite_activations(ctx):
+    """An infinite activation makes infinite logits (of the sign of the table's entry), NaN only where infinities meet."""
+    import torch
+    tb = (torch.randn(500, 136, device="cuda") * 0.05).bfloat16()
+    x = torch.randn(4, 136, device="cuda")
+    x[0, 3], x[1, 70], x[2, 5], x[2, 100] = float("inf"), -float("inf"), float("inf"), -float("inf")
+    want = x @ tb.float().T
+    y = ctx.lm_head(tb.view(torch.int16), x)
+    special = ~torch.isfinite(want)
+    assert bool(torch.isinf(want[:2]).all()) and bool(special[2].all()) and not bool(special[3].any())
+    assert torch.equal(torch.nan_to_num(y[special], 7.0, 8.0, 9.0), torch.nan_to_num(want[special], 7.0, 8.0, 9.0))
+    assert float((y[3] - want[3]).abs().max()) < 1e-5
+    ctx.device_status()

@@ -296,7 +296,6 @@ int32_t mm(qeng_ctx* ctx, qeng_decoder* d, const qeng_weight* w, const float* x,
     }
     int32_t rc = qeng_gemm_q4_decode(ctx, w, x + m0 * ldx, QENG_F32, mm_, ldx, y + m0 * ldy, ldy, true, f, st);
     if (rc != QENG_OK) return rc;
-    d->launches++;
   }
   return QENG_OK;
 }
@@ -339,14 +338,12 @@ int32_t row_split_many(qeng_ctx* ctx, qeng_decoder* d, const qeng_weight* w, con
 int32_t reduce_part(qeng_ctx* ctx, qeng_decoder* d, int64_t rows, cudaStream_t st) {
   const int64_t n = rows * d->cfg.d_model;
   if (qeng_tp_p2p_ready(ctx, n)) {  // push, wait, sum and residual add in one kernel
-    d->launches += 1;
     return qeng_tp_allreduce_add(ctx, d->x, d->part, n, st);
   }
   int32_t rc = qeng_tp_all_reduce_internal(ctx, d->part, n, st);
   if (rc != QENG_OK) return rc;
   add_inplace_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(d->x, d->part, n);
   QENG_LAUNCH_CHECK(ctx);
-  d->launches += 2;
   return QENG_OK;
 }
 
@@ -446,7 +443,6 @@ int32_t run_layer_batch(qeng_ctx* ctx, qeng_decoder* d, int l, int64_t rows, con
   }
   rc = qeng_gemm_rows_prep(ctx, L.wgu, d->x, QENG_F32, rows, dm, L.norm2, d->cfg.rms_eps, eg, st);
   if (rc != QENG_OK) return rc;
-  d->launches += 12;
   if (L.wdown->fmt == QENG_FMT_K4) return qeng_gemm_rows_prep(ctx, L.wdown, d->act, QENG_F32, rows, d->F, nullptr, 0.f, er, st);
   qeng_tc_x x;
   x.data = d->act; x.ld = d->F; x.plane = rows * d->F; x.planes = 2;
@@ -493,14 +489,12 @@ int32_t run_layer(qeng_ctx* ctx, qeng_decoder* d, int l, int64_t rows, int64_t T
     rope_append_kernel<<<(unsigned)rows, 256, 0, st>>>(d->qkv, d->rope_cs, d->pos, table, 1, d->max_pages, (int)d->pages,
                                                        d->Hq, d->Hkv, d->cfg.max_seq, d->q16, pool, ctx->status, L.qnorm, L.knorm, d->cfg.rms_eps);
     QENG_LAUNCH_CHECK(ctx);
-    d->launches++;
   }
   if (f.tp_gather_kind >= 0) x = other(x);  // the gathered rows are the residual stream from here on
   d->view.pages = d->pages; d->view.kv_heads = d->Hkv; d->view.hd = kHD; d->view.data = pool;
   rc = qeng_attn_decode_ex(ctx, &d->view, reinterpret_cast<const uint16_t*>(d->q16), table, d->max_pages, d->lens, rows,
                            d->Hq, 1.0f / sqrtf((float)kHD), d->cfg.attn_softcap, d->cfg.sliding_window, d->att, st);
   if (rc != QENG_OK) return rc;
-  d->launches += 1;
   qeng_gemm_fuse fg;
   fg.norm_gamma = L.norm2; fg.norm_eps = d->cfg.rms_eps; fg.epilogue = QENG_EPI_SWIGLU; fg.two_limbs = true;
   fg.tp_layers = d->cfg.layers;
@@ -536,7 +530,6 @@ int32_t tail_sharded(qeng_ctx* ctx, qeng_decoder* d, const float* x_last, int B,
   t.logits = d->logits; t.v0 = d->v0; t.Vtot = V; t.ldl = V;
   t.gamma = d->final_norm; t.eps = d->cfg.rms_eps; t.softcap = d->cfg.final_softcap;
   if (finalize) { t.pairs = d->tp_pairs; t.pair_slot = R * B; }
-  d->launches += 1;
   int32_t rc = qeng_lm_head_fused(ctx, t, st);
   if (rc != QENG_OK) return rc;
   if (!finalize) {  // prompt end: every rank needs the full logits (zero + x = x, so the sum is exact)
@@ -549,13 +542,11 @@ int32_t tail_sharded(qeng_ctx* ctx, qeng_decoder* d, const float* x_last, int B,
   } else {
     QENG_CUDA(ctx, cudaMemcpyAsync(d->tp_gath, d->tp_pairs, n * 4, cudaMemcpyDeviceToDevice, st));
     rc = qeng_tp_all_reduce_internal(ctx, d->tp_gath, n, st);
-    d->launches += 1;
   }
   if (rc != QENG_OK) return rc;
   tp_pick_kernel<<<1, 256, 0, st>>>(d->tp_gath, W, B, V, dm, d->emb, d->x, d->next, d->pos, d->lens, d->out_tokens,
                                     d->step, ctx->status);
   QENG_LAUNCH_CHECK(ctx);
-  d->launches += 2;
   return QENG_OK;
 }
 
@@ -569,7 +560,6 @@ int32_t tail(qeng_ctx* ctx, qeng_decoder* d, const float* x_last, int B, bool fi
     t.next = d->next; t.emb = d->emb; t.xout = d->x; t.pos = d->pos; t.lens = d->lens;
     t.out_tokens = d->out_tokens; t.step = d->step;
   }
-  d->launches += 1;
   return qeng_lm_head_fused(ctx, t, st);
 }
 
@@ -618,7 +608,6 @@ int32_t decode_step(qeng_ctx* ctx, qeng_decoder* d, cudaStream_t st) {
     // the one gather no matmul absorbs: the parts of the last down projection, added in place
     int32_t rc = qeng_tp_fuse_gather(ctx, x, B, d->cfg.d_model, 1, d->cfg.layers - 1, d->cfg.layers, st);
     if (rc != QENG_OK) return rc;
-    d->launches += 2;
   }
   int32_t rc = tail(ctx, d, x, B, true, st);  // leaves the next token's embedding in d->x
   if (rc == QENG_OK && fused) rc = qeng_tp_fuse_advance(ctx, st);
@@ -764,6 +753,20 @@ static void link_weights(qeng_decoder* d) {
       prev = w;
     }
   }
+}
+
+// kernels of a captured step (for reporting)
+static int kernel_nodes(cudaGraph_t g) {
+  size_t n = 0;
+  if (cudaGraphGetNodes(g, nullptr, &n) != cudaSuccess || n == 0) return 0;
+  std::vector<cudaGraphNode_t> nodes(n);
+  if (cudaGraphGetNodes(g, nodes.data(), &n) != cudaSuccess) return 0;
+  int kernels = 0;
+  for (cudaGraphNode_t node : nodes) {
+    cudaGraphNodeType t;
+    if (cudaGraphNodeGetType(node, &t) == cudaSuccess && t == cudaGraphNodeTypeKernel) ++kernels;
+  }
+  return kernels;
 }
 
 static int32_t pack_fmt(qeng_ctx* ctx, int fmt, const uint8_t* q, const uint16_t* s, int64_t N, int64_t K, qeng_weight** out) {
@@ -1022,7 +1025,7 @@ int32_t qeng_decoder_decode(qeng_ctx* ctx, qeng_decoder* d, int32_t steps, int32
   if (qeng_step_takes(d->fused, B)) {
     // all layers in one persistent kernel, then the LM head (norm, head, sample, advance, embed)
     for (int s = 0; s < steps; ++s) {
-      d->launches = 1;
+      d->launches = 2;
       int32_t rc = qeng_step_launch(ctx, d->fused, B, st);
       if (rc == QENG_OK) rc = tail(ctx, d, d->x, B, true, st);
       if (rc != QENG_OK) return rc;
@@ -1033,11 +1036,11 @@ int32_t qeng_decoder_decode(qeng_ctx* ctx, qeng_decoder* d, int32_t steps, int32
       if (d->graph) { cudaGraphExecDestroy(d->graph); d->graph = nullptr; }
       cudaGraph_t g = nullptr;
       QENG_CUDA(ctx, cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-      d->launches = 0;
       int32_t rc = decode_step(ctx, d, st);
       cudaError_t e = cudaStreamEndCapture(st, &g);
       if (rc != QENG_OK) { if (g) cudaGraphDestroy(g); return rc; }
       if (e != cudaSuccess) return qeng_fail(ctx, QENG_ERR_CUDA, "decoder_decode: capture failed: %s", cudaGetErrorString(e));
+      d->launches = kernel_nodes(g);
       e = cudaGraphInstantiate(&d->graph, g, 0);
       cudaGraphDestroy(g);
       if (e != cudaSuccess) return qeng_fail(ctx, QENG_ERR_CUDA, "decoder_decode: instantiate failed: %s", cudaGetErrorString(e));

@@ -369,3 +369,23 @@ def test_vocabulary_of_several_head_rounds(ctx, batch):
                 break
     assert (toks == want).mean() > 0.9
     dec.free()
+
+
+# per layer, one sequence: q|k|v, attention, o, gate|up, down; five: preparation, matmul and slice sums of each matmul, but
+# that gate|up leaves 4-bit blocks' down projection its operand; with per-head gains the rotation is a kernel of its own
+@pytest.mark.parametrize("fmt,gains,batch,per_layer", [("q4", False, 1, 5), ("q4", False, 5, 12), ("q4", True, 5, 13), ("q4k", False, 5, 13)])
+def test_launches_per_step(ctx, fmt, gains, batch, per_layer):
+    from cyb_b200 import qeng
+    cfg = ref.DecoderConfig(**CFG)
+    W = ref.make_decoder_weights(cfg, seed=5, fmt=fmt)
+    if gains:
+        for lw in W["layers"]:
+            lw["qnorm"] = lw["knorm"] = np.ones(cfg.hd, np.float32)
+    dec = ctx.decoder(layers=cfg.layers, d_model=cfg.d, ffn=cfg.ffn, heads=cfg.heads, kv_heads=cfg.kv_heads,
+                      vocab=cfg.vocab, max_batch=5, max_seq=32)
+    qeng.load_decoder_weights(dec, W, cfg)
+    dec.reset(batch)
+    dec.prefill(np.ones((batch, 3), np.int32))
+    dec.decode(2)
+    assert dec.launches_per_step == per_layer * cfg.layers + 1  # and the LM head
+    dec.free()

@@ -150,7 +150,10 @@ def _cur_stream():
     import torch
     if not torch.cuda.is_initialized():
         torch.cuda.init()
-    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    try:  # the handle without a Stream object around it
+        return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    except AttributeError:  # private functions that another torch may not have
+        return torch.cuda.current_stream().cuda_stream
 
 
 class Context:

@@ -73,3 +73,18 @@ def test_rust_declarations_name_every_symbol():
         c_fields = re.findall(r"([a-z_0-9]+)\s*[,;]", body)
         r_body = re.search(r"pub struct %s \{(.*?)\}" % struct, rs, re.S).group(1)
         assert re.findall(r"pub ([a-z_0-9]+):", r_body) == c_fields, struct
+
+
+@pytest.mark.parametrize("private", [True, False])
+def test_current_stream_does_not_need_private_functions_of_torch(built_lib, monkeypatch, private):
+    import types
+    import torch
+    from cyb_b200 import qeng
+    monkeypatch.setattr(torch.cuda, "is_initialized", lambda: True)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda: types.SimpleNamespace(cuda_stream=77))
+    if private:
+        monkeypatch.setattr(torch._C, "_cuda_getDevice", lambda: 3, raising=False)
+        monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda d: 100 + d, raising=False)
+    else:
+        monkeypatch.delattr(torch._C, "_cuda_getCurrentRawStream", raising=False)
+    assert qeng._cur_stream() == (103 if private else 77)

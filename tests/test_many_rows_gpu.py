@@ -47,6 +47,26 @@ def test_rows_and_widths(ctx, fmt, m):
     ctx.device_status()
 
 
+# Query heads per kv head: one, the most there are, and counts that do not divide the 64 rows of a prompt attention tile
+# (its last rows stay empty); tiles then hold 64, 8, 21, 12, 10 and 9 tokens.
+@pytest.mark.parametrize("heads,kv_heads", [(2, 2), (8, 1), (6, 2), (5, 1), (6, 1), (7, 1)])
+def test_prompt_attention_groups(ctx, heads, kv_heads):
+    from cyb_b200 import qeng
+    cfg = ref.DecoderConfig(layers=2, d=256, ffn=512, heads=heads, kv_heads=kv_heads, vocab=320)
+    W = ref.make_decoder_weights(cfg, seed=5)
+    dec = ctx.decoder(layers=2, d_model=256, ffn=512, heads=heads, kv_heads=kv_heads, vocab=320, max_batch=2, max_seq=128)
+    qeng.load_decoder_weights(dec, W, cfg)
+    prompt = ref.rng_of(heads).integers(0, 320, (2, 86)).astype(np.int32)
+    dec.reset(2)
+    dec.prefill(prompt[:, :65])
+    dec.prefill(prompt[:, 65:])
+    want, logs = ref.Decoder(cfg, W).generate(prompt, 3)
+    assert ref.err_inf(dec.logits(), logs[0]) < 2e-3
+    assert np.array_equal(dec.decode(3), want)
+    ctx.device_status()
+    dec.free()
+
+
 def test_rows_of_more_than_one_pass(ctx):
     """The bf16 planes of f32 rows beyond a gigabyte: two passes, of an odd total, added onto y."""
     import torch

@@ -465,14 +465,14 @@ int32_t qeng_gemm_rows_prep(qeng_ctx* ctx, const qeng_weight* w, const void* x, 
   xx.planes = planes;
   float* sums = w->fmt == QENG_FMT_K4 ? reinterpret_cast<float*>(reinterpret_cast<char*>(sc->planes.ptr) + planes_bytes(w, M, planes)) : nullptr;
   rc = qeng_tc_prep(ctx, x, dtype, M, w->K, ldx, gamma, eps, planes, sc->planes.ptr, sums, stream);
-  return rc == QENG_OK ? qeng_gemm_rows(ctx, w, xx, sums, M, epi, stream) : rc;
+  return rc == QENG_OK ? qeng_gemm_rows(ctx, w, xx, sums, M, epi, stream, sc) : rc;
 }
 
-int32_t qeng_gemm_rows(qeng_ctx* ctx, const qeng_weight* w, const qeng_tc_x& x, const float* xsum, int64_t M, const qeng_tc_epi& epi, cudaStream_t stream) {
+int32_t qeng_gemm_rows(qeng_ctx* ctx, const qeng_weight* w, const qeng_tc_x& x, const float* xsum, int64_t M, const qeng_tc_epi& epi, cudaStream_t stream, qeng_scratch* sc) {
   const RowsPlan pl = rows_plan(ctx, w, M, x.planes);
   if (!pl.ok) return qeng_fail(ctx, QENG_ERR_SHAPE, "gemm_rows: %lld rows over [%lld, %lld] do not fit", (long long)M, (long long)w->N, (long long)w->K);
   if (w->fmt == QENG_FMT_K4 && xsum == nullptr) return qeng_fail(ctx, QENG_ERR_ARG, "gemm_rows: K-quant blocks need the block sums of the activations");
-  qeng_scratch* sc = qeng_scratch_for(ctx, stream);
+  if (sc == nullptr) sc = qeng_scratch_for(ctx, stream);
   const int32_t rc = qeng_scratch_grow(ctx, sc, &sc->part, (size_t)pl.nsl * M * w->N * 4);
   if (rc != QENG_OK) return rc;
   RowsParams p;

@@ -600,13 +600,12 @@ int32_t launch(qeng_ctx* ctx, const qeng_weight* w, const TcParams& p, const Pla
 
 }  // namespace
 
-int32_t qeng_tc::prepare(qeng_ctx* ctx, const qeng_weight* w, const qeng_tc_x& x, int64_t M, const qeng_tc_epi& epi, cudaStream_t stream,
+int32_t qeng_tc::prepare(qeng_ctx* ctx, const qeng_weight* w, const qeng_tc_x& x, int64_t M, const qeng_tc_epi& epi, qeng_scratch* sc,
                          const Plan* pl, TcParams* p, CUtensorMap* map) {
   if ((reinterpret_cast<uintptr_t>(x.data) & 15) != 0 || (x.ld & 7) != 0)
     return qeng_fail(ctx, QENG_ERR_ALIGN, "gemm_tc: activations must be 16-byte aligned with a leading dimension multiple of 8");
   p->ws = nullptr;
   if (pl->sk_tiles > 0) {
-    qeng_scratch* sc = qeng_scratch_for(ctx, stream);
     const int32_t rc = qeng_scratch_grow(ctx, sc, &sc->part, pl->ws_floats * 4);
     if (rc != QENG_OK) return ctx->no_memory ? QENG_ERR_STATE : rc;
     p->ws = reinterpret_cast<float*>(sc->part.ptr);
@@ -660,17 +659,18 @@ int32_t qeng_tc_prep(qeng_ctx* ctx, const void* x, int32_t dtype, int64_t M, int
   return QENG_OK;
 }
 
-int32_t qeng_gemm_tc(qeng_ctx* ctx, const qeng_weight* w, const qeng_tc_x& x, int64_t M, int wp, const qeng_tc_epi& epi, cudaStream_t stream) {
+int32_t qeng_gemm_tc(qeng_ctx* ctx, const qeng_weight* w, const qeng_tc_x& x, int64_t M, int wp, const qeng_tc_epi& epi, cudaStream_t stream, qeng_scratch* sc) {
   const int xp = x.planes;
   if (w->fmt != QENG_FMT_Q4 && wp == 1) return qeng_fail(ctx, QENG_ERR_SHAPE, "gemm_tc: single bf16 weights are for 4-bit blocks only");
   if (wp == 1 && xp != 1) return qeng_fail(ctx, QENG_ERR_ARG, "gemm_tc: two activation planes need two weight planes");
   Plan pl = make_plan(ctx, w, M, wp, xp, true);
   TcParams p;
   CUtensorMap map;
-  int32_t rc = prepare(ctx, w, x, M, epi, stream, &pl, &p, &map);
+  if (pl.sk_tiles > 0 && sc == nullptr) sc = qeng_scratch_for(ctx, stream);
+  int32_t rc = prepare(ctx, w, x, M, epi, sc, &pl, &p, &map);
   if (rc == QENG_ERR_STATE) {  // no memory for the workspace: whole tiles only
     pl = make_plan(ctx, w, M, wp, xp, false);
-    rc = prepare(ctx, w, x, M, epi, stream, &pl, &p, &map);
+    rc = prepare(ctx, w, x, M, epi, sc, &pl, &p, &map);
   }
   if (rc != QENG_OK) return rc;
   if (wp == 1) return launch<QENG_FMT_Q4, 1, 1, 2>(ctx, w, p, pl, map, stream);
@@ -685,14 +685,10 @@ int32_t qeng_gemm_tc(qeng_ctx* ctx, const qeng_weight* w, const qeng_tc_x& x, in
 
 // y[M,N] = x . dequant(W)^T through the kernel above, activations in any type the entry point takes.
 // wp = 1: operands rounded to bf16; wp = 2: two bf16 terms per weight and per f32 / f16 activation.
-int32_t qeng_gemm_many_rows(qeng_ctx* ctx, const qeng_weight* w, const void* x, int32_t x_dtype, int64_t M, int64_t ldx, float* y, int64_t ldy,
-                            int accumulate, int wp, cudaStream_t stream) {
-  qeng_tc_epi e;
-  e.kind = accumulate ? QENG_EPI_ACCUM : QENG_EPI_STORE;
-  e.y = y;
-  e.ldy = ldy;
+int32_t qeng_gemm_many_rows(qeng_ctx* ctx, const qeng_weight* w, const void* x, int32_t x_dtype, int64_t M, int64_t ldx, qeng_tc_epi e, int wp,
+                            cudaStream_t stream) {
+  float* const y = e.y;
   const int planes = wp == 1 || x_dtype == QENG_BF16 ? 1 : 2;
-  if (wp == 2 && qeng_gemm_rows_fits(ctx, w, M, planes)) return qeng_gemm_rows_prep(ctx, w, x, x_dtype, M, ldx, nullptr, 0.f, e, stream);
   qeng_tc_x xx;
   if (x_dtype == QENG_BF16 && ((reinterpret_cast<uintptr_t>(x) | (uintptr_t)(ldx * 2)) & 15) == 0) {
     xx.data = x;
@@ -709,8 +705,8 @@ int32_t qeng_gemm_many_rows(qeng_ctx* ctx, const qeng_weight* w, const void* x, 
     const char* src = reinterpret_cast<const char*>(x) + m0 * ldx * (x_dtype == QENG_F32 ? 4 : 2);
     rc = qeng_tc_prep(ctx, src, x_dtype, rows, w->K, ldx, nullptr, 0.f, planes, sc->planes.ptr, nullptr, stream);
     xx.data = sc->planes.ptr; xx.planes = planes; xx.ld = w->K; xx.plane = rows * w->K;
-    e.y = y + m0 * ldy;
-    if (rc == QENG_OK) rc = qeng_gemm_tc(ctx, w, xx, rows, wp, e, stream);
+    e.y = y + m0 * e.ldy;
+    if (rc == QENG_OK) rc = qeng_gemm_tc(ctx, w, xx, rows, wp, e, stream, sc);
   }
   return rc;
 }

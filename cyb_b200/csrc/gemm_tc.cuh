@@ -288,7 +288,7 @@ struct Plan {
 };
 // gemm_tc.cu: kernel parameters and the tensor map of the activations for a plan; QENG_ERR_STATE when the plan cuts
 // tiles along K and there is no memory for the workspace
-int32_t prepare(qeng_ctx* ctx, const qeng_weight* w, const qeng_tc_x& x, int64_t M, const qeng_tc_epi& epi, cudaStream_t stream,
+int32_t prepare(qeng_ctx* ctx, const qeng_weight* w, const qeng_tc_x& x, int64_t M, const qeng_tc_epi& epi, qeng_scratch* sc,
                 const Plan* pl, TcParams* p, CUtensorMap* map);
 // sums the partials of the tiles cut along K
 int32_t reduce(qeng_ctx* ctx, const TcParams& p, cudaStream_t stream);

@@ -23,8 +23,13 @@ struct qeng_tc_x {
   int planes = 1;
 };
 
-// wp = 1: weights rounded to bf16 (4-bit blocks only); wp = 2: weights as two bf16 terms
-int32_t qeng_gemm_tc(qeng_ctx* ctx, const qeng_weight* w, const qeng_tc_x& x, int64_t M, int wp, const qeng_tc_epi& epi, cudaStream_t stream);
+// wp = 1: weights rounded to bf16 (4-bit blocks only); wp = 2: weights as two bf16 terms.  sc: the stream's working memory
+// where the caller has looked it up already.
+int32_t qeng_gemm_tc(qeng_ctx* ctx, const qeng_weight* w, const qeng_tc_x& x, int64_t M, int wp, const qeng_tc_epi& epi, cudaStream_t stream,
+                     qeng_scratch* sc = nullptr);
+// the same for rows of any type; wp = 1: operands rounded to bf16; wp = 2: two bf16 terms per weight and f32 / f16 activation
+int32_t qeng_gemm_many_rows(qeng_ctx* ctx, const qeng_weight* w, const void* x, int32_t x_dtype, int64_t M, int64_t ldx, qeng_tc_epi e, int wp,
+                            cudaStream_t stream);
 // the driver's cuTensorMapEncodeTiled, or null
 void* qeng_tensor_map_encoder();
 // rows of x (any type), RMS-normalised if gamma is given -> `planes` bf16 planes [M][K]; with `sums` also their sums per
@@ -36,4 +41,5 @@ int32_t qeng_tc_prep(qeng_ctx* ctx, const void* x, int32_t dtype, int64_t M, int
 bool qeng_gemm_rows_fits(const qeng_ctx* ctx, const qeng_weight* w, int64_t M, int planes);
 int32_t qeng_gemm_rows_prep(qeng_ctx* ctx, const qeng_weight* w, const void* x, int32_t dtype, int64_t M, int64_t ldx, const float* gamma, float eps,
                             const qeng_tc_epi& epi, cudaStream_t stream);
-int32_t qeng_gemm_rows(qeng_ctx* ctx, const qeng_weight* w, const qeng_tc_x& x, const float* xsum, int64_t M, const qeng_tc_epi& epi, cudaStream_t stream);
+int32_t qeng_gemm_rows(qeng_ctx* ctx, const qeng_weight* w, const qeng_tc_x& x, const float* xsum, int64_t M, const qeng_tc_epi& epi, cudaStream_t stream,
+                       qeng_scratch* sc = nullptr);

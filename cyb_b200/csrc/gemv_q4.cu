@@ -342,12 +342,18 @@ int32_t qeng_gemm_q4(qeng_ctx* ctx, const qeng_weight* w, const void* x, int32_t
   QENG_ENTER(ctx);
   // A batch on bf16 MMAs (gemm_rows.cu) or a dense contraction on tensor memory (gemm_tc.cu).  Both need working memory;
   // without it the call goes through the integer kernel below in passes, except where that has never taken it.
-  if (M >= kManyRows || qeng_gemm_rows_fits(ctx, w, M, x_dtype == QENG_BF16 ? 1 : 2)) {
+  const bool rows = qeng_gemm_rows_fits(ctx, w, M, x_dtype == QENG_BF16 ? 1 : 2);
+  if (M >= kManyRows || rows) {
     const bool prompt = M >= kPrefillRows && w->fmt == QENG_FMT_Q4;
     if (prompt && x_dtype == QENG_F16)
       return qeng_fail(ctx, QENG_ERR_SHAPE, "gemm_q4 (prefill): f16 activations are not supported, use f32 or bf16");
     ctx->no_memory = false;
-    const int32_t rc = qeng_gemm_many_rows(ctx, w, x, x_dtype, M, ldx, y, ldy, (flags & QENG_GEMM_ACCUMULATE) ? 1 : 0, prompt ? 1 : 2, (cudaStream_t)stream);
+    qeng_tc_epi e;
+    e.kind = (flags & QENG_GEMM_ACCUMULATE) ? QENG_EPI_ACCUM : QENG_EPI_STORE;
+    e.y = y;
+    e.ldy = ldy;
+    const int32_t rc = rows ? qeng_gemm_rows_prep(ctx, w, x, x_dtype, M, ldx, nullptr, 0.f, e, (cudaStream_t)stream)
+                            : qeng_gemm_many_rows(ctx, w, x, x_dtype, M, ldx, e, prompt ? 1 : 2, (cudaStream_t)stream);
     if (rc == QENG_OK || prompt || !ctx->no_memory) return rc;
   }
   qeng_gemm_fuse fuse;

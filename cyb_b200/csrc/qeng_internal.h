@@ -251,10 +251,6 @@ qeng_scratch* qeng_scratch_for(qeng_ctx* ctx, cudaStream_t stream);
 // `zeroed`: a new buffer starts as zeros
 int32_t qeng_scratch_grow(qeng_ctx* ctx, qeng_scratch* sc, qeng_buf* b, size_t bytes, bool zeroed = false);
 
-// gemm_tc.cu: tcgen05 matmul of many rows.  wp = 1: bf16 operands; wp = 2: two bf16 terms per weight and per
-// f32 / f16 activation
-int32_t qeng_gemm_many_rows(qeng_ctx* ctx, const qeng_weight* w, const void* x, int32_t x_dtype, int64_t M, int64_t ldx,
-                            float* y, int64_t ldy, int accumulate, int wp, cudaStream_t stream);
 constexpr int64_t kPrefillRows = 256;  // from this many rows on, 4-bit matmuls run on operands rounded to bf16
 constexpr int64_t kManyRows = 17;      // from this many rows on, prompt layers take the tensor-core path
 

@@ -15,8 +15,8 @@
 // through a scratch buffer (one per stream, one per capture) by the CTA that arrives last.
 //
 // HBM-bound: algorithmic bytes = sum_b len_b * kv_heads * 2 * 128 * 2.  With one producer warp for all slots, clusters of
-// eight and Q as the (mostly empty) 16-row operand: 1 x 15001 tokens, 8 kv heads 36 us, now 16 us (floor 9.5); 16 ragged
-// sequences of 512 to 4096 tokens 39 us, now 32 us (24.5); 16 of 4096: 74 us, now 48 us (42).
+// eight and Q as the (mostly empty) 16-row operand: 1 x 15001 tokens, 8 kv heads 39 us, now 18.5 us (floor 9.4);
+// 16 ragged sequences of 512 to 4096 tokens 41 us, now 32.5 us (24.5); 16 of 4096: 74 us, now 48 us (42).
 #include <cuda.h>
 #include <math.h>
 
@@ -50,7 +50,6 @@ __device__ __forceinline__ void cluster_sync() {
 }
 
 struct AttnParams {
-  const __half* pool;
   const __half* q;
   const int32_t* table;
   const int32_t* lens;
@@ -640,7 +639,7 @@ int32_t qeng_attn_decode_ex(qeng_ctx* ctx, const qeng_kv_pool* pool, const uint1
   int32_t rc0 = attn_configure(ctx);
   if (rc0 != QENG_OK) return rc0;
   AttnParams p;
-  p.pool = pool->data; p.q = reinterpret_cast<const __half*>(q_f16);
+  p.q = reinterpret_cast<const __half*>(q_f16);
   p.table = page_table; p.lens = lens; p.out = out; p.status = ctx->status;
   p.pages = (int)pool->pages; p.Hkv = (int)pool->kv_heads; p.Hq = (int)Hq; p.grp = (int)(Hq / pool->kv_heads);
   p.max_pages = (int)max_pages;
@@ -736,7 +735,7 @@ int32_t qeng_attn_decode_noalloc(qeng_ctx* ctx, const qeng_kv_pool* pool, const 
     g_attn_static_addr[ctx->device] = addr;
   }
   float* scratch = g_attn_static_addr[ctx->device];
-  p.pool = pool->data; p.q = reinterpret_cast<const __half*>(q_f16);
+  p.q = reinterpret_cast<const __half*>(q_f16);
   p.table = page_table; p.lens = lens; p.out = out; p.status = ctx->status;
   p.pages = (int)pool->pages; p.Hkv = (int)pool->kv_heads; p.Hq = (int)Hq; p.grp = (int)(Hq / pool->kv_heads);
   p.max_pages = (int)max_pages;

@@ -8,8 +8,10 @@
 // The probabilities enter the second product as two f16 terms, as in the decode kernel: no precision is
 // lost there.  Three CTAs per SM.
 //
-// Bound by the tensor pipe: 12 MMAs of 2 cycles per 16 x 8 scores; 2 * 128 * 3 * heads * T^2 / 2 multiply-adds
-// for a prompt of T tokens = 73 us per layer at T = 1800 and 32 heads.
+// Least time: 24 MMAs of 2 cycles per 16 x 8 scores (8 for the scores, 16 for the values); 2 * 128 * 3 * heads * T^2 / 2
+// operations for a prompt of T tokens = 73 us per layer at T = 1800 and 32 heads.  It takes 205 to 230 there (ncu): the
+// tensor pipe is busy 53 % of the cycles in which an SM has work (dependent steps of the softmax between the two products,
+// 12 consumer warps per SM), and an SM has work 65 % of the time (904 CTAs of very unequal length on 444 places).
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <math.h>

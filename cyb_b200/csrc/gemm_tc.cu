@@ -503,11 +503,16 @@ EncodeFn encode_fn() {
   return fn;
 }
 
-// Up to this many tokens two chunks of operands in two terms fit shared memory twice, beside the packed ring.
+// Up to this many tokens two stages of two chunks, both operands in two terms, fit shared memory beside the packed ring of
+// every block format.  (8-bit blocks set it: 4-bit and K-quant blocks would fit up to 144 tokens, bf16 rows, which have one
+// term, up to 240 and more.)
 constexpr int64_t kWideStage = 112;
 
 // Tile width and split, by a cost model in cycles.  Per 64 k the MMAs take 2 * bn per product and the dequantisation a
-// fixed time, whichever is longer; tiles cut along K pay for their partials' way through L2 and a second launch.
+// fixed time, whichever is longer; tiles cut along K pay for their partials' way through L2 and a second launch.  The fixed
+// times are what its instructions take to issue.  The stages are slower than that, since the steps of a stage depend on
+// one another: 1320 cycles per 64 k of 4-bit blocks in two terms at 112 tokens, where the MMAs take 670; in one term 620
+// at 160 tokens (320) and 730 at 256 tokens (510).  The model orders plans; it does not predict their times.
 Plan make_plan(const qeng_ctx* ctx, const qeng_weight* w, int64_t M, int wp, int xp, bool may_split) {
   Plan best = {};
   double best_cost = 1e30;

@@ -54,8 +54,7 @@ enum {
   QENG_GEMM_ACCUMULATE = 1, /* y += x.W^T instead of y = x.W^T (fused residual add) */
   QENG_GEMM_FAST_F16 = 2    /* a single activation row is quantised to 15 bits per 32-block
                                instead of 22 (a little faster; costs ~6e-5 of the error
-                               budget instead of ~5e-7); no effect for 2 or more rows, which
-                               always use 15 bits */
+                               budget instead of ~5e-7); no effect for 2 or more rows */
 };
 
 typedef struct qeng_ctx qeng_ctx;
@@ -143,9 +142,7 @@ int32_t qeng_weight_quantize_q4(qeng_ctx* ctx, const void* w_dev, int32_t x_dtyp
 /* ---- 8-bit block weights ("tensor data (Q4/Q8/F16/F32)", decide/pipeline.md:28; the default
  *      model of the reference's catalog was imported as q8, shell/src/worlds/models/mod.rs:68-73)
  * w = q * s with q a signed byte and one f16 scale per 32 consecutive K (the published Q8_0 block).
- * A weight handle of this format is taken by qeng_gemm_q4 / qeng_gemv_q4 (any M: rows in passes of
- * 16 through the decode kernel; the tensor-core prefill kernel is for 4-bit blocks only),
- * qeng_weight_dequant_f32, qeng_weight_set_next and the getters.  Same shape rules as the 4-bit calls. */
+ * A weight handle of this format is taken by qeng_gemm_q4 / qeng_gemv_q4 (any M), qeng_weight_dequant_f32, qeng_weight_set_next and the getters.  Same shape rules as the 4-bit calls. */
 int32_t qeng_weight_pack_q8(qeng_ctx* ctx, const int8_t* q, const uint16_t* s, int64_t N, int64_t K, qeng_weight** out);
 /* Inverse, computed ON THE DEVICE from the packed layout: N*K bytes and N*K/32 scales to HOST buffers. */
 int32_t qeng_weight_unpack_q8(qeng_ctx* ctx, const qeng_weight* w, int8_t* q, uint16_t* s);
@@ -159,7 +156,7 @@ int32_t qeng_weight_quantize_q8(qeng_ctx* ctx, const void* w_dev, int32_t x_dtyp
  * minima, 128 bytes of codes: of every 32 bytes the low nibbles are sub-block 2i, the high nibbles
  * sub-block 2i+1); w = (d * sc_j) * code - (dmin * m_j).  K % 256 == 0, N % 16 == 0.  The weight is
  * expanded to per-32-block f32 (scale, minimum) pairs on the device (0.75 B per weight) and taken by
- * qeng_gemm_q4 / qeng_gemv_q4 (decode kernel, 4 rows per pass), qeng_weight_dequant_f32, the getters. */
+ * qeng_gemm_q4 / qeng_gemv_q4 (any M), qeng_weight_dequant_f32, the getters. */
 int32_t qeng_weight_pack_q4k(qeng_ctx* ctx, const uint8_t* blocks, int64_t N, int64_t K, qeng_weight** out);
 /* Inverse of the device layout (the bit-exactness check): codes [N][K] (0..15) and f32 pairs
  * (scale, minimum) [N][K/32][2] to HOST buffers. */
@@ -180,10 +177,16 @@ int32_t qeng_weight_set_next(qeng_ctx* ctx, qeng_weight* w, const qeng_weight* n
 
 /* ---- quantized matmul (the "QKV / O proj / FFN" steps of decide/pipeline.md:51)
  * y[M,N] (f32, leading dimension ldy) = x[M,K] (x_dtype, leading dimension ldx)
- * . dequant(W)^T, f32 accumulation.  M < 256 runs the decode kernels (weights unpacked in
- * registers, activations in block fixed point: 22 bits for one row, 15 bits per row otherwise,
- * integer tensor-core contraction, per-block f32 scaling); M >= 256 the tensor-core prefill kernel, which rounds
- * activations and dequantised weights to bf16 (tolerance 5e-3 instead of 2e-3). */
+ * . dequant(W)^T, f32 accumulation.
+ *   1 row, 2 to 4 (f32, f16) or 2 (bf16): integer tensor-core contraction on the codes, activations in block
+ *     fixed point (22 bits for one row, 15 bits otherwise), per-block f32 scaling;
+ *   to 16 (f32, f16) or 32 (bf16): the codes as exact bf16 operands, f32 / f16 activations in two bf16 terms
+ *     (17 bits), per-block f32 scaling;
+ *   more, and any of these that do not fit that: dequantised to two bf16 terms (17 bits), activations likewise;
+ *   M >= 256 over 4-bit blocks: activations and dequantised weights rounded to bf16 (tolerance 5e-3 instead
+ *     of 2e-3; f16 activations are refused).
+ * The last three use working memory of the context; without room for it, rows below 256 and 8-bit or K-quant
+ * blocks go through the first form in passes of 16 (K-quant: 4) rows. */
 int32_t qeng_gemm_q4(qeng_ctx* ctx, const qeng_weight* w, const void* x, int32_t x_dtype,
                      int64_t M, int64_t ldx, float* y, int64_t ldy, int32_t flags, void* stream);
 /* M = 1, f32 activations: the decode GEMV. */
@@ -291,8 +294,8 @@ int32_t qeng_decoder_load_matrix(qeng_ctx* ctx, qeng_decoder* dec, int32_t layer
  * (q, k, v of a layer; gate, up of a layer) must come in one format. */
 int32_t qeng_decoder_load_matrix_q8(qeng_ctx* ctx, qeng_decoder* dec, int32_t layer, int32_t which,
                                     const int8_t* q, const uint16_t* s, int64_t N, int64_t K);
-/* The same for Q4_K super-blocks (see qeng_weight_pack_q4k); decode steps of up to 4 sequences take
- * such layers in one pass, batches of 5 to 16 in passes of 4 rows. */
+/* The same for Q4_K super-blocks (see qeng_weight_pack_q4k); decode steps of any batch take such layers in one
+ * pass (with tensor parallelism, batches of 5 to 16 in passes of 4 rows). */
 int32_t qeng_decoder_load_matrix_q4k(qeng_ctx* ctx, qeng_decoder* dec, int32_t layer, int32_t which,
                                      const uint8_t* blocks, int64_t N, int64_t K);
 /* RMSNorm gains of a layer (which = 0: before attention, 1: before FFN), HOST f32[d_model].

@@ -111,8 +111,8 @@ def test_teacher_forced_layer_on_the_tensor_core_path(ctx):
 def test_full_size_layer_teacher_forced(ctx):
     """One layer at BASELINE's full widths (d 4096, FFN 11008, 32/8 heads): 6 prompt rows then one
     decode row, teacher-forced against the float64 oracle (gate 2e-3 on the layer output; measured
-    ~1e-3: the 15-bit block fixed point of the activations entering o / gate|up / down, whose
-    per-matmul error of ~6e-5 is amplified by the heavy-tailed SwiGLU output of these synthetic
+    ~1e-3 for the decode row: the 15-bit block fixed point of the activations entering o / gate|up / down,
+    whose per-matmul error of ~6e-5 is amplified by the heavy-tailed SwiGLU output of these synthetic
     weights)."""
     import torch
     from cyb_b200 import qeng
@@ -208,8 +208,8 @@ def test_qk_norm_decode_matches_the_golden_fixture(ctx):
 
 @pytest.mark.parametrize("batch", [5, 16])
 def test_greedy_decode_at_larger_batches(ctx, batch):
-    """Batches above 4 leave the fused LM head (separate norm, head, argmax, advance, embed) and run
-    the matmuls in row chunks: logits after the prompt and greedy tokens against the float64 teacher."""
+    """Batches above 4 run their matmuls on bf16 MMAs with a preparation and a finishing kernel (their 7-token prompts,
+    35 and 112 rows, on tensor memory): logits after the prompt and greedy tokens against the float64 teacher."""
     cfg, W, dec = _make(ctx, max_batch=batch, max_seq=48)
     teacher = ref.Decoder(cfg, W)
     prompt = ref.rng_of(300 + batch).integers(0, cfg.vocab, (batch, 7)).astype(np.int32)

@@ -59,7 +59,7 @@ def test_decoder_with_kquant_blocks_matches_the_teacher(ctx):
     dec = ctx.decoder(layers=cfg.layers, d_model=cfg.d, ffn=cfg.ffn, heads=cfg.heads, kv_heads=cfg.kv_heads,
                       vocab=cfg.vocab, max_batch=5, max_seq=96)
     qeng.load_decoder_weights(dec, W, cfg)
-    for bn, t in ((1, 23), (5, 9)):  # 5 sequences: passes of 4 rows
+    for bn, t in ((1, 23), (5, 9)):  # 5 sequences: the batch matmul; their prompts: tensor memory
         prompt = ref.rng_of(70 + bn).integers(0, cfg.vocab, (bn, t)).astype(np.int32)
         want, logs = ref.Decoder(cfg, W).generate(prompt, 6)
         dec.reset(bn)

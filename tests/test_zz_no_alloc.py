@@ -51,7 +51,7 @@ def test_noalloc_matches_regular_entry_point_twice(ctx):
 
 
 def test_noalloc_at_the_documented_limit_shape(ctx):
-    """16 sequences x 32 heads with caches of 512..4096 tokens (15 splits): the example the header
+    """16 sequences x 32 heads with caches of 512..4096 tokens, the sequences and heads of the example that the header
     gives for what the built-in array holds.  Checked against the regular entry point and the oracle."""
     import torch
     lens, q, ks, vs, pool_np, table = ref.config4(seed=4)

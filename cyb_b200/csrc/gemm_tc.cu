@@ -7,19 +7,26 @@
 // which makes every store of the epilogue 128 contiguous bytes of a y row.
 //
 // A pair of CTAs (cluster of 2, tcgen05 cta_group::2) computes a tile: each CTA dequantises 128 of the
-// weight rows and loads half of the tokens, so the activation tile crosses L2 -> shared memory once per
-// pair and 64 k cost each SM 32 KB for 2 * 128 * bn * 64 MMA operations.  Roles (24 warps):
-//   warp 0      issues tcgen05.mma (leader CTA, one thread); tcgen05.commit frees stages in both CTAs
+// weight rows into its tensor memory, which is where the MMAs take their A operand from, and loads half of
+// the tokens into shared memory, so the activation tile crosses L2 -> shared memory once per pair.
+// Roles (24 warps):
+//   warp 0      leader CTA: issues tcgen05.mma (one thread); tcgen05.commit frees stages in both CTAs.
+//               Other CTA: passes its dequant warps' arrivals on to the leader, one per stage
 //   warp 1      activation tiles: TMA boxes of 64 k x bn/2 tokens, 128-byte swizzle
 //   warp 2      packed weights: one TMA box of 8 row tiles per stage and plane into a ring of its own,
 //               which keeps tens of KB per SM in flight from HBM independently of the dequant warps
 //   warp 3      tensor memory allocation
-//   warps 4-7   epilogue (tcgen05.ld, one warp per lane quadrant), overlapped with the next tile: two
-//               accumulators of 256 columns
-//   warps 8-23  dequantisation: packed words -> bf16, stored in the swizzled K-major layout the MMA reads;
-//               one warp per 16-row tile, two sets of 8 that take alternate stages
-// A stage is KST chunks of 64 k: two where shared memory allows it (each role then pays its barrier
-// round trips, some 300 cycles of dependent instructions, once per 128 k).
+//   warps 4-7   epilogue (tcgen05.ld, one warp per lane quadrant), overlapped with the next tile where
+//               tensor memory holds two accumulators (up to 160 columns with one weight term)
+//   warps 8-23  dequantisation: packed words -> bf16 -> tensor memory; one warp per 16-row tile, two sets
+//               of 8 that take alternate stages
+// A stage is two chunks of 64 k, with one barrier each way: a hop between the roles costs 100 to 200 cycles
+// of dependent instructions, and with one barrier per chunk the hops of a stage took longer than its MMAs.
+// The weights used to pass through shared memory, which then carried 1.3 times what it can in the time of
+// the MMAs: cycles per 128 k and one term, shared / tensor memory: 1460 / 1024 at 256 columns (the MMAs:
+// 1024), 1240 / 800 to 880 at 160 (640); two terms, 112 columns: 2640 / 1340 (1344).
+// 777 rows f32 over 11008 x 4096 87.6 -> 75.4 us, 101 rows 37.8 -> 35.0, 8192 rows bf16 over 4096 x 11008
+// 645 -> 590 (power limit), a prompt of 1800 tokens 33.2 -> 29.3 ms.
 //
 // Precision.  WP = 1 (prompt path of 4-bit blocks): weights and activations rounded to bf16, as before.
 // WP = 2: a weight is the sum of two bf16 values (4-bit blocks: exact, (c-8)*s has 14 significant bits;
@@ -42,27 +49,40 @@
 namespace {
 using namespace qeng_tc;
 
-constexpr int kDequantWarps = 8;         // per set
-constexpr int kThreads = (8 + 2 * kDequantWarps) * 32;
+constexpr int kDequantWarps = 8, kSets = 2;
+constexpr int kThreads = (8 + kSets * kDequantWarps) * 32;
 
 // ---- dequantisation: one lane's words of one 32-block -> rows g and g+8, 8 consecutive k each ------------------
 // The inner loop of the kernel: its rate is set by the integer pipe (half rate), so the 4-bit form spends two
 // integer instructions per pair of weights (shift, AND-OR) and leaves the rest to the FMA pipe.
 // Codes in the low nibbles of bf16: 0x4300 | c is 128 + c; minus 136 gives c - 8 exactly.  The f16 scale is split
 // into two bf16 terms (8 + 3 bits), so that the fma rounds (c-8)*s once, to the nearest bf16; the remainder is exact.
-template <int WP>
-__device__ __forceinline__ void dequant_q4(uint32_t w, float s, uint32_t (&hi)[4], uint32_t (&lo)[4]) {
+struct Scale2 {
+  __nv_bfloat162 hi, lo;
+};
+__device__ __forceinline__ Scale2 split_scale(float s) {
   const uint32_t sb = __float_as_uint(s);
-  const float rest = s - __uint_as_float(sb & 0xffff0000u);
-  const __nv_bfloat162 s_hi = bf2(__byte_perm(sb, sb, 0x3232)), s_lo = bf2(__byte_perm(__float_as_uint(rest), __float_as_uint(rest), 0x3232));
-  const __nv_bfloat162 off = bf2(0xc308c308u);  // -136
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {  // k = 2i and 2i + 1
-    const __nv_bfloat162 c = __hadd2(bf2(((w >> (4 * i)) & 0x000f000fu) | 0x43004300u), off);
-    const __nv_bfloat162 v = __hfma2(c, s_hi, __hmul2(c, s_lo));
-    hi[i] = u32(v);
-    if (WP == 2) lo[i] = u32(__hfma2(c, s_lo, __hfma2(c, s_hi, __hneg2(v))));
-  }
+  const uint32_t rest = __float_as_uint(s - __uint_as_float(sb & 0xffff0000u));
+  return {bf2(__byte_perm(sb, sb, 0x3232)), bf2(__byte_perm(rest, rest, 0x3232))};
+}
+// (a & b) | c in one instruction, the constants in registers
+__device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t b, uint32_t c) {
+  uint32_t r;
+  asm("lop3.b32 %0, %1, %2, %3, 0xea;\n" : "=r"(r) : "r"(a), "r"(b), "r"(c));
+  return r;
+}
+__device__ __forceinline__ uint32_t in_register(uint32_t v) {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %1;\n" : "=r"(r) : "r"(v));
+  return r;
+}
+// the pair of codes in bits 0..3 and 16..19
+template <int WP>
+__device__ __forceinline__ void pair_q4(uint32_t w, const Scale2& s, uint32_t mask, uint32_t base, uint32_t& hi, uint32_t& lo) {
+  const __nv_bfloat162 c = __hadd2(bf2(and_or(w, mask, base)), bf2(0xc308c308u));  // -136
+  const __nv_bfloat162 v = __hfma2(c, s.hi, __hmul2(c, s.lo));
+  hi = u32(v);
+  if (WP == 2) lo = u32(__hfma2(c, s.lo, __hfma2(c, s.hi, __hneg2(v))));
 }
 // two f32 values -> bf16 pair and the bf16 pair of what the rounding left
 __device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t& lo) {
@@ -70,57 +90,106 @@ __device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t&
   hi = u32(h);
   lo = u32(__floats2bfloat162_rn(a - __low2float(h), b - __high2float(h)));
 }
-// block b (0 or 1) of the chunk at (wbase, sbase): hi/lo[0] row g, hi/lo[1] row g + 8
-template <int FMT, int WP>
-__device__ __forceinline__ void dequant_block(uint32_t wbase, uint32_t sbase, int lane, int b, uint32_t (&hi)[2][4], uint32_t (&lo)[2][4]) {
-  const int g = lane >> 2;
-  if (FMT == QENG_FMT_Q4) {
-    const uint2 w = lds64(wbase + (uint32_t)(lane * 16 + b * 8));
-    const uint32_t sp = lds32(sbase + (uint32_t)(g * 8 + b * 4));
-    const float2 sf = __half22float2(*reinterpret_cast<const __half2*>(&sp));
-    dequant_q4<WP>(w.x, sf.x, hi[0], lo[0]);
-    dequant_q4<WP>(w.y, sf.y, hi[1], lo[1]);
-  } else if (FMT == QENG_FMT_Q8) {
-    const uint4 w = lds128(wbase + (uint32_t)(b * 512 + lane * 16));
-    const uint32_t sp = lds32(sbase + (uint32_t)(g * 8 + b * 4));
-    const float2 sf = __half22float2(*reinterpret_cast<const __half2*>(&sp));
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-      // bytes of k = 0,4,1,5 and of k = 2,6,3,7; a signed byte xor 0x80 under the exponent of 2^23
-      const uint32_t we = (r ? w.y : w.x) ^ 0x80808080u, wo = (r ? w.w : w.z) ^ 0x80808080u;
-      const float s = r ? sf.y : sf.x;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const uint32_t src = (i & 1) ? wo : we;
-        const float a = __uint_as_float(__byte_perm(src, 0x4b000000u, 0x7440 + (i >> 1))) - 8388736.0f;
-        const float c = __uint_as_float(__byte_perm(src, 0x4b000000u, 0x7442 + (i >> 1))) - 8388736.0f;
-        split2(a * s, c * s, hi[r][i], lo[r][i]);
-      }
+// One lane's share of a chunk, in the layout of tmem_st16: quad i = k 16i + 4t .. 16i + 4t + 3 of rows g and g + 8.
+// Packed lane t' of a block holds k = 8t' .. 8t' + 7, so quad i of a block (i = 0, 1) is half t & 1 of the words of packed
+// lane 2i + t / 2: neighbouring lanes read the same 16 bytes, each uses its half.
+template <int FMT>
+struct Words {   // 4-bit and K-quant blocks
+  uint4 q0, q1;  // quad 0 / 1: row g and g + 8 of the first block, of the second
+  uint4 d, m;    // K-quant: De(g), De(g+8), Do(g), Do(g+8) | Me(g), Me(g+8), Mo(g), Mo(g+8); 4-bit: d.x, d.y = f16 pairs
+  __device__ __forceinline__ void load(uint32_t wbase, uint32_t sbase, int lane) {
+    const int g = lane >> 2, t = lane & 3;
+    const uint32_t w0 = wbase + (uint32_t)((g * 4 + (t >> 1)) * 16);
+    q0 = lds128(w0);
+    q1 = lds128(w0 + 32);
+    if (FMT == QENG_FMT_K4) {
+      d = lds128(sbase + (uint32_t)(g * 32));
+      m = lds128(sbase + (uint32_t)(g * 32 + 16));
+    } else {
+      const uint2 s = lds64(sbase + (uint32_t)(g * 8));
+      d = make_uint4(s.x, s.y, 0u, 0u);
+      m = make_uint4(0u, 0u, 0u, 0u);
     }
-  } else {
-    // per lane group: De(g), De(g+8), Do(g), Do(g+8) | Me(g), Me(g+8), Mo(g), Mo(g+8)
-    const uint2 w = lds64(wbase + (uint32_t)(lane * 16 + b * 8));
-    const uint2 d = lds64(sbase + (uint32_t)(g * 32 + b * 8)), m = lds64(sbase + (uint32_t)(g * 32 + 16 + b * 8));
+  }
+  template <int WP>
+  __device__ __forceinline__ void dequant(int lane, uint32_t mask, uint32_t base, uint32_t (&hi)[16], uint32_t (&lo)[16]) const {
+    const uint32_t sh = 8u * (lane & 1);
+    const uint32_t ws[2][2][2] = {{{q0.x, q1.x}, {q0.y, q1.y}}, {{q0.z, q1.z}, {q0.w, q1.w}}};  // [block][row][quad]
 #pragma unroll
-    for (int r = 0; r < 2; ++r) {
-      const uint32_t wv = r ? w.y : w.x;
-      const float D = __uint_as_float(r ? d.y : d.x), mn = __uint_as_float(r ? m.y : m.x);
+    for (int b = 0; b < 2; ++b) {
+      const uint32_t s2 = b ? d.y : d.x;
+      const float2 sf = __half22float2(*reinterpret_cast<const __half2*>(&s2));
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float a = __uint_as_float(0x4b000000u | ((wv >> (4 * i)) & 15u)) - 8388608.0f;
-        const float c = __uint_as_float(0x4b000000u | ((wv >> (4 * i + 16)) & 15u)) - 8388608.0f;
-        split2(fmaf(a, D, -mn), fmaf(c, D, -mn), hi[r][i], lo[r][i]);
+      for (int r = 0; r < 2; ++r) {
+        const Scale2 s = split_scale(r ? sf.y : sf.x);
+        const float D = __uint_as_float(b ? (r ? d.w : d.z) : (r ? d.y : d.x)), mn = __uint_as_float(b ? (r ? m.w : m.z) : (r ? m.y : m.x));
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const uint32_t w = ws[b][r][i] >> sh;
+          const int at = (b * 2 + i) * 4 + r * 2;
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            if (FMT == QENG_FMT_Q4) {
+              pair_q4<WP>(w >> (4 * j), s, mask, base, hi[at + j], lo[at + j]);
+            } else {
+              const float x = __uint_as_float(0x4b000000u | ((w >> (4 * j)) & 15u)) - 8388608.0f;
+              const float y = __uint_as_float(0x4b000000u | ((w >> (4 * j + 16)) & 15u)) - 8388608.0f;
+              split2(fmaf(x, D, -mn), fmaf(y, D, -mn), hi[at + j], lo[at + j]);
+            }
+          }
+        }
       }
     }
   }
-}
+};
+template <>
+struct Words<QENG_FMT_Q8> {
+  uint4 q[2][2];  // [block][quad]
+  uint2 s;
+  __device__ __forceinline__ void load(uint32_t wbase, uint32_t sbase, int lane) {
+    const int g = lane >> 2, t = lane & 3;
+    const uint32_t w0 = wbase + (uint32_t)((g * 4 + (t >> 1)) * 16);
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+      q[b][0] = lds128(w0 + (uint32_t)(b * 512));
+      q[b][1] = lds128(w0 + (uint32_t)(b * 512 + 32));
+    }
+    s = lds64(sbase + (uint32_t)(g * 8));
+  }
+  template <int WP>
+  __device__ __forceinline__ void dequant(int lane, uint32_t, uint32_t, uint32_t (&hi)[16], uint32_t (&lo)[16]) const {
+    // bytes of k = 0,4,1,5 (rows g, g + 8) and of k = 2,6,3,7; a signed byte xor 0x80 under the exponent of 2^23
+    const uint32_t s0 = 0x7440u + (lane & 1), s1 = s0 + 2;
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+      const uint32_t s2 = b ? s.y : s.x;
+      const float2 sf = __half22float2(*reinterpret_cast<const __half2*>(&s2));
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const uint4 w = q[b][i];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const float f = r ? sf.y : sf.x;
+          const int at = (b * 2 + i) * 4 + r * 2;
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            const uint32_t src = (j ? (r ? w.w : w.z) : (r ? w.y : w.x)) ^ 0x80808080u;
+            const float x = __uint_as_float(__byte_perm(src, 0x4b000000u, s0)) - 8388736.0f;
+            const float y = __uint_as_float(__byte_perm(src, 0x4b000000u, s1)) - 8388736.0f;
+            split2(x * f, y * f, hi[at + j], lo[at + j]);
+          }
+        }
+      }
+    }
+  }
+};
 
-template <int FMT, int WP, int XP, int KST>
+template <int FMT, int WP, int XP>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     gemm_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap,
                    const __grid_constant__ CUtensorMap smap) {
   constexpr int kW = Fmt<FMT>::kW, kS = Fmt<FMT>::kS;
-  constexpr uint32_t kSlot = KST * 8 * (kW + kS);
+  constexpr uint32_t kSlot = kST * 8 * (kW + kS), kStageCols = kST * WP * kACols;
   extern __shared__ unsigned char smem_raw[];
   // the swizzle pattern is a function of the address: tiles start on 1024-byte boundaries (the same offset in both CTAs)
   const uint32_t smem = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -132,14 +201,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   asm volatile("mov.u32 %0, %cluster_ctarank;\n" : "=r"(rank));
   const int pair = blockIdx.x >> 1;
   const uint32_t b_plane = (uint32_t)(p.bn >> 1) * 128u;
-  // stage: A [KST][WP] planes, then B [KST][XP] planes
-  const uint32_t stage_bytes = KST * (WP * kAPlane + XP * b_plane);
+  const uint32_t stage_bytes = kST * XP * b_plane;                 // activations: [kST][XP] planes
   const uint32_t ring = smem + (uint32_t)p.nstages * stage_bytes;  // packed-weight slots
 
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   if (tid == 0) {
     for (int s = 0; s < p.nstages; ++s) {
-      mbar_init(smem_u32(full + s), 1 + 2 * kDequantWarps);  // the leader's expect_tx, one set of dequant warps in each CTA
+      // the CTA's own set of dequant warps; in the leader also the peer, once its set has arrived there, and the expect_tx
+      mbar_init(smem_u32(full + s), kDequantWarps + (rank == 0 ? 2 : 0));
       mbar_init(smem_u32(empty + s), 1);
     }
     for (int s = 0; s < p.nslots; ++s) {
@@ -162,51 +231,57 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   cluster_sync();
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
   const uint32_t tmem = tmem_slot;
+  const uint32_t tmem_a = tmem + (uint32_t)(p.nacc * p.acc_cols);  // the weights' stages, behind the accumulators
 
   Segments segs(p, pair);
   Seg sg;
   bool failed = false;
 
   if (warp == 0) {
-    // ===== MMA issuer =====================================================================
     if (rank == 0) {
+      // ===== MMA issuer =====================================================================
       // f32 accumulate, bf16 x bf16, both K-major, N = bn, M = 256
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.bn >> 3) << 17) | (16u << 24);
-      int s = 0, n = 0;
-      uint32_t ph = 0;
+      // What the instructions of a stage are issued from has to be warp-uniform for the compiler (votes and shuffles tell it):
+      // at 160 columns and less the issue of a stage is as long as its MMAs.
+      const uint32_t base = __shfl_sync(0xffffffffu, smem, 0), tm = __shfl_sync(0xffffffffu, tmem, 0), ta = __shfl_sync(0xffffffffu, tmem_a, 0);
+      int s = 0, n = 0, buf = 0;
+      uint32_t ph = 0, acc_ph = 1;
       while (!failed && segs.next(p, sg)) {
-        const int buf = n & 1;
+        if (!mbar_wait_warp(smem_u32(acc_empty + buf), acc_ph)) { failed = true; break; }
+        const uint32_t d = tm + (uint32_t)(buf * p.acc_cols);
+        uint32_t acc = 0;
         for (int kt = sg.k0; kt < sg.k1; ++kt) {
-          if (kt == sg.k0 && !mbar_wait(smem_u32(acc_empty + buf), (((uint32_t)n >> 1) & 1u) ^ 1u)) failed = true;
-          if (failed || !mbar_wait(smem_u32(full + s), ph)) failed = true;
-          if (__any_sync(0xffffffffu, failed)) { failed = true; break; }
+          if (!mbar_wait_warp(smem_u32(full + s), ph)) { failed = true; break; }
           asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-          // (the shuffles tell the compiler what is warp-uniform: MMA operands live in uniform registers)
-          const uint32_t a = __shfl_sync(0xffffffffu, smem + (uint32_t)s * stage_bytes, 0);
-          const uint32_t d = __shfl_sync(0xffffffffu, tmem + (uint32_t)buf * 256u, 0);
           if (elect_one()) {
+            const uint32_t a = ta + (uint32_t)s * kStageCols;
+            const uint64_t bd = make_desc(base + (uint32_t)s * stage_bytes);
 #pragma unroll
-            for (int c = 0; c < KST; ++c) {
-              const uint64_t ah = make_desc(a + c * WP * kAPlane), bh = make_desc(a + KST * WP * kAPlane + c * XP * b_plane);
+            for (int c = 0; c < kST; ++c) {
 #pragma unroll
-              for (int k = 0; k < kBK / 16; ++k) {  // descriptors count 16-byte units: 2 per K step of 16
-                umma_bf16(d, ah + 2 * k, bh + 2 * k, idesc, (kt > sg.k0 || c > 0 || k > 0) ? 1u : 0u);
-                if (WP == 2) umma_bf16(d, ah + (kAPlane >> 4) + 2 * k, bh + 2 * k, idesc, 1u);
-                if (XP == 2) umma_bf16(d, ah + 2 * k, bh + (b_plane >> 4) + 2 * k, idesc, 1u);
+              for (int k = 0; k < kBK / 16; ++k) {  // a K step of 16: 8 columns of A; descriptors count 16-byte units
+                const uint32_t ac = a + c * WP * kACols + 8 * k;
+                const uint64_t bh = bd + c * XP * (b_plane >> 4) + 2 * k;
+                umma_bf16(d, ac, bh, idesc, c > 0 || k > 0 ? 1u : acc);
+                if (WP == 2) umma_bf16(d, ac + kACols, bh, idesc, 1u);
+                if (XP == 2) umma_bf16(d, ac, bh + (b_plane >> 4), idesc, 1u);
               }
             }
             umma_commit_pair(smem_u32(empty + s));
             if (kt + 1 == sg.k1) umma_commit_pair(smem_u32(acc_full + buf));
           }
           __syncwarp();
+          acc = 1;
           if (++s == p.nstages) { s = 0; ph ^= 1u; }
         }
         ++n;
+        if (++buf == p.nacc) { buf = 0; acc_ph ^= 1u; }
       }
       // the last accumulators have been read in both CTAs: nothing of this pair is in flight any more
-      for (int b = 0; b < 2 && b < n; ++b) {
+      for (int b = 0; b < p.nacc && b < n; ++b) {
         const int last = n - 1 - b;
-        if (!failed && !mbar_wait(smem_u32(acc_empty + (last & 1)), ((uint32_t)last >> 1) & 1u)) failed = true;
+        if (!failed && !mbar_wait(smem_u32(acc_empty + last % p.nacc), (uint32_t)(last / p.nacc) & 1u)) failed = true;
       }
       if (failed) {  // what was issued still has to finish before tensor memory is freed
         if (elect_one()) umma_commit_pair(smem_u32(&drained));
@@ -214,6 +289,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         mbar_wait(smem_u32(&drained), 0);
         if (lane == 0) atomicExch(p.status, 4);
       }
+    } else {
+      // ===== the peer's weights: one arrival at the leader per stage, for the eight of its warps =========
+      const int total = segs.stages(p);
+      int s = 0;
+      uint32_t ph = 0;
+      for (int i = 0; i < total; ++i) {
+        if (!mbar_wait(smem_u32(full + s), ph)) failed = true;
+        if (__any_sync(0xffffffffu, failed)) { failed = true; break; }
+        if (lane == 0) mbar_arrive_cluster(map_leader(smem_u32(full + s)));
+        if (++s == p.nstages) { s = 0; ph ^= 1u; }
+      }
+      if (failed && lane == 0) atomicExch(p.status, 4);
     }
   } else if (warp == 1) {
     // ===== activation tiles ==================================================================
@@ -228,12 +315,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         if (!mbar_wait(smem_u32(empty + s), ph ^ 1u)) failed = true;
         if (__any_sync(0xffffffffu, failed)) { failed = true; break; }
         if (elect_one()) {
-          if (rank == 0) mbar_expect_tx(smem_u32(full + s), KST * XP * 2 * b_plane);
-          const uint32_t b = smem + (uint32_t)s * stage_bytes + KST * WP * kAPlane, bar = map_leader(smem_u32(full + s));
+          if (rank == 0) mbar_expect_tx(smem_u32(full + s), 2 * stage_bytes);
+          const uint32_t b = smem + (uint32_t)s * stage_bytes, bar = map_leader(smem_u32(full + s));
 #pragma unroll
-          for (int c = 0; c < KST; ++c)
+          for (int c = 0; c < kST; ++c)
 #pragma unroll
-            for (int pl = 0; pl < XP; ++pl) tma_x(b + (uint32_t)(c * XP + pl) * b_plane, &xmap, (kt * KST + c) * kBK, m0, pl, bar);
+            for (int pl = 0; pl < XP; ++pl) tma_x(b + (uint32_t)(c * XP + pl) * b_plane, &xmap, (kt * kST + c) * kBK, m0, pl, bar);
         }
         __syncwarp();
         if (++s == p.nstages) { s = 0; ph ^= 1u; }
@@ -253,8 +340,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         if (elect_one()) {
           const uint32_t bar = smem_u32(wfull + s), dst = ring + (uint32_t)s * kSlot;
           mbar_expect_tx(bar, kSlot);
-          tma_w(dst, &wmap, kt * KST, nt * 16 + (int)rank * 8, bar);
-          tma_w(dst + KST * 8 * kW, &smap, kt * KST, nt * 16 + (int)rank * 8, bar);
+          tma_w(dst, &wmap, kt * kST, nt * 16 + (int)rank * 8, bar);
+          tma_w(dst + kST * 8 * kW, &smap, kt * kST, nt * 16 + (int)rank * 8, bar);
         }
         __syncwarp();
         if (++s == p.nslots) { s = 0; ph ^= 1u; }
@@ -263,72 +350,60 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     if (failed && lane == 0) atomicExch(p.status, 4);
   } else if (warp >= 8) {
     // ===== dequantisation: warp = one 16-row tile =================================================
-    const int set = (warp - 8) >> 3, rt = (warp - 8) & 7, g = lane >> 2, t = lane & 3;
-    // Lanes with odd g take the chunk's blocks in the other order: a quarter-warp then stores two rows into opposite
-    // halves of the swizzled 128-byte line and touches every bank once.  dst[h]: row g, the h-th block this lane takes
-    // (row g + 8 is 1024 bytes on: the swizzle depends on g alone).
-    const int first = g & 1;
-    uint32_t dst[2];
+    // (whose tensor-memory lanes lie in the quadrant that this warp may write, warp % 4)
+    const int set = (warp - 8) >> 3, rt = (warp & 3) * 2 + ((warp >> 2) & 1);
+    const uint32_t dst0 = tmem_a + ((uint32_t)(rt * 16) << 16);
+    const uint32_t wb0 = ring + (uint32_t)rt * (kST * kW), sb0 = ring + 8u * kST * kW + (uint32_t)rt * (kST * kS);
+    const uint32_t mask = in_register(0x000f000fu), base = in_register(0x43004300u);
+    const int total = segs.stages(p);
+    // Whoever waits on a barrier by parity has to see all of its phases (boxes may land out of order: a set that skipped
+    // one could take the phase before the last for the one it needs), so the number of packed slots is even and a slot
+    // always belongs to one set.  (Stages need no such care: two stages ago this set waited for a consumption no
+    // earlier than the one before the last of this stage, and the MMAs consume in order.)
+    int s = set, ws = set;
+    uint32_t ph = 1, wph = 0;
+    for (int i = set; i < total; i += kSets) {
+      if (!failed && !mbar_wait(smem_u32(wfull + ws), wph)) failed = true;
+      const uint32_t wb = wb0 + (uint32_t)ws * kSlot, sb = sb0 + (uint32_t)ws * kSlot, at = dst0 + (uint32_t)s * kStageCols;
+      Words<FMT> w[kST];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) dst[h] = smem + (uint32_t)((rt * 16 + g) * 128) + (uint32_t)((((h ^ first) * 4 + t) ^ g) << 4);
-    const uint32_t wb0 = ring + (uint32_t)rt * (KST * kW), sb0 = ring + 8u * KST * kW + (uint32_t)rt * (KST * kS);
-    int s = 0, ws = 0, turn = 0;  // turn: the set whose stage comes next
-    uint32_t ph = 0, wph = 0;
-    while (segs.next(p, sg)) {
-      for (int kt = sg.k0; kt < sg.k1; ++kt) {
-        // Whoever waits on a barrier by parity has to see all of its phases (boxes may land out of order: a set that
-        // skipped one could take the phase before the last for the one it needs), so the number of packed slots is
-        // even and a slot always belongs to one set.  (Operand stages need no such care: two stages ago this set waited
-        // for a consumption later than the one before the last of this stage, and the MMAs consume in order.)
-        if (turn == set) {
-          if (!failed && !mbar_wait(smem_u32(wfull + ws), wph)) failed = true;
-          const uint32_t wb = wb0 + (uint32_t)ws * kSlot, sb = sb0 + (uint32_t)ws * kSlot, so = (uint32_t)s * stage_bytes;
-          uint32_t hi[2][2][4], lo[2][2][4];
+      for (int c = 0; c < kST; ++c) w[c].load(wb + (uint32_t)(c * kW), sb + (uint32_t)(c * kS), lane);
 #pragma unroll
-          for (int h = 0; h < 2; ++h) dequant_block<FMT, WP>(wb, sb, lane, h ^ first, hi[h], lo[h]);
-          if (!failed && !mbar_wait(smem_u32(empty + s), ph ^ 1u)) failed = true;
-#pragma unroll
-          for (int c = 0; c < KST; ++c) {
-            if (c > 0) {
-#pragma unroll
-              for (int h = 0; h < 2; ++h)
-                dequant_block<FMT, WP>(wb + (uint32_t)(c * kW), sb + (uint32_t)(c * kS), lane, h ^ first, hi[h], lo[h]);
-            }
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-#pragma unroll
-              for (int r = 0; r < 2; ++r) {
-                const uint32_t at = dst[h] + so + (uint32_t)(c * WP * kAPlane + r * 1024);
-                sts128(at, hi[h][r]);
-                if (WP == 2) sts128(at + kAPlane, lo[h][r]);
-              }
-          }
-          asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+      for (int c = 0; c < kST; ++c) {
+        uint32_t hi[16], lo[16];
+        w[c].template dequant<WP>(lane, mask, base, hi, lo);
+        if (c == 0) {
+          if (!failed && !mbar_wait(smem_u32(empty + s), ph)) failed = true;
           __syncwarp();
-          if (lane == 0) {
-            mbar_arrive_cluster(map_leader(smem_u32(full + s)));
-            mbar_arrive(smem_u32(wempty + ws));
-          }
+          asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         }
-        turn ^= 1;
-        if (++s == p.nstages) { s = 0; ph ^= 1u; }
-        if (++ws == p.nslots) { ws = 0; wph ^= 1u; }
+        tmem_st16(at + (uint32_t)(c * WP * kACols), hi);
+        if (WP == 2) tmem_st16(at + (uint32_t)(c * WP * kACols + kACols), lo);
       }
+      asm volatile("tcgen05.wait::st.sync.aligned;\ntcgen05.fence::before_thread_sync;\n" ::: "memory");
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(smem_u32(full + s));
+        mbar_arrive(smem_u32(wempty + ws));
+      }
+      if ((s += kSets) >= p.nstages) { s -= p.nstages; ph ^= 1u; }
+      if ((ws += kSets) >= p.nslots) { ws -= p.nslots; wph ^= 1u; }
     }
     if (failed && lane == 0) atomicExch(p.status, 4);
   } else if (warp >= 4) {
     // ===== epilogue: warp = one quadrant of tensor-memory lanes =====================================
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
     const int quad = warp & 3;
-    int n = 0;
+    int buf = 0;
+    uint32_t acc_ph = 0;
     while (segs.next(p, sg)) {
       int mt, nt;
       tile_pos(p, sg.tile, mt, nt);
-      const int buf = n & 1, m0 = mt * p.bn, mcnt = min(p.bn, p.M - m0);
+      const int m0 = mt * p.bn, mcnt = min(p.bn, p.M - m0);
       const int row = quad * 32 + lane, wrow = nt * 256 + (int)rank * 128 + row;
-      if (!failed && !mbar_wait(smem_u32(acc_full + buf), ((uint32_t)n >> 1) & 1u)) failed = true;
+      if (!failed && !mbar_wait(smem_u32(acc_full + buf), acc_ph)) failed = true;
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-      const uint32_t tacc = tmem + (uint32_t)buf * 256u + ((uint32_t)(quad * 32) << 16);
+      const uint32_t tacc = tmem + (uint32_t)(buf * p.acc_cols) + ((uint32_t)(quad * 32) << 16);
       const bool whole = sg.k0 == 0 && sg.k1 == p.nk;
       float* mine = whole ? nullptr : partial(p, pair, sg.tile - p.dp_tiles, rank, row);
 #pragma unroll 1
@@ -349,7 +424,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
       asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(map_leader(smem_u32(acc_empty + buf)));
-      ++n;
+      if (++buf == p.nacc) { buf = 0; acc_ph ^= 1u; }
     }
     if (failed && lane == 0) atomicExch(p.status, 4);
   }
@@ -503,88 +578,86 @@ EncodeFn encode_fn() {
   return fn;
 }
 
-// Up to this many tokens two stages of two chunks, both operands in two terms, fit shared memory beside the packed ring of
-// every block format.  (8-bit blocks set it: 4-bit and K-quant blocks would fit up to 144 tokens, bf16 rows, which have one
-// term, up to 240 and more.)
-constexpr int64_t kWideStage = 112;
-
 // Tile width and split, by a cost model in cycles.  Per 64 k the MMAs take 2 * bn per product and the dequantisation a
-// fixed time, whichever is longer; tiles cut along K pay for their partials' way through L2 and a second launch.  The fixed
-// times are what its instructions take to issue.  The stages are slower than that, since the steps of a stage depend on
-// one another: 1320 cycles per 64 k of 4-bit blocks in two terms at 112 tokens, where the MMAs take 670; in one term 620
-// at 160 tokens (320) and 730 at 256 tokens (510).  The model orders plans; it does not predict their times.
-Plan make_plan(const qeng_ctx* ctx, const qeng_weight* w, int64_t M, int wp, int xp, bool may_split) {
+// fixed time, whichever is longer; tiles cut along K pay for their partials' way through L2 and a second launch.
+Plan make_plan(const qeng_ctx* ctx, const qeng_weight* w, int64_t M, int wp, int xp, int epi, bool may_split) {
   Plan best = {};
   double best_cost = 1e30;
-  const int pairs = ctx->sm_count / 2, kst = wp == 1 || M <= kWideStage ? 2 : 1, nk = (int)((w->nchunks + kst - 1) / kst);
-  const int n_tiles = (int)((w->N + 255) / 256), products = wp + xp - 1;
-  const double deq = kst * (w->fmt == QENG_FMT_Q4 ? (wp == 1 ? 330 : 450) : 700);
+  const int pairs = ctx->sm_count / 2, nk = (int)((w->nchunks + kST - 1) / kST);
+  const int n_tiles = (int)((w->N + 255) / 256), products = wp + xp - 1, a_cols = kST * wp * kACols;
+  const double deq = w->fmt == QENG_FMT_Q4 ? (wp == 1 ? 820 : 1250) : 1400;
+  const double per_token = epi == QENG_EPI_QKV ? 80 : epi == QENG_EPI_SWIGLU ? 50 : 20;  // of the epilogue
   const int lo = M <= 256 ? (int)((M + 15) / 16 * 16) : 128, hi = M <= 256 ? lo : 256;
   for (int bn = hi; bn >= lo; bn -= 16) {
     const int m_tiles = (int)((M + bn - 1) / bn), T = m_tiles * n_tiles;
-    const double mma = 2.0 * kst * (bn < 32 ? 32 : bn) * products, stage = mma > deq ? mma : deq;
+    // Tensor memory: two accumulators if three stages of weights fit beside them, else one.  (With two stages the MMAs wait
+    // for the refill: 192 columns, 86 stages: 63 us a tile against 55 with one accumulator and five stages.)
+    const int acc_cols = (bn + 31) / 32 * 32, nacc = 2 * acc_cols + 3 * a_cols <= 512 ? 2 : 1;
+    const double mma = 2.0 * kST * (bn < 32 ? 32 : bn) * products, stage = mma > deq ? mma : deq;
     const int waves = (T + pairs - 1) / pairs, rem = T % pairs;
-    const double dp = waves * nk * stage + 25.0 * bn;
-    const double sk = (T / pairs) * nk * stage + (double)rem * nk / pairs * stage + 50.0 * bn + 6000;
+    // the next tile hides an epilogue where there are two accumulators
+    const double ep = per_token * bn, tile = nacc == 1 ? nk * stage + ep : std::max(nk * stage, ep);
+    const double dp = waves * tile + (nacc == 1 ? 0.0 : ep);
+    const double sk = (T / pairs) * tile + (double)rem * nk / pairs * stage + 50.0 * bn + 6000;
     // shares of at least two stages (with no whole tiles the number of pairs is reduced instead, below)
     const bool cut = may_split && rem != 0 && sk < dp && (T < pairs || (int64_t)rem * nk >= 2 * (int64_t)pairs);
     const double cost = cut ? sk : dp;
     if (cost < best_cost) {
       best_cost = cost;
       best.bn = bn; best.m_tiles = m_tiles; best.n_tiles = n_tiles;
+      best.nacc = nacc; best.acc_cols = acc_cols;
       best.sk_tiles = cut ? rem : 0;
       best.dp_tiles = T - best.sk_tiles;
     }
   }
-  best.kst = kst;
   best.nk = nk;
   best.npairs = best.sk_tiles > 0 ? pairs : (best.dp_tiles < pairs ? best.dp_tiles : pairs);
   if (best.sk_tiles > 0 && best.dp_tiles == 0) {
     const int64_t units = (int64_t)best.sk_tiles * nk;
     if (units / 2 < best.npairs) best.npairs = units / 2 > 0 ? (int)(units / 2) : 1;
   }
-  // Operand stages first, but at least two slots of packed weights; what is left goes to the packed ring (few
-  // tokens: the weights come from HBM and want tens of KB in flight, and then a stage leaves room for it).
-  const size_t stage = (size_t)kst * (wp * kAPlane + xp * (best.bn / 2) * 128), slot = (size_t)slot_bytes_of(w->fmt, kst);
+  // As many stages as tensor memory holds of the weights and shared memory of the activations beside four slots of packed
+  // weights (never fewer than two); what is left goes to the packed ring (few tokens: the weights come from HBM and want
+  // tens of KB in flight, and then a stage leaves room for it).
+  const size_t stage = (size_t)kST * xp * (best.bn / 2) * 128, slot = (size_t)slot_bytes_of(w->fmt);
   const size_t room = kSmemBudget - 1024 - 1024;  // alignment, static shared memory
-  best.nstages = (int)((room - 2 * slot) / stage);
-  const int most = wp == 2 ? 4 : kMaxStages;
-  if (best.nstages > most) best.nstages = most;
+  best.nstages = (512 - best.nacc * best.acc_cols) / a_cols;
+  if (best.nstages > kMaxStages) best.nstages = kMaxStages;
+  if (best.nstages > (int)((room - 2 * kSets * slot) / stage)) best.nstages = (int)((room - 2 * kSets * slot) / stage);
   best.nslots = (int)((room - best.nstages * stage) / slot);
-  best.nslots = (best.nslots < kMaxSlots ? best.nslots : kMaxSlots) & ~1;  // a slot belongs to one dequant set
+  best.nslots = (best.nslots < kMaxSlots ? best.nslots : kMaxSlots) / kSets * kSets;  // a slot belongs to one dequant set
   best.box_rows = best.bn / 2;
   best.smem = best.nstages * stage + best.nslots * slot + 1024;
   best.ws_floats = best.sk_tiles > 0 ? (size_t)best.npairs * 4 * best.bn * 128 : 0;
   return best;
 }
 
-// tensor maps of the packed planes, boxes of kst chunks x 8 row tiles of 64-bit words; kept with the weight
+// tensor maps of the packed planes, boxes of kST chunks x 8 row tiles of 64-bit words; kept with the weight
 bool weight_maps(const qeng_weight* w) {
   std::lock_guard<std::mutex> hold(w->lock);
   if (w->tc_maps_ready) return true;
   EncodeFn enc = encode_fn();
-  for (int kst = 1; kst <= 2; ++kst)
-    for (int plane = 0; plane < 2; ++plane) {
-      const cuuint64_t words = (cuuint64_t)(plane == 0 ? chunk_w(w->fmt) : chunk_s(w->fmt)) / 8;
-      const cuuint64_t dims[3] = {words, (cuuint64_t)w->nchunks, (cuuint64_t)w->ntiles};
-      const cuuint64_t strides[2] = {words * 8, words * 8 * (cuuint64_t)w->nchunks};
-      const cuuint32_t box[3] = {(cuuint32_t)words, (cuuint32_t)kst, 8}, es[3] = {1, 1, 1};
-      void* base = plane == 0 ? reinterpret_cast<void*>(w->qs) : reinterpret_cast<void*>(w->sc);
-      if (enc(reinterpret_cast<CUtensorMap*>(w->tc_maps[kst - 1][plane]), CU_TENSOR_MAP_DATA_TYPE_UINT64, 3, base, dims, strides, box, es,
-              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-        return false;
-    }
+  for (int plane = 0; plane < 2; ++plane) {
+    const cuuint64_t words = (cuuint64_t)(plane == 0 ? chunk_w(w->fmt) : chunk_s(w->fmt)) / 8;
+    const cuuint64_t dims[3] = {words, (cuuint64_t)w->nchunks, (cuuint64_t)w->ntiles};
+    const cuuint64_t strides[2] = {words * 8, words * 8 * (cuuint64_t)w->nchunks};
+    const cuuint32_t box[3] = {(cuuint32_t)words, kST, 8}, es[3] = {1, 1, 1};
+    void* base = plane == 0 ? reinterpret_cast<void*>(w->qs) : reinterpret_cast<void*>(w->sc);
+    if (enc(reinterpret_cast<CUtensorMap*>(w->tc_maps[plane]), CU_TENSOR_MAP_DATA_TYPE_UINT64, 3, base, dims, strides, box, es,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+      return false;
+  }
   w->tc_maps_ready = true;
   return true;
 }
 
-template <int FMT, int WP, int XP, int KST>
+template <int FMT, int WP, int XP>
 int32_t launch(qeng_ctx* ctx, const qeng_weight* w, const TcParams& p, const Plan& pl, const CUtensorMap& map, cudaStream_t stream) {
   static bool configured_on[64] = {};  // the opt-in shared-memory size is set per device
   bool& configured = configured_on[ctx->device & 63];
   if (!configured) {
-    QENG_CUDA(ctx, cudaFuncSetAttribute(gemm_tc_kernel<FMT, WP, XP, KST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
+    QENG_CUDA(ctx, cudaFuncSetAttribute(gemm_tc_kernel<FMT, WP, XP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
     configured = true;
   }
   cudaLaunchConfig_t cfg = {};
@@ -597,9 +670,9 @@ int32_t launch(qeng_ctx* ctx, const qeng_weight* w, const TcParams& p, const Pla
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = ctx->pdl ? 1 : 0;
-  const CUtensorMap* wm = reinterpret_cast<const CUtensorMap*>(w->tc_maps[KST - 1][0]);
-  const CUtensorMap* sm = reinterpret_cast<const CUtensorMap*>(w->tc_maps[KST - 1][1]);
-  QENG_CUDA(ctx, cudaLaunchKernelEx(&cfg, gemm_tc_kernel<FMT, WP, XP, KST>, p, map, *wm, *sm));
+  const CUtensorMap* wm = reinterpret_cast<const CUtensorMap*>(w->tc_maps[0]);
+  const CUtensorMap* sm = reinterpret_cast<const CUtensorMap*>(w->tc_maps[1]);
+  QENG_CUDA(ctx, cudaLaunchKernelEx(&cfg, gemm_tc_kernel<FMT, WP, XP>, p, map, *wm, *sm));
   return p.sk_tiles > 0 ? reduce(ctx, p, stream) : QENG_OK;
 }
 
@@ -625,7 +698,7 @@ int32_t qeng_tc::prepare(qeng_ctx* ctx, const qeng_weight* w, const qeng_tc_x& x
     return qeng_fail(ctx, QENG_ERR_CUDA, "gemm_tc: tensor map rejected (M=%lld, K=%lld, ld=%lld)", (long long)M, (long long)w->K, (long long)x.ld);
   p->nk = pl->nk; p->M = (int)M; p->N = (int)w->N;
   p->bn = pl->bn; p->m_tiles = pl->m_tiles; p->n_tiles = pl->n_tiles; p->dp_tiles = pl->dp_tiles; p->sk_tiles = pl->sk_tiles;
-  p->nstages = pl->nstages; p->nslots = pl->nslots; p->npairs = pl->npairs; p->e = epi;
+  p->nstages = pl->nstages; p->nslots = pl->nslots; p->nacc = pl->nacc; p->acc_cols = pl->acc_cols; p->npairs = pl->npairs; p->e = epi;
   p->status = ctx->status;
   return QENG_OK;
 }
@@ -668,18 +741,18 @@ int32_t qeng_gemm_tc(qeng_ctx* ctx, const qeng_weight* w, const qeng_tc_x& x, in
   const int xp = x.planes;
   if (w->fmt != QENG_FMT_Q4 && wp == 1) return qeng_fail(ctx, QENG_ERR_SHAPE, "gemm_tc: single bf16 weights are for 4-bit blocks only");
   if (wp == 1 && xp != 1) return qeng_fail(ctx, QENG_ERR_ARG, "gemm_tc: two activation planes need two weight planes");
-  Plan pl = make_plan(ctx, w, M, wp, xp, true);
+  Plan pl = make_plan(ctx, w, M, wp, xp, epi.kind, true);
   TcParams p;
   CUtensorMap map;
   if (pl.sk_tiles > 0 && sc == nullptr) sc = qeng_scratch_for(ctx, stream);
   int32_t rc = prepare(ctx, w, x, M, epi, sc, &pl, &p, &map);
   if (rc == QENG_ERR_STATE) {  // no memory for the workspace: whole tiles only
-    pl = make_plan(ctx, w, M, wp, xp, false);
+    pl = make_plan(ctx, w, M, wp, xp, epi.kind, false);
     rc = prepare(ctx, w, x, M, epi, sc, &pl, &p, &map);
   }
   if (rc != QENG_OK) return rc;
-  if (wp == 1) return launch<QENG_FMT_Q4, 1, 1, 2>(ctx, w, p, pl, map, stream);
-#define QENG_TC(F, X) (pl.kst == 2 ? launch<F, 2, X, 2>(ctx, w, p, pl, map, stream) : launch<F, 2, X, 1>(ctx, w, p, pl, map, stream))
+  if (wp == 1) return launch<QENG_FMT_Q4, 1, 1>(ctx, w, p, pl, map, stream);
+#define QENG_TC(F, X) launch<F, 2, X>(ctx, w, p, pl, map, stream)
   switch (w->fmt) {
     case QENG_FMT_Q4: return xp == 1 ? QENG_TC(QENG_FMT_Q4, 1) : QENG_TC(QENG_FMT_Q4, 2);
     case QENG_FMT_Q8: return xp == 1 ? QENG_TC(QENG_FMT_Q8, 1) : QENG_TC(QENG_FMT_Q8, 2);

@@ -9,7 +9,8 @@
 namespace qeng_tc {
 
 constexpr int kBK = 64;                  // k per chunk: one 128-byte swizzled row of bf16
-constexpr int kAPlane = 128 * kBK * 2;   // 16 KB: this CTA's 128 weight rows of a chunk
+constexpr int kST = 2;                   // chunks per stage
+constexpr int kACols = kBK / 2;          // tensor-memory columns of one plane of a chunk of weights
 constexpr int kMaxStages = 8, kMaxSlots = 12;
 constexpr size_t kSmemBudget = 226 * 1024;
 
@@ -19,14 +20,15 @@ template <> struct Fmt<QENG_FMT_Q8> { static constexpr int kW = 1024, kS = 64; }
 template <> struct Fmt<QENG_FMT_K4> { static constexpr int kW = 512, kS = 256; };
 inline int chunk_w(int fmt) { return fmt == QENG_FMT_Q8 ? 1024 : 512; }
 inline int chunk_s(int fmt) { return fmt == QENG_FMT_K4 ? 256 : 64; }
-inline int slot_bytes_of(int fmt, int kst) { return kst * 8 * (chunk_w(fmt) + chunk_s(fmt)); }
+inline int slot_bytes_of(int fmt) { return kST * 8 * (chunk_w(fmt) + chunk_s(fmt)); }
 
 struct TcParams {
-  int nk;                    // stages of KST chunks along K
+  int nk;                    // stages of kST chunks along K
   int M, N;
   int bn, m_tiles, n_tiles;  // tokens per tile, token tiles, 256-row weight tiles
   int dp_tiles, sk_tiles;    // whole tiles (round-robin), tiles cut along K
-  int nstages, nslots;       // rings: operand tiles, packed weights
+  int nstages, nslots;       // rings: operands (weights in tensor memory, activations in shared memory), packed weights
+  int nacc, acc_cols;        // accumulators (1 or 2), tensor-memory columns of each
   qeng_tc_epi e;
   int npairs;
   float* ws;                 // stream-K partials: [pair][2][CTA of the pair][bn][128]
@@ -77,6 +79,10 @@ __device__ __forceinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity) {
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
   return mbar_try_wait(bar, parity) || mbar_wait_slow(bar, parity);
 }
+// The same for a converged warp; all lanes learn the outcome by vote, so that what follows stays warp-uniform.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) {
+  return __all_sync(0xffffffffu, mbar_try_wait(bar, parity)) || __all_sync(0xffffffffu, mbar_wait_slow(bar, parity));
+}
 // one box of a packed plane: `box` chunks x 8 row tiles (beyond the matrix: zeros)
 __device__ __forceinline__ void tma_w(uint32_t dst, const CUtensorMap* map, int chunk, int tile, uint32_t bar) {
   asm volatile(
@@ -105,11 +111,20 @@ __device__ __forceinline__ uint64_t make_desc(uint32_t saddr) {
   d |= (uint64_t)2 << 61;                   // 128-byte swizzle
   return d;
 }
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
+// A from tensor memory (each CTA's 128 rows in its own), B from both CTAs' shared memory
+__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
   asm volatile(
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc)
+      " tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(tmem_d),
+      "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(acc)
+      : "memory");
+}
+// 16 lanes x 32 columns; a lane's registers 4i, 4i + 1: row g, columns 8i + 2t and the next; 4i + 2, 4i + 3: row g + 8
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.16x256b.x4.b32 [%16], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};\n" ::"r"(v[0]), "r"(v[1]),
+      "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]),
+      "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(taddr)
       : "memory");
 }
 // arrives at the barrier at this offset in both CTAs once the MMAs issued so far have finished
@@ -148,9 +163,6 @@ __device__ __forceinline__ uint2 lds64(uint32_t a) {
   asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];\n" : "=r"(v.x), "=r"(v.y) : "r"(a) : "memory");
   return v;
 }
-__device__ __forceinline__ void sts128(uint32_t a, const uint32_t (&o)[4]) {
-  asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};\n" ::"r"(a), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
-}
 
 // ---- the sequence of (tile, K range) segments of one CTA pair; every role walks the same one ----------
 struct Seg {
@@ -162,6 +174,9 @@ struct Segments {
     const long long U = (long long)p.sk_tiles * p.nk;
     u = (int)(U * pair / npairs);
     u1 = (int)(U * (pair + 1) / npairs);
+  }
+  __device__ int stages(const TcParams& p) const {  // of all segments still to come
+    return (next_dp < p.dp_tiles ? (p.dp_tiles - next_dp + npairs - 1) / npairs * p.nk : 0) + (u1 - u);
   }
   __device__ bool next(const TcParams& p, Seg& s) {
     if (next_dp < p.dp_tiles) {
@@ -240,49 +255,88 @@ __device__ __forceinline__ void finish(const qeng_tc_epi& e, int N, int32_t* sta
   // SWIGLU and QKV combine rows r and r + 8 of a 16-row tile: lanes with bit 3 clear take the even tokens, the others
   // the odd ones, so one exchange per token pair keeps every lane busy
   const int odd = (lane >> 3) & 1, r = lane & 7, tile = n >> 4;
+  if (e.kind == QENG_EPI_SWIGLU) {
 #pragma unroll
-  for (int i = 0; i < NT; i += 2) {
-    const float got = __shfl_xor_sync(0xffffffffu, odd ? v[i] : v[i + 1], 8);
-    const float a = odd ? got : v[i], b = odd ? v[i + 1] : got;  // rows r and r + 8
-    const int t = i + odd, m = m0 + t;
-    if (t >= cnt || n >= N) continue;
-    if (e.kind == QENG_EPI_SWIGLU) {
+    for (int i = 0; i < NT; i += 2) {
+      const float got = __shfl_xor_sync(0xffffffffu, odd ? v[i] : v[i + 1], 8);
+      const float a = odd ? got : v[i], b = odd ? v[i + 1] : got;  // rows r and r + 8
+      const int t = i + odd, m = m0 + t;
+      if (t >= cnt || n >= N) continue;
       const float f = a / (1.0f + __expf(-a)) * b;
       if (e.yb != nullptr) st_planes(e, (size_t)m * e.ldyb + (size_t)tile * 8 + r, f);
       else e.y[(size_t)m * e.ldy + (size_t)tile * 8 + r] = f;
-    } else {
-      const qeng_qkv_epi& q = e.qkv;
-      const int head = tile >> 3, d = ((tile & 7) << 3) + r, ps = q.pos[m];
-      if (ps < 0 || ps >= q.max_seq || (ps >> 4) >= q.max_pages) {
-        atomicExch(status, 2);
-        continue;
-      }
-      float lo = a, hi = b;
-      if (head < q.Hq + q.Hkv) {
-        const float c = q.cs[(size_t)ps * 128 + d], sn = q.cs[(size_t)ps * 128 + 64 + d];
-        lo = a * c - b * sn;
-        hi = b * c + a * sn;
-      }
-      __half* dst;
-      if (head < q.Hq) {
-        dst = q.q16 + ((size_t)m * q.Hq + head) * 128 + d;
-      } else {
-        const int pid = q.table[(size_t)(m / q.rows_per_seq) * q.max_pages + (ps >> 4)];
-        if ((unsigned)pid >= (unsigned)q.pages) {
-          atomicExch(status, 1);
-          continue;
-        }
-        const int kh = head - q.Hq, isv = kh >= q.Hkv ? 1 : 0;
-        dst = q.pool + (((size_t)pid * q.Hkv + (kh - isv * q.Hkv)) * 2 + isv) * (16 * 128) + (ps & 15) * 128 + d;
-      }
-      dst[0] = __float2half_rn(lo);
-      dst[64] = __float2half_rn(hi);
     }
+    return;
+  }
+  // QKV: the loads of all tokens (positions, then angles, then pages) are issued together: one after the other they were
+  // three trips to L2 per token pair, and the epilogue of 1800 rows took twice as long as its matmul.
+  const qeng_qkv_epi& q = e.qkv;
+  const int head = tile >> 3, d = ((tile & 7) << 3) + r;
+  constexpr int kP = NT / 2;
+  int ps[kP];
+#pragma unroll
+  for (int i = 0; i < kP; ++i) ps[i] = 2 * i + odd < cnt && n < N ? q.pos[m0 + 2 * i + odd] : 0;
+  float lo[kP], hi[kP];
+#pragma unroll
+  for (int i = 0; i < kP; ++i) {
+    const float got = __shfl_xor_sync(0xffffffffu, odd ? v[2 * i] : v[2 * i + 1], 8);
+    lo[i] = odd ? got : v[2 * i];
+    hi[i] = odd ? v[2 * i + 1] : got;
+  }
+  bool ok[kP];
+#pragma unroll
+  for (int i = 0; i < kP; ++i) {
+    ok[i] = 2 * i + odd < cnt && n < N;
+    if (ok[i] && (ps[i] < 0 || ps[i] >= q.max_seq || (ps[i] >> 4) >= q.max_pages)) {
+      atomicExch(status, 2);
+      ok[i] = false;
+    }
+    if (!ok[i]) ps[i] = 0;
+  }
+  if (head < q.Hq + q.Hkv) {
+    float c[kP], sn[kP];
+#pragma unroll
+    for (int i = 0; i < kP; ++i) {
+      c[i] = __ldg(q.cs + (size_t)ps[i] * 128 + d);
+      sn[i] = __ldg(q.cs + (size_t)ps[i] * 128 + 64 + d);
+    }
+#pragma unroll
+    for (int i = 0; i < kP; ++i) {
+      const float a = lo[i], b = hi[i];
+      lo[i] = a * c[i] - b * sn[i];
+      hi[i] = b * c[i] + a * sn[i];
+    }
+  }
+  if (head < q.Hq) {
+    __half* dst = q.q16 + ((size_t)(m0 + odd) * q.Hq + head) * 128 + d;
+#pragma unroll
+    for (int i = 0; i < kP; ++i) {
+      if (!ok[i]) continue;
+      dst[(size_t)(2 * i) * q.Hq * 128] = __float2half_rn(lo[i]);
+      dst[(size_t)(2 * i) * q.Hq * 128 + 64] = __float2half_rn(hi[i]);
+    }
+    return;
+  }
+  const int kh = head - q.Hq, isv = kh >= q.Hkv ? 1 : 0;
+  int pid[kP];
+#pragma unroll
+  for (int i = 0; i < kP; ++i)
+    pid[i] = ok[i] ? q.table[(size_t)((m0 + 2 * i + odd) / q.rows_per_seq) * q.max_pages + (ps[i] >> 4)] : 0;
+#pragma unroll
+  for (int i = 0; i < kP; ++i) {
+    if (!ok[i]) continue;
+    if ((unsigned)pid[i] >= (unsigned)q.pages) {
+      atomicExch(status, 1);
+      continue;
+    }
+    __half* dst = q.pool + (((size_t)pid[i] * q.Hkv + (kh - isv * q.Hkv)) * 2 + isv) * (16 * 128) + (ps[i] & 15) * 128 + d;
+    dst[0] = __float2half_rn(lo[i]);
+    dst[64] = __float2half_rn(hi[i]);
   }
 }
 
 struct Plan {
-  int kst, nk, bn, m_tiles, n_tiles, dp_tiles, sk_tiles, npairs, nstages, nslots;
+  int nk, bn, m_tiles, n_tiles, dp_tiles, sk_tiles, npairs, nstages, nslots, nacc, acc_cols;
   int box_rows;  // rows of an activation box
   size_t smem, ws_floats;
 };

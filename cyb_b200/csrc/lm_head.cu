@@ -24,6 +24,7 @@ using namespace qeng_tc;
 constexpr int kM = 16, kCols = 3 * kM;   // rows per launch, their three planes
 constexpr int kEpi = 8, kConv = 4, kThreadsL = (2 + kEpi + kConv) * 32;
 constexpr int kMaxStagesL = 24;
+constexpr int kTilePlane = 128 * kBK * 2;  // 128 table rows of a chunk
 constexpr size_t kHeadSmem = kSmemBudget - 4096;  // dynamic; the static arrays take the rest
 constexpr uint32_t kBBytes = kCols * 128u;
 
@@ -119,7 +120,7 @@ __global__ void __launch_bounds__(kThreadsL, 1) lm_head_kernel(const HeadParams 
           for (int k = 0; k < kBK / 16; ++k) {
             const uint32_t acc = k > 0 ? 1u : 0u;
             umma1(d, ad + 2 * k, bd + 2 * k, idesc, acc);
-            if (groups > 1) umma1(d + 64u, ad + (kAPlane >> 4) + 2 * k, bd + 2 * k, idesc, acc);
+            if (groups > 1) umma1(d + 64u, ad + (kTilePlane >> 4) + 2 * k, bd + 2 * k, idesc, acc);
           }
           commit1(smem_u32(empty + s));
           commit1(smem_u32(acc_full + buf));

@@ -47,6 +47,24 @@ def test_rows_and_widths(ctx, fmt, m):
     ctx.device_status()
 
 
+# One-term operands: the smallest and largest token tiles with two accumulators and with one, remainders of both, tiles cut
+# along K and whole ones, more tiles than CTA pairs.  Against operands rounded to bf16, only the sums differ: bound as above.
+@pytest.mark.parametrize("m,n,k", [(256, 272, 736), (257, 4096, 992), (320, 1040, 4096), (416, 4112, 2048), (777, 2064, 4064), (2049, 4096, 544)])
+def test_prompt_rows_and_widths(ctx, m, n, k):
+    import torch
+    w = _weight(ctx, "q4", n, k)
+    wd = w.dequant().bfloat16().double()
+    for dt in DT[:2]:
+        x = torch.randn(m, k, device="cuda").to(getattr(torch, dt))
+        y = torch.full((m, n + 8), 0.25, device="cuda")[:, :n]
+        acc = m % 2
+        ctx.gemm_q4(w, x, out=y, flags=acc)
+        want = x.bfloat16().double() @ wd.T + (0.25 if acc else 0.0)
+        err = float((y.double() - want).abs().max() / want.abs().max())
+        assert err < 3e-5, (m, n, k, dt, err)
+    ctx.device_status()
+
+
 # Query heads per kv head: one, the most there are, and counts that do not divide the 64 rows of a prompt attention tile
 # (its last rows stay empty); tiles then hold 64, 8, 21, 12, 10 and 9 tokens.
 @pytest.mark.parametrize("heads,kv_heads", [(2, 2), (8, 1), (6, 2), (5, 1), (6, 1), (7, 1)])

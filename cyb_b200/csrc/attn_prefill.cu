@@ -9,9 +9,9 @@
 // lost there.  Three CTAs per SM.
 //
 // Least time: 24 MMAs of 2 cycles per 16 x 8 scores (8 for the scores, 16 for the values); 2 * 128 * 3 * heads * T^2 / 2
-// operations for a prompt of T tokens = 73 us per layer at T = 1800 and 32 heads.  It takes 205 to 230 there (ncu): the
-// tensor pipe is busy 53 % of the cycles in which an SM has work (dependent steps of the softmax between the two products,
-// 12 consumer warps per SM), and an SM has work 65 % of the time (904 CTAs of very unequal length on 444 places).
+// operations for a prompt of T tokens = 73 us per layer at T = 1800 and 32 heads.  It takes 148 there (ncu; 212 with the
+// CTAs in head order): the tensor pipe is busy 53 % of the cycles in which an SM has work (dependent steps of the softmax
+// between the two products, 12 consumer warps per SM).
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <math.h>
@@ -118,7 +118,10 @@ __global__ void __launch_bounds__(kThreads, 3) attn_prefill_kernel(const qeng_pr
   __shared__ volatile int gave_up;  // a consumer stopped waiting: nobody waits for the producer's copies any more
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int grp = p.Hq / p.Hkv, tpt = kRows / grp;             // tokens per tile
-  const int b = blockIdx.z, h = blockIdx.y, tt0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * tpt;  // long tiles first
+  // long tiles first, of all heads and sequences together: head after head, the long tiles of the last heads started late
+  // and an SM had work 65 % of the time
+  const int hb = blockIdx.x % (unsigned)(p.Hkv * p.B), b = hb / p.Hkv, h = hb - b * p.Hkv;
+  const int tt0 = (int)((gridDim.x - 1 - blockIdx.x) / (unsigned)(p.Hkv * p.B)) * tpt;
   const int ntok = min(tpt, p.T - tt0);
 
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
@@ -393,7 +396,7 @@ int32_t qeng_attn_prefill(qeng_ctx* ctx, const qeng_prefill_attn& p, const void*
   }
   const int tpt = kRows / (p.Hq / p.Hkv);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)((p.T + tpt - 1) / tpt), (unsigned)p.Hkv, (unsigned)p.B);
+  cfg.gridDim = dim3((unsigned)((p.T + tpt - 1) / tpt * p.Hkv * p.B));
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = kSmem;
   cfg.stream = stream;

@@ -586,7 +586,7 @@ Plan make_plan(const qeng_ctx* ctx, const qeng_weight* w, int64_t M, int wp, int
   const int pairs = ctx->sm_count / 2, nk = (int)((w->nchunks + kST - 1) / kST);
   const int n_tiles = (int)((w->N + 255) / 256), products = wp + xp - 1, a_cols = kST * wp * kACols;
   const double deq = w->fmt == QENG_FMT_Q4 ? (wp == 1 ? 820 : 1250) : 1400;
-  const double per_token = epi == QENG_EPI_QKV ? 80 : epi == QENG_EPI_SWIGLU ? 50 : 20;  // of the epilogue
+  const double per_token = epi == QENG_EPI_QKV ? 80 : epi == QENG_EPI_SWIGLU ? 60 : 20;  // of the epilogue
   const int lo = M <= 256 ? (int)((M + 15) / 16 * 16) : 128, hi = M <= 256 ? lo : 256;
   for (int bn = hi; bn >= lo; bn -= 16) {
     const int m_tiles = (int)((M + bn - 1) / bn), T = m_tiles * n_tiles;

@@ -224,11 +224,6 @@ __device__ __forceinline__ uint32_t u32(__nv_bfloat162 v) { return *reinterpret_
 
 // ---- epilogue of up to NT (8 or 16) tokens of this lane's weight row -------------------------------------------------
 // n = weight row of this lane (rows of a warp are 32 consecutive ones, so whole 16-row tiles); v[i] = sum of token m0 + i
-__device__ __forceinline__ void st_planes(const qeng_tc_epi& e, size_t at, float f) {
-  const __nv_bfloat16 h = __float2bfloat16_rn(f);
-  e.yb[at] = h;
-  if (e.yb_planes == 2) e.yb[at + e.yb_plane] = __float2bfloat16_rn(f - __bfloat162float(h));
-}
 template <int NT>
 __device__ __forceinline__ void finish(const qeng_tc_epi& e, int N, int32_t* status, int n, int m0, int cnt, const float (&v)[NT], int lane) {
   if (e.kind == QENG_EPI_STORE || e.kind == QENG_EPI_ACCUM) {
@@ -255,16 +250,38 @@ __device__ __forceinline__ void finish(const qeng_tc_epi& e, int N, int32_t* sta
   // SWIGLU and QKV combine rows r and r + 8 of a 16-row tile: lanes with bit 3 clear take the even tokens, the others
   // the odd ones, so one exchange per token pair keeps every lane busy
   const int odd = (lane >> 3) & 1, r = lane & 7, tile = n >> 4;
-  if (e.kind == QENG_EPI_SWIGLU) {
+  constexpr int kP = NT / 2;
+  float lo[kP], hi[kP];  // rows r and r + 8 of token 2 i + odd
 #pragma unroll
-    for (int i = 0; i < NT; i += 2) {
-      const float got = __shfl_xor_sync(0xffffffffu, odd ? v[i] : v[i + 1], 8);
-      const float a = odd ? got : v[i], b = odd ? v[i + 1] : got;  // rows r and r + 8
-      const int t = i + odd, m = m0 + t;
-      if (t >= cnt || n >= N) continue;
-      const float f = a / (1.0f + __expf(-a)) * b;
-      if (e.yb != nullptr) st_planes(e, (size_t)m * e.ldyb + (size_t)tile * 8 + r, f);
-      else e.y[(size_t)m * e.ldy + (size_t)tile * 8 + r] = f;
+  for (int i = 0; i < kP; ++i) {
+    const float got = __shfl_xor_sync(0xffffffffu, odd ? v[2 * i] : v[2 * i + 1], 8);
+    lo[i] = odd ? got : v[2 * i];
+    hi[i] = odd ? v[2 * i + 1] : got;
+  }
+  if (e.kind == QENG_EPI_SWIGLU) {
+    // each step for all tokens before the next: token after token, with a branch for each, the chain of exchange, exponential,
+    // division and stores took 4500 cycles per 16 tokens, more than the matmul of the next tile hides
+    float den[kP];
+#pragma unroll
+    for (int i = 0; i < kP; ++i) den[i] = 1.0f + __expf(-lo[i]);
+#pragma unroll
+    for (int i = 0; i < kP; ++i) lo[i] = lo[i] / den[i] * hi[i];
+    if (n >= N) return;
+    if (e.yb != nullptr) {
+      __nv_bfloat16* dst = e.yb + (size_t)(m0 + odd) * e.ldyb + (size_t)tile * 8 + r;
+#pragma unroll
+      for (int i = 0; i < kP; ++i) {
+        const __nv_bfloat16 h = __float2bfloat16_rn(lo[i]);
+        if (2 * i + odd < cnt) {
+          dst[(size_t)(2 * i) * e.ldyb] = h;
+          if (e.yb_planes == 2) dst[(size_t)(2 * i) * e.ldyb + e.yb_plane] = __float2bfloat16_rn(lo[i] - __bfloat162float(h));
+        }
+      }
+    } else {
+      float* dst = e.y + (size_t)(m0 + odd) * e.ldy + (size_t)tile * 8 + r;
+#pragma unroll
+      for (int i = 0; i < kP; ++i)
+        if (2 * i + odd < cnt) dst[(size_t)(2 * i) * e.ldy] = lo[i];
     }
     return;
   }
@@ -272,17 +289,9 @@ __device__ __forceinline__ void finish(const qeng_tc_epi& e, int N, int32_t* sta
   // three trips to L2 per token pair, and the epilogue of 1800 rows took twice as long as its matmul.
   const qeng_qkv_epi& q = e.qkv;
   const int head = tile >> 3, d = ((tile & 7) << 3) + r;
-  constexpr int kP = NT / 2;
   int ps[kP];
 #pragma unroll
   for (int i = 0; i < kP; ++i) ps[i] = 2 * i + odd < cnt && n < N ? q.pos[m0 + 2 * i + odd] : 0;
-  float lo[kP], hi[kP];
-#pragma unroll
-  for (int i = 0; i < kP; ++i) {
-    const float got = __shfl_xor_sync(0xffffffffu, odd ? v[2 * i] : v[2 * i + 1], 8);
-    lo[i] = odd ? got : v[2 * i];
-    hi[i] = odd ? v[2 * i + 1] : got;
-  }
   bool ok[kP];
 #pragma unroll
   for (int i = 0; i < kP; ++i) {

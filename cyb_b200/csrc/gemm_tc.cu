@@ -20,7 +20,7 @@
 //               tensor memory holds two accumulators (up to 160 columns with one weight term)
 //   warps 8-23  dequantisation: packed words -> bf16 -> tensor memory; one warp per 16-row tile, two sets
 //               of 8 that take alternate stages
-// A stage is two chunks of 64 k, with one barrier each way: a hop between the roles costs 100 to 200 cycles
+// A stage is two chunks of 64 k (KST; one for more than 128 columns in two weight terms), with one barrier each way: a hop between the roles costs 100 to 200 cycles
 // of dependent instructions, and with one barrier per chunk the hops of a stage took longer than its MMAs.
 // The weights used to pass through shared memory, which then carried 1.3 times what it can in the time of
 // the MMAs: cycles per 128 k and one term, shared / tensor memory: 1460 / 1024 at 256 columns (the MMAs:
@@ -184,12 +184,12 @@ struct Words<QENG_FMT_Q8> {
   }
 };
 
-template <int FMT, int WP, int XP>
+template <int FMT, int WP, int XP, int KST>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     gemm_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap,
                    const __grid_constant__ CUtensorMap smap) {
   constexpr int kW = Fmt<FMT>::kW, kS = Fmt<FMT>::kS;
-  constexpr uint32_t kSlot = kST * 8 * (kW + kS), kStageCols = kST * WP * kACols;
+  constexpr uint32_t kSlot = KST * 8 * (kW + kS), kStageCols = KST * WP * kACols;
   extern __shared__ unsigned char smem_raw[];
   // the swizzle pattern is a function of the address: tiles start on 1024-byte boundaries (the same offset in both CTAs)
   const uint32_t smem = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -201,7 +201,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   asm volatile("mov.u32 %0, %cluster_ctarank;\n" : "=r"(rank));
   const int pair = blockIdx.x >> 1;
   const uint32_t b_plane = (uint32_t)(p.bn >> 1) * 128u;
-  const uint32_t stage_bytes = kST * XP * b_plane;                 // activations: [kST][XP] planes
+  const uint32_t stage_bytes = KST * XP * b_plane;                 // activations: [KST][XP] planes
   const uint32_t ring = smem + (uint32_t)p.nstages * stage_bytes;  // packed-weight slots
 
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
@@ -258,7 +258,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             const uint32_t a = ta + (uint32_t)s * kStageCols;
             const uint64_t bd = make_desc(base + (uint32_t)s * stage_bytes);
 #pragma unroll
-            for (int c = 0; c < kST; ++c) {
+            for (int c = 0; c < KST; ++c) {
 #pragma unroll
               for (int k = 0; k < kBK / 16; ++k) {  // a K step of 16: 8 columns of A; descriptors count 16-byte units
                 const uint32_t ac = a + c * WP * kACols + 8 * k;
@@ -318,9 +318,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
           if (rank == 0) mbar_expect_tx(smem_u32(full + s), 2 * stage_bytes);
           const uint32_t b = smem + (uint32_t)s * stage_bytes, bar = map_leader(smem_u32(full + s));
 #pragma unroll
-          for (int c = 0; c < kST; ++c)
+          for (int c = 0; c < KST; ++c)
 #pragma unroll
-            for (int pl = 0; pl < XP; ++pl) tma_x(b + (uint32_t)(c * XP + pl) * b_plane, &xmap, (kt * kST + c) * kBK, m0, pl, bar);
+            for (int pl = 0; pl < XP; ++pl) tma_x(b + (uint32_t)(c * XP + pl) * b_plane, &xmap, (kt * KST + c) * kBK, m0, pl, bar);
         }
         __syncwarp();
         if (++s == p.nstages) { s = 0; ph ^= 1u; }
@@ -340,8 +340,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         if (elect_one()) {
           const uint32_t bar = smem_u32(wfull + s), dst = ring + (uint32_t)s * kSlot;
           mbar_expect_tx(bar, kSlot);
-          tma_w(dst, &wmap, kt * kST, nt * 16 + (int)rank * 8, bar);
-          tma_w(dst + kST * 8 * kW, &smap, kt * kST, nt * 16 + (int)rank * 8, bar);
+          tma_w(dst, &wmap, kt * KST, nt * 16 + (int)rank * 8, bar);
+          tma_w(dst + KST * 8 * kW, &smap, kt * KST, nt * 16 + (int)rank * 8, bar);
         }
         __syncwarp();
         if (++s == p.nslots) { s = 0; ph ^= 1u; }
@@ -353,7 +353,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     // (whose tensor-memory lanes lie in the quadrant that this warp may write, warp % 4)
     const int set = (warp - 8) >> 3, rt = (warp & 3) * 2 + ((warp >> 2) & 1);
     const uint32_t dst0 = tmem_a + ((uint32_t)(rt * 16) << 16);
-    const uint32_t wb0 = ring + (uint32_t)rt * (kST * kW), sb0 = ring + 8u * kST * kW + (uint32_t)rt * (kST * kS);
+    const uint32_t wb0 = ring + (uint32_t)rt * (KST * kW), sb0 = ring + 8u * KST * kW + (uint32_t)rt * (KST * kS);
     const uint32_t mask = in_register(0x000f000fu), base = in_register(0x43004300u);
     const int total = segs.stages(p);
     // Whoever waits on a barrier by parity has to see all of its phases (boxes may land out of order: a set that skipped
@@ -365,11 +365,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     for (int i = set; i < total; i += kSets) {
       if (!failed && !mbar_wait(smem_u32(wfull + ws), wph)) failed = true;
       const uint32_t wb = wb0 + (uint32_t)ws * kSlot, sb = sb0 + (uint32_t)ws * kSlot, at = dst0 + (uint32_t)s * kStageCols;
-      Words<FMT> w[kST];
+      Words<FMT> w[KST];
 #pragma unroll
-      for (int c = 0; c < kST; ++c) w[c].load(wb + (uint32_t)(c * kW), sb + (uint32_t)(c * kS), lane);
+      for (int c = 0; c < KST; ++c) w[c].load(wb + (uint32_t)(c * kW), sb + (uint32_t)(c * kS), lane);
 #pragma unroll
-      for (int c = 0; c < kST; ++c) {
+      for (int c = 0; c < KST; ++c) {
         uint32_t hi[16], lo[16];
         w[c].template dequant<WP>(lane, mask, base, hi, lo);
         if (c == 0) {
@@ -606,9 +606,13 @@ EncodeFn encode_fn() {
 Plan make_plan(const qeng_ctx* ctx, const qeng_weight* w, int64_t M, int wp, int xp, int epi, bool may_split) {
   Plan best = {};
   double best_cost = 1e30;
-  const int pairs = ctx->sm_count / 2, nk = (int)((w->nchunks + kST - 1) / kST);
-  const int n_tiles = (int)((w->N + 255) / 256), products = wp + xp - 1, a_cols = kST * wp * kACols;
-  const double deq = w->fmt == QENG_FMT_Q4 ? (wp == 1 ? 820 : 1250) : 1400;
+  // two weight terms of two chunks are 128 columns of tensor memory, of which only two stages fit beside an accumulator of more
+  // than 128: then stages of one chunk (8-bit blocks, 144 rows f32 over 11008 x 4096: 41.7 us, so 37.9)
+  const int kst = wp == 2 && M > 128 ? 1 : 2;
+  const int pairs = ctx->sm_count / 2, nk = (int)((w->nchunks + kst - 1) / kst);
+  const int n_tiles = (int)((w->N + 255) / 256), products = wp + xp - 1, a_cols = kst * wp * kACols;
+  // measured: the dequantisation of 64 k where it, not the MMAs, sets the pace
+  const double deq = kst * (w->fmt == QENG_FMT_Q4 ? (wp == 1 ? 410 : 625) : 700);
   const double per_token = epi == QENG_EPI_QKV ? 80 : epi == QENG_EPI_SWIGLU ? 60 : 20;  // of the epilogue
   const int lo = M <= 256 ? (int)((M + 15) / 16 * 16) : 128, hi = M <= 256 ? lo : 256;
   for (int bn = hi; bn >= lo; bn -= 16) {
@@ -616,7 +620,7 @@ Plan make_plan(const qeng_ctx* ctx, const qeng_weight* w, int64_t M, int wp, int
     // Tensor memory: two accumulators if three stages of weights fit beside them, else one.  (With two stages the MMAs wait
     // for the refill: 192 columns, 86 stages: 63 us a tile against 55 with one accumulator and five stages.)
     const int acc_cols = (bn + 31) / 32 * 32, nacc = 2 * acc_cols + 3 * a_cols <= 512 ? 2 : 1;
-    const double mma = 2.0 * kST * (bn < 32 ? 32 : bn) * products, stage = mma > deq ? mma : deq;
+    const double mma = 2.0 * kst * (bn < 32 ? 32 : bn) * products, stage = mma > deq ? mma : deq;
     const int waves = (T + pairs - 1) / pairs, rem = T % pairs;
     // the next tile hides an epilogue where there are two accumulators
     const double ep = per_token * bn, tile = nacc == 1 ? nk * stage + ep : std::max(nk * stage, ep);
@@ -633,6 +637,7 @@ Plan make_plan(const qeng_ctx* ctx, const qeng_weight* w, int64_t M, int wp, int
       best.dp_tiles = T - best.sk_tiles;
     }
   }
+  best.kst = kst;
   best.nk = nk;
   best.npairs = best.sk_tiles > 0 ? pairs : (best.dp_tiles < pairs ? best.dp_tiles : pairs);
   if (best.sk_tiles > 0 && best.dp_tiles == 0) {
@@ -642,7 +647,7 @@ Plan make_plan(const qeng_ctx* ctx, const qeng_weight* w, int64_t M, int wp, int
   // As many stages as tensor memory holds of the weights and shared memory of the activations beside four slots of packed
   // weights (never fewer than two); what is left goes to the packed ring (few tokens: the weights come from HBM and want
   // tens of KB in flight, and then a stage leaves room for it).
-  const size_t stage = (size_t)kST * xp * (best.bn / 2) * 128, slot = (size_t)slot_bytes_of(w->fmt);
+  const size_t stage = (size_t)kst * xp * (best.bn / 2) * 128, slot = (size_t)slot_bytes_of(w->fmt, kst);
   size_t room = kSmemBudget - 1024 - 1024;  // alignment, static shared memory
   // the old values of y where two stages fit beside them (8-bit blocks, two planes of more than 224 tokens: they do not)
   const size_t old = epi == QENG_EPI_ACCUM && room >= kOldBytes + 4 * slot + 2 * stage ? (size_t)kOldBytes : 0;
@@ -659,32 +664,33 @@ Plan make_plan(const qeng_ctx* ctx, const qeng_weight* w, int64_t M, int wp, int
   return best;
 }
 
-// tensor maps of the packed planes, boxes of kST chunks x 8 row tiles of 64-bit words; kept with the weight
+// tensor maps of the packed planes, boxes of kst chunks x 8 row tiles of 64-bit words; kept with the weight
 bool weight_maps(const qeng_weight* w) {
   std::lock_guard<std::mutex> hold(w->lock);
   if (w->tc_maps_ready) return true;
   EncodeFn enc = encode_fn();
-  for (int plane = 0; plane < 2; ++plane) {
-    const cuuint64_t words = (cuuint64_t)(plane == 0 ? chunk_w(w->fmt) : chunk_s(w->fmt)) / 8;
-    const cuuint64_t dims[3] = {words, (cuuint64_t)w->nchunks, (cuuint64_t)w->ntiles};
-    const cuuint64_t strides[2] = {words * 8, words * 8 * (cuuint64_t)w->nchunks};
-    const cuuint32_t box[3] = {(cuuint32_t)words, kST, 8}, es[3] = {1, 1, 1};
-    void* base = plane == 0 ? reinterpret_cast<void*>(w->qs) : reinterpret_cast<void*>(w->sc);
-    if (enc(reinterpret_cast<CUtensorMap*>(w->tc_maps[plane]), CU_TENSOR_MAP_DATA_TYPE_UINT64, 3, base, dims, strides, box, es,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-      return false;
-  }
+  for (int kst = 1; kst <= 2; ++kst)
+    for (int plane = 0; plane < 2; ++plane) {
+      const cuuint64_t words = (cuuint64_t)(plane == 0 ? chunk_w(w->fmt) : chunk_s(w->fmt)) / 8;
+      const cuuint64_t dims[3] = {words, (cuuint64_t)w->nchunks, (cuuint64_t)w->ntiles};
+      const cuuint64_t strides[2] = {words * 8, words * 8 * (cuuint64_t)w->nchunks};
+      const cuuint32_t box[3] = {(cuuint32_t)words, (cuuint32_t)kst, 8}, es[3] = {1, 1, 1};
+      void* base = plane == 0 ? reinterpret_cast<void*>(w->qs) : reinterpret_cast<void*>(w->sc);
+      if (enc(reinterpret_cast<CUtensorMap*>(w->tc_maps[kst - 1][plane]), CU_TENSOR_MAP_DATA_TYPE_UINT64, 3, base, dims, strides, box, es,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return false;
+    }
   w->tc_maps_ready = true;
   return true;
 }
 
-template <int FMT, int WP, int XP>
+template <int FMT, int WP, int XP, int KST>
 int32_t launch(qeng_ctx* ctx, const qeng_weight* w, const TcParams& p, const Plan& pl, const CUtensorMap& map, cudaStream_t stream) {
   static bool configured_on[64] = {};  // the opt-in shared-memory size is set per device
   bool& configured = configured_on[ctx->device & 63];
   if (!configured) {
-    QENG_CUDA(ctx, cudaFuncSetAttribute(gemm_tc_kernel<FMT, WP, XP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
+    QENG_CUDA(ctx, cudaFuncSetAttribute(gemm_tc_kernel<FMT, WP, XP, KST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
     configured = true;
   }
   cudaLaunchConfig_t cfg = {};
@@ -697,9 +703,9 @@ int32_t launch(qeng_ctx* ctx, const qeng_weight* w, const TcParams& p, const Pla
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = ctx->pdl ? 1 : 0;
-  const CUtensorMap* wm = reinterpret_cast<const CUtensorMap*>(w->tc_maps[0]);
-  const CUtensorMap* sm = reinterpret_cast<const CUtensorMap*>(w->tc_maps[1]);
-  QENG_CUDA(ctx, cudaLaunchKernelEx(&cfg, gemm_tc_kernel<FMT, WP, XP>, p, map, *wm, *sm));
+  const CUtensorMap* wm = reinterpret_cast<const CUtensorMap*>(w->tc_maps[KST - 1][0]);
+  const CUtensorMap* sm = reinterpret_cast<const CUtensorMap*>(w->tc_maps[KST - 1][1]);
+  QENG_CUDA(ctx, cudaLaunchKernelEx(&cfg, gemm_tc_kernel<FMT, WP, XP, KST>, p, map, *wm, *sm));
   return p.sk_tiles > 0 ? reduce(ctx, p, stream) : QENG_OK;
 }
 
@@ -778,8 +784,8 @@ int32_t qeng_gemm_tc(qeng_ctx* ctx, const qeng_weight* w, const qeng_tc_x& x, in
     rc = prepare(ctx, w, x, M, epi, sc, &pl, &p, &map);
   }
   if (rc != QENG_OK) return rc;
-  if (wp == 1) return launch<QENG_FMT_Q4, 1, 1>(ctx, w, p, pl, map, stream);
-#define QENG_TC(F, X) launch<F, 2, X>(ctx, w, p, pl, map, stream)
+  if (wp == 1) return launch<QENG_FMT_Q4, 1, 1, 2>(ctx, w, p, pl, map, stream);
+#define QENG_TC(F, X) (pl.kst == 2 ? launch<F, 2, X, 2>(ctx, w, p, pl, map, stream) : launch<F, 2, X, 1>(ctx, w, p, pl, map, stream))
   switch (w->fmt) {
     case QENG_FMT_Q4: return xp == 1 ? QENG_TC(QENG_FMT_Q4, 1) : QENG_TC(QENG_FMT_Q4, 2);
     case QENG_FMT_Q8: return xp == 1 ? QENG_TC(QENG_FMT_Q8, 1) : QENG_TC(QENG_FMT_Q8, 2);

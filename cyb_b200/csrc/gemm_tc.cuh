@@ -9,7 +9,6 @@
 namespace qeng_tc {
 
 constexpr int kBK = 64;                  // k per chunk: one 128-byte swizzled row of bf16
-constexpr int kST = 2;                   // chunks per stage
 constexpr int kACols = kBK / 2;          // tensor-memory columns of one plane of a chunk of weights
 constexpr int kMaxStages = 8, kMaxSlots = 12;
 constexpr int kOldTokens = 64, kOldBytes = kOldTokens * 128 * 4;
@@ -21,10 +20,10 @@ template <> struct Fmt<QENG_FMT_Q8> { static constexpr int kW = 1024, kS = 64; }
 template <> struct Fmt<QENG_FMT_K4> { static constexpr int kW = 512, kS = 256; };
 inline int chunk_w(int fmt) { return fmt == QENG_FMT_Q8 ? 1024 : 512; }
 inline int chunk_s(int fmt) { return fmt == QENG_FMT_K4 ? 256 : 64; }
-inline int slot_bytes_of(int fmt) { return kST * 8 * (chunk_w(fmt) + chunk_s(fmt)); }
+inline int slot_bytes_of(int fmt, int kst) { return kst * 8 * (chunk_w(fmt) + chunk_s(fmt)); }
 
 struct TcParams {
-  int nk;                    // stages of kST chunks along K
+  int nk;                    // stages of KST chunks along K
   int M, N;
   int bn, m_tiles, n_tiles;  // tokens per tile, token tiles, 256-row weight tiles
   int dp_tiles, sk_tiles;    // whole tiles (round-robin), tiles cut along K
@@ -357,7 +356,7 @@ __device__ __forceinline__ void cp_async_wait() {
 }
 
 struct Plan {
-  int nk, bn, m_tiles, n_tiles, dp_tiles, sk_tiles, npairs, nstages, nslots, nacc, acc_cols, old_at;
+  int kst, nk, bn, m_tiles, n_tiles, dp_tiles, sk_tiles, npairs, nstages, nslots, nacc, acc_cols, old_at;
   int box_rows;  // rows of an activation box
   size_t smem, ws_floats;
 };

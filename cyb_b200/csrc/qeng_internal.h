@@ -43,9 +43,9 @@ struct qeng_weight {
   int64_t bytes;       // device bytes held
   // What the matmuls work out on first use.  The lock guards it: contexts in several threads may share a weight.
   mutable std::mutex lock;
-  // tensor maps of both planes for the tensor-core matmul (gemm_tc.cu), unchanged once encoded: codes, scales
+  // tensor maps of both planes for the tensor-core matmul (gemm_tc.cu), unchanged once encoded: [1 or 2 chunks per box][codes, scales]
   mutable bool tc_maps_ready = false;
-  alignas(64) mutable unsigned char tc_maps[2][128];
+  alignas(64) mutable unsigned char tc_maps[2][2][128];
   mutable int rows_plan[4][10] = {};  // gemm_rows.cu: plans of the last few row counts
   mutable int rows_plan_next = 0;
   const qeng_weight* next = nullptr;  // matrix the caller multiplies by after this one (L2 prefetch hint)

@@ -248,11 +248,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
       int s = 0, n = 0, buf = 0;
       uint32_t ph = 0, acc_ph = 1;
       while (!failed && segs.next(p, sg)) {
-        if (!mbar_wait_warp(smem_u32(acc_empty + buf), acc_ph)) { failed = true; break; }
+        if (!mbar_wait_cluster(smem_u32(acc_empty + buf), acc_ph)) { failed = true; break; }
         const uint32_t d = tm + (uint32_t)(buf * p.acc_cols);
         uint32_t acc = 0;
         for (int kt = sg.k0; kt < sg.k1; ++kt) {
-          if (!mbar_wait_warp(smem_u32(full + s), ph)) { failed = true; break; }
+          if (!mbar_wait_cluster(smem_u32(full + s), ph)) { failed = true; break; }
           asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
           if (elect_one()) {
             const uint32_t a = ta + (uint32_t)s * kStageCols;
@@ -281,7 +281,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
       // the last accumulators have been read in both CTAs: nothing of this pair is in flight any more
       for (int b = 0; b < p.nacc && b < n; ++b) {
         const int last = n - 1 - b;
-        if (!failed && !mbar_wait(smem_u32(acc_empty + last % p.nacc), (uint32_t)(last / p.nacc) & 1u)) failed = true;
+        if (!failed && !mbar_wait_cluster(smem_u32(acc_empty + last % p.nacc), (uint32_t)(last / p.nacc) & 1u)) failed = true;
       }
       if (failed) {  // what was issued still has to finish before tensor memory is freed
         if (elect_one()) umma_commit_pair(smem_u32(&drained));
@@ -297,6 +297,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
       for (int i = 0; i < total; ++i) {
         if (!mbar_wait(smem_u32(full + s), ph)) failed = true;
         if (__any_sync(0xffffffffu, failed)) { failed = true; break; }
+        asm volatile("tcgen05.fence::after_thread_sync;\ntcgen05.fence::before_thread_sync;\n" ::: "memory");
         if (lane == 0) mbar_arrive_cluster(map_leader(smem_u32(full + s)));
         if (++s == p.nstages) { s = 0; ph ^= 1u; }
       }

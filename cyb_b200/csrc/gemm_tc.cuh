@@ -48,30 +48,41 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
 }
-// arrive on a barrier of either CTA of the pair (address from map_leader)
+// Arrive on a barrier of either CTA of the pair (address from map_leader).  Without the qualifiers the arrival would order
+// this CTA's accesses for threads of this CTA alone; whoever waits for it uses mbar_wait_cluster.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];\n" ::"r"(bar) : "memory");
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
 }
+// CLUSTER: what the other CTA of the pair did before its arrival is seen, too
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
+  if (CLUSTER)
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+  else
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
   return ok != 0;
 }
 // Bounded wait: gives up (false) two seconds after the first failed attempt; a healthy wait ends
 // in microseconds.  The clock is read once per 64 attempts.
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity) {
   unsigned long long t0;
   asm volatile("mov.u64 %0, %globaltimer;\n" : "=l"(t0));
   for (;;) {
     for (int i = 0; i < 64; ++i)
-      if (mbar_try_wait(bar, parity)) return true;
+      if (mbar_try_wait<CLUSTER>(bar, parity)) return true;
     unsigned long long t1;
     asm volatile("mov.u64 %0, %globaltimer;\n" : "=l"(t1));
     if (t1 - t0 > 2000000000ull) return false;
@@ -80,9 +91,10 @@ __device__ __forceinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity) {
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
   return mbar_try_wait(bar, parity) || mbar_wait_slow(bar, parity);
 }
-// The same for a converged warp; all lanes learn the outcome by vote, so that what follows stays warp-uniform.
-__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) {
-  return __all_sync(0xffffffffu, mbar_try_wait(bar, parity)) || __all_sync(0xffffffffu, mbar_wait_slow(bar, parity));
+// The same for a converged warp and a barrier on which the other CTA arrives; all lanes learn the outcome by vote, so that
+// what follows stays warp-uniform.
+__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity) {
+  return __all_sync(0xffffffffu, mbar_try_wait<true>(bar, parity)) || __all_sync(0xffffffffu, mbar_wait_slow<true>(bar, parity));
 }
 // one box of a packed plane: `box` chunks x 8 row tiles (beyond the matrix: zeros)
 __device__ __forceinline__ void tma_w(uint32_t dst, const CUtensorMap* map, int chunk, int tile, uint32_t bar) {

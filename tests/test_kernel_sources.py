@@ -1,0 +1,33 @@
+"""What the kernel sources have to say for the hardware to keep it: the scope of barriers between CTAs (a missing one
+shows in no run that happens to go well)."""
+import glob
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "cyb_b200", "csrc")
+
+
+def _sources():
+    return {os.path.basename(p): open(p).read() for p in sorted(glob.glob(os.path.join(CSRC, "*.cu*")))}
+
+
+def test_arrivals_at_another_cta_release_to_the_cluster():
+    found = 0
+    for name, text in _sources().items():
+        for ins in re.findall(r"mbarrier\.arrive[\w.:]*", text):
+            if "shared::cluster" in ins:
+                found += 1
+                assert ".release.cluster" in ins, (name, ins)
+    assert found
+
+
+def test_waits_for_another_ctas_arrivals_acquire_from_the_cluster():
+    """In the matmul of CTA pairs these are the leader's waits for operand stages and for emptied accumulators."""
+    text = _sources()["gemm_tc.cu"]
+    assert not re.search(r"mbar_wait\(smem_u32\(acc_empty", text)
+    issuer = text[text.index("if (rank == 0) {\n      // ===== MMA issuer"):text.index("the peer's weights: one arrival")]
+    assert not re.search(r"mbar_wait\(smem_u32\(full", issuer) and "mbar_wait_cluster(smem_u32(full" in issuer
+    relay = text[text.index("the peer's weights: one arrival"):text.index("===== activation tiles")]
+    fences = relay.index("fence::after_thread_sync"), relay.index("fence::before_thread_sync")
+    assert relay.index("mbar_wait(") < fences[0] < fences[1] < relay.index("mbar_arrive_cluster(")
+    assert "try_wait.parity.acquire.cluster" in _sources()["gemm_tc.cuh"]

@@ -441,7 +441,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
           finish<16>(p.e, p.N, p.status, wrow, m0 + c0, mcnt - c0, f, lane);
         } else {
 #pragma unroll
-          for (int i = 0; i < 16; ++i) __stcg(mine + (size_t)(c0 + i) * 128, f[i]);
+          for (int i = 0; i < 16; i += 4) __stcg(reinterpret_cast<float4*>(mine + (size_t)(c0 + i) * 128), make_float4(f[i], f[i + 1], f[i + 2], f[i + 3]));
         }
       }
       if (ahead) cp_async_wait<0>();
@@ -459,10 +459,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 }
 
 // ---- tiles cut along K: the parts, added in K order, through the epilogue -----------------------------------
-// Grid: (split tile, CTA of the pair) x 16 tokens; thread = weight row.
+// Grid: (split tile, CTA of the pair) x kSumTokens tokens; thread = weight row.  Its time is the latency of the parts (2 to 6 of
+// a tile): three are requested together.  f32 rows, one part at a time / so: 101 over 4096 x 4096 23.9 / 20.9 us a call, 240 over
+// 11008 x 4096 57.1 / 56.9; 8 tokens a thread 20.4 / 58.0, 4 tokens 20.0 / 61.3 (a CTA's start costs more than its sums).
+constexpr int kSumTokens = 16, kSumAhead = 3;
 __global__ void __launch_bounds__(128) tc_reduce_kernel(const TcParams p) {
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
-  const int r = blockIdx.x >> 1, rank = blockIdx.x & 1, c0 = blockIdx.y * 16, row = threadIdx.x;
+  const int r = blockIdx.x >> 1, rank = blockIdx.x & 1, c0 = blockIdx.y * kSumTokens, row = threadIdx.x;
   const long long U = (long long)p.sk_tiles * p.nk;
   int mt, nt;
   tile_pos(p, p.dp_tiles + r, mt, nt);
@@ -470,15 +473,30 @@ __global__ void __launch_bounds__(128) tc_reduce_kernel(const TcParams p) {
   const int q0 = pair_of_unit(U, p.npairs, r * p.nk), q1 = pair_of_unit(U, p.npairs, (r + 1) * p.nk - 1);
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
   if (q0 == q1 || c0 >= mcnt) return;  // one pair had all of K: its epilogue is done
-  float f[16];
+  float f[kSumTokens];
 #pragma unroll
-  for (int i = 0; i < 16; ++i) f[i] = 0.f;
-  for (int q = q0; q <= q1; ++q) {
-    const float* src = partial(p, q, r, (uint32_t)rank, row) + (size_t)c0 * 128;
+  for (int i = 0; i < kSumTokens; ++i) f[i] = 0.f;
+  for (int q = q0; q <= q1; q += kSumAhead) {
+    float4 v[kSumAhead][kSumTokens / 4];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) f[i] += __ldcg(src + (size_t)i * 128);
+    for (int j = 0; j < kSumAhead; ++j) {
+      const float4* src = reinterpret_cast<const float4*>(partial(p, min(q + j, q1), r, (uint32_t)rank, row) + (size_t)c0 * 128);
+#pragma unroll
+      for (int i = 0; i < kSumTokens / 4; ++i) v[j][i] = __ldcg(src + i * 128);
+    }
+#pragma unroll
+    for (int j = 0; j < kSumAhead; ++j) {
+      if (q + j > q1) break;
+#pragma unroll
+      for (int i = 0; i < kSumTokens / 4; ++i) {
+        f[4 * i] += v[j][i].x;
+        f[4 * i + 1] += v[j][i].y;
+        f[4 * i + 2] += v[j][i].z;
+        f[4 * i + 3] += v[j][i].w;
+      }
+    }
   }
-  finish<16>(p.e, p.N, p.status, nt * 256 + rank * 128 + row, m0 + c0, mcnt - c0, f, row & 31);
+  finish<kSumTokens>(p.e, p.N, p.status, nt * 256 + rank * 128 + row, m0 + c0, mcnt - c0, f, row & 31);
 }
 
 // ---- activation rows -> one or two bf16 planes, optionally RMS-normalised on the way ----------------------
@@ -739,7 +757,7 @@ int32_t qeng_tc::prepare(qeng_ctx* ctx, const qeng_weight* w, const qeng_tc_x& x
 
 int32_t qeng_tc::reduce(qeng_ctx* ctx, const TcParams& p, cudaStream_t stream) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(2 * p.sk_tiles), (unsigned)(p.bn / 16));
+  cfg.gridDim = dim3((unsigned)(2 * p.sk_tiles), (unsigned)(p.bn / kSumTokens));
   cfg.blockDim = dim3(128);
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];

@@ -17,9 +17,9 @@
 //               which keeps tens of KB per SM in flight from HBM independently of the dequant warps
 //   warp 3      tensor memory allocation
 //   warps 4-7   epilogue (tcgen05.ld, one warp per lane quadrant), overlapped with the next tile where
-//               tensor memory holds two accumulators (up to 160 columns with one weight term)
+//               there are two accumulators
 //   warps 8-23  dequantisation: packed words -> bf16 -> tensor memory; one warp per 16-row tile, two sets
-//               of 8 that take alternate stages
+//               of 8 that take alternate stages; with one accumulator that is added to y also its epilogue
 // A stage is two chunks of 64 k (KST; one for more than 128 columns in two weight terms), with one barrier each way: a hop between the roles costs 100 to 200 cycles
 // of dependent instructions, and with one barrier per chunk the hops of a stage took longer than its MMAs.
 // The weights used to pass through shared memory, which then carried 1.3 times what it can in the time of
@@ -50,7 +50,8 @@ namespace {
 using namespace qeng_tc;
 
 constexpr int kDequantWarps = 8, kSets = 2;
-constexpr int kThreads = (8 + kSets * kDequantWarps) * 32;
+constexpr int kHelpers = kSets * kDequantWarps;
+constexpr int kThreads = (8 + kHelpers) * 32;
 
 // ---- dequantisation: one lane's words of one 32-block -> rows g and g+8, 8 consecutive k each ------------------
 // The inner loop of the kernel: its rate is set by the integer pipe (half rate), so the 4-bit form spends two
@@ -184,7 +185,32 @@ struct Words<QENG_FMT_Q8> {
   }
 };
 
-template <int FMT, int WP, int XP, int KST>
+// ---- one warp's part of a finished accumulator: groups of 16 tokens from c0 on, every `step` tokens -------------------
+template <bool ACCUM_ONLY>
+__device__ __forceinline__ void drain(const TcParams& p, int tile, bool whole, int pair, uint32_t rank, uint32_t tacc, int quad, int lane, int c0, int step) {
+  int mt, nt;
+  tile_pos(p, tile, mt, nt);
+  const int m0 = mt * p.bn, mcnt = min(p.bn, p.M - m0), row = quad * 32 + lane;
+  float* const mine = whole ? nullptr : partial(p, pair, tile - p.dp_tiles, rank, row);
+  qeng_tc_epi e = p.e;
+  if (ACCUM_ONLY) e.kind = QENG_EPI_ACCUM;
+#pragma unroll 1
+  for (; c0 < mcnt; c0 += step) {
+    uint32_t v[16];
+    tmem_ld16(tacc + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, v);
+    float f[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) f[i] = __uint_as_float(v[i]);
+    if (whole) {
+      finish<16>(e, p.N, p.status, nt * 256 + (int)rank * 128 + row, m0 + c0, mcnt - c0, f, lane);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 16; i += 4) __stcg(reinterpret_cast<float4*>(mine + (size_t)(c0 + i) * 128), make_float4(f[i], f[i + 1], f[i + 2], f[i + 3]));
+    }
+  }
+}
+
+template <int FMT, int WP, int XP, int KST, bool HELP>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     gemm_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap,
                    const __grid_constant__ CUtensorMap smap) {
@@ -217,7 +243,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(acc_full + b), 1);
-      mbar_init(smem_u32(acc_empty + b), 8);  // the epilogue warps of both CTAs
+      mbar_init(smem_u32(acc_empty + b), HELP ? 2 * (4 + kHelpers) : 8);  // who empties it, in both CTAs
     }
     mbar_init(smem_u32(&drained), 1);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -363,32 +389,58 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     // earlier than the one before the last of this stage, and the MMAs consume in order.)
     int s = set, ws = set;
     uint32_t ph = 1, wph = 0;
-    for (int i = set; i < total; i += kSets) {
-      if (!failed && !mbar_wait(smem_u32(wfull + ws), wph)) failed = true;
-      const uint32_t wb = wb0 + (uint32_t)ws * kSlot, sb = sb0 + (uint32_t)ws * kSlot, at = dst0 + (uint32_t)s * kStageCols;
-      Words<FMT> w[KST];
+    // HELP: one accumulator, added to y.  The MMAs stand still while it is emptied, and so would these warps as soon as all
+    // stages are full: they take four fifths of it instead, as it is the latency of the old values that makes it long.  A segment
+    // is due once the stage ahead (i) is one that the first stage of the next segment has to free; up to there a warp has filled
+    // all that the segment's MMAs need.  4096 rows bf16 over 22016 x 4096 803 -> 633 us, over 4096 x 4096 152 -> 123, 1800 rows
+    // over 4096 x 11008 149 -> 134.  (Stores and parts are no faster for it: those are bound by the way to L2.)
+    bool owed = HELP && segs.next(p, sg);
+    int due = owed ? sg.k1 - sg.k0 + p.nstages : 0;
+    uint32_t acc_ph = 0;
+    for (int i = set;;) {
+      const int stop = owed ? min(total, due) : total;
+#pragma unroll 1
+      for (; i < stop; i += kSets) {
+        if (!failed && !mbar_wait(smem_u32(wfull + ws), wph)) failed = true;
+        const uint32_t wb = wb0 + (uint32_t)ws * kSlot, sb = sb0 + (uint32_t)ws * kSlot, at = dst0 + (uint32_t)s * kStageCols;
+        Words<FMT> w[KST];
 #pragma unroll
-      for (int c = 0; c < KST; ++c) w[c].load(wb + (uint32_t)(c * kW), sb + (uint32_t)(c * kS), lane);
+        for (int c = 0; c < KST; ++c) w[c].load(wb + (uint32_t)(c * kW), sb + (uint32_t)(c * kS), lane);
 #pragma unroll
-      for (int c = 0; c < KST; ++c) {
-        uint32_t hi[16], lo[16];
-        w[c].template dequant<WP>(lane, mask, base, hi, lo);
-        if (c == 0) {
-          if (!failed && !mbar_wait(smem_u32(empty + s), ph)) failed = true;
-          __syncwarp();
-          asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        for (int c = 0; c < KST; ++c) {
+          uint32_t hi[16], lo[16];
+          w[c].template dequant<WP>(lane, mask, base, hi, lo);
+          if (c == 0) {
+            if (!failed && !mbar_wait(smem_u32(empty + s), ph)) failed = true;
+            __syncwarp();
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+          }
+          tmem_st16(at + (uint32_t)(c * WP * kACols), hi);
+          if (WP == 2) tmem_st16(at + (uint32_t)(c * WP * kACols + kACols), lo);
         }
-        tmem_st16(at + (uint32_t)(c * WP * kACols), hi);
-        if (WP == 2) tmem_st16(at + (uint32_t)(c * WP * kACols + kACols), lo);
+        asm volatile("tcgen05.wait::st.sync.aligned;\ntcgen05.fence::before_thread_sync;\n" ::: "memory");
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive(smem_u32(full + s));
+          mbar_arrive(smem_u32(wempty + ws));
+        }
+        if ((s += kSets) >= p.nstages) { s -= p.nstages; ph ^= 1u; }
+        if ((ws += kSets) >= p.nslots) { ws -= p.nslots; wph ^= 1u; }
       }
-      asm volatile("tcgen05.wait::st.sync.aligned;\ntcgen05.fence::before_thread_sync;\n" ::: "memory");
+      if (!owed) break;
+      asm volatile("griddepcontrol.wait;\n" ::: "memory");
+      if (!failed && !mbar_wait(smem_u32(acc_full), acc_ph)) failed = true;
+      acc_ph ^= 1u;
       __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(smem_u32(full + s));
-        mbar_arrive(smem_u32(wempty + ws));
-      }
-      if ((s += kSets) >= p.nstages) { s -= p.nstages; ph ^= 1u; }
-      if ((ws += kSets) >= p.nslots) { ws -= p.nslots; wph ^= 1u; }
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+      const bool whole = sg.k0 == 0 && sg.k1 == p.nk;
+      if (!__any_sync(0xffffffffu, failed) && whole)
+        drain<true>(p, sg.tile, whole, pair, rank, tmem, warp & 3, lane, 16 * (1 + ((warp - 8) >> 2)), 16 * (1 + kHelpers / 4));
+      asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(map_leader(smem_u32(acc_empty)));
+      owed = segs.next(p, sg);
+      if (owed) due += sg.k1 - sg.k0;
     }
     if (failed && lane == 0) atomicExch(p.status, 4);
   } else if (warp >= 4) {
@@ -398,53 +450,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     int buf = 0;
     uint32_t acc_ph = 0;
     while (segs.next(p, sg)) {
-      int mt, nt;
-      tile_pos(p, sg.tile, mt, nt);
-      const int m0 = mt * p.bn, mcnt = min(p.bn, p.M - m0);
-      const int row = quad * 32 + lane, wrow = nt * 256 + (int)rank * 128 + row;
       const bool whole = sg.k0 == 0 && sg.k1 == p.nk;
-      // y += ... of a whole tile: the old values come through shared memory, kOldTokens tokens ahead of their use and each
-      // through the lane that asked for it.  Loaded group by group into registers they cost a trip to L2 per 16 tokens: 100
-      // cycles a token instead of 30, which one accumulator leaves exposed
-      // (1800 rows over 4096 x 4096: 79 us, now 69; over 4096 x 11008: 137, now 126).
-      const bool ahead = whole && p.old_at >= 0;
-      float* const ycol = ahead ? p.e.y + (size_t)m0 * p.e.ldy + wrow : nullptr;
-      const uint32_t old = smem + (uint32_t)max(p.old_at, 0) + (uint32_t)row * 4u;
-      const int live = wrow < p.N ? mcnt : 0;  // tokens of this lane
-      const auto request = [&](int c0) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i)
-          if (c0 + i < live) cp_async4(old + (uint32_t)((c0 + i) % kOldTokens) * 512u, ycol + (size_t)(c0 + i) * p.e.ldy);
-        cp_async_commit();
-      };
-      if (ahead)
-        for (int c0 = 0; c0 < kOldTokens; c0 += 16) request(c0);
       if (!failed && !mbar_wait(smem_u32(acc_full + buf), acc_ph)) failed = true;
+      __syncwarp();
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-      const uint32_t tacc = tmem + (uint32_t)(buf * p.acc_cols) + ((uint32_t)(quad * 32) << 16);
-      float* mine = whole ? nullptr : partial(p, pair, sg.tile - p.dp_tiles, rank, row);
-#pragma unroll 1
-      for (int c0 = 0; c0 < mcnt; c0 += 16) {
-        uint32_t v[16];
-        tmem_ld16(tacc + (uint32_t)c0, v);
-        float f[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) f[i] = __uint_as_float(v[i]);
-        if (failed) continue;
-        if (ahead) {
-          cp_async_wait<kOldTokens / 16 - 1>();
-#pragma unroll
-          for (int i = 0; i < 16; ++i)
-            if (c0 + i < live) ycol[(size_t)(c0 + i) * p.e.ldy] = __uint_as_float(lds32(old + (uint32_t)((c0 + i) % kOldTokens) * 512u)) + f[i];
-          request(c0 + kOldTokens);
-        } else if (whole) {
-          finish<16>(p.e, p.N, p.status, wrow, m0 + c0, mcnt - c0, f, lane);
-        } else {
-#pragma unroll
-          for (int i = 0; i < 16; i += 4) __stcg(reinterpret_cast<float4*>(mine + (size_t)(c0 + i) * 128), make_float4(f[i], f[i + 1], f[i + 2], f[i + 3]));
-        }
-      }
-      if (ahead) cp_async_wait<0>();
+      if (!__any_sync(0xffffffffu, failed)) 
+        drain<HELP>(p, sg.tile, whole, pair, rank, tmem + (uint32_t)(buf * p.acc_cols), quad, lane, 0, HELP && whole ? 16 * (1 + kHelpers / 4) : 16);
       asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(map_leader(smem_u32(acc_empty + buf)));
@@ -667,18 +678,14 @@ Plan make_plan(const qeng_ctx* ctx, const qeng_weight* w, int64_t M, int wp, int
   // weights (never fewer than two); what is left goes to the packed ring (few tokens: the weights come from HBM and want
   // tens of KB in flight, and then a stage leaves room for it).
   const size_t stage = (size_t)kst * xp * (best.bn / 2) * 128, slot = (size_t)slot_bytes_of(w->fmt, kst);
-  size_t room = kSmemBudget - 1024 - 1024;  // alignment, static shared memory
-  // the old values of y where two stages fit beside them (8-bit blocks, two planes of more than 224 tokens: they do not)
-  const size_t old = epi == QENG_EPI_ACCUM && room >= kOldBytes + 4 * slot + 2 * stage ? (size_t)kOldBytes : 0;
-  room -= old;
+  const size_t room = kSmemBudget - 1024 - 1024;  // alignment, static shared memory
   best.nstages = (512 - best.nacc * best.acc_cols) / a_cols;
   if (best.nstages > kMaxStages) best.nstages = kMaxStages;
   if (best.nstages > (int)((room - 4 * slot) / stage)) best.nstages = (int)((room - 4 * slot) / stage);
   best.nslots = (int)((room - best.nstages * stage) / slot);
   best.nslots = (best.nslots < kMaxSlots ? best.nslots : kMaxSlots) / kSets * kSets;  // a slot belongs to one dequant set
   best.box_rows = best.bn / 2;
-  best.old_at = old > 0 ? (int)(best.nstages * stage + best.nslots * slot) : -1;
-  best.smem = best.nstages * stage + best.nslots * slot + old + 1024;
+  best.smem = best.nstages * stage + best.nslots * slot + 1024;
   best.ws_floats = best.sk_tiles > 0 ? (size_t)best.npairs * 4 * best.bn * 128 : 0;
   return best;
 }
@@ -704,12 +711,12 @@ bool weight_maps(const qeng_weight* w) {
   return true;
 }
 
-template <int FMT, int WP, int XP, int KST>
+template <int FMT, int WP, int XP, int KST, bool HELP>
 int32_t launch(qeng_ctx* ctx, const qeng_weight* w, const TcParams& p, const Plan& pl, const CUtensorMap& map, cudaStream_t stream) {
   static bool configured_on[64] = {};  // the opt-in shared-memory size is set per device
   bool& configured = configured_on[ctx->device & 63];
   if (!configured) {
-    QENG_CUDA(ctx, cudaFuncSetAttribute(gemm_tc_kernel<FMT, WP, XP, KST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
+    QENG_CUDA(ctx, cudaFuncSetAttribute(gemm_tc_kernel<FMT, WP, XP, KST, HELP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
     configured = true;
   }
   cudaLaunchConfig_t cfg = {};
@@ -724,7 +731,7 @@ int32_t launch(qeng_ctx* ctx, const qeng_weight* w, const TcParams& p, const Pla
   cfg.numAttrs = ctx->pdl ? 1 : 0;
   const CUtensorMap* wm = reinterpret_cast<const CUtensorMap*>(w->tc_maps[KST - 1][0]);
   const CUtensorMap* sm = reinterpret_cast<const CUtensorMap*>(w->tc_maps[KST - 1][1]);
-  QENG_CUDA(ctx, cudaLaunchKernelEx(&cfg, gemm_tc_kernel<FMT, WP, XP, KST>, p, map, *wm, *sm));
+  QENG_CUDA(ctx, cudaLaunchKernelEx(&cfg, gemm_tc_kernel<FMT, WP, XP, KST, HELP>, p, map, *wm, *sm));
   return p.sk_tiles > 0 ? reduce(ctx, p, stream) : QENG_OK;
 }
 
@@ -750,7 +757,7 @@ int32_t qeng_tc::prepare(qeng_ctx* ctx, const qeng_weight* w, const qeng_tc_x& x
     return qeng_fail(ctx, QENG_ERR_CUDA, "gemm_tc: tensor map rejected (M=%lld, K=%lld, ld=%lld)", (long long)M, (long long)w->K, (long long)x.ld);
   p->nk = pl->nk; p->M = (int)M; p->N = (int)w->N;
   p->bn = pl->bn; p->m_tiles = pl->m_tiles; p->n_tiles = pl->n_tiles; p->dp_tiles = pl->dp_tiles; p->sk_tiles = pl->sk_tiles;
-  p->nstages = pl->nstages; p->nslots = pl->nslots; p->nacc = pl->nacc; p->acc_cols = pl->acc_cols; p->old_at = pl->old_at; p->npairs = pl->npairs; p->e = epi;
+  p->nstages = pl->nstages; p->nslots = pl->nslots; p->nacc = pl->nacc; p->acc_cols = pl->acc_cols; p->npairs = pl->npairs; p->e = epi;
   p->status = ctx->status;
   return QENG_OK;
 }
@@ -803,14 +810,17 @@ int32_t qeng_gemm_tc(qeng_ctx* ctx, const qeng_weight* w, const qeng_tc_x& x, in
     rc = prepare(ctx, w, x, M, epi, sc, &pl, &p, &map);
   }
   if (rc != QENG_OK) return rc;
-  if (wp == 1) return launch<QENG_FMT_Q4, 1, 1, 2>(ctx, w, p, pl, map, stream);
-#define QENG_TC(F, X) (pl.kst == 2 ? launch<F, 2, X, 2>(ctx, w, p, pl, map, stream) : launch<F, 2, X, 1>(ctx, w, p, pl, map, stream))
+  const bool help = pl.nacc == 1 && epi.kind == QENG_EPI_ACCUM;
+  if (wp == 1) return help ? launch<QENG_FMT_Q4, 1, 1, 2, true>(ctx, w, p, pl, map, stream) : launch<QENG_FMT_Q4, 1, 1, 2, false>(ctx, w, p, pl, map, stream);
+#define QENG_TC_K(F, X, K) (help ? launch<F, 2, X, K, true>(ctx, w, p, pl, map, stream) : launch<F, 2, X, K, false>(ctx, w, p, pl, map, stream))
+#define QENG_TC(F, X) (pl.kst == 2 ? QENG_TC_K(F, X, 2) : QENG_TC_K(F, X, 1))
   switch (w->fmt) {
     case QENG_FMT_Q4: return xp == 1 ? QENG_TC(QENG_FMT_Q4, 1) : QENG_TC(QENG_FMT_Q4, 2);
     case QENG_FMT_Q8: return xp == 1 ? QENG_TC(QENG_FMT_Q8, 1) : QENG_TC(QENG_FMT_Q8, 2);
     default: return xp == 1 ? QENG_TC(QENG_FMT_K4, 1) : QENG_TC(QENG_FMT_K4, 2);
   }
 #undef QENG_TC
+#undef QENG_TC_K
 }
 
 // y[M,N] = x . dequant(W)^T through the kernel above, activations in any type the entry point takes.

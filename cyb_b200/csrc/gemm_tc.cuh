@@ -11,7 +11,6 @@ namespace qeng_tc {
 constexpr int kBK = 64;                  // k per chunk: one 128-byte swizzled row of bf16
 constexpr int kACols = kBK / 2;          // tensor-memory columns of one plane of a chunk of weights
 constexpr int kMaxStages = 8, kMaxSlots = 12;
-constexpr int kOldTokens = 64, kOldBytes = kOldTokens * 128 * 4;
 constexpr size_t kSmemBudget = 226 * 1024;
 
 template <int FMT> struct Fmt;
@@ -29,7 +28,6 @@ struct TcParams {
   int dp_tiles, sk_tiles;    // whole tiles (round-robin), tiles cut along K
   int nstages, nslots;       // rings: operands (weights in tensor memory, activations in shared memory), packed weights
   int nacc, acc_cols;        // accumulators (1 or 2), tensor-memory columns of each
-  int old_at;                // ACCUM: where in shared memory the old values of y pass through (kOldTokens rows of 128)
   qeng_tc_epi e;
   int npairs;
   float* ws;                 // stream-K partials: [pair][2][CTA of the pair][bn / 4][128][4]
@@ -362,18 +360,8 @@ __device__ __forceinline__ void finish(const qeng_tc_epi& e, int N, int32_t* sta
   }
 }
 
-// y += ... of whole tiles: four bytes of y on their way into shared memory, and the wait for all but the last N groups of them
-__device__ __forceinline__ void cp_async4(uint32_t dst, const float* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
-
 struct Plan {
-  int kst, nk, bn, m_tiles, n_tiles, dp_tiles, sk_tiles, npairs, nstages, nslots, nacc, acc_cols, old_at;
+  int kst, nk, bn, m_tiles, n_tiles, dp_tiles, sk_tiles, npairs, nstages, nslots, nacc, acc_cols;
   int box_rows;  // rows of an activation box
   size_t smem, ws_floats;
 };

@@ -2,9 +2,9 @@
 //   y[m][n] (f32) = sum_k x[m][k] * dequant(W)[n][k], f32 accumulation in tensor memory.
 //
 // The weights are the M side of the MMA, the activation rows ("tokens") its N side: an output tile is
-// 256 weight rows x `bn` tokens, bn any multiple of 16 up to 256, so a token count that fits no tile
-// wastes at most 15 columns of one, and the accumulator has one weight row per tensor-memory lane,
-// which makes every store of the epilogue 128 contiguous bytes of a y row.
+// 256 weight rows x `bn` tokens, bn any multiple of 16 up to 256 (a plan may leave more than 15 columns of
+// the last tile empty: 257 rows over 11008 x 4096 are two tiles of 144), and the accumulator has one weight
+// row per tensor-memory lane, which makes every store of the epilogue 128 contiguous bytes of a y row.
 //
 // A pair of CTAs (cluster of 2, tcgen05 cta_group::2) computes a tile: each CTA dequantises 128 of the
 // weight rows into its tensor memory, which is where the MMAs take their A operand from, and loads half of
@@ -20,13 +20,15 @@
 //               there are two accumulators
 //   warps 8-23  dequantisation: packed words -> bf16 -> tensor memory; one warp per 16-row tile, two sets
 //               of 8 that take alternate stages; with one accumulator that is added to y also its epilogue
-// A stage is two chunks of 64 k (KST; one for more than 128 columns in two weight terms), with one barrier each way: a hop between the roles costs 100 to 200 cycles
-// of dependent instructions, and with one barrier per chunk the hops of a stage took longer than its MMAs.
-// The weights used to pass through shared memory, which then carried 1.3 times what it can in the time of
-// the MMAs: cycles per 128 k and one term, shared / tensor memory: 1460 / 1024 at 256 columns (the MMAs:
-// 1024), 1240 / 800 to 880 at 160 (640); two terms, 112 columns: 2640 / 1340 (1344).
-// 777 rows f32 over 11008 x 4096 87.6 -> 75.4 us, 101 rows 37.8 -> 35.0, 8192 rows bf16 over 4096 x 11008
-// 645 -> 590 (power limit), a prompt of 1800 tokens 33.2 -> 29.3 ms.
+// A stage is two chunks of 64 k or (two weight terms, as the plan finds better) one, with one barrier each way: a hop between
+// the roles costs 100 to 200 cycles of dependent instructions, and with one barrier per chunk the hops of a stage took longer
+// than its MMAs.
+// The weights used to pass through shared memory, which then carried 1.3 times what it can in the time of the MMAs; cycles per
+// 128 k and one term, shared / tensor memory: 1460 / 1024 at 256 columns (the MMAs: 1024), 1240 / 800 to 880 at 160 (640); two
+// terms, 112 columns: 2640 / 1340 (1344).  With it went the second accumulator of more than 160 columns (96 to 192 in two terms).
+// Calls with weights through shared memory / now: 777 rows f32 over 11008 x 4096 86 / 68 us, 101 rows 36.0 / 30.8, 240 rows
+// 57.0 / 57.2, over 4096 x 4096 32.6 / 27.8; 8192 rows bf16 over 4096 x 11008 627 / 549, 4096 rows added to y over 22016 x 4096
+// 652 / 652; a prompt of 1800 tokens 33.2 / 24.4 ms.
 //
 // Precision.  WP = 1 (prompt path of 4-bit blocks): weights and activations rounded to bf16, as before.
 // WP = 2: a weight is the sum of two bf16 values (4-bit blocks: exact, (c-8)*s has 14 significant bits;
@@ -631,61 +633,72 @@ EncodeFn encode_fn() {
   return fn;
 }
 
-// Tile width and split, by a cost model in cycles.  Per 64 k the MMAs take 2 * bn per product and the dequantisation a
-// fixed time, whichever is longer; tiles cut along K pay for their partials' way through L2 and a second launch.
+// As many stages as tensor memory holds of the weights and shared memory of the activations, beside four slots of packed
+// weights; what is left goes to the packed ring (few tokens: the weights come from HBM and want tens of KB in flight, and then a
+// stage leaves room for it).  False where two stages do not fit.
+bool fit_rings(Plan* pl, int fmt, int wp, int xp) {
+  const size_t stage = (size_t)pl->kst * xp * (pl->bn / 2) * 128, slot = (size_t)slot_bytes_of(fmt, pl->kst);
+  const size_t room = kSmemBudget - 1024 - 1024;  // alignment, static shared memory
+  pl->nstages = std::min(std::min((512 - pl->nacc * pl->acc_cols) / (pl->kst * wp * kACols), kMaxStages), (int)((room - 4 * slot) / stage));
+  if (pl->nstages < 2) return false;
+  pl->nslots = (int)((room - pl->nstages * stage) / slot);
+  pl->nslots = (pl->nslots < kMaxSlots ? pl->nslots : kMaxSlots) / kSets * kSets;  // a slot belongs to one dequant set
+  pl->smem = pl->nstages * stage + pl->nslots * slot + 1024;
+  return true;
+}
+
+// Tile width, stages and split, by a cost model in cycles.  Its constants were fitted to 1265 calls (three formats, f32 and bf16
+// rows, 17 to 4096 of them, seven matrices, store and accumulate) and to 68 prompts, each timed with every plan that fits: the
+// plan it picks takes 1.0 % longer than the best one in the mean.  Per 64 k:
+//   the MMAs take 2 * bn per product, the dequantisation 430 (4-bit blocks, one term), 735 (two), 870 (8-bit) or 1020 (K-quant),
+//   a stage what is longer; stages of one chunk add 34 to the former and 76 to the latter (each has its barriers), two stages in
+//   all 106 and 163 (one waits for the other's refill).
+// Emptying an accumulator takes 17 cycles a token (store), 27 (accumulate), 12 with the dequantising warps' help, 100 (SWIGLU)
+// and 250 (QKV, whose pages and angles come from L2); the next tile hides it where there are two of them (a last store then takes
+// 11).  Every tile of the first round costs 29 (the pairs' first loads meet).  Tiles cut along K pay for their parts (64 a token,
+// 0.6 of it where another segment hides one), their sums (700 a part) and the second launch (9400).
 Plan make_plan(const qeng_ctx* ctx, const qeng_weight* w, int64_t M, int wp, int xp, int epi, bool may_split) {
   Plan best = {};
   double best_cost = 1e30;
-  // two weight terms of two chunks are 128 columns of tensor memory, of which only two stages fit beside an accumulator of more
-  // than 128: then stages of one chunk (8-bit blocks, 144 rows f32 over 11008 x 4096: 41.7 us, so 37.9)
-  const int kst = wp == 2 && M > 128 ? 1 : 2;
-  const int pairs = ctx->sm_count / 2, nk = (int)((w->nchunks + kst - 1) / kst);
-  const int n_tiles = (int)((w->N + 255) / 256), products = wp + xp - 1, a_cols = kst * wp * kACols;
-  // measured: the dequantisation of 64 k where it, not the MMAs, sets the pace
-  const double deq = kst * (w->fmt == QENG_FMT_Q4 ? (wp == 1 ? 410 : 625) : 700);
-  const double per_token = epi == QENG_EPI_QKV ? 80 : epi == QENG_EPI_SWIGLU ? 60 : 20;  // of the epilogue
-  const int lo = M <= 256 ? (int)((M + 15) / 16 * 16) : 128, hi = M <= 256 ? lo : 256;
-  for (int bn = hi; bn >= lo; bn -= 16) {
-    const int m_tiles = (int)((M + bn - 1) / bn), T = m_tiles * n_tiles;
-    // Tensor memory: two accumulators if three stages of weights fit beside them, else one.  (With two stages the MMAs wait
-    // for the refill: 192 columns, 86 stages: 63 us a tile against 55 with one accumulator and five stages.)
-    const int acc_cols = (bn + 31) / 32 * 32, nacc = 2 * acc_cols + 3 * a_cols <= 512 ? 2 : 1;
-    const double mma = 2.0 * kst * (bn < 32 ? 32 : bn) * products, stage = mma > deq ? mma : deq;
-    const int waves = (T + pairs - 1) / pairs, rem = T % pairs;
-    // the next tile hides an epilogue where there are two accumulators
-    const double ep = per_token * bn, tile = nacc == 1 ? nk * stage + ep : std::max(nk * stage, ep);
-    const double dp = waves * tile + (nacc == 1 ? 0.0 : ep);
-    const double sk = (T / pairs) * tile + (double)rem * nk / pairs * stage + 50.0 * bn + 6000;
-    // shares of at least two stages (with no whole tiles the number of pairs is reduced instead, below)
-    const bool cut = may_split && rem != 0 && sk < dp && (T < pairs || (int64_t)rem * nk >= 2 * (int64_t)pairs);
-    const double cost = cut ? sk : dp;
-    if (cost < best_cost) {
+  const int pairs = ctx->sm_count / 2, n_tiles = (int)((w->N + 255) / 256), products = wp + xp - 1;
+  const double deq = w->fmt == QENG_FMT_Q4 ? (wp == 1 ? 430 : 735) : w->fmt == QENG_FMT_Q8 ? 870 : 1020;
+  const int widest = M <= 256 ? (int)((M + 15) / 16 * 16) : 256, narrowest = M <= 128 ? widest : 80;
+  for (int bn = widest; bn >= narrowest; bn -= 16) {
+    for (int form = 0; form < (wp == 1 ? 2 : 4); ++form) {  // stages of two chunks or (two terms) of one; one accumulator or two
+      Plan c = {};
+      c.kst = form < 2 ? 2 : 1;
+      c.nacc = 1 + form % 2;
+      c.acc_cols = (bn + 31) / 32 * 32;
+      c.bn = bn;
+      if (!fit_rings(&c, w->fmt, wp, xp)) continue;
+      c.m_tiles = (int)((M + bn - 1) / bn);
+      c.n_tiles = n_tiles;
+      c.nk = (int)((w->nchunks + c.kst - 1) / c.kst);
+      const int T = c.m_tiles * n_tiles, waves = (T + pairs - 1) / pairs, rem = T % pairs, nk = c.nk;
+      const bool two = c.nstages == 2, one = c.kst == 1;
+      const double mma = 2.0 * c.kst * std::max(bn, 32) * products + (one ? 34 : 0) + (two ? 106 : 0);
+      const double convert = c.kst * deq + (one ? 76 : 0) + (two ? 163 : 0);
+      const double stage = std::max(mma, convert);
+      const double per_token = epi == QENG_EPI_QKV ? 250 : epi == QENG_EPI_SWIGLU ? 100 : epi == QENG_EPI_STORE ? (c.nacc == 1 ? 17 : 11) : c.nacc == 1 ? 12 : 27;
+      const double ep = per_token * bn, body = nk * stage, tile = c.nacc == 1 ? body + ep : std::max(body, ep);
+      const double dp = waves * tile + (c.nacc == 1 ? 0.0 : ep) + 29.0 * std::min(T, pairs);
+      // shares of at least two stages (with no whole tiles the number of pairs is reduced instead)
+      const int sharing = T < pairs ? std::min(pairs, std::max(1, (int)((int64_t)rem * nk / 2))) : pairs;
+      const double share = (double)rem * nk / sharing, parts = 1 + std::max(1.0, nk / std::max(share, 1.0));
+      // the share of a cut tile has to hide the epilogue of the pair's last whole one, old values of y from HBM among it
+      const double tail = c.nacc == 1 || T < pairs ? 0.0 : std::max(0.0, (epi == QENG_EPI_ACCUM ? 100 : per_token) * bn - share * stage);
+      const double sk = (T / pairs) * tile + share * stage + tail + (c.nacc == 1 ? 64.0 : 38.0) * bn + 700 * parts + 9400;
+      const bool cut = may_split && rem != 0 && sk < dp && (T < pairs || (int64_t)rem * nk >= 2 * (int64_t)pairs);
+      const double cost = cut ? sk : dp;
+      if (cost >= best_cost) continue;
       best_cost = cost;
-      best.bn = bn; best.m_tiles = m_tiles; best.n_tiles = n_tiles;
-      best.nacc = nacc; best.acc_cols = acc_cols;
-      best.sk_tiles = cut ? rem : 0;
-      best.dp_tiles = T - best.sk_tiles;
+      c.sk_tiles = cut ? rem : 0;
+      c.dp_tiles = T - c.sk_tiles;
+      c.npairs = cut ? sharing : std::min(T, pairs);
+      best = c;
     }
   }
-  best.kst = kst;
-  best.nk = nk;
-  best.npairs = best.sk_tiles > 0 ? pairs : (best.dp_tiles < pairs ? best.dp_tiles : pairs);
-  if (best.sk_tiles > 0 && best.dp_tiles == 0) {
-    const int64_t units = (int64_t)best.sk_tiles * nk;
-    if (units / 2 < best.npairs) best.npairs = units / 2 > 0 ? (int)(units / 2) : 1;
-  }
-  // As many stages as tensor memory holds of the weights and shared memory of the activations beside four slots of packed
-  // weights (never fewer than two); what is left goes to the packed ring (few tokens: the weights come from HBM and want
-  // tens of KB in flight, and then a stage leaves room for it).
-  const size_t stage = (size_t)kst * xp * (best.bn / 2) * 128, slot = (size_t)slot_bytes_of(w->fmt, kst);
-  const size_t room = kSmemBudget - 1024 - 1024;  // alignment, static shared memory
-  best.nstages = (512 - best.nacc * best.acc_cols) / a_cols;
-  if (best.nstages > kMaxStages) best.nstages = kMaxStages;
-  if (best.nstages > (int)((room - 4 * slot) / stage)) best.nstages = (int)((room - 4 * slot) / stage);
-  best.nslots = (int)((room - best.nstages * stage) / slot);
-  best.nslots = (best.nslots < kMaxSlots ? best.nslots : kMaxSlots) / kSets * kSets;  // a slot belongs to one dequant set
   best.box_rows = best.bn / 2;
-  best.smem = best.nstages * stage + best.nslots * slot + 1024;
   best.ws_floats = best.sk_tiles > 0 ? (size_t)best.npairs * 4 * best.bn * 128 : 0;
   return best;
 }

@@ -863,3 +863,11 @@ int32_t qeng_gemm_many_rows(qeng_ctx* ctx, const qeng_weight* w, const void* x, 
   }
   return rc;
 }
+
+// For the tests, which have to meet every kind of plan: chunks a stage, tokens a tile, accumulators, whole tiles, cut tiles, pairs.
+extern "C" int32_t qeng_many_rows_plan(const qeng_ctx* ctx, const qeng_weight* w, int64_t M, int32_t wp, int32_t xp, int32_t epilogue, int32_t* out) {
+  const Plan pl = make_plan(ctx, w, M, wp, xp, epilogue, true);
+  const int v[6] = {pl.kst, pl.bn, pl.nacc, pl.dp_tiles, pl.sk_tiles, pl.npairs};
+  std::copy(v, v + 6, out);
+  return QENG_OK;
+}

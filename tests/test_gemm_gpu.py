@@ -172,8 +172,8 @@ def _sample_rows(m):
 
 @pytest.mark.parametrize("m,n,k", [(2048, 11008, 4096), (8192, 11008, 4096), (8192, 4096, 11008), (2049, 11024, 4096)])
 def test_prefill_wide_tile_kernel(ctx, m, n, k):
-    """The M = 2048 and 8192 cases of the prefill sweep select the 256-wide output tile (all 512
-    tensor-memory columns); (2049, 11024) adds a partial last row tile and a partial last column
+    """The M = 2048 and 8192 cases of the prefill sweep take the widest output tiles (one accumulator of
+    256 tensor-memory columns); (2049, 11024) adds a partial last row tile and a partial last column
     tile.  The device computes every row; the oracle checks a sample of rows that covers every
     position inside a tile (the float64 product of the full matrix would take minutes)."""
     import torch

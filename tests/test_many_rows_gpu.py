@@ -47,22 +47,75 @@ def test_rows_and_widths(ctx, fmt, m):
     ctx.device_status()
 
 
-# One-term operands: the smallest and largest token tiles with two accumulators and with one, remainders of both, tiles cut
-# along K and whole ones, more tiles than CTA pairs.  Against operands rounded to bf16, only the sums differ: bound as above.
-@pytest.mark.parametrize("m,n,k", [(256, 272, 736), (257, 4096, 992), (320, 1040, 4096), (416, 4112, 2048), (777, 2064, 4064), (2049, 4096, 544)])
-def test_prompt_rows_and_widths(ctx, m, n, k):
+def _plan(ctx, w, m, wp, xp, epilogue):
+    """What the planner of the many-row matmul chose, for the tests below to know what they ran."""
+    import ctypes
+    from cyb_b200 import qeng
+    out = (ctypes.c_int32 * 6)()
+    fn = qeng._lib.qeng_many_rows_plan
+    fn.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32, ctypes.c_void_p]
+    assert fn(ctx.h, w.h, m, wp, xp, epilogue, out) == 0
+    chunks, width, accumulators, whole, cut, pairs = out
+    kind = "mixed" if whole and cut else "cut" if cut else "rounds" if whole > pairs else "one round"
+    return chunks, width, accumulators, kind
+
+
+# Every kind of plan: stages of two chunks or one, one accumulator (which the dequantising warps help to add to y) or two,
+# tiles all whole (one round, or several to a pair), all cut along K, or both; rows and widths that fill no tile; the widest
+# tile.  Stored and added to y.  One weight term (256 rows of 4-bit blocks and more) against operands rounded to bf16, two
+# against exact ones; bound as above.
+@pytest.mark.parametrize("fmt,m,n,k,plan", [
+    ("q4", 412, 7360, 288, (2, 208, 1, "one round")), ("q4", 649, 12432, 544, (2, 224, 1, "rounds")),
+    ("q4", 823, 1840, 5792, (2, 208, 1, "cut")), ("q4", 321, 10720, 5504, (2, 176, 1, "mixed")),
+    ("q4", 260, 19792, 544, (2, 144, 2, "rounds")), ("q4", 271, 272, 3488, (2, 80, 2, "cut")),
+    ("q4", 274, 9536, 4480, (2, 96, 2, "mixed")), ("q4", 2025, 4112, 4096, (2, 256, 1, "rounds")),
+    ("q4", 206, 10288, 320, (1, 208, 1, "one round")), ("q8", 167, 18960, 1408, (1, 176, 1, "rounds")),
+    ("q8", 197, 5424, 3616, (1, 208, 1, "cut")), ("q8", 196, 21072, 1472, (1, 208, 1, "mixed")),
+    ("q4", 207, 19232, 256, (1, 112, 2, "rounds")), ("q4", 161, 304, 3488, (1, 80, 2, "cut")),
+    ("q8", 33, 21568, 1504, (1, 48, 2, "mixed")), ("q8", 73, 448, 480, (2, 80, 1, "one round")),
+    ("q4", 78, 19776, 864, (2, 80, 1, "rounds")), ("q8", 65, 10400, 3168, (2, 80, 1, "cut")),
+    ("q4", 67, 20512, 2816, (2, 80, 1, "mixed")), ("q4", 33, 336, 1984, (2, 48, 2, "cut")),
+    ("q8", 38, 21712, 1920, (2, 48, 2, "mixed"))])
+def test_every_kind_of_plan(ctx, fmt, m, n, k, plan):
     import torch
-    w = _weight(ctx, "q4", n, k)
-    wd = w.dequant().bfloat16().double()
-    for dt in DT[:2]:
-        x = torch.randn(m, k, device="cuda").to(getattr(torch, dt))
-        y = torch.full((m, n + 8), 0.25, device="cuda")[:, :n]
-        acc = m % 2
-        ctx.gemm_q4(w, x, out=y, flags=acc)
-        want = x.bfloat16().double() @ wd.T + (0.25 if acc else 0.0)
-        err = float((y.double() - want).abs().max() / want.abs().max())
-        assert err < 3e-5, (m, n, k, dt, err)
+    w = _weight(ctx, fmt, n, k)
+    one_term = fmt == "q4" and m >= 256
+    rounded = (lambda t: t.bfloat16()) if one_term else (lambda t: t)
+    wd = rounded(w.dequant()).double()
+    for acc in (0, 1):
+        assert _plan(ctx, w, m, 1 if one_term else 2, 1 if one_term else 2, acc) == plan
+        for dt in DT[:2] if one_term else DT[:1]:
+            x = torch.randn(m, k, device="cuda").to(getattr(torch, dt))
+            y = torch.full((m + 1, n + 8), 0.25, device="cuda")
+            ctx.gemm_q4(w, x, out=y[:m, :n], flags=acc)
+            want = rounded(x).double() @ wd.T + (0.25 if acc else 0.0)
+            err = float((y[:m, :n].double() - want).abs().max() / want.abs().max())
+            assert err < 3e-5, (fmt, m, n, k, acc, dt, err)
+            assert bool((y[m] == 0.25).all()) and bool((y[:, n:] == 0.25).all())
     ctx.device_status()
+
+
+def test_prompt_epilogues_over_several_tiles(ctx):
+    """Rotary embedding with KV append, SwiGLU and the residual adds where CTA pairs run several tiles through one
+    accumulator, then cut ones: a layer over 895 rows against the float64 teacher (operands rounded to bf16: 5e-3)."""
+    import torch
+    from cyb_b200 import qeng
+    T = 895
+    cfg = ref.DecoderConfig(layers=1, d=512, ffn=4096, heads=32, kv_heads=8, vocab=320)
+    W = ref.make_decoder_weights(cfg, seed=5)
+    dec = ctx.decoder(layers=1, d_model=512, ffn=4096, heads=32, kv_heads=8, vocab=320, max_batch=1, max_seq=896)
+    qeng.load_decoder_weights(dec, W, cfg)
+    SWIGLU, QKV = 3, 4
+    assert _plan(ctx, dec.weight(0, 0), T, 1, 1, QKV)[2:] == (1, "mixed")
+    assert _plan(ctx, dec.weight(0, 2), T, 1, 1, SWIGLU)[2:] == (1, "mixed")
+    teacher = ref.Decoder(cfg, W)
+    teacher.reset(1)
+    x = ref.rng_of(41).standard_normal((1, T, cfg.d), dtype=np.float32)
+    want = teacher.layer(0, x.astype(np.float64), np.arange(T)[None])
+    got = dec.layer(0, torch.from_numpy(x[0]).cuda(), np.arange(T)).cpu().numpy()
+    ctx.device_status()
+    assert ref.err_inf(got, want[0]) < 5e-3
+    dec.free()
 
 
 # Query heads per kv head: one, the most there are, and counts that do not divide the 64 rows of a prompt attention tile

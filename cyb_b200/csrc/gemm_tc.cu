@@ -456,7 +456,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
       if (!failed && !mbar_wait(smem_u32(acc_full + buf), acc_ph)) failed = true;
       __syncwarp();
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-      if (!__any_sync(0xffffffffu, failed)) 
+      if (!__any_sync(0xffffffffu, failed))
         drain<HELP>(p, sg.tile, whole, pair, rank, tmem + (uint32_t)(buf * p.acc_cols), quad, lane, 0, HELP && whole ? 16 * (1 + kHelpers / 4) : 16);
       asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
       __syncwarp();
@@ -687,7 +687,9 @@ Plan make_plan(const qeng_ctx* ctx, const qeng_weight* w, int64_t M, int wp, int
       const double share = (double)rem * nk / sharing, parts = 1 + std::max(1.0, nk / std::max(share, 1.0));
       // the share of a cut tile has to hide the epilogue of the pair's last whole one, old values of y from HBM among it
       const double tail = c.nacc == 1 || T < pairs ? 0.0 : std::max(0.0, (epi == QENG_EPI_ACCUM ? 100 : per_token) * bn - share * stage);
-      const double sk = (T / pairs) * tile + share * stage + tail + (c.nacc == 1 ? 64.0 : 38.0) * bn + 700 * parts + 9400;
+      // (whole and cut tiles added to y took 1.5 to 5 us more than stored ones, cut tiles alone 1)
+      const double mixed = epi == QENG_EPI_ACCUM && T >= pairs ? 4000.0 : 0.0;
+      const double sk = (T / pairs) * tile + share * stage + tail + mixed + (c.nacc == 1 ? 64.0 : 38.0) * bn + 700 * parts + 9400;
       const bool cut = may_split && rem != 0 && sk < dp && (T < pairs || (int64_t)rem * nk >= 2 * (int64_t)pairs);
       const double cost = cut ? sk : dp;
       if (cost >= best_cost) continue;

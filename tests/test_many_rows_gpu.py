@@ -68,11 +68,11 @@ def _plan(ctx, w, m, wp, xp, epilogue):
     ("q4", 412, 7360, 288, (2, 208, 1, "one round")), ("q4", 649, 12432, 544, (2, 224, 1, "rounds")),
     ("q4", 823, 1840, 5792, (2, 208, 1, "cut")), ("q4", 321, 10720, 5504, (2, 176, 1, "mixed")),
     ("q4", 260, 19792, 544, (2, 144, 2, "rounds")), ("q4", 271, 272, 3488, (2, 80, 2, "cut")),
-    ("q4", 274, 9536, 4480, (2, 96, 2, "mixed")), ("q4", 2025, 4112, 4096, (2, 256, 1, "rounds")),
+    ("q4", 260, 9504, 5248, (2, 96, 2, "mixed")), ("q4", 2025, 4112, 4096, (2, 256, 1, "rounds")),
     ("q4", 206, 10288, 320, (1, 208, 1, "one round")), ("q8", 167, 18960, 1408, (1, 176, 1, "rounds")),
-    ("q8", 197, 5424, 3616, (1, 208, 1, "cut")), ("q8", 196, 21072, 1472, (1, 208, 1, "mixed")),
+    ("q8", 197, 5424, 3616, (1, 208, 1, "cut")), ("q8", 194, 20864, 1664, (1, 208, 1, "mixed")),
     ("q4", 207, 19232, 256, (1, 112, 2, "rounds")), ("q4", 161, 304, 3488, (1, 80, 2, "cut")),
-    ("q8", 33, 21568, 1504, (1, 48, 2, "mixed")), ("q8", 73, 448, 480, (2, 80, 1, "one round")),
+    ("q8", 33, 20640, 2144, (1, 48, 2, "mixed")), ("q8", 73, 448, 480, (2, 80, 1, "one round")),
     ("q4", 78, 19776, 864, (2, 80, 1, "rounds")), ("q8", 65, 10400, 3168, (2, 80, 1, "cut")),
     ("q4", 67, 20512, 2816, (2, 80, 1, "mixed")), ("q4", 33, 336, 1984, (2, 48, 2, "cut")),
     ("q8", 38, 21712, 1920, (2, 48, 2, "mixed"))])

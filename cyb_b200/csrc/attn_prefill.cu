@@ -10,7 +10,7 @@
 //
 // Least time: 24 MMAs of 2 cycles per 16 x 8 scores (8 for the scores, 16 for the values); 2 * 128 * 3 * heads * T^2 / 2
 // operations for a prompt of T tokens = 73 us per layer at T = 1800 and 32 heads.  It takes 148 there (ncu; 212 with the
-// CTAs in head order): the tensor pipe is busy 53 % of the cycles in which an SM has work (dependent steps of the softmax
+// CTAs in head order): the tensor pipe is busy 57 % of the cycles in which an SM has work (dependent steps of the softmax
 // between the two products, 12 consumer warps per SM).
 #include <cuda.h>
 #include <cuda_bf16.h>

@@ -28,8 +28,9 @@ constexpr int kMaxRing = 16;
 // Fewer rows: the integer kernel is faster (11008 x 4096, f32: 4 rows 11.0 against 13.2 us, 8 rows 15.2 against 14; bf16: 3 rows
 // 4096 x 4096 7.1 against 5.4).
 constexpr int kLeastF32 = 5, kLeastBf16 = 3;
-// Beyond this many columns the tensor-memory kernel is faster: 11008 x 4096, 32 rows: bf16 (32 columns) 24.6 against 31.9 us,
-// f32 (64 columns) 41.7 against 28.8.
+// Beyond this many columns the tensor-memory kernel (gemm_tc.cu) takes over.  Here / there, 11008 x 4096, 4-bit: 16 rows bf16 14.2 /
+// 21.9 us, 32 rows 21.4 / 22.3, 16 rows f32 (32 columns) 19.7 / 24.6; 8-bit, 32 rows bf16 27.1 / 26.3, 16 rows f32 24.0 / 28.3;
+// K-quant, 17 rows bf16 29.7 / 28.6, 32 rows 32.5 / 28.8, 16 rows f32 22.4 / 30.8.  (Over 4096 x 4096 all are faster here.)
 constexpr int kMostCols = 32;
 constexpr size_t kBudget = 226 * 1024 - 1024;
 

@@ -71,7 +71,6 @@ struct StepParams {
   unsigned* sync;       // [0] steps completed (the tag base), [1] grid-barrier arrivals
   int32_t* status;
   int nstages;          // ring slots
-  uint32_t zero_bytes;  // bytes of the zero region at the head of the staging area
   unsigned long long* trace;  // [2 CTAs (first, last)][layers][16] %globaltimer stamps of the phases
 };
 
@@ -167,10 +166,6 @@ __global__ void __launch_bounds__(kThreads, 1) decode_step_kernel(const StepPara
   int tcount = 0;        // tiles of this CTA so far (all operators): tile -> group tcount % kTG
   int buf = 0;
   bool ring_failed = false;
-
-  // zero region of the staging area (the lanes of other blocks' columns read it)
-  for (uint32_t o = (uint32_t)tid * 16u; o < p.zero_bytes; o += kCT * 16u)
-    asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};\n" ::"r"(xbase + 64u + o), "r"(0u) : "memory");
 
   // the residual stream: this thread owns k = 8 tid .. 8 tid + 7 of every row
   const int k0 = tid * 8;
@@ -274,7 +269,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_step_kernel(const StepPara
         q += (unsigned)spt;  // another group's tile
         continue;
       }
-      float acc[2] = {0.f, 0.f};
+      f32x2 acc[2] = {0ull, 0ull};
       for (int c0 = 0; c0 < M.nchunks; c0 += kStageChunks, ++q) {
         const int s = (int)(q % (unsigned)NS);
         const uint32_t ph = (q / (unsigned)NS) & 1u;
@@ -282,24 +277,18 @@ __global__ void __launch_bounds__(kThreads, 1) decode_step_kernel(const StepPara
         const int nc = min(kStageChunks, M.nchunks - c0);
         const uint32_t wb = smem_u32(ring) + (uint32_t)s * kSlotBytes;
         const uint32_t sb = wb + kStageChunks * 512u;
-        if (mode == kM1L3) consume_m1l3<kGW>(acc, wb, sb, nc, c0 * 2, L, xbase, wi, lane);
-        else if (mode == kM1L2) consume_g4<kGW>(acc, wb, sb, nc, c0 * 2, L, xbase, wi, lane);
-        else consume_g2<kGW>(acc, wb, sb, nc, c0 * 2, L, xbase, wi, lane);
+        const uint32_t wl = wb + (uint32_t)lane * 16u, sl = sb + (uint32_t)g * 8u;
+        if (mode == kM1L2) consume_x4<kGW>(acc, wl, sl + (uint32_t)(t & 1) * 64u, nc, c0 * 2, lane_x4(L, xbase, lane), wi, lane);
+        else consume_x2<kGW>(acc, wl, sl, nc, c0 * 2, lane_x2(L, xbase, mode == kM1L3 ? 3 : 4, lane), wi);
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(empty + s));
       }
       float* myred = red + (((size_t)gi * 2 + buf) * kGW + wi) * red_stride;
-      if (B == 1) {
-        acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 1);
-        acc[1] += __shfl_xor_sync(0xffffffffu, acc[1], 1);
-        acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 2);
-        acc[1] += __shfl_xor_sync(0xffffffffu, acc[1], 2);
-        if (t == 0) { myred[g] = acc[0]; myred[g + 8] = acc[1]; }
-      } else {
-        acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 1);
-        acc[1] += __shfl_xor_sync(0xffffffffu, acc[1], 1);
-        if ((t & 1) == 0) { myred[(t >> 1) * 16 + g] = acc[0]; myred[(t >> 1) * 16 + g + 8] = acc[1]; }
-      }
+      float a0 = sum2(acc[0]), a1 = sum2(acc[1]);
+      if (mode == kM1L3 && t == 3) a0 = a1 = 0.f;
+      const float part = quad_rows(a0, a1, lane, B == 1);
+      if (B != 1) myred[(t >> 1) * 16 + g + 8 * (t & 1)] = part;
+      else if (t < 2) myred[g + 8 * t] = part;
       group_sync(gi);
       if (wi == (tg_count % kGW)) {
         const float* rb = red + ((size_t)gi * 2 + buf) * kGW * red_stride;
@@ -381,7 +370,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_step_kernel(const StepPara
     if (l > 0) gather(1, tag_d - 2u);
     {
       const int mode = B == 1 ? kM1L3 : kM2L2;
-      const XLayout L = x_layout(B == 1 ? 3 : 4, Ly.m[0].nchunks, true, p.zero_bytes);
+      const XLayout L = x_layout(B == 1 ? 3 : 4, Ly.m[0].nchunks, true);
       stamp(l, 1);
       stage_norm(gain1, mode, L);
       stamp(l, 2);
@@ -401,8 +390,8 @@ __global__ void __launch_bounds__(kThreads, 1) decode_step_kernel(const StepPara
         const int npages = min((len + 15) >> 4, p.max_pages);
         const int S = max(1, min(kMaxSplit, (npages + kCW - 1) / kCW));
         if (s < S) {
-          // staging area (behind the zero region): q as f32 [grp][128], then the warps' partials
-          float* qsm = reinterpret_cast<float*>(xreg + 64 + ((p.zero_bytes + 127) & ~127u));
+          // staging area: q as f32 [grp][128], then the warps' partials
+          float* qsm = reinterpret_cast<float*>(xreg);
           float* sm_o = qsm + 4 * kHD;                     // [kCW][4][128]
           float* sm_ml = sm_o + kCW * 4 * kHD;             // [kCW][4][2]
           for (int i = tid; i < p.grp * kHD; i += kCT)
@@ -523,7 +512,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_step_kernel(const StepPara
     {
       const int mode = B == 1 ? kM1L2 : kM2L2;
       const int K = p.Hq * kHD;
-      const XLayout L = x_layout(2 * B, B == 1 ? (Ly.m[1].nchunks + 1) & ~1 : Ly.m[1].nchunks, true, p.zero_bytes);
+      const XLayout L = x_layout(2 * B, B == 1 ? (Ly.m[1].nchunks + 1) & ~1 : Ly.m[1].nchunks, B == 2);
       stage_plain(
           [&](int b, int kk, bool valid, float(&v)[8]) {
 #pragma unroll
@@ -563,7 +552,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_step_kernel(const StepPara
     stamp(l, 9);
     {
       const int mode = B == 1 ? kM1L2 : kM2L2;
-      const XLayout L = x_layout(2 * B, B == 1 ? (Ly.m[2].nchunks + 1) & ~1 : Ly.m[2].nchunks, true, p.zero_bytes);
+      const XLayout L = x_layout(2 * B, B == 1 ? (Ly.m[2].nchunks + 1) & ~1 : Ly.m[2].nchunks, B == 2);
       stage_norm(gain2, mode, L);
       stamp(l, 10);
       run_tiles(Ly.m[2], mode, L, kEpiSwiglu, l, tag_o, 0);
@@ -573,7 +562,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_step_kernel(const StepPara
     // ---- down ------------------------------------------------------------------------------------------
     {
       const int mode = B == 1 ? kM1L2 : kM2L2;
-      const XLayout L = x_layout(2 * B, B == 1 ? (Ly.m[3].nchunks + 1) & ~1 : Ly.m[3].nchunks, true, p.zero_bytes);
+      const XLayout L = x_layout(2 * B, B == 1 ? (Ly.m[3].nchunks + 1) & ~1 : Ly.m[3].nchunks, B == 2);
       stage_plain(
           [&](int b, int kk, bool valid, float(&v)[8]) {
 #pragma unroll
@@ -645,7 +634,7 @@ int32_t qeng_step_create(qeng_ctx* ctx, const qeng_step_desc& d, qeng_step** out
   if (d.dm % 128 != 0 || d.dm > 8 * kCT || grp < 1 || grp > 4 || d.F % 8 != 0) return QENG_OK;
   if (kMaxB * d.Hkv * kMaxSplit > ctx->sm_count) return QENG_OK;
   if (d.world > 1 && !d.peer_inbox[0]) return QENG_OK;
-  // staging area: zero region + the widest operand (down: K = F, or q|k|v in three limbs), or the attention buffers
+  // staging area: the widest operand (down: K = F, or q|k|v in three limbs), or the attention buffers
   int max_chunks = 0;
   for (const auto& L : d.layers)
     for (int i = 0; i < 4; ++i) {
@@ -653,13 +642,12 @@ int32_t qeng_step_create(qeng_ctx* ctx, const qeng_step_desc& d, qeng_step** out
       max_chunks = (int)L.w[i]->nchunks > max_chunks ? (int)L.w[i]->nchunks : max_chunks;
     }
   const int alloc = (max_chunks + 1) & ~1;
-  const uint32_t zero_bytes = x_zero_bytes(x_layout(2, alloc, true));
   size_t xbytes = 0;
   for (int cols : {3, 4}) {
-    const XLayout L = x_layout(cols, alloc, true, zero_bytes);
+    const XLayout L = x_layout(cols, alloc, true);
     xbytes = L.bytes > xbytes ? L.bytes : xbytes;
   }
-  const size_t attn = 64 + ((zero_bytes + 127) & ~127u) + kAttnBytes + 256;
+  const size_t attn = kAttnBytes + 256;
   if (attn > xbytes) xbytes = attn;
   xbytes = (xbytes + 127) & ~(size_t)127;
   const size_t budget = 226 * 1024 - 6 * 1024;  // static shared memory of the kernel comes on top
@@ -708,7 +696,7 @@ int32_t qeng_step_create(qeng_ctx* ctx, const qeng_step_desc& d, qeng_step** out
   p.world = d.world; p.rank = d.rank;
   for (int r = 0; r < 8; ++r) p.inbox[r] = d.world == 1 ? (r == 0 ? s->own_inbox : nullptr) : reinterpret_cast<uint2*>(d.peer_inbox[r]);
   p.sync = s->sync; p.status = ctx->status;
-  p.nstages = ns; p.zero_bytes = zero_bytes; p.trace = s->trace;
+  p.nstages = ns; p.trace = s->trace;
   s->smem = (size_t)ns * kSlotBytes + xbytes;
   s->grid = ctx->sm_count;
   // opt-in dynamic shared memory: the kernel's static arrays come on top, so ask for what is used

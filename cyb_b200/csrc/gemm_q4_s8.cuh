@@ -19,22 +19,17 @@
 // f32 accumulation.  One-hot or power-of-two activations are exact.
 //
 // Column use of the 8-wide MMA tile.  One activation row in two limbs: the 8 columns hold
-// (limb, block) for FOUR consecutive blocks; the MMA of block j gets activation bytes only in the
-// two columns of block j (the other lanes' bytes are masked to zero), so four blocks share one
-// accumulator fragment and the f32 post-processing is paid once per four blocks.  One row in three
-// limbs, or two rows: two blocks per fragment (the lanes of the other block read a zero region).
+// (limb, block) for FOUR consecutive blocks of activations.  Each of the four blocks of weights is multiplied
+// by all of them, into an accumulator of its own; the two columns that belong to it are picked out afterwards
+// (four selects, where masking the other blocks' activations was eight ANDs and a chain of dependent MMAs),
+// and the f32 post-processing is paid once per four blocks, two values an instruction.  One row in three
+// limbs, or two rows: two blocks, whose columns lie in one lane: nothing to select.
 // Three or four rows: one block per fragment, columns = (row, limb).  More rows: several such
 // 8-column tiles.
 #pragma once
 #include "qeng_internal.h"
 
-#ifndef QENG_G4_UNROLL
-#define QENG_G4_UNROLL 2
-#endif
-
 namespace q4s8 {
-constexpr int kG4Unroll = QENG_G4_UNROLL;  // items of the one-row loop in flight per warp
-
 constexpr int kCW = 16;               // consumer warps
 constexpr int kCT = kCW * 32;         // consumer threads
 constexpr int kThreads = kCT + 32;    // + producer warp
@@ -103,27 +98,47 @@ __device__ __forceinline__ uint32_t lds32(uint32_t addr) {
 __device__ __forceinline__ void sts64(uint32_t addr, uint32_t a, uint32_t b) {
   asm volatile("st.shared.v2.u32 [%0], {%1,%2};\n" ::"r"(addr), "r"(a), "r"(b) : "memory");
 }
-// d += a.b : 16 rows x 32 k of u8 codes (a) times 32 k x 8 columns of s8 activation bytes (b), s32
+// d = c + a.b : 16 rows x 32 k of u8 codes (a) times 32 k x 8 columns of s8 activation bytes (b), s32
 __device__ __forceinline__ void imma(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                     uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-      : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+                                     uint32_t b1, const int (&c)[4]) {
+  asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};\n"
+      : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(c[0]), "r"(c[1]), "r"(c[2]), "r"(c[3]));
 }
 // one 32-block of 16 weight rows: lane (g, t) holds w0 = codes of row g, w1 = codes of row g+8, each
 // the 8 codes of k = 8t + j in nibble qeng_nib(j).  The even nibbles (j = 0,4,1,5) land in the MMA's k
 // slots 4t..4t+3, the odd ones (j = 2,6,3,7) in 16+4t..16+4t+3; the staged activation bytes use the same order.
-__device__ __forceinline__ void block_mma(int (&d)[4], uint32_t w0, uint32_t w1, uint32_t b0, uint32_t b1) {
+__device__ __forceinline__ void block_mma(int (&d)[4], uint32_t w0, uint32_t w1, uint32_t b0, uint32_t b1, const int (&c)[4]) {
   const uint32_t m = 0x0f0f0f0fu;
-  imma(d, w0 & m, w1 & m, (w0 >> 4) & m, (w1 >> 4) & m, b0, b1);
+  imma(d, w0 & m, w1 & m, (w0 >> 4) & m, (w1 >> 4) & m, b0, b1, c);
 }
 // the same contraction for 8-bit block weights (signed bytes): no unpacking, no zero point
 __device__ __forceinline__ void imma_s8(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                        uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-      : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+                                        uint32_t b1, const int (&c)[4]) {
+  asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};\n"
+      : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(c[0]), "r"(c[1]), "r"(c[2]), "r"(c[3]));
 }
+// two f32 values in a register pair: one instruction works on both
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pair2(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};\n" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float sum2(f32x2 v) { return __uint_as_float((uint32_t)v) + __uint_as_float((uint32_t)(v >> 32)); }
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;\n" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+// d += a * b
+__device__ __forceinline__ void fma2(f32x2& d, f32x2 a, f32x2 b) { asm("fma.rn.f32x2 %0, %1, %2, %0;\n" : "+l"(d) : "l"(a), "l"(b)); }
 // Weight format of a matmul: Q4 = 4-bit codes (two 32-blocks per uint4 and lane, 512 B per 64-wide
 // chunk of a row tile); Q8 = signed bytes (one 32-block per uint4 and lane: the bytes of row g at
 // k = 8t + 0,4,1,5, of row g+8 likewise, then k = 8t + 2,6,3,7 of both rows, i.e. the A registers of
@@ -135,22 +150,23 @@ struct WBlocks {
 };
 template <bool Q8>
 __device__ __forceinline__ uint32_t chunk_bytes() { return Q8 ? 1024u : 512u; }
+// `lane_addr`: the chunk's address + 16 * lane
 template <bool Q8>
-__device__ __forceinline__ WBlocks<Q8> load_chunk(uint32_t chunk_addr, int lane) {
+__device__ __forceinline__ WBlocks<Q8> load_chunk(uint32_t lane_addr) {
   WBlocks<Q8> w;
-  w.lo = lds128(chunk_addr + (uint32_t)lane * 16u);
-  if (Q8) w.hi = lds128(chunk_addr + 512u + (uint32_t)lane * 16u);
+  w.lo = lds128(lane_addr);
+  if (Q8) w.hi = lds128(lane_addr + 512u);
   return w;
 }
-// d += block j (0 or 1) of the chunk times the activation bytes (b0, b1)
+// d = c + block j (0 or 1) of the chunk times the activation bytes (b0, b1)
 template <bool Q8>
-__device__ __forceinline__ void chunk_mma(int (&d)[4], const WBlocks<Q8>& w, int j, uint32_t b0, uint32_t b1) {
+__device__ __forceinline__ void chunk_mma(int (&d)[4], const WBlocks<Q8>& w, int j, uint32_t b0, uint32_t b1, const int (&c)[4]) {
   if (Q8) {
     const uint4& a = j == 0 ? w.lo : w.hi;
-    imma_s8(d, a.x, a.y, a.z, a.w, b0, b1);
+    imma_s8(d, a.x, a.y, a.z, a.w, b0, b1, c);
   } else {
-    if (j == 0) block_mma(d, w.lo.x, w.lo.y, b0, b1);
-    else block_mma(d, w.lo.z, w.lo.w, b0, b1);
+    if (j == 0) block_mma(d, w.lo.x, w.lo.y, b0, b1, c);
+    else block_mma(d, w.lo.z, w.lo.w, b0, b1, c);
   }
 }
 __device__ __forceinline__ float unbias(int d) { return __int_as_float(d) - kBiasF; }
@@ -193,42 +209,56 @@ __device__ __forceinline__ float act_f32(const void* x, int dtype, long long i) 
   return __uint_as_float((uint32_t)reinterpret_cast<const uint16_t*>(x)[i] << 16);
 }
 
+// The same as (even block, odd block) pairs of row g (d0, m0) and row g+8 (d1, m1); `at`: the chunk's scales + the lane group's
+// offset (8 g, or 32 g with KQ)
+template <bool KQ>
+struct PairScales {
+  f32x2 d0, d1, m0, m1;
+};
+template <bool KQ>
+__device__ __forceinline__ PairScales<KQ> load_pairs(uint32_t at, bool live = true) {
+  PairScales<KQ> r;
+  if (KQ) {
+    uint4 a = lds128(at), b = lds128(at + 16u);
+    if (!live) a = b = make_uint4(0u, 0u, 0u, 0u);
+    r.d0 = pair2(__uint_as_float(a.x), __uint_as_float(a.z));
+    r.d1 = pair2(__uint_as_float(a.y), __uint_as_float(a.w));
+    r.m0 = pair2(-__uint_as_float(b.x), -__uint_as_float(b.z));
+    r.m1 = pair2(-__uint_as_float(b.y), -__uint_as_float(b.w));
+  } else {
+    uint2 s2 = lds64(at);
+    if (!live) s2 = make_uint2(0u, 0u);
+    const uint32_t g0 = __byte_perm(s2.x, s2.y, 0x5410), g8 = __byte_perm(s2.x, s2.y, 0x7632);
+    const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&g0)), b = __half22float2(*reinterpret_cast<const __half2*>(&g8));
+    r.d0 = pair2(a.x, a.y);
+    r.d1 = pair2(b.x, b.y);
+    r.m0 = r.m1 = 0ull;
+  }
+  return r;
+}
+
 // Shared-memory geometry of the staged activations of one K slice (bytes, relative to `base`).
 //   xq   : [cols][col_stride]  s8 bytes; column c = 2 * row + limb; inside a column the 32 bytes of
 //          block b start at 32 b: [t 0..3][k = 8t + 0,4,1,5,2,6,3,7]
-//   zero : col_stride bytes of zeros (only when several blocks share a fragment)
 //   zin  : [cols][nblk] int32   kBias - 8 * (sum of the column's bytes in the block)
 //   fex  : [cols][nblk] float   2^e (x 128 for the hi limb), 0 for blocks beyond K
 struct XLayout {
-  uint32_t col_stride, xq, zero, zin, fex, bytes;
+  uint32_t col_stride, xq, zin, fex, bytes;
   uint32_t fsx;  // [cols][nblk] float: fex * (sum of the column's bytes in the block); 0 = not staged (only
                  // weight formats with a per-block minimum need the block sums of the activations)
   uint32_t zs;  // bytes per column of zin / fex (padded so that the columns read together fall in different banks)
   int nblk;
 };
-// zeroed = true when several blocks share an accumulator fragment (the lanes of the other blocks
-// read zeros); chunks = 64-wide K chunks of the slice.  zero_reserved > 0 puts the zero region
-// first, at a fixed place and size whatever the columns are (a kernel that stages several
-// different operands clears it once); it must be >= x_zero_bytes of every layout used.
-__host__ __device__ inline XLayout x_layout(int cols, int chunks, bool zeroed, uint32_t zero_reserved = 0, bool sums = false) {
+// chunks = 64-wide K chunks of the slice.  two_blocks: the 8 MMA columns are four (row, limb) columns x two blocks.
+__host__ __device__ inline XLayout x_layout(int cols, int chunks, bool two_blocks, bool sums = false) {
   XLayout L;
   L.nblk = chunks * 2;
   const uint32_t raw = ((uint32_t)chunks * 64u + 127u) / 128u * 128u;
-  // Bank rule for the 64-bit activation loads: a half-warp (lane groups g = 0..3 or 4..7) reads at
-  // most two different columns plus the zero region, 32 bytes each.  Columns sit 32 bytes apart
-  // (mod 128); the zero region starts 64 bytes off (mod 128) and the upper half-warp enters it
-  // another 64 bytes further on.
-  L.col_stride = raw + 32u;
-  uint32_t after;
-  if (zero_reserved > 0) {
-    L.zero = 64u;
-    L.xq = (64u + zero_reserved + 127u) / 128u * 128u;
-    after = L.xq + (uint32_t)cols * L.col_stride;
-  } else {
-    L.xq = 0;
-    L.zero = ((uint32_t)cols * L.col_stride + 127u) / 128u * 128u + 64u;
-    after = zeroed ? L.zero + raw + 128u : (uint32_t)cols * L.col_stride;
-  }
+  // Bank rule for the 64-bit activation loads: a half-warp (lane groups g = 0..3 or 4..7) reads 32 bytes each of four
+  // neighbouring columns, of two columns x two blocks, or of four blocks of a column: all in different banks.
+  L.col_stride = raw + (two_blocks ? 64u : 32u);
+  L.xq = 0;
+  const uint32_t after = (uint32_t)cols * L.col_stride;
   L.zin = (after + 127u) & ~127u;
   L.zs = ((uint32_t)L.nblk * 4u + 127u) / 128u * 128u + 16u;
   L.fex = L.zin + (uint32_t)cols * L.zs;
@@ -240,9 +270,6 @@ __host__ __device__ inline XLayout x_layout(int cols, int chunks, bool zeroed, u
   }
   return L;
 }
-// bytes of the zero region (to be cleared once per kernel)
-__host__ __device__ inline uint32_t x_zero_bytes(const XLayout& L) { return L.col_stride - 32u + 128u; }
-
 // Quantise 8 consecutive activations (one (block, t) group of a row) and store its limbs.
 // `v` are the final f32 values (norm applied).  The four lanes of a quad hold one 32-block.
 // Every lane of the warp must call this (shuffles); `valid` gates the stores.
@@ -320,151 +347,122 @@ __device__ __forceinline__ void quantise_group(const float (&v)[8], bool valid, 
 }
 
 // ---- the per-stage contraction ------------------------------------------------------------
-// One call processes this warp's share of a stage: `nc` chunks of 64 k of one 16-row tile, already
-// in shared memory at `wbase` (nibbles, 512 B per chunk) and `sbase` (scales, 64 B per chunk).
-// blk0 = index (inside the staged slice) of the stage's first block.  Warp `wi` of `NW` takes the
-// work items wi, wi + NW, ...; an item is max(G/2, 1) chunks.
+// One call processes this warp's share of a stage: `nc` chunks of 64 k of one 16-row tile, already in shared memory.
+// Warp `wi` of `NW` takes the work items wi, wi + NW, ...
+// What a lane reads of the staged activations, as addresses for block 0 of the slice: worked out once per kernel, as are its
+// offsets into a stage.  What bounds these loops is the instructions around the MMAs (40 per 16 x 32 block and warp with addresses
+// and ring positions worked out per stage, masked activations and one f32 operation a value: the issue slots of 1280 of the 1440
+// cycles that HBM takes per tile).  One row, 15 bits / 22 bits, microseconds before and now, L2 cold: 22016 x 4096 13.6 / 14.0 ->
+// 11.4 / 12.4, 11008 x 4096 7.8 / 8.2 -> 7.0 / 7.5, 4096 x 11008 8.7 / 9.4 -> 8.0 / 8.5, 4096 x 4096 4.6 / 4.8 -> 4.4 / 4.4.
+struct LaneX {
+  uint32_t xa, zin, fex, fsx;
+};
+// one row in two limbs, four blocks an item: B column g = (limb g >> 2, block g & 3); the outputs of lane t are
+// limb t >> 1, blocks 2 (t & 1) and the next
+__device__ __forceinline__ LaneX lane_x4(const XLayout& L, uint32_t xbase, int lane) {
+  const uint32_t g = (uint32_t)lane >> 2, t = (uint32_t)lane & 3u, o = (t >> 1) * L.zs + (t & 1u) * 8u;
+  return {xbase + L.xq + (g >> 2) * L.col_stride + (g & 3u) * 32u + t * 8u, xbase + L.zin + o, xbase + L.fex + o, xbase + L.fsx + o};
+}
+// `cols` (row, limb) columns (3 or 4), two blocks an item: B column g = (column g >> 1, block g & 1); the outputs of lane t are
+// column t, both blocks (three limbs: what lane 3 has is nobody's)
+__device__ __forceinline__ LaneX lane_x2(const XLayout& L, uint32_t xbase, int cols, int lane) {
+  const uint32_t g = (uint32_t)lane >> 2, t = (uint32_t)lane & 3u, c = (uint32_t)cols - 1u, o = min(t, c) * L.zs;
+  return {xbase + L.xq + min(g >> 1, c) * L.col_stride + (g & 1u) * 32u + t * 8u, xbase + L.zin + o, xbase + L.fex + o, xbase + L.fsx + o};
+}
 
-// G = 4: one activation row.  acc[0] += row g, acc[1] += row g+8 (partial over this lane's columns).
+// d: the item's exact sums of row g / g+8 (even, odd block); acc: sums so far of row g, row g+8 (a pair each)
+template <bool KQ>
+__device__ __forceinline__ void add_item(f32x2 (&acc)[2], int e0, int o0, int e1, int o1, const PairScales<KQ>& S, f32x2 f, uint32_t fsx) {
+  const f32x2 bias = pair2(-kBiasF, -kBiasF);
+  const f32x2 v0 = add2(pair2(__int_as_float(e0), __int_as_float(o0)), bias), v1 = add2(pair2(__int_as_float(e1), __int_as_float(o1)), bias);
+  fma2(acc[0], mul2(S.d0, f), v0);
+  fma2(acc[1], mul2(S.d1, f), v1);
+  if (KQ) {  // - M * (block sum of the activations)
+    const uint2 q = lds64(fsx);
+    const f32x2 q2 = pair2(__uint_as_float(q.x), __uint_as_float(q.y));
+    fma2(acc[0], S.m0, q2);
+    fma2(acc[1], S.m1, q2);
+  }
+}
+// two blocks (one chunk) an item.  wl = weights of the stage + 16 * lane, sl = its scales + the lane group's offset; blk0 = index
+// (inside the staged slice) of the stage's first block.
 template <int NW, bool Q8 = false, bool KQ = false>
-__device__ __forceinline__ void consume_g4(float (&acc)[2], uint32_t wbase, uint32_t sbase, int nc, int blk0,
-                                           const XLayout& L, uint32_t xbase, int wi, int lane) {
-  const int g = lane >> 2, t = lane & 3;
-  const int limb = t >> 1;      // this lane's output columns: limb, blocks 2(t&1), 2(t&1)+1 of the item
-  const int myblk = g & 3;      // this lane's B column: limb g>>2, block g&3 of the item
-  // The lane reads the activation bytes of its own column once per item; in the MMA of another
-  // block its B registers are zero (selected, not loaded: shared-memory bandwidth is the scarcer
-  // resource in this loop).
-  const uint32_t xa = xbase + L.xq + (uint32_t)(g >> 2) * L.col_stride + (uint32_t)t * 8u + (uint32_t)(blk0 + myblk) * 32u;
-  const uint32_t zin = xbase + L.zin + (uint32_t)limb * L.zs + (uint32_t)(blk0 + 2 * (t & 1)) * 4u;
-  const uint32_t fex = xbase + L.fex + (uint32_t)limb * L.zs + (uint32_t)(blk0 + 2 * (t & 1)) * 4u;
-  const uint32_t fsx = xbase + L.fsx + (uint32_t)limb * L.zs + (uint32_t)(blk0 + 2 * (t & 1)) * 4u;
-  const uint32_t k0 = myblk == 0 ? 0xffffffffu : 0u, k1 = myblk == 1 ? 0xffffffffu : 0u, k2 = myblk == 2 ? 0xffffffffu : 0u,
-                 k3 = myblk == 3 ? 0xffffffffu : 0u;
+__device__ __forceinline__ void consume_x2(f32x2 (&acc)[2], uint32_t wl, uint32_t sl, int nc, int blk0, const LaneX& X, int wi) {
+  auto item = [&](uint32_t w, uint32_t s, uint32_t x, uint32_t o) {
+    const WBlocks<Q8> W = load_chunk<Q8>(w);
+    const PairScales<KQ> S = load_pairs<KQ>(s);
+    const uint2 f = lds64(X.fex + o), b = lds64(X.xa + x);
+    int c[4] = {(int)kBias, (int)kBias, (int)kBias, (int)kBias};  // signed bytes / codes with a minimum: no zero point
+    if (!Q8 && !KQ) {
+      const uint2 z = lds64(X.zin + o);
+      c[0] = c[2] = (int)z.x;
+      c[1] = c[3] = (int)z.y;
+    }
+    int d0[4], d1[4];
+    chunk_mma<Q8>(d0, W, 0, b.x, b.y, c);
+    chunk_mma<Q8>(d1, W, 1, b.x, b.y, c);
+    add_item<KQ>(acc, d0[0], d1[1], d0[2], d1[3], S, pair2(__uint_as_float(f.x), __uint_as_float(f.y)), X.fsx + o);
+  };
+  constexpr uint32_t kWC = Q8 ? 1024u : 512u, kSC = KQ ? 256u : 64u;
+  int it = wi;
+  uint32_t w = wl + (uint32_t)it * kWC, s = sl + (uint32_t)it * kSC, x = (uint32_t)(2 * it + blk0) * 32u, o = (uint32_t)(2 * it + blk0) * 4u;
+#pragma unroll 1
+  for (; it + NW < nc; it += 2 * NW) {
+    item(w, s, x, o);
+    item(w + NW * kWC, s + NW * kSC, x + NW * 64u, o + NW * 8u);
+    w += 2u * NW * kWC; s += 2u * NW * kSC; x += NW * 128u; o += NW * 16u;
+  }
+  if (it < nc) item(w, s, x, o);
+}
+// four blocks (two chunks) an item; sl also holds the offset of the lane's chunk of the two (t & 1)
+template <int NW, bool Q8 = false, bool KQ = false>
+__device__ __forceinline__ void consume_x4(f32x2 (&acc)[2], uint32_t wl, uint32_t sl, int nc, int blk0, const LaneX& X, int wi, int lane) {
+  const bool second = (lane & 1) != 0;  // this lane's outputs belong to the second chunk
+  auto item = [&](uint32_t w, uint32_t s, uint32_t x, uint32_t o, bool live) {
+    const WBlocks<Q8> A = load_chunk<Q8>(w), B = load_chunk<Q8>(w + (Q8 ? 1024u : 512u));
+    const PairScales<KQ> S = load_pairs<KQ>(s, live);
+    const uint2 f = lds64(X.fex + o), b = lds64(X.xa + x);
+    int c[4] = {(int)kBias, (int)kBias, (int)kBias, (int)kBias};
+    if (!Q8 && !KQ) {
+      const uint2 z = lds64(X.zin + o);
+      c[0] = c[2] = (int)z.x;
+      c[1] = c[3] = (int)z.y;
+    }
+    int d0[4], d1[4], d2[4], d3[4];
+    chunk_mma<Q8>(d0, A, 0, b.x, b.y, c);
+    chunk_mma<Q8>(d1, A, 1, b.x, b.y, c);
+    chunk_mma<Q8>(d2, B, 0, b.x, b.y, c);
+    chunk_mma<Q8>(d3, B, 1, b.x, b.y, c);
+    add_item<KQ>(acc, second ? d2[0] : d0[0], second ? d3[1] : d1[1], second ? d2[2] : d0[2], second ? d3[3] : d1[3], S,
+                 pair2(__uint_as_float(f.x), __uint_as_float(f.y)), X.fsx + o);
+  };
+  constexpr uint32_t kWC = Q8 ? 2048u : 1024u, kSC = KQ ? 512u : 128u;
   const int nitems = (nc + 1) >> 1;
-#pragma unroll kG4Unroll
-  for (int it = wi; it < nitems; it += NW) {
-    const WBlocks<Q8> wA = load_chunk<Q8>(wbase + (uint32_t)(2 * it) * chunk_bytes<Q8>(), lane);
-    const WBlocks<Q8> wB = load_chunk<Q8>(wbase + (uint32_t)(2 * it + 1) * chunk_bytes<Q8>(), lane);
-    const int ch = 2 * it + (t & 1);
-    // a chunk past the stage's data: whatever the slot holds must not count
-    const BlkScales<KQ> S = load_scales<KQ>(sbase, ch, g, ch < nc);
-    const uint2 z2 = lds64(zin + (uint32_t)it * 16u);
-    const uint2 f2 = lds64(fex + (uint32_t)it * 16u);
-    const uint2 b = lds64(xa + (uint32_t)it * 128u);
-    int d[4] = {(int)z2.x, (int)z2.y, (int)z2.x, (int)z2.y};
-    if (Q8 || KQ) d[0] = d[1] = d[2] = d[3] = (int)kBias;  // signed bytes / codes with a minimum: no zero point
-    chunk_mma<Q8>(d, wA, 0, b.x & k0, b.y & k0);
-    chunk_mma<Q8>(d, wA, 1, b.x & k1, b.y & k1);
-    chunk_mma<Q8>(d, wB, 0, b.x & k2, b.y & k2);
-    chunk_mma<Q8>(d, wB, 1, b.x & k3, b.y & k3);
-
-    const float fe = __uint_as_float(f2.x), fo = __uint_as_float(f2.y);
-    acc[0] = fmaf(S.se.x * fe, unbias(d[0]), acc[0]);
-    acc[0] = fmaf(S.so.x * fo, unbias(d[1]), acc[0]);
-    acc[1] = fmaf(S.se.y * fe, unbias(d[2]), acc[1]);
-    acc[1] = fmaf(S.so.y * fo, unbias(d[3]), acc[1]);
-    if (KQ) {  // - M * (block sum of the activations)
-      const uint2 q2 = lds64(fsx + (uint32_t)it * 16u);
-      const float qe = __uint_as_float(q2.x), qo = __uint_as_float(q2.y);
-      acc[0] = fmaf(-S.me.x, qe, acc[0]);
-      acc[0] = fmaf(-S.mo.x, qo, acc[0]);
-      acc[1] = fmaf(-S.me.y, qe, acc[1]);
-      acc[1] = fmaf(-S.mo.y, qo, acc[1]);
+  int it = wi;
+  uint32_t w = wl + (uint32_t)it * kWC, s = sl + (uint32_t)it * kSC, x = (uint32_t)(4 * it + blk0) * 32u, o = (uint32_t)(4 * it + blk0) * 4u;
+  if ((nc & 1) == 0) {
+#pragma unroll 1
+    for (; it + NW < nitems; it += 2 * NW) {
+      item(w, s, x, o, true);
+      item(w + NW * kWC, s + NW * kSC, x + NW * 128u, o + NW * 16u, true);
+      w += 2u * NW * kWC; s += 2u * NW * kSC; x += NW * 256u; o += NW * 32u;
+    }
+    if (it < nitems) item(w, s, x, o, true);
+  } else {
+#pragma unroll 1
+    for (; it < nitems; it += NW) {  // a chunk past the stage's data: whatever the slot holds must not count
+      item(w, s, x, o, 2 * it + (second ? 1 : 0) < nc);
+      w += NW * kWC; s += NW * kSC; x += NW * 128u; o += NW * 16u;
     }
   }
 }
-
-// One activation row in three limbs (22 bits): the 8 columns hold (limb, block) for the TWO blocks of
-// a chunk (6 used); lane t < 3 owns limb t of both blocks, lane t = 3 idles.  acc[0] += row g,
-// acc[1] += row g+8.
-template <int NW, bool Q8 = false, bool KQ = false>
-__device__ __forceinline__ void consume_m1l3(float (&acc)[2], uint32_t wbase, uint32_t sbase, int nc, int blk0,
-                                             const XLayout& L, uint32_t xbase, int wi, int lane) {
-  const int g = lane >> 2, t = lane & 3;
-  const int limb = min(t, 2);
-  const uint32_t xcol = xbase + L.xq + (uint32_t)(g >> 1) * L.col_stride + (uint32_t)t * 8u;  // B column g: limb g>>1, block g&1
-  const uint32_t zcol = xbase + L.zero + (uint32_t)(g >> 2) * 64u + (uint32_t)t * 8u;
-  uint32_t xa[2];
-#pragma unroll
-  for (int j = 0; j < 2; ++j) xa[j] = ((g < 6 && (g & 1) == j) ? xcol : zcol) + (uint32_t)(blk0 + j) * 32u;
-  const uint32_t zin = xbase + L.zin + (uint32_t)limb * L.zs + (uint32_t)blk0 * 4u;
-  const uint32_t fex = xbase + L.fex + (uint32_t)limb * L.zs + (uint32_t)blk0 * 4u;
-  const uint32_t fsx = xbase + L.fsx + (uint32_t)limb * L.zs + (uint32_t)blk0 * 4u;
-  const float live = t < 3 ? 1.f : 0.f;
-#pragma unroll 2
-  for (int it = wi; it < nc; it += NW) {
-    const WBlocks<Q8> w = load_chunk<Q8>(wbase + (uint32_t)it * chunk_bytes<Q8>(), lane);
-    const BlkScales<KQ> S = load_scales<KQ>(sbase, it, g);
-    const uint2 z2 = lds64(zin + (uint32_t)it * 8u);
-    const uint2 f2 = lds64(fex + (uint32_t)it * 8u);
-    int d[4] = {(int)z2.x, (int)z2.y, (int)z2.x, (int)z2.y};
-    if (Q8 || KQ) d[0] = d[1] = d[2] = d[3] = (int)kBias;
-    const uint32_t xo = (uint32_t)it * 64u;
-    uint2 b, b2;
-    b = lds64(xa[0] + xo);
-    b2 = lds64(xa[1] + xo);
-    chunk_mma<Q8>(d, w, 0, b.x, b.y);
-    chunk_mma<Q8>(d, w, 1, b2.x, b2.y);
-    const float fe = __uint_as_float(f2.x) * live, fo = __uint_as_float(f2.y) * live;
-    acc[0] = fmaf(S.se.x * fe, unbias(d[0]), acc[0]);
-    acc[0] = fmaf(S.so.x * fo, unbias(d[1]), acc[0]);
-    acc[1] = fmaf(S.se.y * fe, unbias(d[2]), acc[1]);
-    acc[1] = fmaf(S.so.y * fo, unbias(d[3]), acc[1]);
-    if (KQ) {
-      const uint2 q2 = lds64(fsx + (uint32_t)it * 8u);
-      const float qe = __uint_as_float(q2.x) * live, qo = __uint_as_float(q2.y) * live;
-      acc[0] = fmaf(-S.me.x, qe, acc[0]);
-      acc[0] = fmaf(-S.mo.x, qo, acc[0]);
-      acc[1] = fmaf(-S.me.y, qe, acc[1]);
-      acc[1] = fmaf(-S.mo.y, qo, acc[1]);
-    }
-  }
-}
-
-// G = 2: two activation rows; columns = (row, limb) x 2 blocks; an item is one chunk.
-// This lane's output columns: column pair t = (row t>>1, limb t&1), blocks 0 and 1 of the chunk.
-template <int NW, bool Q8 = false, bool KQ = false>
-__device__ __forceinline__ void consume_g2(float (&acc)[2], uint32_t wbase, uint32_t sbase, int nc, int blk0,
-                                           const XLayout& L, uint32_t xbase, int wi, int lane) {
-  const int g = lane >> 2, t = lane & 3;
-  const int myblk = g & 1;
-  const uint32_t xcol = xbase + L.xq + (uint32_t)(g >> 1) * L.col_stride + (uint32_t)t * 8u;
-  const uint32_t zcol = xbase + L.zero + (uint32_t)(g >> 2) * 64u + (uint32_t)t * 8u;
-  uint32_t xa[2];
-#pragma unroll
-  for (int j = 0; j < 2; ++j) xa[j] = (myblk == j ? xcol : zcol) + (uint32_t)(blk0 + j) * 32u;
-  const uint32_t zin = xbase + L.zin + (uint32_t)t * L.zs + (uint32_t)blk0 * 4u;
-  const uint32_t fex = xbase + L.fex + (uint32_t)t * L.zs + (uint32_t)blk0 * 4u;
-  const uint32_t fsx = xbase + L.fsx + (uint32_t)t * L.zs + (uint32_t)blk0 * 4u;
-#pragma unroll 2
-  for (int it = wi; it < nc; it += NW) {
-    const WBlocks<Q8> w = load_chunk<Q8>(wbase + (uint32_t)it * chunk_bytes<Q8>(), lane);
-    const BlkScales<KQ> S = load_scales<KQ>(sbase, it, g);
-    const uint2 z2 = lds64(zin + (uint32_t)it * 8u);
-    const uint2 f2 = lds64(fex + (uint32_t)it * 8u);
-    int d[4] = {(int)z2.x, (int)z2.y, (int)z2.x, (int)z2.y};
-    if (Q8 || KQ) d[0] = d[1] = d[2] = d[3] = (int)kBias;
-    const uint32_t xo = (uint32_t)it * 64u;
-    uint2 b;
-    b = lds64(xa[0] + xo);
-    chunk_mma<Q8>(d, w, 0, b.x, b.y);
-    b = lds64(xa[1] + xo);
-    chunk_mma<Q8>(d, w, 1, b.x, b.y);
-    const float fe = __uint_as_float(f2.x), fo = __uint_as_float(f2.y);
-    acc[0] = fmaf(S.se.x * fe, unbias(d[0]), acc[0]);
-    acc[0] = fmaf(S.so.x * fo, unbias(d[1]), acc[0]);
-    acc[1] = fmaf(S.se.y * fe, unbias(d[2]), acc[1]);
-    acc[1] = fmaf(S.so.y * fo, unbias(d[3]), acc[1]);
-    if (KQ) {
-      const uint2 q2 = lds64(fsx + (uint32_t)it * 8u);
-      const float qe = __uint_as_float(q2.x), qo = __uint_as_float(q2.y);
-      acc[0] = fmaf(-S.me.x, qe, acc[0]);
-      acc[0] = fmaf(-S.mo.x, qo, acc[0]);
-      acc[1] = fmaf(-S.me.y, qe, acc[1]);
-      acc[1] = fmaf(-S.mo.y, qo, acc[1]);
-    }
-  }
+// a lane's sums of a tile, added over the lanes that share a row: afterwards lane t has row g + 8 (t & 1)
+__device__ __forceinline__ float quad_rows(float a0, float a1, int lane, bool four) {
+  const bool odd = (lane & 1) != 0;
+  float keep = odd ? a1 : a0;
+  keep += __shfl_xor_sync(0xffffffffu, odd ? a0 : a1, 1);
+  if (four) keep += __shfl_xor_sync(0xffffffffu, keep, 2);
+  return keep;
 }
 
 // G = 1: NT tiles of 8 columns = 4 activation rows each; lane t of tile nt owns row 4 nt + t, both
@@ -486,7 +484,7 @@ __device__ __forceinline__ void consume_g1(float (&acc)[NT][2], uint32_t wbase, 
   const uint32_t lo_off = L.zs;  // column + 1
 #pragma unroll 2
   for (int it = wi; it < nc; it += NW) {
-    const WBlocks<Q8> wq = load_chunk<Q8>(wbase + (uint32_t)it * chunk_bytes<Q8>(), lane);
+    const WBlocks<Q8> wq = load_chunk<Q8>(wbase + (uint32_t)it * chunk_bytes<Q8>() + (uint32_t)lane * 16u);
     const uint4 w = wq.lo;
     const BlkScales<KQ> S = load_scales<KQ>(sbase, it, g);
     const float2 se = S.se, so = S.so;
@@ -503,19 +501,15 @@ __device__ __forceinline__ void consume_g1(float (&acc)[NT][2], uint32_t wbase, 
       const uint2 fh = lds64(fex + zo);                                  // 2^e * 128 of (even, odd); lo factor = / 128
       const uint2 be = lds64(xa[nt] + (uint32_t)it * 64u);
       const uint2 bo = lds64(xa[nt] + (uint32_t)it * 64u + 32u);
-      int de[4] = {(int)zh.x, (int)zl.x, (int)zh.x, (int)zl.x};
-      int dd[4] = {(int)zh.y, (int)zl.y, (int)zh.y, (int)zl.y};
+      int ce[4] = {(int)zh.x, (int)zl.x, (int)zh.x, (int)zl.x}, co[4] = {(int)zh.y, (int)zl.y, (int)zh.y, (int)zl.y};
+      int de[4], dd[4];
+      if (Q8 || KQ) ce[0] = ce[1] = ce[2] = ce[3] = co[0] = co[1] = co[2] = co[3] = (int)kBias;
       if (Q8) {
-        de[0] = de[1] = de[2] = de[3] = dd[0] = dd[1] = dd[2] = dd[3] = (int)kBias;
-        imma_s8(de, e0, e1, e2, e3, be.x, be.y);
-        imma_s8(dd, o0, o1, o2, o3, bo.x, bo.y);
-      } else if (KQ) {
-        de[0] = de[1] = de[2] = de[3] = dd[0] = dd[1] = dd[2] = dd[3] = (int)kBias;
-        imma(de, e0, e1, e2, e3, be.x, be.y);
-        imma(dd, o0, o1, o2, o3, bo.x, bo.y);
+        imma_s8(de, e0, e1, e2, e3, be.x, be.y, ce);
+        imma_s8(dd, o0, o1, o2, o3, bo.x, bo.y, co);
       } else {
-        imma(de, e0, e1, e2, e3, be.x, be.y);
-        imma(dd, o0, o1, o2, o3, bo.x, bo.y);
+        imma(de, e0, e1, e2, e3, be.x, be.y, ce);
+        imma(dd, o0, o1, o2, o3, bo.x, bo.y, co);
       }
       const float fe = __uint_as_float(fh.x), fo = __uint_as_float(fh.y);
       // 128 hi + lo, in units of 2^e / 128 ... fe already carries the 128: v = fe * (hi + lo / 128)

@@ -22,7 +22,8 @@
 // Weight formats: 4-bit blocks (nibbles unpacked in registers, zero point 8), 8-bit blocks (the
 // bytes are the MMA operand as stored), 4-bit K-quant blocks (f32 scale and minimum per block, up to
 // 4 rows).  HBM-bound: algorithmic bytes = N*K*{0.5625, 1.0625, 0.75} + activations + outputs.
-#include <cstdlib>
+#include <type_traits>
+
 #include "gemm_q4_s8.cuh"
 
 namespace {
@@ -186,13 +187,13 @@ __global__ void __launch_bounds__(kCT + 32 * (kTG == 0 ? 1 : kTG), 1) gemv_q4_st
   constexpr int kGW = kCW / kTGe;         // warps per tile group
   constexpr int kMR = MODE == kMN ? 4 * NT : (MODE == kM2L2 ? 2 : 1);  // activation rows the fragment layout holds
   constexpr int kLimbs = MODE == kM1L3 ? 3 : 2;
-  constexpr bool kZeroed = MODE != kMN;
+  constexpr bool kTwoBlocks = MODE == kM1L3 || MODE == kM2L2;
   extern __shared__ __align__(128) unsigned char smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int NS = p.nstages;
   const uint32_t stage_bytes = (uint32_t)p.stage_chunks * (kWChunk + kSChunk);
   const int sl_alloc = MODE == kM1L2 ? (p.slice_chunks + 1) & ~1 : p.slice_chunks;
-  const XLayout L = x_layout(p.cols, sl_alloc, kZeroed, 0, KQ);
+  const XLayout L = x_layout(p.cols, sl_alloc, kTwoBlocks, KQ);
   // carve: ring | activations (128-byte aligned) | reduction buffers | slice accumulators | barriers
   unsigned char* ring = smem;
   unsigned char* xreg = smem + (((size_t)NS * stage_bytes + 127) & ~(size_t)127);
@@ -298,13 +299,8 @@ __global__ void __launch_bounds__(kCT + 32 * (kTG == 0 ? 1 : kTG), 1) gemv_q4_st
   // The weights never change, so only the consumers wait for the kernel that produced the
   // activations (a no-op unless launched with programmatic stream serialization).
   QENG_STAMP(1);
-  const XLayout& Lz = L;
-  // Work that does not depend on the kernel before: the zero region other blocks' lanes read (several
-  // blocks per fragment), and the norm gains of this thread's groups, requested into L1 so that the
+  // Work that does not depend on the kernel before: the norm gains of this thread's groups, requested into L1 so that the
   // loads behind the reduction below find them there.
-  if (kZeroed)
-    for (uint32_t o = (uint32_t)tid * 16u; o < x_zero_bytes(Lz); o += kCT * 16u)
-      asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};\n" ::"r"(xbase + Lz.zero + o), "r"(0u) : "memory");
   if (p.gamma != nullptr && p.ximage == nullptr)
     for (int k0 = tid * 8; k0 < p.K; k0 += kCT * 8) asm volatile("prefetch.global.L1 [%0];\n" ::"l"(p.gamma + k0));
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
@@ -466,7 +462,7 @@ __global__ void __launch_bounds__(kCT + 32 * (kTG == 0 ? 1 : kTG), 1) gemv_q4_st
   // phases are seen strictly in order however far the groups drift apart.
   const int gi = warp / kGW, wi = warp % kGW;
   bool failed = false;
-  int tcount = 0, buf = 0, use = 0;
+  [[maybe_unused]] int tcount = 0, buf = 0, use = 0;
 
   // the fused epilogue of one row tile, run by one warp; total(a, r) = the finished sum for activation
   // row a and weight row r of the tile
@@ -532,55 +528,50 @@ __global__ void __launch_bounds__(kCT + 32 * (kTG == 0 ? 1 : kTG), 1) gemv_q4_st
     }
   };
   // this lane's partial accumulators of a tile -> `dst` ([row a][16]) (one or two activation rows)
-  auto park = [&](float* dst, float (&acc1)[2]) {
-    if (MODE == kM1L3 || MODE == kM1L2) {
-      acc1[0] += __shfl_xor_sync(0xffffffffu, acc1[0], 1);
-      acc1[1] += __shfl_xor_sync(0xffffffffu, acc1[1], 1);
-      acc1[0] += __shfl_xor_sync(0xffffffffu, acc1[0], 2);
-      acc1[1] += __shfl_xor_sync(0xffffffffu, acc1[1], 2);
-      if (t == 0) { dst[g] = acc1[0]; dst[g + 8] = acc1[1]; }
-    } else {
-      acc1[0] += __shfl_xor_sync(0xffffffffu, acc1[0], 1);
-      acc1[1] += __shfl_xor_sync(0xffffffffu, acc1[1], 1);
-      if ((t & 1) == 0) { dst[(t >> 1) * 16 + g] = acc1[0]; dst[(t >> 1) * 16 + g + 8] = acc1[1]; }
-    }
+  auto park = [&](float* dst, const f32x2 (&acc)[2]) {
+    float a0 = sum2(acc[0]), a1 = sum2(acc[1]);
+    if (MODE == kM1L3 && t == 3) a0 = a1 = 0.f;
+    const float v = quad_rows(a0, a1, lane, MODE != kM2L2);
+    if (MODE == kM2L2) dst[(t >> 1) * 16 + g + 8 * (t & 1)] = v;
+    else if (t < 2) dst[g + 8 * t] = v;
+  };
+  const LaneX X = MODE == kM1L2 ? lane_x4(L, xbase, lane) : lane_x2(L, xbase, MODE == kM1L3 ? 3 : 4, lane);
+  const uint32_t wl0 = smem_u32(ring) + (uint32_t)lane * 16u;
+  const uint32_t sl0 = smem_u32(ring) + (uint32_t)p.stage_chunks * kWChunk + (uint32_t)g * (KQ ? 32u : 8u) + (MODE == kM1L2 ? (uint32_t)(t & 1) * kSChunk : 0u);
+  auto consume = [&](f32x2 (&acc)[2], int s, int nc, int blk0, int wi, auto warps) {
+    const uint32_t at = (uint32_t)s * stage_bytes;
+    if constexpr (MODE == kM1L2) consume_x4<decltype(warps)::value, Q8, KQ>(acc, wl0 + at, sl0 + at, nc, blk0, X, wi, lane);
+    else consume_x2<decltype(warps)::value, Q8, KQ>(acc, wl0 + at, sl0 + at, nc, blk0, X, wi);
   };
 
   if constexpr (kDefer) {
     // ---- one activation slice, up to two rows: no per-tile meeting -------------------------------
-    int tl = 0, rot = 0;
-    for (int tile = blockIdx.x; tile < p.ntiles; tile += gridDim.x, ++tl) {
-      float acc1[2] = {0.f, 0.f};
-      for (int c0 = 0; c0 < p.nchunks; c0 += p.stage_chunks, ++use) {
-        const int s = use % NS;
-        const uint32_t ph = (uint32_t)(use / NS) & 1u;
+    int slot = 0, rot = 0, s = 0;
+    uint32_t ph = 0;
+    for (int tile = blockIdx.x; tile < p.ntiles; tile += gridDim.x) {
+      f32x2 acc[2] = {0ull, 0ull};
+      for (int c0 = 0; c0 < p.nchunks; c0 += p.stage_chunks) {
         QENG_TICK(tc0);
         if (!failed && !mbar_wait(smem_u32(full + s), ph)) failed = true;
         QENG_TOCK(tc0, 8, warp == 0);
         QENG_TICK(tc1);
         const int nc = min(p.stage_chunks, p.nchunks - c0);
-        const uint32_t wb = smem_u32(ring) + (uint32_t)s * stage_bytes;
-        const uint32_t sb = wb + (uint32_t)p.stage_chunks * kWChunk;
-        const int blk0 = c0 * 2;
         // the warp that takes a stage's first item rotates, so that stages whose item count is not a
         // multiple of 16 load the warps evenly over a tile
-        const int wr = (warp + kCW - rot) & (kCW - 1);
-        if (MODE == kM1L3) consume_m1l3<kCW, Q8, KQ>(acc1, wb, sb, nc, blk0, L, xbase, wr, lane);
-        else if (MODE == kM1L2) consume_g4<kCW, Q8, KQ>(acc1, wb, sb, nc, blk0, L, xbase, wr, lane);
-        else consume_g2<kCW, Q8, KQ>(acc1, wb, sb, nc, blk0, L, xbase, wr, lane);
+        consume(acc, s, nc, c0 * 2, (warp + kCW - rot) & (kCW - 1), std::integral_constant<int, kCW>());
         rot = (rot + (MODE == kM1L2 ? (nc + 1) >> 1 : nc)) & (kCW - 1);
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(empty + s));
+        if (++s == NS) { s = 0; ph ^= 1u; }
         QENG_TOCK(tc1, 9, warp == 0);
         QENG_COUNT(11, warp == 0);
       }
       QENG_TICK(tc2);
-      const int slot = tl % kDeferTiles;
-      park(red + ((size_t)slot * kCW + warp) * red_stride, acc1);
+      park(red + ((size_t)slot * kCW + warp) * red_stride, acc);
       const bool last_tile = tile + (int)gridDim.x >= p.ntiles;
       if (slot == kDeferTiles - 1 || last_tile) {
         consumer_sync();
-        if (tl < kDeferTiles) QENG_STAMP(4);
+        QENG_STAMP(4);
         for (int j = warp; j <= slot; j += kCW) {
           const float* rb = red + (size_t)j * kCW * red_stride;
           finish(tile - (slot - j) * (int)gridDim.x, [&](int a, int r) {
@@ -591,7 +582,9 @@ __global__ void __launch_bounds__(kCT + 32 * (kTG == 0 ? 1 : kTG), 1) gemv_q4_st
           });
         }
         if (!last_tile) consumer_sync();  // the parking area is free again
+        slot = -1;
       }
+      ++slot;
       QENG_TOCK(tc2, 10, warp == 0);
     }
   } else {
@@ -627,7 +620,7 @@ __global__ void __launch_bounds__(kCT + 32 * (kTG == 0 ? 1 : kTG), 1) gemv_q4_st
     int tl = 0;  // index of the tile among this CTA's tiles
     for (int tile = blockIdx.x; tile < p.ntiles; tile += gridDim.x, ++tcount, ++tl) {
       if ((tcount % kTGe) != gi) continue;  // another group's tile
-      float acc1[2] = {0.f, 0.f};
+      f32x2 acc[2] = {0ull, 0ull};
       float accn[NT][2];
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt) accn[nt][0] = accn[nt][1] = 0.f;
@@ -642,10 +635,8 @@ __global__ void __launch_bounds__(kCT + 32 * (kTG == 0 ? 1 : kTG), 1) gemv_q4_st
         const uint32_t wb = smem_u32(ring) + (uint32_t)s * stage_bytes;
         const uint32_t sb = wb + (uint32_t)p.stage_chunks * kWChunk;
         const int blk0 = (c0 - cs0) * 2;
-        if (MODE == kM1L3) consume_m1l3<kGW, Q8, KQ>(acc1, wb, sb, nc, blk0, L, xb, wi, lane);
-        else if (MODE == kM1L2) consume_g4<kGW, Q8, KQ>(acc1, wb, sb, nc, blk0, L, xb, wi, lane);
-        else if (MODE == kM2L2) consume_g2<kGW, Q8, KQ>(acc1, wb, sb, nc, blk0, L, xb, wi, lane);
-        else consume_g1<kGW, NT, Q8, KQ>(accn, wb, sb, nc, blk0, L, xb, p.cols, wi, lane);
+        if constexpr (MODE == kMN) consume_g1<kGW, NT, Q8, KQ>(accn, wb, sb, nc, blk0, L, xb, p.cols, wi, lane);
+        else consume(acc, s, nc, blk0, wi, std::integral_constant<int, kGW>());
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(empty + s));  // this warp is done with the stage
         QENG_TOCK(tc1, 9, warp == 0);
@@ -658,7 +649,7 @@ __global__ void __launch_bounds__(kCT + 32 * (kTG == 0 ? 1 : kTG), 1) gemv_q4_st
       // the next tile's barrier, and buffer `buf` is written again only after that barrier
       float* myred = red + (((size_t)gi * 2 + buf) * kGW + wi) * red_stride;
       if (MODE != kMN) {
-        park(myred, acc1);
+        park(myred, acc);
       } else {
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) {
@@ -758,7 +749,7 @@ StreamFit stream_fit(const qeng_ctx* ctx, const qeng_weight* w, int64_t M, bool 
     const int nsl = (nch + slice - 1) / slice;
     if (!f.imaged && nsl == 1 && nch * 64 > 8 * kGroups * kCT) return false;  // single-slice staging goes through registers: K <= 12288
     const int alloc = f.mode == kM1L2 ? (slice + 1) & ~1 : slice;
-    const XLayout L = x_layout(f.cols, alloc, f.mode != kMN, 0, kq);
+    const XLayout L = x_layout(f.cols, alloc, f.mode == kM1L3 || f.mode == kM2L2, kq);
     f.defer = f.mode != kMN && nsl == 1 && (ctx->stream_groups == 0 || w->fmt != QENG_FMT_Q4);
     const size_t red = (size_t)(f.defer ? kDeferTiles : 2) * kCW * kMR * 16 * 4;  // grouped: the same for every number of groups
     const size_t accs = nsl > 1 ? (size_t)tiles_per_cta * kMR * 16 * 4 : 0;

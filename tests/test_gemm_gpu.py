@@ -279,3 +279,26 @@ def test_device_quantizer_matches_the_golden_fixture(ctx):
     assert np.array_equal(q, GOLD["quant_q"])
     assert np.array_equal(s.view(np.uint16), GOLD["quant_s"].view(np.uint16))
     w.free()
+
+
+# One and two rows: shares of a warp of no, one, two or more items, odd chunk counts, several stages a tile, one row tile
+# or more than a CTA parks (16).  Bounds: 22 bits 2e-6 of max|y|, 15 bits (two rows, or asked for) TIGHT.
+@pytest.mark.parametrize("fmt,n,k", [(f, n, k) for n, k in [(48, 32), (16, 96), (64, 992), (2400, 1056), (48, 2016), (16, 3008), (48, 4160), (16, 8224),
+                                                            (40000, 64)] for f in ("q4", "q8")] + [("q4k", 48, 256), ("q4k", 16, 4352), ("q4k", 2400, 2304)])
+def test_one_and_two_rows_of_every_share(ctx, fmt, n, k):
+    import torch
+    rng = ref.rng_of(n * 31 + k)
+    if fmt == "q4k":
+        blocks = rng.integers(0, 256, (n * k // 256, 144), dtype=np.uint8)
+        blocks[:, :4] = rng.uniform(2e-4, 6e-4, (n * k // 256, 2)).astype(np.float16).view(np.uint8)
+        w = ctx.pack_q4k(blocks, n, k)
+    else:
+        wf = _t((rng.standard_normal((n, k)) * 0.05).astype(np.float32))
+        w = ctx.quantize_q4(wf) if fmt == "q4" else ctx.quantize_q8(wf)
+    x = _t(rng.standard_normal((2, k)).astype(np.float32))
+    want = (x.double() @ w.dequant().double().T).cpu().numpy()
+    assert ref.err_inf(ctx.gemm_q4(w, x[:1]).cpu().numpy(), want[:1]) < 2e-6
+    assert ref.err_inf(ctx.gemm_q4(w, x[:1], flags=2).cpu().numpy(), want[:1]) < TIGHT
+    assert ref.err_inf(ctx.gemm_q4(w, x).cpu().numpy(), want) < TIGHT
+    assert torch.equal(ctx.gemm_q4(w, x[:1]), ctx.gemm_q4(w, x[:1].clone()))
+    w.free()

@@ -419,7 +419,7 @@ int32_t run_layer_batch(qeng_ctx* ctx, qeng_decoder* d, int l, int64_t rows, con
   } else {
     e.y = d->qkv; e.ldy = d->nqkv;
   }
-  int32_t rc = qeng_gemm_rows_prep(ctx, L.wqkv, d->x, QENG_F32, rows, dm, L.norm1, d->cfg.rms_eps, e, st);
+  int32_t rc = qeng_gemm_rows_prep(ctx, L.wqkv, d->x, rows, dm, L.norm1, d->cfg.rms_eps, e, st);
   if (rc != QENG_OK) return rc;
   if (L.qnorm != nullptr) {
     rope_append_kernel<<<(unsigned)rows, 256, 0, st>>>(d->qkv, d->rope_cs, d->pos, table, 1, d->max_pages, (int)d->pages,
@@ -432,7 +432,7 @@ int32_t run_layer_batch(qeng_ctx* ctx, qeng_decoder* d, int l, int64_t rows, con
   if (rc != QENG_OK) return rc;
   qeng_tc_epi er;
   er.kind = QENG_EPI_ACCUM; er.y = d->x; er.ldy = dm;
-  rc = qeng_gemm_rows_prep(ctx, L.wo, d->att, QENG_F32, rows, nq, nullptr, 0.f, er, st);
+  rc = qeng_gemm_rows_prep(ctx, L.wo, d->att, rows, nq, nullptr, 0.f, er, st);
   if (rc != QENG_OK) return rc;
   qeng_tc_epi eg;
   eg.kind = QENG_EPI_SWIGLU;
@@ -441,12 +441,12 @@ int32_t run_layer_batch(qeng_ctx* ctx, qeng_decoder* d, int l, int64_t rows, con
   } else {
     eg.yb = reinterpret_cast<__nv_bfloat16*>(d->act); eg.ldyb = d->F; eg.yb_plane = rows * d->F; eg.yb_planes = 2;
   }
-  rc = qeng_gemm_rows_prep(ctx, L.wgu, d->x, QENG_F32, rows, dm, L.norm2, d->cfg.rms_eps, eg, st);
+  rc = qeng_gemm_rows_prep(ctx, L.wgu, d->x, rows, dm, L.norm2, d->cfg.rms_eps, eg, st);
   if (rc != QENG_OK) return rc;
-  if (L.wdown->fmt == QENG_FMT_K4) return qeng_gemm_rows_prep(ctx, L.wdown, d->act, QENG_F32, rows, d->F, nullptr, 0.f, er, st);
+  if (L.wdown->fmt == QENG_FMT_K4) return qeng_gemm_rows_prep(ctx, L.wdown, d->act, rows, d->F, nullptr, 0.f, er, st);
   qeng_tc_x x;
   x.data = d->act; x.ld = d->F; x.plane = rows * d->F; x.planes = 2;
-  return qeng_gemm_rows(ctx, L.wdown, x, nullptr, rows, er, st);
+  return qeng_gemm_rows(ctx, L.wdown, x, rows, er, st);
 }
 
 // One layer over `rows` rows whose positions / lengths / page-table rows are on the device.

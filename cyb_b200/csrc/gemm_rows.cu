@@ -38,9 +38,10 @@ struct RowsParams {
   const char* qs;
   const char* sc;
   int ntiles, nchunks, K;
-  const __nv_bfloat16* x;  // planes [XP][M][ldx]
+  const void* x;           // bf16 planes [XP][M][ldx], brought in as they are, or rows of any type
+  int x_dtype, made;
   long long ldx, plane;
-  const float* xsum;       // K-quant blocks: [XP][M][nchunks * 2] block sums of the planes
+  const float* xsum;       // K-quant blocks, planes: [XP][M][nchunks * 2] their block sums
   int M, nsl, cps, slice;  // rows, slices of `slice` chunks, CTAs per slice
   int nring, park;         // ring slots (a multiple of the groups), units parked between meetings
   float* ws;               // [nsl][M][16 * ntiles]
@@ -60,6 +61,16 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], 
 }
 __device__ __forceinline__ uint4 ld128(uint32_t a) { return *reinterpret_cast<const uint4*>(__cvta_shared_to_generic((size_t)a)); }
 __device__ __forceinline__ uint2 ld64(uint32_t a) { return *reinterpret_cast<const uint2*>(__cvta_shared_to_generic((size_t)a)); }
+__device__ __forceinline__ void sts128(uint32_t a, const uint32_t (&w)[4]) {
+  asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};\n" ::"r"(a), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
+}
+__device__ __forceinline__ void stsf(uint32_t a, float v) { asm volatile("st.shared.f32 [%0], %1;\n" ::"r"(a), "f"(v) : "memory"); }
+// two f32 values -> bf16 pair and the bf16 pair of what the rounding left
+__device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t& lo) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+  hi = u32(h);
+  lo = u32(__floats2bfloat162_rn(a - __low2float(h), b - __high2float(h)));
+}
 __device__ __forceinline__ float ldf(uint32_t a) { return *reinterpret_cast<const float*>(__cvta_shared_to_generic((size_t)a)); }
 
 // (a & b) | c in one instruction: with the constants as literals the compiler spends two, which is 16 of 150 per 64 k
@@ -98,7 +109,10 @@ __device__ __forceinline__ void fma2(unsigned long long& d, unsigned long long a
 __device__ __forceinline__ float lo_of(unsigned long long v) { return __uint_as_float((uint32_t)v); }
 __device__ __forceinline__ float hi_of(unsigned long long v) { return __uint_as_float((uint32_t)(v >> 32)); }
 
-template <int FMT, int XP, int NT>
+// RAW: rows of any type, split into planes here, by every CTA its slice: a call is one launch and one pass through memory less.  f32
+// rows over 4-bit blocks, as before / so: 8 over 4096 x 11008 15.5 / 13.5 us, 16 20.9 / 19.4; 8 over 22016 x 4096 23.9 / 21.8; 8
+// over 6144 x 4096 12.8 / 10.7; 8-bit blocks 4 to 18 % less.
+template <int FMT, int XP, int NT, bool RAW>
 // Compiled for more threads than it has: 80 registers leave room on the SM for the CTAs of the second kernel, which are
 // then waiting there when this one ends.
 __global__ void __launch_bounds__(kThreadsR + 160, 1) gemm_rows_kernel(const RowsParams p) {
@@ -151,28 +165,109 @@ __global__ void __launch_bounds__(kThreadsR + 160, 1) gemm_rows_kernel(const Row
 
   // ===== activations: the columns of this slice ================================================================
   const int kbeg = c0 * 64, kval = min(nc * 64, p.K - kbeg);  // values of K in the slice (a multiple of 32)
-  if (kval < nc * 64)  // the padding block of an odd block count has zero scales: its activations only have to be finite
-    for (int i = tid; i < 8 * NT * 4; i += kWarps * 32)
-      asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};\n" ::"r"(xs + (uint32_t)(i >> 2) * xstride + (uint32_t)kval * 2u + (uint32_t)(i & 3) * 16u), "r"(0u) : "memory");
-  asm volatile("griddepcontrol.wait;\n" ::: "memory");
-  if (warp == 0) {
-    const int cols = XP * p.M;
-    if (lane == 0) mbar_expect_tx(smem_u32(&xbar), (uint32_t)(cols * kval * 2));
-    __syncwarp();
-    for (int c = lane; c < cols; c += 32) {  // column of row m, plane pl: pl * kRows + m
-      const int pl = c / p.M, m = c - pl * p.M;
-      bulk_g2s(xs + (uint32_t)(pl * kRows + m) * xstride, p.x + (size_t)pl * p.plane + (size_t)m * p.ldx + kbeg, (uint32_t)kval * 2u, smem_u32(&xbar));
+  if (!RAW) {
+    if (kval < nc * 64)  // the padding block of an odd block count has zero scales: its activations only have to be finite
+      for (int i = tid; i < 8 * NT * 4; i += kWarps * 32)
+        asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};\n" ::"r"(xs + (uint32_t)(i >> 2) * xstride + (uint32_t)kval * 2u + (uint32_t)(i & 3) * 16u), "r"(0u) : "memory");
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    if (warp == 0) {
+      const int cols = XP * p.M;
+      if (lane == 0) mbar_expect_tx(smem_u32(&xbar), (uint32_t)(cols * kval * 2));
+      __syncwarp();
+      for (int c = lane; c < cols; c += 32) {  // column of row m, plane pl: pl * kRows + m
+        const int pl = c / p.M, m = c - pl * p.M;
+        bulk_g2s(xs + (uint32_t)(pl * kRows + m) * xstride, reinterpret_cast<const __nv_bfloat16*>(p.x) + (size_t)pl * p.plane + (size_t)m * p.ldx + kbeg, (uint32_t)kval * 2u, smem_u32(&xbar));
+      }
     }
-  }
-  if (FMT == QENG_FMT_K4) {
-    for (int i = tid; i < XP * p.M * nc * 2; i += kWarps * 32) {
-      const int c = i / (nc * 2), b = i - c * nc * 2;  // plane-major: c = plane * M + m
-      const float v = p.xsum[(size_t)c * p.nchunks * 2 + c0 * 2 + b];
-      asm volatile("st.shared.f32 [%0], %1;\n" ::"r"(sums + (uint32_t)(c / p.M * kRows + c % p.M) * sstride + (uint32_t)b * 4u), "f"(v) : "memory");
+    if (FMT == QENG_FMT_K4) {
+      for (int i = tid; i < XP * p.M * nc * 2; i += kWarps * 32) {
+        const int c = i / (nc * 2), b = i - c * nc * 2;  // plane-major: c = plane * M + m
+        const float v = p.xsum[(size_t)c * p.nchunks * 2 + c0 * 2 + b];
+        asm volatile("st.shared.f32 [%0], %1;\n" ::"r"(sums + (uint32_t)(c / p.M * kRows + c % p.M) * sstride + (uint32_t)b * 4u), "f"(v) : "memory");
+      }
+    }
+  } else {
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    const int ngrp = nc * 8, segs = (ngrp + 31) >> 5;  // groups of 8 k, segments of 32 of them
+    const int esz = p.x_dtype == QENG_F32 ? 4 : 2;
+    const bool vec = ((reinterpret_cast<uintptr_t>(p.x) | (uintptr_t)(p.ldx * esz)) & 15) == 0;
+    const int items = p.M * segs;
+    constexpr int kU = 3;  // items of a warp whose loads are on their way together
+#pragma unroll 1
+    for (int it0 = warp; it0 < items; it0 += kWarps * kU) {
+      uint4 raw[kU][2];
+#pragma unroll
+      for (int u = 0; u < kU; ++u) {
+        const int it = it0 + u * kWarps, m = it / segs, k = ((it - m * segs) * 32 + lane) * 8;
+        raw[u][0] = raw[u][1] = make_uint4(0u, 0u, 0u, 0u);
+        if (it < items && k < kval) {
+          const char* src = reinterpret_cast<const char*>(p.x) + ((long long)m * p.ldx + kbeg + k) * esz;
+          if (vec) {
+            raw[u][0] = *reinterpret_cast<const uint4*>(src);
+            if (esz == 4) raw[u][1] = *reinterpret_cast<const uint4*>(src + 16);
+          } else {
+            uint32_t w[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) w[i] = esz == 4 ? reinterpret_cast<const uint32_t*>(src)[i] : reinterpret_cast<const uint16_t*>(src)[i];
+            if (esz == 4) {
+              raw[u][0] = make_uint4(w[0], w[1], w[2], w[3]);
+              raw[u][1] = make_uint4(w[4], w[5], w[6], w[7]);
+            } else {
+              raw[u][0] = make_uint4(w[0] | w[1] << 16, w[2] | w[3] << 16, w[4] | w[5] << 16, w[6] | w[7] << 16);
+            }
+          }
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kU; ++u) {
+        const int it = it0 + u * kWarps;
+        if (it >= items) break;
+        const int m = it / segs, grp = (it - m * segs) * 32 + lane, k = grp * 8;
+        uint32_t hi[4] = {raw[u][0].x, raw[u][0].y, raw[u][0].z, raw[u][0].w}, lo[4] = {0u, 0u, 0u, 0u};
+        if (XP == 2) {
+          float v[8];
+          if (p.x_dtype == QENG_F32) {
+            const uint32_t w[8] = {raw[u][0].x, raw[u][0].y, raw[u][0].z, raw[u][0].w, raw[u][1].x, raw[u][1].y, raw[u][1].z, raw[u][1].w};
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(w[i]);
+          } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const float2 f = p.x_dtype == QENG_F16 ? __half22float2(*reinterpret_cast<const __half2*>(&hi[i])) : __bfloat1622float2(bf2(hi[i]));
+              v[2 * i] = f.x;
+              v[2 * i + 1] = f.y;
+            }
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i) split2(v[2 * i], v[2 * i + 1], hi[i], lo[i]);
+        }
+        if (grp < ngrp) {
+          sts128(xs + (uint32_t)m * xstride + (uint32_t)k * 2u, hi);
+          if (XP == 2) sts128(xs + (uint32_t)(kRows + m) * xstride + (uint32_t)k * 2u, lo);
+        }
+        if (FMT == QENG_FMT_K4) {  // per block and plane, the sum of the values as stored (the factor of the minimum)
+          float q = 0.f, ql = 0.f;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float2 f = __bfloat1622float2(bf2(hi[i])), fl = __bfloat1622float2(bf2(lo[i]));
+            q += f.x + f.y;
+            ql += fl.x + fl.y;
+          }
+#pragma unroll
+          for (int o = 1; o <= 2; o <<= 1) {
+            q += __shfl_xor_sync(0xffffffffu, q, o);
+            ql += __shfl_xor_sync(0xffffffffu, ql, o);
+          }
+          if ((lane & 3) == 0 && grp < ngrp) {
+            stsf(sums + (uint32_t)m * sstride + (uint32_t)(grp >> 2) * 4u, q);
+            if (XP == 2) stsf(sums + (uint32_t)(kRows + m) * sstride + (uint32_t)(grp >> 2) * 4u, ql);
+          }
+        }
+      }
     }
   }
   asm volatile("bar.sync 1, %0;\n" ::"n"(kWarps * 32) : "memory");
-  bool failed = !mbar_wait(smem_u32(&xbar), 0);
+  bool failed = !RAW && !mbar_wait(smem_u32(&xbar), 0);
 
   const int gi = warp / kGroupWarps, wi = warp % kGroupWarps;
   const uint32_t xa = xs + (uint32_t)g * xstride + (uint32_t)t * 16u;  // column g of tile 0, this lane's 8 k
@@ -397,12 +492,12 @@ RowsPlan rows_plan(const qeng_ctx* ctx, const qeng_weight* w, int64_t M, int xp)
   return r;
 }
 
-template <int FMT, int XP, int NT>
+template <int FMT, int XP, int NT, bool RAW>
 int32_t launch_rows(qeng_ctx* ctx, const RowsParams& p, const RowsPlan& pl, const qeng_tc_epi& e, int N, cudaStream_t stream) {
   static bool configured_on[64] = {};  // the opt-in shared-memory size is set per device
   bool& configured = configured_on[ctx->device & 63];
   if (!configured) {
-    QENG_CUDA(ctx, cudaFuncSetAttribute(gemm_rows_kernel<FMT, XP, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBudget));
+    QENG_CUDA(ctx, cudaFuncSetAttribute(gemm_rows_kernel<FMT, XP, NT, RAW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBudget));
     configured = true;
   }
   cudaLaunchConfig_t cfg = {};
@@ -415,7 +510,7 @@ int32_t launch_rows(qeng_ctx* ctx, const RowsParams& p, const RowsPlan& pl, cons
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = ctx->pdl ? 1 : 0;
-  QENG_CUDA(ctx, cudaLaunchKernelEx(&cfg, gemm_rows_kernel<FMT, XP, NT>, p));
+  QENG_CUDA(ctx, cudaLaunchKernelEx(&cfg, gemm_rows_kernel<FMT, XP, NT, RAW>, p));
   const bool split = p.nsl > 4;
   cfg.gridDim = dim3((unsigned)(split ? (N + 31) / 32 : (N + 127) / 128), (unsigned)((p.M + 3) / 4));
   cfg.blockDim = dim3(128);
@@ -424,17 +519,18 @@ int32_t launch_rows(qeng_ctx* ctx, const RowsParams& p, const RowsPlan& pl, cons
   return QENG_OK;
 }
 
-template <int FMT, int XP>
+template <int FMT, int XP, bool RAW>
 int32_t launch_nt(qeng_ctx* ctx, const RowsParams& p, const RowsPlan& pl, const qeng_tc_epi& e, int N, cudaStream_t stream) {
   switch (pl.nt) {
-    case 1: return launch_rows<FMT, 1, 1>(ctx, p, pl, e, N, stream);  // one plane only
-    case 2: return launch_rows<FMT, XP, 2>(ctx, p, pl, e, N, stream);
-    default: return launch_rows<FMT, XP, 4>(ctx, p, pl, e, N, stream);
+    case 1: return launch_rows<FMT, 1, 1, RAW>(ctx, p, pl, e, N, stream);  // one plane only
+    case 2: return launch_rows<FMT, XP, 2, RAW>(ctx, p, pl, e, N, stream);
+    default: return launch_rows<FMT, XP, 4, RAW>(ctx, p, pl, e, N, stream);
   }
 }
 template <int FMT>
 int32_t launch_xp(qeng_ctx* ctx, const RowsParams& p, const RowsPlan& pl, int xp, const qeng_tc_epi& e, int N, cudaStream_t stream) {
-  return xp == 1 ? launch_nt<FMT, 1>(ctx, p, pl, e, N, stream) : launch_nt<FMT, 2>(ctx, p, pl, e, N, stream);
+  if (p.made) return xp == 1 ? launch_nt<FMT, 1, false>(ctx, p, pl, e, N, stream) : launch_nt<FMT, 2, false>(ctx, p, pl, e, N, stream);
+  return xp == 1 ? launch_nt<FMT, 1, true>(ctx, p, pl, e, N, stream) : launch_nt<FMT, 2, true>(ctx, p, pl, e, N, stream);
 }
 
 }  // namespace
@@ -445,41 +541,39 @@ bool qeng_gemm_rows_fits(const qeng_ctx* ctx, const qeng_weight* w, int64_t M, i
 
 static size_t planes_bytes(const qeng_weight* w, int64_t M, int planes) { return ((size_t)planes * M * w->K * 2 + 15) & ~(size_t)15; }
 
-// rows of any type through the kernels above; with `gamma` they are RMS-normalised first
-int32_t qeng_gemm_rows_prep(qeng_ctx* ctx, const qeng_weight* w, const void* x, int32_t dtype, int64_t M, int64_t ldx, const float* gamma, float eps,
+static int32_t rows_call(qeng_ctx* ctx, const qeng_weight* w, const qeng_tc_x& x, int32_t dtype, bool made, const float* xsum, int64_t M, const qeng_tc_epi& epi,
+                         cudaStream_t stream, qeng_scratch* sc);
+
+// f32 rows as planes made (and RMS-normalised, if `gamma` is given) by a kernel of its own
+int32_t qeng_gemm_rows_prep(qeng_ctx* ctx, const qeng_weight* w, const float* x, int64_t M, int64_t ldx, const float* gamma, float eps,
                             const qeng_tc_epi& epi, cudaStream_t stream) {
-  const int planes = dtype == QENG_BF16 && gamma == nullptr ? 1 : 2;
-  if (planes == 1 && w->fmt != QENG_FMT_K4 && ((reinterpret_cast<uintptr_t>(x) | (uintptr_t)(ldx * 2)) & 15) == 0) {
-    qeng_tc_x xx;
-    xx.data = x;
-    xx.ld = ldx;
-    return qeng_gemm_rows(ctx, w, xx, nullptr, M, epi, stream);
-  }
   qeng_scratch* sc = qeng_scratch_for(ctx, stream);
-  const size_t sum_bytes = w->fmt == QENG_FMT_K4 ? (size_t)planes * M * w->nchunks * 8 : 0;
-  int32_t rc = qeng_scratch_grow(ctx, sc, &sc->planes, planes_bytes(w, M, planes) + sum_bytes);
+  const size_t sum_bytes = w->fmt == QENG_FMT_K4 ? (size_t)2 * M * w->nchunks * 8 : 0;
+  int32_t rc = qeng_scratch_grow(ctx, sc, &sc->planes, planes_bytes(w, M, 2) + sum_bytes);
   if (rc != QENG_OK) return rc;
   qeng_tc_x xx;
   xx.data = sc->planes.ptr;
   xx.ld = w->K;
   xx.plane = M * w->K;
-  xx.planes = planes;
-  float* sums = w->fmt == QENG_FMT_K4 ? reinterpret_cast<float*>(reinterpret_cast<char*>(sc->planes.ptr) + planes_bytes(w, M, planes)) : nullptr;
-  rc = qeng_tc_prep(ctx, x, dtype, M, w->K, ldx, gamma, eps, planes, sc->planes.ptr, sums, stream);
-  return rc == QENG_OK ? qeng_gemm_rows(ctx, w, xx, sums, M, epi, stream, sc) : rc;
+  xx.planes = 2;
+  float* sums = w->fmt == QENG_FMT_K4 ? reinterpret_cast<float*>(reinterpret_cast<char*>(sc->planes.ptr) + planes_bytes(w, M, 2)) : nullptr;
+  rc = qeng_tc_prep(ctx, x, QENG_F32, M, w->K, ldx, gamma, eps, 2, sc->planes.ptr, sums, stream);
+  return rc == QENG_OK ? rows_call(ctx, w, xx, QENG_BF16, true, sums, M, epi, stream, sc) : rc;
 }
 
-int32_t qeng_gemm_rows(qeng_ctx* ctx, const qeng_weight* w, const qeng_tc_x& x, const float* xsum, int64_t M, const qeng_tc_epi& epi, cudaStream_t stream, qeng_scratch* sc) {
+// made: x holds bf16 planes, with their block sums in xsum; otherwise rows of any type
+static int32_t rows_call(qeng_ctx* ctx, const qeng_weight* w, const qeng_tc_x& x, int32_t dtype, bool made, const float* xsum, int64_t M, const qeng_tc_epi& epi,
+                         cudaStream_t stream, qeng_scratch* sc) {
   const RowsPlan pl = rows_plan(ctx, w, M, x.planes);
   if (!pl.ok) return qeng_fail(ctx, QENG_ERR_SHAPE, "gemm_rows: %lld rows over [%lld, %lld] do not fit", (long long)M, (long long)w->N, (long long)w->K);
-  if (w->fmt == QENG_FMT_K4 && xsum == nullptr) return qeng_fail(ctx, QENG_ERR_ARG, "gemm_rows: K-quant blocks need the block sums of the activations");
+  if (made && w->fmt == QENG_FMT_K4 && xsum == nullptr) return qeng_fail(ctx, QENG_ERR_ARG, "gemm_rows: K-quant blocks need the block sums of the activations");
   if (sc == nullptr) sc = qeng_scratch_for(ctx, stream);
   const int32_t rc = qeng_scratch_grow(ctx, sc, &sc->part, (size_t)pl.nsl * M * w->N * 4);
   if (rc != QENG_OK) return rc;
   RowsParams p;
   p.qs = reinterpret_cast<const char*>(w->qs); p.sc = reinterpret_cast<const char*>(w->sc);
   p.ntiles = (int)w->ntiles; p.nchunks = (int)w->nchunks; p.K = (int)w->K;
-  p.x = reinterpret_cast<const __nv_bfloat16*>(x.data); p.ldx = x.ld; p.plane = x.plane; p.xsum = xsum;
+  p.x = x.data; p.x_dtype = dtype; p.made = made; p.ldx = x.ld; p.plane = x.plane; p.xsum = xsum;
   p.M = (int)M; p.nsl = pl.nsl; p.cps = pl.cps; p.slice = pl.slice; p.nring = pl.nring; p.park = pl.park;
   p.ws = reinterpret_cast<float*>(sc->part.ptr);
   p.status = ctx->status;
@@ -488,4 +582,17 @@ int32_t qeng_gemm_rows(qeng_ctx* ctx, const qeng_weight* w, const qeng_tc_x& x, 
     case QENG_FMT_Q8: return launch_xp<QENG_FMT_Q8>(ctx, p, pl, x.planes, epi, (int)w->N, stream);
     default: return launch_xp<QENG_FMT_K4>(ctx, p, pl, x.planes, epi, (int)w->N, stream);
   }
+}
+
+int32_t qeng_gemm_rows(qeng_ctx* ctx, const qeng_weight* w, const qeng_tc_x& x, int64_t M, const qeng_tc_epi& epi, cudaStream_t stream) {
+  return rows_call(ctx, w, x, QENG_BF16, true, nullptr, M, epi, stream, nullptr);
+}
+
+int32_t qeng_gemm_rows_raw(qeng_ctx* ctx, const qeng_weight* w, const void* x, int32_t dtype, int64_t M, int64_t ldx, const qeng_tc_epi& epi, cudaStream_t stream) {
+  qeng_tc_x xx;
+  xx.data = x;
+  xx.ld = ldx;
+  xx.planes = dtype == QENG_BF16 ? 1 : 2;
+  const bool made = dtype == QENG_BF16 && w->fmt != QENG_FMT_K4 && ((reinterpret_cast<uintptr_t>(x) | (uintptr_t)(ldx * 2)) & 15) == 0;
+  return rows_call(ctx, w, xx, dtype, made, nullptr, M, epi, stream, nullptr);
 }

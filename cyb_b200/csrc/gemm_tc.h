@@ -39,7 +39,11 @@ int32_t qeng_tc_prep(qeng_ctx* ctx, const void* x, int32_t dtype, int64_t M, int
 
 // gemm_rows.cu: a few rows (all formats) at the precision of wp = 2; planes: 1 for bf16 rows, else 2
 bool qeng_gemm_rows_fits(const qeng_ctx* ctx, const qeng_weight* w, int64_t M, int planes);
-int32_t qeng_gemm_rows_prep(qeng_ctx* ctx, const qeng_weight* w, const void* x, int32_t dtype, int64_t M, int64_t ldx, const float* gamma, float eps,
+// rows of any type, converted by the matmul itself
+int32_t qeng_gemm_rows_raw(qeng_ctx* ctx, const qeng_weight* w, const void* x, int32_t dtype, int64_t M, int64_t ldx, const qeng_tc_epi& epi, cudaStream_t stream);
+// f32 rows, converted (and normalised, if gamma is given) by a kernel of its own: what the layers of a decoder take, where that kernel
+// starts before the one in front of it has ended (sixteen rows converted and normalised by the matmul itself: 3270 us a step, so 2680)
+int32_t qeng_gemm_rows_prep(qeng_ctx* ctx, const qeng_weight* w, const float* x, int64_t M, int64_t ldx, const float* gamma, float eps,
                             const qeng_tc_epi& epi, cudaStream_t stream);
-int32_t qeng_gemm_rows(qeng_ctx* ctx, const qeng_weight* w, const qeng_tc_x& x, const float* xsum, int64_t M, const qeng_tc_epi& epi, cudaStream_t stream,
-                       qeng_scratch* sc = nullptr);
+// rows that are bf16 planes already (not K-quant blocks, which need the planes' block sums)
+int32_t qeng_gemm_rows(qeng_ctx* ctx, const qeng_weight* w, const qeng_tc_x& x, int64_t M, const qeng_tc_epi& epi, cudaStream_t stream);

@@ -352,7 +352,7 @@ int32_t qeng_gemm_q4(qeng_ctx* ctx, const qeng_weight* w, const void* x, int32_t
     e.kind = (flags & QENG_GEMM_ACCUMULATE) ? QENG_EPI_ACCUM : QENG_EPI_STORE;
     e.y = y;
     e.ldy = ldy;
-    const int32_t rc = rows ? qeng_gemm_rows_prep(ctx, w, x, x_dtype, M, ldx, nullptr, 0.f, e, (cudaStream_t)stream)
+    const int32_t rc = rows ? qeng_gemm_rows_raw(ctx, w, x, x_dtype, M, ldx, e, (cudaStream_t)stream)
                             : qeng_gemm_many_rows(ctx, w, x, x_dtype, M, ldx, e, prompt ? 1 : 2, (cudaStream_t)stream);
     if (rc == QENG_OK || prompt || !ctx->no_memory) return rc;
   }

@@ -47,6 +47,21 @@ def test_rows_and_widths(ctx, fmt, m):
     ctx.device_status()
 
 
+# Rows that the matmul converts itself: odd row starts and strides (no 16-byte loads), f16, bf16 rows that are not aligned, slices of
+# which the last is short, rows that fill no column tile.  Bound as above.
+@pytest.mark.parametrize("fmt", ["q4", "q8", "q4k"])
+@pytest.mark.parametrize("m,n,k,off,pad", [(5, 272, 768, 1, 0), (16, 1040, 4352, 3, 5), (7, 2064, 2304, 0, 1), (11, 48, 11008, 2, 0)])
+def test_few_rows_of_any_alignment(ctx, fmt, m, n, k, off, pad):
+    import torch
+    w = _weight(ctx, fmt, n, k)
+    wd = w.dequant().double()
+    for dt in DT:
+        x = torch.randn(off + m * (k + pad), device="cuda").to(getattr(torch, dt))[off:].view(m, k + pad)[:, :k]
+        want = x.double() @ wd.T
+        assert float((ctx.gemm_q4(w, x).double() - want).abs().max() / want.abs().max()) < 3e-5, (fmt, m, n, k, dt)
+    ctx.device_status()
+
+
 def _plan(ctx, w, m, wp, xp, epilogue):
     """What the planner of the many-row matmul chose, for the tests below to know what they ran."""
     import ctypes

@@ -1,31 +1,36 @@
-// Causal attention of prompt rows (GQA) over the paged f16 KV cache.
+// Causal attention of prompt rows (GQA) over the paged f16 KV cache, on the 5th-generation tensor cores.
 //
-// One CTA serves 64 MMA rows = 64 / group tokens x the query heads of one kv head, so a K / V tile fetched
-// once is used by every head of the group (the decode kernel, called once per prompt row, fetched the whole
-// context for every token: 16 GB per layer at 1800 tokens).  A producer warp brings pages into a ring of
-// 32-token tiles, one TMA box of 8 KB per page, 128-byte swizzled so that ldmatrix reads are free of bank
-// conflicts; four consumer warps own 16 rows each (mma.sync m16n8k16, f32 accumulation, online softmax).
-// The probabilities enter the second product as two f16 terms, as in the decode kernel: no precision is
-// lost there.  Three CTAs per SM.
+// A tile is 128 MMA rows = 128 / group tokens x the query heads of one kv head, so a K / V page fetched once is used by every
+// head of the group; a CTA works on two tiles of neighbouring tokens against the same keys, 64 at a time (four pages).  All
+// operands but K and V live in tensor memory, 256 columns a tile: the queries (A operand of S = Q K^T), S, which the
+// probabilities (A operand of O += P V, two f16 terms, so that no precision is lost there) overwrite, and O.  A page is one TMA
+// box of 8 KB with a 128-byte swizzle; its K rows are a K-major B operand of 16 columns, its V rows an MN-major one of 128.
+// Warps: 0-7 and 8-15 softmax of the two tiles, 16 MMA issue, 17 pages.  A lane of the softmax is a row and half of a tile's
+// keys (no exchange between lanes; the two halves meet once a tile for the row's maximum).  The MMAs of one tile run while the
+// other is in its softmax.  O is rescaled in tensor memory, only when a row's maximum has grown by more
+// than 2^8 since it was last (the probabilities stay below 256, exact in two f16 terms as before).
 //
-// Least time: 24 MMAs of 2 cycles per 16 x 8 scores (8 for the scores, 16 for the values); 2 * 128 * 3 * heads * T^2 / 2
-// operations for a prompt of T tokens = 73 us per layer at T = 1800 and 32 heads.  It takes 148 there (ncu; 212 with the
-// CTAs in head order): the tensor pipe is busy 57 % of the cycles in which an SM has work (dependent steps of the softmax
-// between the two products, 12 consumer warps per SM).
+// Least time: 64 keys of a tile are 32 MMAs of 16 columns (9.4 cycles each) and 8 of 128 (64): 815 cycles a tile, 37 K cycles
+// for the 450 tiles of 1800 tokens, 32 query and 8 kv heads, on 148 SMs.  There a layer takes 68 us (ncu; 152 with mma.sync,
+// whose pipe alone needs 73): what is left is the chain of a tile (scores, softmax, values, the hops between them), which two
+// tiles a CTA hide by half.  128 tokens behind nothing 13.7 us (15.5), 16 x 45 tokens 13-16 (14.8): launch, first page, one
+// chain.  A softmax of four warps a tile, a lane all 64 keys: 77 us.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <math.h>
-
-#include <type_traits>
 
 #include "attn_prefill.h"
 
 namespace {
 
-constexpr int kHD = 128, kNW = 4, kRows = 16 * kNW, kThreads = (kNW + 1) * 32;
-constexpr int kTile = 32, kStages = 3, kPageBytes = 8192, kStageBytes = 2 * kPageBytes;
-constexpr int kQBytes = kRows * kHD * 2;
-constexpr size_t kSmem = kQBytes + kStages * kStageBytes + 1024;
+constexpr int kHD = 128, kRows = 128, kTile = 64, kPages = kTile / 16, kStages = 3;
+constexpr int kSoftWarps = 16, kMmaWarp = kSoftWarps, kLoadWarp = kMmaWarp + 1, kThreads = (kLoadWarp + 1) * 32;
+constexpr int kKeys = kTile / 2;  // of a softmax warp
+constexpr uint32_t kPageBytes = 8192, kStageBytes = kPages * kPageBytes;
+constexpr uint32_t kScratch = kTile * kRows * 4;  // probabilities of a tile that goes key by key
+constexpr size_t kSmem = kStages * kStageBytes + 2 * kScratch + 1024;
+constexpr uint32_t kTileCols = 256, kO = 64, kS = 192;  // tensor-memory columns: queries at 0
+constexpr float kGrow = 8.f;                            // log2 of how far a row's maximum may grow before O is rescaled
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
@@ -60,97 +65,135 @@ __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity) {
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
   return mbar_try_wait(bar, parity) || mbar_wait_slow(bar, parity);
 }
-__device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t (&r)[4]) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(addr)
-               : "memory");
-}
-__device__ __forceinline__ void ldsm4_t(uint32_t addr, uint32_t (&r)[4]) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(addr)
-               : "memory");
-}
-__device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+// the same for a converged warp, which learns the outcome by vote
+__device__ __forceinline__ bool wait_warp(uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); }
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n selp.u32 %0, 1, 0, q;\n}\n" : "=r"(p));
+  return p != 0;
 }
 __device__ __forceinline__ uint32_t pack_h2(float a, float b) {
   __half2 h = __floats2half2_rn(a, b);
   return *reinterpret_cast<uint32_t*>(&h);
 }
-// byte offset of 16-byte chunk c (0..15) of row r in a tile of [2 halves][rows][128 B], 128-byte swizzled
-__device__ __forceinline__ uint32_t chunk_at(int rows, int r, int c) {
-  return (uint32_t)((c >> 3) * rows * 128 + r * 128 + (((c & 7) ^ (r & 7)) << 4));
+__device__ __forceinline__ uint32_t pack_b2(float a, float b) {
+  __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<uint32_t*>(&h);
+}
+// 2^x, results below 2^-126 as zero
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;\n" : "=f"(y) : "f"(x));
+  return y;
+}
+// shared-memory matrix descriptor, 128-byte swizzle.  K-major: 8-row groups `sbo` bytes apart (lbo unused); MN-major: groups of 64
+// columns `lbo` apart, of 8 k `sbo` apart
+__device__ __forceinline__ uint64_t make_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
+  uint64_t d = 0;
+  d |= (uint64_t)((saddr & 0x3ffff) >> 4);
+  d |= (uint64_t)(lbo >> 4) << 16;
+  d |= (uint64_t)(sbo >> 4) << 32;
+  d |= (uint64_t)1 << 46;  // descriptor version of this architecture
+  d |= (uint64_t)2 << 61;  // 128-byte swizzle
+  return d;
+}
+__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(tmem_d),
+      "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(acc)
+      : "memory");
+}
+__device__ __forceinline__ void umma_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar) : "memory");
+}
+#define R4(v, i) "=r"(v[i]), "=r"(v[i + 1]), "=r"(v[i + 2]), "=r"(v[i + 3])
+#define R16(v, i) R4(v, i), R4(v, i + 4), R4(v, i + 8), R4(v, i + 12)
+#define W4(v, i) "r"(v[i]), "r"(v[i + 1]), "r"(v[i + 2]), "r"(v[i + 3])
+#define W16(v, i) W4(v, i), W4(v, i + 4), W4(v, i + 8), W4(v, i + 12)
+// 32 columns of this warp's lanes (complete on return)
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* v) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,"
+      "%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
+      "tcgen05.wait::ld.sync.aligned;\n"
+      : R16(v, 0), R16(v, 16)
+      : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* v) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%32], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,"
+      "%24,%25,%26,%27,%28,%29,%30,%31};\n" ::W16(v, 0), W16(v, 16), "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* v) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};\n" ::W16(v, 0), "r"(taddr) : "memory");
+}
+#undef R4
+#undef R16
+#undef W4
+#undef W16
+__device__ __forceinline__ void st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }
+__device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
+__device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
+// address of 16-byte chunk c (0..15) of row r (16..31: V) of a page, [2 halves][32 rows][128 B], 128-byte swizzled
+__device__ __forceinline__ uint32_t chunk_at(uint32_t page, int r, int c) {
+  return page + (uint32_t)((c >> 3) * 4096 + r * 128 + (((c & 7) ^ (r & 7)) << 4));
 }
 
-__device__ __forceinline__ __half2 ldh2(uint32_t a) {
-  uint32_t v;
-  asm volatile("ld.shared.u32 %0, [%1];\n" : "=r"(v) : "r"(a) : "memory");
-  return *reinterpret_cast<__half2*>(&v);
-}
-// whether the values of a tile's keys up to kv1 hold an infinity or a NaN (asked by whole warps)
-__device__ __forceinline__ bool tile_not_finite(uint32_t kv, int key0, int kv1, int lane) {
-  uint32_t worst = 0;  // largest magnitude bits of the halves: an exponent of all ones has 0x7c00 and more
-  if (key0 + lane < kv1) {  // lane = key
-    const uint32_t row = kv + (uint32_t)(lane >> 4) * kPageBytes;
-#pragma unroll
-    for (int c = 0; c < 16; ++c) {
-      uint4 v;
-      asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];\n"
-                   : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-                   : "r"(row + chunk_at(32, 16 + (lane & 15), c))
-                   : "memory");
-      worst = __vmaxu2(worst, __vmaxu2(__vmaxu2(v.x & 0x7fff7fffu, v.y & 0x7fff7fffu), __vmaxu2(v.z & 0x7fff7fffu, v.w & 0x7fff7fffu)));
-    }
-  }
-  return __any_sync(0xffffffffu, (worst & 0xffffu) >= 0x7c00u || (worst >> 16) >= 0x7c00u);
-}
-
-__global__ void __launch_bounds__(kThreads, 3) attn_prefill_kernel(const qeng_prefill_attn p, const __grid_constant__ CUtensorMap kvmap) {
+__global__ void __launch_bounds__(kThreads, 1) attn_prefill_kernel(const qeng_prefill_attn p, const int per_cta, const __grid_constant__ CUtensorMap kvmap) {
   extern __shared__ unsigned char smem_raw[];
-  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const uint32_t ring = base + kQBytes;
-  __shared__ __align__(8) uint64_t full[kStages], empty[kStages];
-  __shared__ volatile int gave_up;  // a consumer stopped waiting: nobody waits for the producer's copies any more
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  const int grp = p.Hq / p.Hkv, tpt = kRows / grp;             // tokens per tile
-  // long tiles first, of all heads and sequences together: head after head, the long tiles of the last heads started late
-  // and an SM had work 65 % of the time
+  const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  __shared__ __align__(8) uint64_t kfull[kStages], kempty[kStages], sfull[2], pready[2], qready, odone, drained;
+  __shared__ uint32_t tmem_slot;
+  __shared__ volatile int skip_pv[2], not_finite[2][2][8];
+  __shared__ float met[2][2][2][kRows];  // [turn][tile][half]: maxima of the rows, at the end their sums
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int grp = p.Hq / p.Hkv, tpt = kRows / grp;  // tokens per tile
+  // long tiles first, of all heads and sequences together
   const int hb = blockIdx.x % (unsigned)(p.Hkv * p.B), b = hb / p.Hkv, h = hb - b * p.Hkv;
-  const int tt0 = (int)((gridDim.x - 1 - blockIdx.x) / (unsigned)(p.Hkv * p.B)) * tpt;
-  const int ntok = min(tpt, p.T - tt0);
+  const int tt0 = (int)((gridDim.x - 1 - blockIdx.x) / (unsigned)(p.Hkv * p.B)) * tpt * per_cta;
+  const int ntok = min(tpt * per_cta, p.T - tt0), tiles = (ntok + tpt - 1) / tpt;
 
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   if (tid == 0) {
     for (int s = 0; s < kStages; ++s) {
-      mbar_init(smem_u32(full + s), 1);
-      mbar_init(smem_u32(empty + s), kNW);
+      mbar_init(smem_u32(kfull + s), 1);
+      mbar_init(smem_u32(kempty + s), 1);
     }
-    gave_up = 0;
+    for (int x = 0; x < 2; ++x) {
+      mbar_init(smem_u32(sfull + x), 1);
+      mbar_init(smem_u32(pready + x), kSoftWarps / 2);
+      skip_pv[x] = 0;
+    }
+    mbar_init(smem_u32(&qready), kSoftWarps / 2 * tiles);
+    mbar_init(smem_u32(&odone), 1);
+    mbar_init(smem_u32(&drained), 1);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
-  asm volatile("griddepcontrol.wait;\n" ::: "memory");
-  // queries of this tile, zero rows where there is no token
-  for (int i = tid; i < kRows * 16; i += kThreads) {
-    const int r = i >> 4, c = i & 15, tok = r / grp;
-    uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (tok < ntok)
-      v = *reinterpret_cast<const uint4*>(p.q16 + (((size_t)b * p.T + tt0 + tok) * p.Hq + (size_t)h * grp + (r - tok * grp)) * kHD + c * 8);
-    asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};\n" ::"r"(base + chunk_at(kRows, r, c)), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+  if (warp == kMmaWarp) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;\n" ::"r"(smem_u32(&tmem_slot)));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
   }
-  // keys any row of the tile attends to: [kv0, kv1)
+  fence_before();
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  __syncthreads();
+  fence_after();
+  const uint32_t tmem = tmem_slot;
+
+  // keys any row of the CTA attends to: [kv0, kv1); of this warp's own tile: what all its rows attend ends at len_min, begins at win_max
   const int32_t* lens = p.lens + (size_t)b * p.T + tt0;
+  const int mine = warp < kSoftWarps ? warp >> 3 : 0;
   int kv1 = 0, kv0 = 0x7fffffff, len_min = 0x7fffffff, win_max = 0;
   for (int i = lane; i < ntok; i += 32) {
     const int l = min(lens[i], p.max_pages * 16), w0 = p.window > 0 ? max(0, l - p.window) : 0;
     kv1 = max(kv1, l);
-    len_min = min(len_min, l);
     kv0 = min(kv0, w0);
-    win_max = max(win_max, w0);
+    if (i / tpt == mine) {
+      len_min = min(len_min, l);
+      win_max = max(win_max, w0);
+    }
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -159,28 +202,26 @@ __global__ void __launch_bounds__(kThreads, 3) attn_prefill_kernel(const qeng_pr
     len_min = min(len_min, __shfl_xor_sync(0xffffffffu, len_min, o));
     win_max = max(win_max, __shfl_xor_sync(0xffffffffu, win_max, o));
   }
-  const int t0 = kv0 / kTile, t1 = (kv1 + kTile - 1) / kTile;
-  __syncthreads();
-
+  const int t0 = kv0 / kTile, t1 = (kv1 + kTile - 1) / kTile, n = max(t1 - t0, 0);
   bool failed = false;
-  if (warp == kNW) {
-    // ===== producer: two pages per tile; a page beyond the context repeats the last one (its keys are masked) ======
+
+  if (warp == kLoadWarp) {
+    // ===== pages: four per stage; a page beyond the context repeats the last one (its keys are masked) ==============
     const int last_page = (kv1 - 1) >> 4;
     int s = 0;
-    uint32_t ph = 0;
-    for (int kt = t0; kt < t1; ++kt) {
-      const int pg = min(kt * 2 + (lane & 1), last_page);
+    uint32_t ph = 1;
+    for (int j = 0; j < n; ++j) {
+      const int pg = min((t0 + j) * kPages + (lane & 3), last_page);
       int pid = p.table[(size_t)b * p.max_pages + pg];
       if ((unsigned)pid >= (unsigned)p.pages) {  // malformed page table: record it, read a page that exists
         atomicExch(p.status, 1);
         pid = 0;
       }
-      if (!failed && !mbar_wait(smem_u32(empty + s), ph ^ 1u)) failed = true;
-      if (__any_sync(0xffffffffu, failed)) { failed = true; break; }
-      const uint32_t bar = smem_u32(full + s);
+      if (!wait_warp(smem_u32(kempty + s), ph)) { failed = true; break; }
+      const uint32_t bar = smem_u32(kfull + s);
       if (lane == 0) mbar_expect_tx(bar, kStageBytes);
       __syncwarp();
-      if (lane < 2) {
+      if (lane < kPages) {
         const int row = (pid * p.Hkv + h) * 32;
         asm volatile(
             "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];\n" ::"r"(
@@ -190,186 +231,257 @@ __global__ void __launch_bounds__(kThreads, 3) attn_prefill_kernel(const qeng_pr
       }
       if (++s == kStages) { s = 0; ph ^= 1u; }
     }
-    if (failed && lane == 0) atomicExch(p.status, 4);
-    if (failed || gave_up) grace();
-    return;
-  }
-
-  // ===== consumers: rows warp * 16 + g and + 8 =========================================================
-  auto token_of = [&](int i) { return (warp * 16 + g + 8 * i) / grp; };  // worked out where needed: registers are short
-  const float sc = p.scale * 1.4426950408889634f;
-  float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
-  float o[16][4];
+  } else if (warp == kMmaWarp) {
+    // ===== MMA issue ================================================================================================
+    const uint32_t base = __shfl_sync(0xffffffffu, ring, 0), tm = __shfl_sync(0xffffffffu, tmem, 0);
+    if (elect_one()) {
+      // f16 x f16 -> f32, M = 128; S: N = 16, B K-major; O: N = 128, B MN-major
+      constexpr uint32_t kIdescS = (1u << 4) | (2u << 17) | (8u << 24), kIdescO = (1u << 4) | (1u << 16) | (16u << 17) | (8u << 24);
+      auto scores = [&](int x, int s) {
+        const uint32_t q = tm + (uint32_t)x * kTileCols, page = base + (uint32_t)s * kStageBytes;
 #pragma unroll
-  for (int j = 0; j < 16; ++j)
+        for (int pg = 0; pg < kPages; ++pg) {
+          const uint64_t kd = make_desc(page + pg * kPageBytes, 16, 1024);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) o[j][i] = 0.f;
-
-  // ldmatrix row of this lane: A (queries): rows 0..15, chunk lane/16; K: row lane%8, chunk lane/8; V: row lane%16, chunk lane/16
-  const int qrow = warp * 16 + (lane & 15), qc = lane >> 4, krow = lane & 7, kc = lane >> 3, vrow = 16 + (lane & 15), vc = lane >> 4;
-  // one tile of 32 keys; kEdge: not every row attends every key of it
-  auto tile = [&](int kt, uint32_t kv, auto edge_tile) {
-    constexpr bool kEdge = decltype(edge_tile)::value;
-    int len[2], win[2];  // the keys that the lane's two rows attend: [win, len)
-    if (kEdge) {
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        len[i] = token_of(i) < ntok ? min(lens[token_of(i)], p.max_pages * 16) : 0;
-        win[i] = p.window > 0 ? max(0, len[i] - p.window) : 0;
-      }
-    }
-    float sa[4][4];
-#pragma unroll
-    for (int n = 0; n < 4; ++n) sa[n][0] = sa[n][1] = sa[n][2] = sa[n][3] = 0.f;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {  // 32 of the 128 dims
-      uint32_t qa[2][4];
-#pragma unroll
-      for (int k = 0; k < 2; ++k) ldsm4(base + chunk_at(kRows, qrow, 4 * j + 2 * k + qc), qa[k]);
-#pragma unroll
-      for (int n = 0; n < 4; ++n) {
-        uint32_t kb[4];
-        ldsm4(kv + (uint32_t)(n >> 1) * kPageBytes + chunk_at(32, (n & 1) * 8 + krow, 4 * j + kc), kb);
-        mma16816(sa[n], qa[0], kb[0], kb[1]);
-        mma16816(sa[n], qa[1], kb[2], kb[3]);
-      }
-    }
-    // scale (optionally soft-capped), log2 domain, mask
-    float mx[2] = {-INFINITY, -INFINITY};
-#pragma unroll
-    for (int n = 0; n < 4; ++n)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        float x = sa[n][c];
-        if (p.softcap > 0.f) x = p.softcap * tanhf(x * p.scale / p.softcap) * 1.4426950408889634f;
-        else x *= sc;
-        if (kEdge) {
-          const int key = kt * kTile + n * 8 + 2 * t + (c & 1), i = c >> 1;
-          if (key >= len[i] || key < win[i]) x = -INFINITY;
+          for (int k = 0; k < 8; ++k) umma_f16(q + kS + 16 * pg, q + 8 * k, kd + (k >> 2) * (4096 >> 4) + (k & 3) * 2, kIdescS, k > 0);
         }
-        sa[n][c] = x;
-        mx[c >> 1] = fmaxf(mx[c >> 1], x);
-      }
-    float alpha[2];
+        umma_commit(smem_u32(sfull + x));
+      };
+      uint32_t begun = 0;  // bit x: tile x's O holds sums already
+      auto values = [&](int x, int s) {
+        const uint32_t t = tm + (uint32_t)x * kTileCols, page = base + (uint32_t)s * kStageBytes + 2048;
+        if (!skip_pv[x]) {
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 1));
-      mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 2));
-      const float mn = fmaxf(m_run[i], mx[i]);
-      const float ref = mn == -INFINITY ? 0.f : mn;  // nothing attended yet: all weights below are zero
-      alpha[i] = exp2f(m_run[i] - ref);
-      m_run[i] = mn;
-      l_run[i] *= alpha[i];
-      mx[i] = ref;
+          for (int pg = 0; pg < kPages; ++pg) {
+            const uint64_t vd = make_desc(page + pg * kPageBytes, 4096, 1024);
+            umma_f16(t + kO, t + kS + 8 * pg, vd, kIdescO, pg > 0 ? 1u : (begun >> x) & 1u);
+            umma_f16(t + kO, t + kS + 32 + 8 * pg, vd, kIdescO, 1u);
+          }
+        }
+        begun |= 1u << x;
+      };
+      failed = !mbar_wait(smem_u32(&qready), 0);
+      if (!failed && n > 0) {
+        failed = !mbar_wait(smem_u32(kfull), 0);
+        fence_after();
+        for (int x = 0; x < tiles && !failed; ++x) scores(x, 0);
+      }
+      int s = 0;
+      uint32_t ph = 0;
+      for (int j = 0; j < n && !failed; ++j) {
+        const int s1 = s + 1 == kStages ? 0 : s + 1;
+        const uint32_t ph1 = s1 == 0 ? ph ^ 1u : ph;
+        for (int x = 0; x < tiles; ++x) {
+          if (!mbar_wait(smem_u32(pready + x), (uint32_t)j & 1u)) { failed = true; break; }
+          fence_after();
+          values(x, s);
+          if (x + 1 == tiles) umma_commit(smem_u32(j + 1 < n ? kempty + s : &odone));
+          if (j + 1 < n) {
+            if (x == 0 && !mbar_wait(smem_u32(kfull + s1), ph1)) { failed = true; break; }
+            scores(x, s1);
+          }
+        }
+        s = s1;
+        ph = ph1;
+      }
+      if (failed) {  // what was issued still has to finish before tensor memory is freed
+        umma_commit(smem_u32(&drained));
+        mbar_wait(smem_u32(&drained), 0);
+      }
     }
+    failed = __any_sync(0xffffffffu, failed);
+  } else if (mine < tiles) {
+    // ===== softmax: this lane's row of tile `mine`, keys kKeys * half and on of each 64 ================================
+    const int quad = warp & 3, half = (warp >> 2) & 1, row = quad * 32 + lane, tok = row / grp, at = mine * tpt + tok;
+    const bool live = tok < tpt && at < ntok;
+    const size_t token = (size_t)b * p.T + tt0 + at;
+    const int head = h * grp + row - tok * grp;
+    const uint32_t mem = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)mine * kTileCols;
+    auto meet = [&] { asm volatile("bar.sync %0, %1;\n" ::"r"(1 + mine), "n"(kSoftWarps / 2 * 32) : "memory"); };  // the tile's warps
+    {
+      uint32_t q[32];
 #pragma unroll
-    for (int n = 0; n < 4; ++n)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        sa[n][c] = exp2f(sa[n][c] - mx[c >> 1]);
-        l_run[c >> 1] += sa[n][c];
+      for (int i = 0; i < 8; ++i) {
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (live) v = *reinterpret_cast<const uint4*>(p.q16 + (token * p.Hq + head) * kHD + half * 64 + i * 8);
+        q[4 * i] = v.x; q[4 * i + 1] = v.y; q[4 * i + 2] = v.z; q[4 * i + 3] = v.w;
       }
-    if (__any_sync(0xffffffffu, alpha[0] != 1.0f || alpha[1] != 1.0f)) {
-#pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        o[j][0] *= alpha[0]; o[j][1] *= alpha[0];
-        o[j][2] *= alpha[1]; o[j][3] *= alpha[1];
-      }
+      tmem_st32(mem + 32 * half, q);
+      st_wait();
+      fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&qready));
     }
-    // Where the rows attend different keys, a value that is not finite would reach rows that do not attend it (their weight
-    // is zero, but zero times infinity is NaN): such a tile, which real caches do not hold, goes key by key.
-    if (kEdge && tile_not_finite(kv, kt * kTile, kv1, lane)) {
+    // a row without a token attends everything, to nobody's use
+    const int len = live ? min(lens[at], p.max_pages * 16) : 0x7fffffff, win = live && p.window > 0 ? max(0, len - p.window) : 0;
+    const float sc = p.softcap > 0.f ? 1.f : p.scale * 1.4426950408889634f;
+    float m_run = -INFINITY, l_run = 0.f;  // the row's maximum; the sum of this half's keys
+    int slot = 0;
+    uint32_t slot_ph = 0;
 #pragma unroll 1
-      for (int k = 0; k < kTile; ++k) {
-        const int n = k >> 3, c = k & 1, src = (lane & ~3) | ((k & 7) >> 1), key = kt * kTile + k;
-        float w[2];  // weights of the lane's two rows for this key, from the lane of the quad that holds them
+    for (int j = 0; j < n; ++j) {
+      const int key0 = (t0 + j) * kTile;
+      const bool edge = key0 + kTile > len_min || key0 < win_max;  // not every row attends every key (the same in all warps of the tile)
+      if (!failed && !wait_warp(smem_u32(sfull + mine), (uint32_t)j & 1u)) failed = true;
+      fence_after();
+      float s[kKeys];
+      tmem_ld32(mem + kS + kKeys * half, reinterpret_cast<uint32_t*>(s));
+      if (p.softcap > 0.f) {
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          float x = 0.f;
+        for (int i = 0; i < kKeys; ++i) s[i] = p.softcap * tanhf(s[i] * p.scale / p.softcap) * 1.4426950408889634f;
+      }
+      if (edge) {
+        const int end = len - key0 - kKeys * half, begin = win - key0 - kKeys * half;
 #pragma unroll
-          for (int m = 0; m < 4; ++m)
-            if (m == n) x = c ? sa[m][2 * i + 1] : sa[m][2 * i];
-          w[i] = __shfl_sync(0xffffffffu, x, src);
+        for (int i = 0; i < kKeys; ++i)
+          if (i >= end || i < begin) s[i] = -INFINITY;
+        // Where the rows attend different keys, a value that is not finite would reach rows that do not attend it (their weight
+        // is zero, but zero times infinity is NaN): such a tile, which real caches do not hold, goes key by key.  Values of keys
+        // past the context, which nobody attends, are cleared.  A warp looks after half the dims of one page.
+        if (!failed && !wait_warp(smem_u32(kfull + slot), slot_ph)) failed = true;
+        const uint32_t page = ring + (uint32_t)slot * kStageBytes + (uint32_t)quad * kPageBytes;
+        const int r = 16 + (lane & 15), c0 = half * 8 + (lane >> 4) * 4;
+        uint32_t worst = 0;  // largest magnitude bits of the halves: an exponent of all ones has 0x7c00 and more
+        if (key0 + quad * 16 + (lane & 15) < kv1) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            uint4 v;
+            asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(chunk_at(page, r, c0 + c)) : "memory");
+            worst = __vmaxu2(worst, __vmaxu2(__vmaxu2(v.x & 0x7fff7fffu, v.y & 0x7fff7fffu), __vmaxu2(v.z & 0x7fff7fffu, v.w & 0x7fff7fffu)));
+          }
+        } else if (mine == 0) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};\n" ::"r"(chunk_at(page, r, c0 + c)), "r"(0u) : "memory");
+          asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
         }
-        const bool on0 = key < len[0] && key >= win[0], on1 = key < len[1] && key >= win[1];
+        const bool any = __any_sync(0xffffffffu, (worst & 0xffffu) >= 0x7c00u || (worst >> 16) >= 0x7c00u);
+        if (lane == 0) not_finite[mine][j & 1][warp & 7] = any;
+      }
+      float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const float2 v = __half22float2(ldh2(kv + (uint32_t)(k >> 4) * kPageBytes + chunk_at(32, 16 + (k & 15), j) + (uint32_t)t * 4u));
-          if (on0) { o[j][0] = fmaf(w[0], v.x, o[j][0]); o[j][1] = fmaf(w[0], v.y, o[j][1]); }
-          if (on1) { o[j][2] = fmaf(w[1], v.x, o[j][2]); o[j][3] = fmaf(w[1], v.y, o[j][3]); }
+      for (int i = 0; i < kKeys; ++i) mx4[i & 3] = fmaxf(mx4[i & 3], s[i]);
+      float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+      met[j & 1][mine][half][row] = mx;
+      meet();
+      mx = fmaxf(mx, met[j & 1][mine][half ^ 1][row]);
+      bool bad = false;
+      if (edge) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) bad = bad || not_finite[mine][j & 1][i];
+      }
+      // the reference of the row's exponentials moves when its maximum has left it far behind
+      const bool moved = mx > m_run && (m_run == -INFINITY || (mx - m_run) * sc > kGrow);
+      const float alpha = moved ? ex2((m_run - mx) * sc) : 1.f;
+      if (moved) m_run = mx;
+      l_run *= alpha;
+      if (j > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {  // this half's 64 dims
+#pragma unroll 1
+        for (int c = 0; c < 2; ++c) {
+          uint32_t o[32];
+          tmem_ld32(mem + kO + 64 * half + 32 * c, o);
+#pragma unroll
+          for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+          tmem_st32(mem + kO + 64 * half + 32 * c, o);
         }
       }
-    } else {
-      const bool tail = kEdge && (kt + 1) * kTile > kv1;
+      const float off = m_run == -INFINITY ? 0.f : -m_run * sc;  // nothing attended yet: all weights are zero
+      float sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-      for (int pg = 0; pg < 2; ++pg) {
-        uint32_t hi[4], lo[4];
+      for (int i = 0; i < kKeys; ++i) {
+        s[i] = ex2(fmaf(s[i], sc, off));
+        sum[i & 3] += s[i];
+      }
+      l_run += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+      if (!bad) {
+        uint32_t hi[16], lo[16];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {  // a0: keys 2t row g, a1: row g+8, a2 / a3: keys 2t + 8
-          const float x = sa[2 * pg + (q >> 1)][2 * (q & 1)], y = sa[2 * pg + (q >> 1)][2 * (q & 1) + 1];
-          hi[q] = pack_h2(x, y);
-          const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hi[q]));
-          lo[q] = pack_h2(x - f.x, y - f.y);
+        for (int i = 0; i < 16; ++i) {
+          hi[i] = pack_h2(s[2 * i], s[2 * i + 1]);
+          const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hi[i]));
+          lo[i] = pack_h2(s[2 * i] - f.x, s[2 * i + 1] - f.y);
         }
-        // keys past the context: their weight is zero, but zero times whatever the page holds there may be NaN
-        uint32_t keep[2] = {0xffffffffu, 0xffffffffu};
-        if (tail) {
+        tmem_st16(mem + kS + 16 * half, hi);
+        tmem_st16(mem + kS + 32 + 16 * half, lo);
+      } else {
+        const uint32_t w0 = ring + kStages * kStageBytes + (uint32_t)mine * kScratch + (uint32_t)row * 4u, pages = ring + (uint32_t)slot * kStageBytes;
 #pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            const int key = kt * kTile + pg * 16 + q * 8 + 2 * t;
-            keep[q] = (key < kv1 ? 0xffffu : 0u) | (key + 1 < kv1 ? 0xffff0000u : 0u);
+        for (int i = 0; i < kKeys; ++i) asm volatile("st.shared.f32 [%0], %1;\n" ::"r"(w0 + (uint32_t)(kKeys * half + i) * (kRows * 4)), "f"(s[i]) : "memory");
+        meet();
+        st_wait();
+#pragma unroll 1
+        for (int c = 2 * half; c < 2 * half + 2; ++c) {  // 32 of the 128 dims
+          uint32_t o[32];
+          if (j > 0) tmem_ld32(mem + kO + 32 * c, o);
+          else
+#pragma unroll
+            for (int i = 0; i < 32; ++i) o[i] = 0u;
+#pragma unroll 1
+          for (int k = 0; k < kTile; ++k) {
+            const bool on = key0 + k < len && key0 + k >= win;
+            float w;
+            asm volatile("ld.shared.f32 %0, [%1];\n" : "=f"(w) : "r"(w0 + (uint32_t)k * (kRows * 4)) : "memory");
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              uint32_t v[4];
+              asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];\n"
+                           : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+                           : "r"(chunk_at(pages + (uint32_t)(k >> 4) * kPageBytes, 16 + (k & 15), 4 * c + q))
+                           : "memory");
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&v[i]));
+                uint32_t* const d = o + 8 * q + 2 * i;
+                if (on) {
+                  d[0] = __float_as_uint(fmaf(w, f.x, __uint_as_float(d[0])));
+                  d[1] = __float_as_uint(fmaf(w, f.y, __uint_as_float(d[1])));
+                }
+              }
+            }
           }
+          tmem_st32(mem + kO + 32 * c, o);
         }
+      }
+      st_wait();
+      fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        if ((warp & 7) == 0) skip_pv[mine] = bad;
+        mbar_arrive(smem_u32(pready + mine));
+      }
+      if (++slot == kStages) { slot = 0; slot_ph ^= 1u; }
+    }
+    if (n > 0 && !failed && !wait_warp(smem_u32(&odone), 0)) failed = true;
+    fence_after();
+    met[n & 1][mine][half][row] = l_run;
+    meet();
+    l_run += met[n & 1][mine][half ^ 1][row];
+    const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
+    __nv_bfloat16* const dst = p.out + token * p.ldo + (size_t)head * kHD + half * 64;
+#pragma unroll 1
+    for (int c = 0; c < 2; ++c) {
+      uint32_t o[32];
+      tmem_ld32(mem + kO + 64 * half + 32 * c, o);
 #pragma unroll
-        for (int c = 0; c < 16; c += 2) {
-          uint32_t vb[4];
-          ldsm4_t(kv + (uint32_t)pg * kPageBytes + chunk_at(32, vrow, c + vc), vb);
-          if (tail) {
-            vb[0] &= keep[0]; vb[1] &= keep[1];
-            vb[2] &= keep[0]; vb[3] &= keep[1];
-          }
-          mma16816(o[c], hi, vb[0], vb[1]);
-          mma16816(o[c + 1], hi, vb[2], vb[3]);
-          mma16816(o[c], lo, vb[0], vb[1]);
-          mma16816(o[c + 1], lo, vb[2], vb[3]);
+      for (int i = 0; i < 32; i += 8) {
+        uint32_t hw[4], lw[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const float x = l_run > 0.f ? __uint_as_float(o[i + 2 * q]) * inv : 0.f, y = l_run > 0.f ? __uint_as_float(o[i + 2 * q + 1]) * inv : 0.f;
+          hw[q] = pack_b2(x, y);
+          const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&hw[q]));
+          lw[q] = pack_b2(x - f.x, y - f.y);
+        }
+        if (live) {
+          *reinterpret_cast<uint4*>(dst + 32 * c + i) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
+          if (p.planes == 2) *reinterpret_cast<uint4*>(dst + p.plane + 32 * c + i) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
         }
       }
     }
-  };
-  int s = 0;
-  uint32_t ph = 0;
-  for (int kt = t0; kt < t1; ++kt) {
-    if (!failed && !mbar_wait(smem_u32(full + s), ph)) failed = true;
-    const uint32_t kv = ring + (uint32_t)s * kStageBytes;
-    if ((kt + 1) * kTile > len_min || kt * kTile < win_max || ntok < tpt) tile(kt, kv, std::true_type());
-    else tile(kt, kv, std::false_type());
-    __syncwarp();
-    if (lane == 0) mbar_arrive(smem_u32(empty + s));
-    if (++s == kStages) { s = 0; ph ^= 1u; }
   }
-  if (failed) {
-    gave_up = 1;
-    if (lane == 0) atomicExch(p.status, 4);
-    grace();
-  }
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], 1);
-    l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], 2);
-    const int tok = token_of(i);
-    if (tok >= ntok) continue;
-    const float inv = l_run[i] > 0.f ? 1.f / l_run[i] : 0.f;
-    const int head = h * grp + (warp * 16 + g + 8 * i) - tok * grp;
-    const size_t at = ((size_t)b * p.T + tt0 + tok) * p.ldo + (size_t)head * kHD + 2 * t;
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      const float x = o[j][2 * i] * inv, y = o[j][2 * i + 1] * inv;
-      const __nv_bfloat162 hb = __floats2bfloat162_rn(x, y);
-      *reinterpret_cast<__nv_bfloat162*>(p.out + at + j * 8) = hb;
-      if (p.planes == 2)
-        *reinterpret_cast<__nv_bfloat162*>(p.out + p.plane + at + j * 8) = __floats2bfloat162_rn(x - __low2float(hb), y - __high2float(hb));
-    }
-  }
+  if (failed && lane == 0) atomicExch(p.status, 4);
+  fence_before();
+  if (__syncthreads_or(failed)) grace();
+  if (warp == kMmaWarp) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;\n" ::"r"(tmem));
 }
 
 }  // namespace
@@ -394,9 +506,11 @@ int32_t qeng_attn_prefill(qeng_ctx* ctx, const qeng_prefill_attn& p, const void*
     QENG_CUDA(ctx, cudaFuncSetAttribute(attn_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
     configured = true;
   }
-  const int tpt = kRows / (p.Hq / p.Hkv);
+  // Two tiles a CTA take turns on the tensor cores; with no more tiles than SMs each has one to itself.
+  const int tpt = kRows / (p.Hq / p.Hkv), tiles = (p.T + tpt - 1) / tpt;
+  const int per_cta = (int64_t)tiles * p.Hkv * p.B > ctx->sm_count ? 2 : 1;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)((p.T + tpt - 1) / tpt * p.Hkv * p.B));
+  cfg.gridDim = dim3((unsigned)((tiles + per_cta - 1) / per_cta * p.Hkv * p.B));
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = kSmem;
   cfg.stream = stream;
@@ -405,6 +519,6 @@ int32_t qeng_attn_prefill(qeng_ctx* ctx, const qeng_prefill_attn& p, const void*
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = ctx->pdl ? 1 : 0;
-  QENG_CUDA(ctx, cudaLaunchKernelEx(&cfg, attn_prefill_kernel, p, *reinterpret_cast<const CUtensorMap*>(map)));
+  QENG_CUDA(ctx, cudaLaunchKernelEx(&cfg, attn_prefill_kernel, p, per_cta, *reinterpret_cast<const CUtensorMap*>(map)));
   return QENG_OK;
 }

@@ -133,8 +133,8 @@ def test_prompt_epilogues_over_several_tiles(ctx):
     dec.free()
 
 
-# Query heads per kv head: one, the most there are, and counts that do not divide the 64 rows of a prompt attention tile
-# (its last rows stay empty); tiles then hold 64, 8, 21, 12, 10 and 9 tokens.
+# Query heads per kv head: one, the most there are, and counts that do not divide the 128 rows of a prompt attention tile
+# (its last rows stay empty); tiles then hold 128, 16, 42, 25, 21 and 18 tokens.
 @pytest.mark.parametrize("heads,kv_heads", [(2, 2), (8, 1), (6, 2), (5, 1), (6, 1), (7, 1)])
 def test_prompt_attention_groups(ctx, heads, kv_heads):
     from cyb_b200 import qeng
@@ -149,6 +149,33 @@ def test_prompt_attention_groups(ctx, heads, kv_heads):
     want, logs = ref.Decoder(cfg, W).generate(prompt, 3)
     assert ref.err_inf(dec.logits(), logs[0]) < 2e-3
     assert np.array_equal(dec.decode(3), want)
+    ctx.device_status()
+    dec.free()
+
+
+# More tiles of the prompt attention than SMs: two to a CTA, an odd number of them, ten tiles of keys through a ring of three, and
+# scores spread so far that rows are rescaled on the way.  Against the teacher the operands of the matmuls, rounded to bf16 (2^-9
+# each, of scores of some tens), leave 1e-2 (as much with any attention); against the same prompt in two calls, one tile a CTA,
+# only sums in another order differ, and the bf16 roundings of its output that they tip: far below 1e-3.
+@pytest.mark.parametrize("window", [0, 100])
+def test_long_prompt_attention_two_tiles_a_cta(ctx, window):
+    from cyb_b200 import qeng
+    cfg = ref.DecoderConfig(layers=1, d=256, ffn=512, heads=8, kv_heads=1, vocab=320, sliding_window=window)
+    W = ref.make_decoder_weights(cfg, seed=6)
+    q, s = W["layers"][0]["wq"]
+    W["layers"][0]["wq"] = (q, (s.astype(np.float32) * 4).astype(np.float16))
+    dec = ctx.decoder(layers=1, d_model=256, ffn=512, heads=8, kv_heads=1, vocab=320, max_batch=4, max_seq=640, sliding_window=window)
+    qeng.load_decoder_weights(dec, W, cfg)
+    prompt = ref.rng_of(77).integers(0, 320, (4, 601)).astype(np.int32)
+    dec.reset(4)
+    dec.prefill(prompt)
+    one = dec.logits()
+    _, logs = ref.Decoder(cfg, W).generate(prompt, 1)
+    assert ref.err_inf(one, logs[0]) < 2e-2
+    dec.reset(4)
+    dec.prefill(prompt[:, :301])
+    dec.prefill(prompt[:, 301:])
+    assert ref.err_inf(dec.logits(), one) < 1e-3
     ctx.device_status()
     dec.free()
 
@@ -223,7 +250,7 @@ def test_lm_head_edges(ctx, v, d):
     ctx.device_status()
 
 
-# A 64-row tile of the prompt attention holds tokens that attend different keys.  Token 20's values overflow f16: the rows
+# A tile of the prompt attention holds tokens that attend different keys.  Token 20's values overflow f16: the rows
 # that do not attend it (before it, and with a window of 8 those from 28 on) give what they give without it.
 @pytest.mark.parametrize("window", [0, 8])
 def test_prompt_rows_do_not_see_infinite_values_they_do_not_attend(ctx, window):

@@ -187,15 +187,113 @@ struct Words<QENG_FMT_Q8> {
   }
 };
 
+// ---- the same for the epilogues that combine rows r and r + 8 of a 16-row tile (SWIGLU into planes, QKV), of a whole tile -------
+// 16 tokens of the warp's 32 rows are turned in shared memory, so that a lane has the 16 rows of one row tile for one token: its
+// angles are four loads of 16 bytes, its results one or two stores of 16.  With a lane's row of every token the exchange between
+// lanes, the addresses and the 2-byte stores were some 30 instructions a token, which the epilogue's four warps issue between
+// those of sixteen dequantising ones: 160 tokens of q|k|v took longer than the tile's MMAs.  1800 tokens (ncu): q|k|v 6144 x 4096
+// 118 us and 9 for the sums of its cut tiles -> 86 with none cut, gate|up 290 and 8 -> 274; a prompt of 16 x 45 tokens through 32
+// layers 9.46 -> 8.07 ms, of 1800 20.1 -> 18.2.  (Asking for positions, angles and pages ahead, row by row, gave nothing: 130 us.)
+constexpr uint32_t kTurnRow = 36 * 4, kTurnBytes = 4 * 16 * kTurnRow;  // 16 bytes between rows: no bank conflicts either way
+__device__ __forceinline__ void drain_pairs(const TcParams& p, int tile, uint32_t rank, uint32_t tacc, int quad, int lane, uint32_t turn) {
+  int mt, nt;
+  tile_pos(p, tile, mt, nt);
+  const int m0 = mt * p.bn, mcnt = min(p.bn, p.M - m0), tl = lane >> 1;
+  const int t16 = nt * 16 + (int)rank * 8 + quad * 2 + (lane & 1);  // this lane's row tile, token c0 + tl
+  const bool live = t16 * 16 < p.N, swiglu = p.e.kind == QENG_EPI_SWIGLU;
+  const qeng_qkv_epi& q = p.e.qkv;
+  const int head = t16 >> 3, d = (t16 & 7) << 3, kh = head - q.Hq;
+  const bool rotate = !swiglu && head < q.Hq + q.Hkv;
+  const uint32_t buf = turn + (uint32_t)quad * (16 * kTurnRow);
+  int ps = !swiglu && tl < mcnt && live ? q.pos[m0 + tl] : 0;  // a group ahead
+#pragma unroll 1
+  for (int c0 = 0; c0 < mcnt; c0 += 16) {
+    const int m = c0 + tl;
+    bool on = m < mcnt && live;
+    float4 cs[4];
+    int pid = 0;
+    if (!swiglu) {
+      if (on && (ps < 0 || ps >= q.max_seq || (ps >> 4) >= q.max_pages)) {
+        atomicExch(p.status, 2);
+        on = false;
+      }
+      if (on && rotate) {
+        const float4* a = reinterpret_cast<const float4*>(q.cs + (size_t)ps * 128 + d);
+        cs[0] = __ldg(a); cs[1] = __ldg(a + 1); cs[2] = __ldg(a + 16); cs[3] = __ldg(a + 17);
+      }
+      if (on && kh >= 0) pid = q.table[(size_t)((m0 + m) / q.rows_per_seq) * q.max_pages + (ps >> 4)];
+    }
+    const int at = ps;
+    if (!swiglu && m + 16 < mcnt && live) ps = q.pos[m0 + m + 16];
+    uint32_t v[16];
+    tmem_ld16(tacc + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, v);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) asm volatile("st.shared.u32 [%0], %1;\n" ::"r"(buf + (uint32_t)i * kTurnRow + (uint32_t)lane * 4u), "r"(v[i]) : "memory");
+    __syncwarp();
+    float lo[8], hi[8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint4 w = lds128(buf + (uint32_t)tl * kTurnRow + (uint32_t)((lane & 1) * 64 + i * 16));
+      float* const o = i < 2 ? lo + 4 * i : hi + 4 * (i - 2);
+      o[0] = __uint_as_float(w.x); o[1] = __uint_as_float(w.y); o[2] = __uint_as_float(w.z); o[3] = __uint_as_float(w.w);
+    }
+    __syncwarp();
+    if (swiglu) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) lo[i] = lo[i] / (1.0f + __expf(-lo[i])) * hi[i];
+      if (!on) continue;
+      __nv_bfloat16* const dst = p.e.yb + (size_t)(m0 + m) * p.e.ldyb + (size_t)t16 * 8;
+      uint32_t h[4], l[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) split2(lo[2 * i], lo[2 * i + 1], h[i], l[i]);
+      *reinterpret_cast<uint4*>(dst) = make_uint4(h[0], h[1], h[2], h[3]);
+      if (p.e.yb_planes == 2) *reinterpret_cast<uint4*>(dst + p.e.yb_plane) = make_uint4(l[0], l[1], l[2], l[3]);
+      continue;
+    }
+    if (!on) continue;
+    if (rotate) {
+      const float c[8] = {cs[0].x, cs[0].y, cs[0].z, cs[0].w, cs[1].x, cs[1].y, cs[1].z, cs[1].w};
+      const float sn[8] = {cs[2].x, cs[2].y, cs[2].z, cs[2].w, cs[3].x, cs[3].y, cs[3].z, cs[3].w};
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float a = lo[i], b = hi[i];
+        lo[i] = a * c[i] - b * sn[i];
+        hi[i] = b * c[i] + a * sn[i];
+      }
+    }
+    __half* dst;
+    if (kh < 0) {
+      dst = q.q16 + ((size_t)(m0 + m) * q.Hq + head) * 128 + d;
+    } else {
+      if ((unsigned)pid >= (unsigned)q.pages) {
+        atomicExch(p.status, 1);
+        continue;
+      }
+      const int isv = kh >= q.Hkv ? 1 : 0;
+      dst = q.pool + (((size_t)pid * q.Hkv + (kh - isv * q.Hkv)) * 2 + isv) * (16 * 128) + (at & 15) * 128 + d;
+    }
+    uint32_t w[8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const __half2 a = __floats2half2_rn(lo[2 * i], lo[2 * i + 1]), b = __floats2half2_rn(hi[2 * i], hi[2 * i + 1]);
+      w[i] = *reinterpret_cast<const uint32_t*>(&a);
+      w[4 + i] = *reinterpret_cast<const uint32_t*>(&b);
+    }
+    *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+    *reinterpret_cast<uint4*>(dst + 64) = make_uint4(w[4], w[5], w[6], w[7]);
+  }
+}
+
 // ---- one warp's part of a finished accumulator: groups of 16 tokens from c0 on, every `step` tokens -------------------
-template <bool ACCUM_ONLY>
+// (FIXED: only parts of cut tiles and whole ones added to y)
+template <bool FIXED>
 __device__ __forceinline__ void drain(const TcParams& p, int tile, bool whole, int pair, uint32_t rank, uint32_t tacc, int quad, int lane, int c0, int step) {
   int mt, nt;
   tile_pos(p, tile, mt, nt);
   const int m0 = mt * p.bn, mcnt = min(p.bn, p.M - m0), row = quad * 32 + lane;
   float* const mine = whole ? nullptr : partial(p, pair, tile - p.dp_tiles, rank, row);
   qeng_tc_epi e = p.e;
-  if (ACCUM_ONLY) e.kind = QENG_EPI_ACCUM;
+  if (FIXED) e.kind = QENG_EPI_ACCUM;
 #pragma unroll 1
   for (; c0 < mcnt; c0 += step) {
     uint32_t v[16];
@@ -212,10 +310,14 @@ __device__ __forceinline__ void drain(const TcParams& p, int tile, bool whole, i
   }
 }
 
-template <int FMT, int WP, int XP, int KST, bool HELP>
+// What empties an accumulator: the four epilogue warps row by row; they and the dequantising ones (a single accumulator, added to
+// y); or the four by drain_pairs
+enum { kPlain = 0, kHelp = 1, kPairs = 2 };
+template <int FMT, int WP, int XP, int KST, int MODE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     gemm_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap,
                    const __grid_constant__ CUtensorMap smap) {
+  constexpr bool HELP = MODE == kHelp;
   constexpr int kW = Fmt<FMT>::kW, kS = Fmt<FMT>::kS;
   constexpr uint32_t kSlot = KST * 8 * (kW + kS), kStageCols = KST * WP * kACols;
   extern __shared__ unsigned char smem_raw[];
@@ -456,8 +558,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
       if (!failed && !mbar_wait(smem_u32(acc_full + buf), acc_ph)) failed = true;
       __syncwarp();
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-      if (!__any_sync(0xffffffffu, failed))
-        drain<HELP>(p, sg.tile, whole, pair, rank, tmem + (uint32_t)(buf * p.acc_cols), quad, lane, 0, HELP && whole ? 16 * (1 + kHelpers / 4) : 16);
+      if (!__any_sync(0xffffffffu, failed)) {
+        if (MODE == kPairs && whole) drain_pairs(p, sg.tile, rank, tmem + (uint32_t)(buf * p.acc_cols), quad, lane, ring + (uint32_t)p.nslots * kSlot);
+        else drain<HELP || MODE == kPairs>(p, sg.tile, whole, pair, rank, tmem + (uint32_t)(buf * p.acc_cols), quad, lane, 0, HELP && whole ? 16 * (1 + kHelpers / 4) : 16);
+      }
       asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(map_leader(smem_u32(acc_empty + buf)));
@@ -638,12 +742,12 @@ EncodeFn encode_fn() {
 // stage leaves room for it).  False where two stages do not fit.
 bool fit_rings(Plan* pl, int fmt, int wp, int xp) {
   const size_t stage = (size_t)pl->kst * xp * (pl->bn / 2) * 128, slot = (size_t)slot_bytes_of(fmt, pl->kst);
-  const size_t room = kSmemBudget - 1024 - 1024;  // alignment, static shared memory
+  const size_t turn = pl->pairs ? kTurnBytes : 0, room = kSmemBudget - 1024 - 1024 - turn;  // alignment, static shared memory
   pl->nstages = std::min(std::min((512 - pl->nacc * pl->acc_cols) / (pl->kst * wp * kACols), kMaxStages), (int)((room - 4 * slot) / stage));
   if (pl->nstages < 2) return false;
   pl->nslots = (int)((room - pl->nstages * stage) / slot);
   pl->nslots = (pl->nslots < kMaxSlots ? pl->nslots : kMaxSlots) / kSets * kSets;  // a slot belongs to one dequant set
-  pl->smem = pl->nstages * stage + pl->nslots * slot + 1024;
+  pl->smem = pl->nstages * stage + pl->nslots * slot + turn + 1024;
   return true;
 }
 
@@ -653,11 +757,12 @@ bool fit_rings(Plan* pl, int fmt, int wp, int xp) {
 //   the MMAs take 2 * bn per product, the dequantisation 430 (4-bit blocks, one term), 735 (two), 870 (8-bit) or 1020 (K-quant),
 //   a stage what is longer; stages of one chunk add 34 to the former and 76 to the latter (each has its barriers), two stages in
 //   all 106 and 163 (one waits for the other's refill).
-// Emptying an accumulator takes 17 cycles a token (store), 27 (accumulate), 12 with the dequantising warps' help, 100 (SWIGLU)
-// and 250 (QKV, whose pages and angles come from L2); the next tile hides it where there are two of them (a last store then takes
+// Emptying an accumulator takes 17 cycles a token (store), 27 (accumulate), 12 with the dequantising warps' help, 100 (SWIGLU row by
+// row) and 250 (QKV row by row), 60 of both by drain_pairs (fitted to K of 4096: 40, 60, 80, 90 and 100 for either, prompts of 45 to
+// 1800 tokens; below 2048 the former two are kept); the next tile hides it where there are two of them (a last store then takes
 // 11).  Every tile of the first round costs 29 (the pairs' first loads meet).  Tiles cut along K pay for their parts (64 a token,
 // 0.6 of it where another segment hides one), their sums (700 a part) and the second launch (9400).
-Plan make_plan(const qeng_ctx* ctx, const qeng_weight* w, int64_t M, int wp, int xp, int epi, bool may_split) {
+Plan make_plan(const qeng_ctx* ctx, const qeng_weight* w, int64_t M, int wp, int xp, int epi, bool pairs_ok, bool may_split) {
   Plan best = {};
   double best_cost = 1e30;
   const int pairs = ctx->sm_count / 2, n_tiles = (int)((w->N + 255) / 256), products = wp + xp - 1;
@@ -670,6 +775,7 @@ Plan make_plan(const qeng_ctx* ctx, const qeng_weight* w, int64_t M, int wp, int
       c.nacc = 1 + form % 2;
       c.acc_cols = (bn + 31) / 32 * 32;
       c.bn = bn;
+      c.pairs = pairs_ok;
       if (!fit_rings(&c, w->fmt, wp, xp)) continue;
       c.m_tiles = (int)((M + bn - 1) / bn);
       c.n_tiles = n_tiles;
@@ -679,7 +785,8 @@ Plan make_plan(const qeng_ctx* ctx, const qeng_weight* w, int64_t M, int wp, int
       const double mma = 2.0 * c.kst * std::max(bn, 32) * products + (one ? 34 : 0) + (two ? 106 : 0);
       const double convert = c.kst * deq + (one ? 76 : 0) + (two ? 163 : 0);
       const double stage = std::max(mma, convert);
-      const double per_token = epi == QENG_EPI_QKV ? 250 : epi == QENG_EPI_SWIGLU ? 100 : epi == QENG_EPI_STORE ? (c.nacc == 1 ? 17 : 11) : c.nacc == 1 ? 12 : 27;
+      const bool turned = pairs_ok && w->nchunks >= 32;
+      const double per_token = epi == QENG_EPI_QKV ? (turned ? 60 : 250) : epi == QENG_EPI_SWIGLU ? (turned ? 60 : 100) : epi == QENG_EPI_STORE ? (c.nacc == 1 ? 17 : 11) : c.nacc == 1 ? 12 : 27;
       const double ep = per_token * bn, body = nk * stage, tile = c.nacc == 1 ? body + ep : std::max(body, ep);
       const double dp = waves * tile + (c.nacc == 1 ? 0.0 : ep) + 29.0 * std::min(T, pairs);
       // shares of at least two stages (with no whole tiles the number of pairs is reduced instead)
@@ -699,6 +806,10 @@ Plan make_plan(const qeng_ctx* ctx, const qeng_weight* w, int64_t M, int wp, int
       c.npairs = cut ? sharing : std::min(T, pairs);
       best = c;
     }
+  }
+  if (best.pairs && best.dp_tiles == 0) {  // (nothing but parts, whose sums another kernel finishes: their room goes to the packed ring)
+    best.pairs = false;
+    fit_rings(&best, w->fmt, wp, xp);
   }
   best.box_rows = best.bn / 2;
   best.ws_floats = best.sk_tiles > 0 ? (size_t)best.npairs * 4 * best.bn * 128 : 0;
@@ -726,12 +837,12 @@ bool weight_maps(const qeng_weight* w) {
   return true;
 }
 
-template <int FMT, int WP, int XP, int KST, bool HELP>
+template <int FMT, int WP, int XP, int KST, int MODE>
 int32_t launch(qeng_ctx* ctx, const qeng_weight* w, const TcParams& p, const Plan& pl, const CUtensorMap& map, cudaStream_t stream) {
   static bool configured_on[64] = {};  // the opt-in shared-memory size is set per device
   bool& configured = configured_on[ctx->device & 63];
   if (!configured) {
-    QENG_CUDA(ctx, cudaFuncSetAttribute(gemm_tc_kernel<FMT, WP, XP, KST, HELP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
+    QENG_CUDA(ctx, cudaFuncSetAttribute(gemm_tc_kernel<FMT, WP, XP, KST, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
     configured = true;
   }
   cudaLaunchConfig_t cfg = {};
@@ -746,7 +857,7 @@ int32_t launch(qeng_ctx* ctx, const qeng_weight* w, const TcParams& p, const Pla
   cfg.numAttrs = ctx->pdl ? 1 : 0;
   const CUtensorMap* wm = reinterpret_cast<const CUtensorMap*>(w->tc_maps[KST - 1][0]);
   const CUtensorMap* sm = reinterpret_cast<const CUtensorMap*>(w->tc_maps[KST - 1][1]);
-  QENG_CUDA(ctx, cudaLaunchKernelEx(&cfg, gemm_tc_kernel<FMT, WP, XP, KST, HELP>, p, map, *wm, *sm));
+  QENG_CUDA(ctx, cudaLaunchKernelEx(&cfg, gemm_tc_kernel<FMT, WP, XP, KST, MODE>, p, map, *wm, *sm));
   return p.sk_tiles > 0 ? reduce(ctx, p, stream) : QENG_OK;
 }
 
@@ -815,19 +926,25 @@ int32_t qeng_gemm_tc(qeng_ctx* ctx, const qeng_weight* w, const qeng_tc_x& x, in
   const int xp = x.planes;
   if (w->fmt != QENG_FMT_Q4 && wp == 1) return qeng_fail(ctx, QENG_ERR_SHAPE, "gemm_tc: single bf16 weights are for 4-bit blocks only");
   if (wp == 1 && xp != 1) return qeng_fail(ctx, QENG_ERR_ARG, "gemm_tc: two activation planes need two weight planes");
-  Plan pl = make_plan(ctx, w, M, wp, xp, epi.kind, true);
+  // drain_pairs makes 16-byte accesses: rows of planes, pages and angles allow them (the decoder's buffers)
+  const bool pairs_ok = epi.kind == QENG_EPI_QKV || (epi.kind == QENG_EPI_SWIGLU && epi.yb != nullptr &&
+                        ((reinterpret_cast<uintptr_t>(epi.yb) | (uintptr_t)(epi.ldyb * 2) | (uintptr_t)(epi.yb_plane * 2)) & 15) == 0);
+  Plan pl = make_plan(ctx, w, M, wp, xp, epi.kind, pairs_ok, true);
   TcParams p;
   CUtensorMap map;
   if (pl.sk_tiles > 0 && sc == nullptr) sc = qeng_scratch_for(ctx, stream);
   int32_t rc = prepare(ctx, w, x, M, epi, sc, &pl, &p, &map);
   if (rc == QENG_ERR_STATE) {  // no memory for the workspace: whole tiles only
-    pl = make_plan(ctx, w, M, wp, xp, epi.kind, false);
+    pl = make_plan(ctx, w, M, wp, xp, epi.kind, pairs_ok, false);
     rc = prepare(ctx, w, x, M, epi, sc, &pl, &p, &map);
   }
   if (rc != QENG_OK) return rc;
   const bool help = pl.nacc == 1 && epi.kind == QENG_EPI_ACCUM;
-  if (wp == 1) return help ? launch<QENG_FMT_Q4, 1, 1, 2, true>(ctx, w, p, pl, map, stream) : launch<QENG_FMT_Q4, 1, 1, 2, false>(ctx, w, p, pl, map, stream);
-#define QENG_TC_K(F, X, K) (help ? launch<F, 2, X, K, true>(ctx, w, p, pl, map, stream) : launch<F, 2, X, K, false>(ctx, w, p, pl, map, stream))
+#define QENG_TC_M(F, W, X, K)                                                 \
+  (help ? launch<F, W, X, K, kHelp>(ctx, w, p, pl, map, stream)               \
+        : pl.pairs ? launch<F, W, X, K, kPairs>(ctx, w, p, pl, map, stream) : launch<F, W, X, K, kPlain>(ctx, w, p, pl, map, stream))
+  if (wp == 1) return QENG_TC_M(QENG_FMT_Q4, 1, 1, 2);
+#define QENG_TC_K(F, X, K) QENG_TC_M(F, 2, X, K)
 #define QENG_TC(F, X) (pl.kst == 2 ? QENG_TC_K(F, X, 2) : QENG_TC_K(F, X, 1))
   switch (w->fmt) {
     case QENG_FMT_Q4: return xp == 1 ? QENG_TC(QENG_FMT_Q4, 1) : QENG_TC(QENG_FMT_Q4, 2);
@@ -836,6 +953,7 @@ int32_t qeng_gemm_tc(qeng_ctx* ctx, const qeng_weight* w, const qeng_tc_x& x, in
   }
 #undef QENG_TC
 #undef QENG_TC_K
+#undef QENG_TC_M
 }
 
 // y[M,N] = x . dequant(W)^T through the kernel above, activations in any type the entry point takes.
@@ -868,7 +986,7 @@ int32_t qeng_gemm_many_rows(qeng_ctx* ctx, const qeng_weight* w, const void* x, 
 
 // For the tests, which have to meet every kind of plan: chunks a stage, tokens a tile, accumulators, whole tiles, cut tiles, pairs.
 extern "C" int32_t qeng_many_rows_plan(const qeng_ctx* ctx, const qeng_weight* w, int64_t M, int32_t wp, int32_t xp, int32_t epilogue, int32_t* out) {
-  const Plan pl = make_plan(ctx, w, M, wp, xp, epilogue, true);
+  const Plan pl = make_plan(ctx, w, M, wp, xp, epilogue, epilogue == QENG_EPI_QKV || epilogue == QENG_EPI_SWIGLU, true);
   const int v[6] = {pl.kst, pl.bn, pl.nacc, pl.dp_tiles, pl.sk_tiles, pl.npairs};
   std::copy(v, v + 6, out);
   return QENG_OK;

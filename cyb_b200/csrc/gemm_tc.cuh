@@ -362,6 +362,7 @@ __device__ __forceinline__ void finish(const qeng_tc_epi& e, int N, int32_t* sta
 
 struct Plan {
   int kst, nk, bn, m_tiles, n_tiles, dp_tiles, sk_tiles, npairs, nstages, nslots, nacc, acc_cols;
+  bool pairs;    // whole tiles by drain_pairs
   int box_rows;  // rows of an activation box
   size_t smem, ws_floats;
 };

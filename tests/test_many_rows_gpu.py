@@ -133,6 +133,42 @@ def test_prompt_epilogues_over_several_tiles(ctx):
     dec.free()
 
 
+def test_prompt_epilogues_of_whole_tiles(ctx):
+    """The same where the planner's constants are the ones fitted to values turned in shared memory (K of 2048 and more): whole
+    tiles of more tokens than a multiple of 16.  Against the teacher the operands rounded to bf16 leave 1e-2 here (the second
+    matrix sees products of two of them); against the same rows in two calls, in other tiles, only
+    the roundings tipped by sums in another order differ (2^-9 of single operands: 1e-3).  Three sequences give the same in another
+    order."""
+    import torch
+    from cyb_b200 import qeng
+    T = 601
+    cfg = ref.DecoderConfig(layers=1, d=2048, ffn=4096, heads=16, kv_heads=8, vocab=320)
+    W = ref.make_decoder_weights(cfg, seed=5)
+    dec = ctx.decoder(layers=1, d_model=2048, ffn=4096, heads=16, kv_heads=8, vocab=320, max_batch=3, max_seq=640)
+    qeng.load_decoder_weights(dec, W, cfg)
+    SWIGLU, QKV = 3, 4
+    for rows in (T, 3 * 173):
+        assert _plan(ctx, dec.weight(0, 0), rows, 1, 1, QKV)[3] != "cut" and _plan(ctx, dec.weight(0, 2), rows, 1, 1, SWIGLU)[3] != "cut"
+    teacher = ref.Decoder(cfg, W)
+    teacher.reset(1)
+    x = ref.rng_of(41).standard_normal((1, T, cfg.d), dtype=np.float32)
+    want = teacher.layer(0, x.astype(np.float64), np.arange(T)[None])
+    xs = torch.from_numpy(x[0]).cuda()
+    got = dec.layer(0, xs, np.arange(T)).cpu().numpy()
+    assert ref.err_inf(got, want[0]) < 2e-2
+    halves = [dec.layer(0, xs[a:b], np.arange(a, b)).cpu().numpy() for a, b in ((0, 301), (301, T))]
+    assert ref.err_inf(np.concatenate(halves), got) < 4e-3
+    prompt = ref.rng_of(43).integers(0, 320, (3, 173)).astype(np.int32)
+    logits = []
+    for order in ([0, 1, 2], [2, 0, 1]):
+        dec.reset(3)
+        dec.prefill(prompt[order])
+        logits.append(dec.logits()[np.argsort(order)])
+    assert ref.err_inf(logits[1], logits[0]) < 1e-3
+    ctx.device_status()
+    dec.free()
+
+
 # Query heads per kv head: one, the most there are, and counts that do not divide the 128 rows of a prompt attention tile
 # (its last rows stay empty); tiles then hold 128, 16, 42, 25, 21 and 18 tokens.
 @pytest.mark.parametrize("heads,kv_heads", [(2, 2), (8, 1), (6, 2), (5, 1), (6, 1), (7, 1)])

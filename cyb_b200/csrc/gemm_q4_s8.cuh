@@ -353,7 +353,7 @@ __device__ __forceinline__ void quantise_group(const float (&v)[8], bool valid, 
 // offsets into a stage.  What bounds these loops is the instructions around the MMAs (40 per 16 x 32 block and warp with addresses
 // and ring positions worked out per stage, masked activations and one f32 operation a value: the issue slots of 1280 of the 1440
 // cycles that HBM takes per tile).  One row, 15 bits / 22 bits, microseconds before and now, L2 cold: 22016 x 4096 13.6 / 14.0 ->
-// 11.4 / 12.4, 11008 x 4096 7.8 / 8.2 -> 7.0 / 7.5, 4096 x 11008 8.7 / 9.4 -> 8.0 / 8.5, 4096 x 4096 4.6 / 4.8 -> 4.4 / 4.4.
+// 10.4 / 11.4, 11008 x 4096 7.8 / 8.2 -> 6.7 / 7.1, 4096 x 11008 8.7 / 9.4 -> 7.5 / 8.1, 4096 x 4096 4.6 / 4.8 -> 4.4 / 4.5.
 struct LaneX {
   uint32_t xa, zin, fex, fsx;
 };
@@ -456,6 +456,33 @@ __device__ __forceinline__ void consume_x4(f32x2 (&acc)[2], uint32_t wl, uint32_
     }
   }
 }
+// ---- 4-bit blocks, every tile one stage of an even number of chunks: a warp's share lies at the same k in all of them ---------
+// (two items of two chunks at most), so its activations stay in registers and a tile is straight-line code.
+struct HeldX {
+  uint2 z[2][2], f[2][2], b[2][2];  // [item][chunk]
+  __device__ __forceinline__ void load(int j, int it, const LaneX& X) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const uint32_t blk = (uint32_t)(4 * it + 2 * i);
+      z[j][i] = lds64(X.zin + blk * 4u);
+      f[j][i] = lds64(X.fex + blk * 4u);
+      b[j][i] = lds64(X.xa + blk * 32u);
+    }
+  }
+  // item j of a tile: its weights + 16 * lane at w, its scales + the lane group's offset at s
+  __device__ __forceinline__ void contract(f32x2 (&acc)[2], int j, uint32_t w, uint32_t s) const {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const WBlocks<false> W = load_chunk<false>(w + (uint32_t)i * 512u);
+      const PairScales<false> S = load_pairs<false>(s + (uint32_t)i * 64u);
+      const int c[4] = {(int)z[j][i].x, (int)z[j][i].y, (int)z[j][i].x, (int)z[j][i].y};
+      int d0[4], d1[4];
+      chunk_mma<false>(d0, W, 0, b[j][i].x, b[j][i].y, c);
+      chunk_mma<false>(d1, W, 1, b[j][i].x, b[j][i].y, c);
+      add_item<false>(acc, d0[0], d1[1], d0[2], d1[3], S, pair2(__uint_as_float(f[j][i].x), __uint_as_float(f[j][i].y)), 0u);
+    }
+  }
+};
 // a lane's sums of a tile, added over the lanes that share a row: afterwards lane t has row g + 8 (t & 1)
 __device__ __forceinline__ float quad_rows(float a0, float a1, int lane, bool four) {
   const bool odd = (lane & 1) != 0;

@@ -183,6 +183,11 @@ __global__ void __launch_bounds__(kCT + 32 * (kTG == 0 ? 1 : kTG), 1) gemv_q4_st
   // partial sums of a tile in shared memory and moves on; the CTA meets once at the end (or every
   // kDeferTiles tiles), where the warps sum the partials and run the epilogues of the tiles in parallel
   constexpr bool kDefer = kTG == 0;
+  // 4-bit blocks, items of one chunk (one row in three limbs, or two rows): a matrix whose tiles are one stage has a loop of its own
+  // (22016 x 4096, 22 bits 11.4 -> 9.9 us, 11008 x 4096 7.1 -> 6.5, 4096 x 4096 4.5 -> 4.4; decode steps +-0).  One row in two
+  // limbs has not: alone it gains as much (10.4 -> 9.6), but a decode step runs that kernel over both kinds of matrix in turn, and
+  // with both loops in it the step takes 1328 us where it takes 1270 with one.
+  constexpr bool kHold = !Q8 && !KQ && (MODE == kM1L3 || MODE == kM2L2);
   constexpr int kTGe = kDefer ? 1 : kTG;  // tile groups (rings, producer warps)
   constexpr int kGW = kCW / kTGe;         // warps per tile group
   constexpr int kMR = MODE == kMN ? 4 * NT : (MODE == kM2L2 ? 2 : 1);  // activation rows the fragment layout holds
@@ -546,46 +551,87 @@ __global__ void __launch_bounds__(kCT + 32 * (kTG == 0 ? 1 : kTG), 1) gemv_q4_st
 
   if constexpr (kDefer) {
     // ---- one activation slice, up to two rows: no per-tile meeting -------------------------------
-    int slot = 0, rot = 0, s = 0;
+    // the parked sums of tiles `tile`, `tile` - gridDim.x, ... (slot + 1 of them)
+    auto meet = [&](int tile, int slot, bool last_tile) {
+      consumer_sync();
+      QENG_STAMP(4);
+      for (int j = warp; j <= slot; j += kCW) {
+        const float* rb = red + (size_t)j * kCW * red_stride;
+        finish(tile - (slot - j) * (int)gridDim.x, [&](int a, int r) {
+          float v = 0.f;
+#pragma unroll
+          for (int w = 0; w < kCW; ++w) v += rb[w * red_stride + a * 16 + r];
+          return v;
+        });
+      }
+      if (!last_tile) consumer_sync();  // the parking area is free again
+    };
+    int slot = 0, s = 0;
     uint32_t ph = 0;
-    for (int tile = blockIdx.x; tile < p.ntiles; tile += gridDim.x) {
-      f32x2 acc[2] = {0ull, 0ull};
-      for (int c0 = 0; c0 < p.nchunks; c0 += p.stage_chunks) {
+    if (kHold && p.nchunks <= p.stage_chunks && (p.nchunks & 1) == 0) {
+      const int items = p.nchunks >> 1;
+      const bool has0 = warp < items, has1 = warp + kCW < items;
+      HeldX held;
+      if (has0) held.load(0, warp, X);
+      if (has1) held.load(1, warp + kCW, X);
+      const uint32_t wl = wl0 + (uint32_t)warp * 1024u, sl = sl0 + (uint32_t)warp * 128u;
+      uint32_t at = 0;
+      float* park_at = red + (size_t)warp * red_stride;
+#pragma unroll 1
+      for (int tile = blockIdx.x; tile < p.ntiles; tile += gridDim.x) {
+        f32x2 acc[2] = {0ull, 0ull};
         QENG_TICK(tc0);
         if (!failed && !mbar_wait(smem_u32(full + s), ph)) failed = true;
         QENG_TOCK(tc0, 8, warp == 0);
         QENG_TICK(tc1);
-        const int nc = min(p.stage_chunks, p.nchunks - c0);
-        // the warp that takes a stage's first item rotates, so that stages whose item count is not a
-        // multiple of 16 load the warps evenly over a tile
-        consume(acc, s, nc, c0 * 2, (warp + kCW - rot) & (kCW - 1), std::integral_constant<int, kCW>());
-        rot = (rot + (MODE == kM1L2 ? (nc + 1) >> 1 : nc)) & (kCW - 1);
+        if (has0) held.contract(acc, 0, wl + at, sl + at);
+        if (has1) held.contract(acc, 1, wl + at + kCW * 1024u, sl + at + kCW * 128u);
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(empty + s));
-        if (++s == NS) { s = 0; ph ^= 1u; }
+        at += stage_bytes;
+        if (++s == NS) { s = 0; ph ^= 1u; at = 0; }
         QENG_TOCK(tc1, 9, warp == 0);
         QENG_COUNT(11, warp == 0);
-      }
-      QENG_TICK(tc2);
-      park(red + ((size_t)slot * kCW + warp) * red_stride, acc);
-      const bool last_tile = tile + (int)gridDim.x >= p.ntiles;
-      if (slot == kDeferTiles - 1 || last_tile) {
-        consumer_sync();
-        QENG_STAMP(4);
-        for (int j = warp; j <= slot; j += kCW) {
-          const float* rb = red + (size_t)j * kCW * red_stride;
-          finish(tile - (slot - j) * (int)gridDim.x, [&](int a, int r) {
-            float v = 0.f;
-#pragma unroll
-            for (int w = 0; w < kCW; ++w) v += rb[w * red_stride + a * 16 + r];
-            return v;
-          });
+        park(park_at, acc);
+        park_at += kCW * red_stride;
+        const bool last_tile = tile + (int)gridDim.x >= p.ntiles;
+        if (slot == kDeferTiles - 1 || last_tile) {
+          meet(tile, slot, last_tile);
+          slot = -1;
+          park_at = red + (size_t)warp * red_stride;
         }
-        if (!last_tile) consumer_sync();  // the parking area is free again
-        slot = -1;
+        ++slot;
       }
-      ++slot;
-      QENG_TOCK(tc2, 10, warp == 0);
+    } else {
+      int rot = 0;
+      for (int tile = blockIdx.x; tile < p.ntiles; tile += gridDim.x) {
+        f32x2 acc[2] = {0ull, 0ull};
+        for (int c0 = 0; c0 < p.nchunks; c0 += p.stage_chunks) {
+          QENG_TICK(tc0);
+          if (!failed && !mbar_wait(smem_u32(full + s), ph)) failed = true;
+          QENG_TOCK(tc0, 8, warp == 0);
+          QENG_TICK(tc1);
+          const int nc = min(p.stage_chunks, p.nchunks - c0);
+          // the warp that takes a stage's first item rotates, so that stages whose item count is not a
+          // multiple of 16 load the warps evenly over a tile
+          consume(acc, s, nc, c0 * 2, (warp + kCW - rot) & (kCW - 1), std::integral_constant<int, kCW>());
+          rot = (rot + (MODE == kM1L2 ? (nc + 1) >> 1 : nc)) & (kCW - 1);
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(empty + s));
+          if (++s == NS) { s = 0; ph ^= 1u; }
+          QENG_TOCK(tc1, 9, warp == 0);
+          QENG_COUNT(11, warp == 0);
+        }
+        QENG_TICK(tc2);
+        park(red + ((size_t)slot * kCW + warp) * red_stride, acc);
+        const bool last_tile = tile + (int)gridDim.x >= p.ntiles;
+        if (slot == kDeferTiles - 1 || last_tile) {
+          meet(tile, slot, last_tile);
+          slot = -1;
+        }
+        ++slot;
+        QENG_TOCK(tc2, 10, warp == 0);
+      }
     }
   } else {
   for (int sl = 0; sl < p.nslices; ++sl) {

@@ -618,21 +618,28 @@ __global__ void __launch_bounds__(128) tc_reduce_kernel(const TcParams p) {
 
 // ---- activation rows -> one or two bf16 planes, optionally RMS-normalised on the way ----------------------
 // One CTA per row, or several (grid.y) where no norm has to see the whole row: with a few rows the chain of loads of
-// one CTA is the time (16 rows x 11008: 6 us with 256 threads a row, 2 us split).
-constexpr int kPrepThreads = 512;
-__global__ void __launch_bounds__(kPrepThreads) tc_prep_kernel(const void* __restrict__ x, int dtype, long long ldx, int K,
+// one CTA is the time (16 rows x 11008: 6 us with a row to a CTA, 2 us split).  With many rows the time is the chain of a row (loads,
+// the sum of its squares, stores) times the rounds of CTAs on an SM: 256 threads with four loads of 16 bytes on their way each take
+// 4096 values at once and leave room for 5 or 6 rows on an SM at 48 or 40 registers, where 512 threads had half of their registers
+// idle and room for 4 (a norm of 1800 rows 2 us less, prompts of 1800 tokens 18.36 -> 18.19 ms; 777 f32 rows over 11008 x 4096
+// 75.4 -> 74.8 us, of which the conversion is 7).
+constexpr int kPrepThreads = 256;
+constexpr int kPrepKeep = 4;  // loads of a thread in flight
+template <bool NORM>
+__global__ void __launch_bounds__(kPrepThreads, NORM ? 5 : 6) tc_prep_kernel(const void* __restrict__ x, int dtype, long long ldx, int K,
                                                       const float* __restrict__ gamma, float eps,
                                                       __nv_bfloat16* __restrict__ out, long long plane, int planes,
                                                       float* __restrict__ sums, int sum_blocks) {
   __shared__ float sh[kPrepThreads / 32];
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
-  if (gamma != nullptr)  // the weights of a layer pass through L2 between two uses of its gains
+  if (NORM)  // the weights of a layer pass through L2 between two uses of its gains
     for (int k = threadIdx.x * 8; k < K; k += 8 * kPrepThreads) asm volatile("prefetch.global.L1 [%0];\n" ::"l"(gamma + k));
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
   const int tid = threadIdx.x;
   const long long row = blockIdx.x;
   // K is a multiple of 32; a row of f32 may start at any 4-byte boundary
   const bool vec = dtype == QENG_F32 && ((reinterpret_cast<uintptr_t>(x) | (uintptr_t)(ldx * 4)) & 15) == 0;
+  const bool gvec = NORM && (reinterpret_cast<uintptr_t>(gamma) & 15) == 0;
   auto load4 = [&](int k, float (&v)[4]) {
     if (vec) {
       const float4 a = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(x) + row * ldx + k);
@@ -651,9 +658,17 @@ __global__ void __launch_bounds__(kPrepThreads) tc_prep_kernel(const void* __res
   auto emit = [&](int k, float (&v)[4]) {  // whole warps: the block sums are shuffled
     uint2 hi = make_uint2(0u, 0u), lo = make_uint2(0u, 0u);
     if (k < K) {
-      if (gamma != nullptr) {
+      if (NORM) {
+        float g[4];
+        if (gvec) {
+          const float4 a = *reinterpret_cast<const float4*>(gamma + k);
+          g[0] = a.x; g[1] = a.y; g[2] = a.z; g[3] = a.w;
+        } else {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) v[i] = v[i] * rs * gamma[k + i];
+          for (int i = 0; i < 4; ++i) g[i] = gamma[k + i];
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = v[i] * rs * g[i];
       }
       split2(v[0], v[1], hi.x, lo.x);
       split2(v[2], v[3], hi.y, lo.y);
@@ -677,28 +692,37 @@ __global__ void __launch_bounds__(kPrepThreads) tc_prep_kernel(const void* __res
       }
     }
   };
-  if (gamma == nullptr) {
-    for (int k = ((int)blockIdx.y * kPrepThreads + tid) * 4; (k & ~127) < K; k += 4 * kPrepThreads * (int)gridDim.y) {
-      float v[4] = {};
-      if (k < K) load4(k, v);
-      emit(k, v);
+  float v[kPrepKeep][4];
+  if (!NORM) {
+    const int step = 4 * kPrepThreads * (int)gridDim.y;
+    for (int k0 = ((int)blockIdx.y * kPrepThreads + tid) * 4; (k0 & ~127) < K; k0 += kPrepKeep * step) {
+#pragma unroll
+      for (int j = 0; j < kPrepKeep; ++j) {
+        const int k = k0 + j * step;
+        v[j][0] = v[j][1] = v[j][2] = v[j][3] = 0.f;
+        if (k < K) load4(k, v[j]);
+      }
+#pragma unroll
+      for (int j = 0; j < kPrepKeep; ++j) {
+        const int k = k0 + j * step;
+        if ((k & ~127) < K) emit(k, v[j]);
+      }
     }
     return;
   }
-  // the first kKeep * 2048 values of the row stay in registers across the reduction
-  constexpr int kKeep = 4;
-  float v[kKeep][4], ss = 0.f;
+  // the first kPrepKeep * 1024 values of the row stay in registers across the reduction
+  float ss = 0.f;
 #pragma unroll
-  for (int j = 0; j < kKeep; ++j) {
+  for (int j = 0; j < kPrepKeep; ++j) {
     const int k = (j * kPrepThreads + tid) * 4;
     v[j][0] = v[j][1] = v[j][2] = v[j][3] = 0.f;
     if (k < K) load4(k, v[j]);
   }
 #pragma unroll
-  for (int j = 0; j < kKeep; ++j)
+  for (int j = 0; j < kPrepKeep; ++j)
 #pragma unroll
     for (int i = 0; i < 4; ++i) ss = fmaf(v[j][i], v[j][i], ss);
-  for (int k = (kKeep * kPrepThreads + tid) * 4; k < K; k += 4 * kPrepThreads) {
+  for (int k = (kPrepKeep * kPrepThreads + tid) * 4; k < K; k += 4 * kPrepThreads) {
     float w[4];
     load4(k, w);
 #pragma unroll
@@ -713,11 +737,11 @@ __global__ void __launch_bounds__(kPrepThreads) tc_prep_kernel(const void* __res
   for (int w = 0; w < kPrepThreads / 32; ++w) tot += sh[w];
   rs = rsqrtf(tot / (float)K + eps);
 #pragma unroll
-  for (int j = 0; j < kKeep; ++j) {
+  for (int j = 0; j < kPrepKeep; ++j) {
     const int k = (j * kPrepThreads + tid) * 4;
     if ((k & ~127) < K) emit(k, v[j]);
   }
-  for (int k = (kKeep * kPrepThreads + tid) * 4; (k & ~127) < K; k += 4 * kPrepThreads) {
+  for (int k = (kPrepKeep * kPrepThreads + tid) * 4; (k & ~127) < K; k += 4 * kPrepThreads) {
     float w[4] = {};
     if (k < K) load4(k, w);
     emit(k, w);
@@ -916,7 +940,7 @@ int32_t qeng_tc_prep(qeng_ctx* ctx, const void* x, int32_t dtype, int64_t M, int
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = ctx->pdl ? 1 : 0;
-  QENG_CUDA(ctx, cudaLaunchKernelEx(&cfg, tc_prep_kernel, x, (int)dtype, (long long)ldx, (int)K, gamma, eps,
+  QENG_CUDA(ctx, cudaLaunchKernelEx(&cfg, gamma != nullptr ? tc_prep_kernel<true> : tc_prep_kernel<false>, x, (int)dtype, (long long)ldx, (int)K, gamma, eps,
                                     reinterpret_cast<__nv_bfloat16*>(out), (long long)(M * K), planes, sums,
                                     (int)((K / 32 + 1) / 2 * 2)));
   return QENG_OK;

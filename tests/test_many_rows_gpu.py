@@ -189,6 +189,24 @@ def test_prompt_attention_groups(ctx, heads, kv_heads):
     dec.free()
 
 
+# Norms of prompt rows wider than the 4096 values that a thread block keeps in registers: the rest is read twice, here all of
+# one warp's loads and two blocks of 1024 with a remainder.  20 rows: operands of 17 bits, so rounding stays far below 2e-3.
+@pytest.mark.parametrize("d", [4224, 6528])
+def test_norm_of_wide_prompt_rows(ctx, d):
+    from cyb_b200 import qeng
+    cfg = ref.DecoderConfig(layers=1, d=d, ffn=512, heads=2, kv_heads=1, vocab=320)
+    W = ref.make_decoder_weights(cfg, seed=7)
+    dec = ctx.decoder(layers=1, d_model=d, ffn=512, heads=2, kv_heads=1, vocab=320, max_batch=1, max_seq=32)
+    qeng.load_decoder_weights(dec, W, cfg)
+    prompt = ref.rng_of(d).integers(0, 320, (1, 20)).astype(np.int32)
+    dec.reset(1)
+    dec.prefill(prompt)
+    _, logs = ref.Decoder(cfg, W).generate(prompt, 1)
+    assert ref.err_inf(dec.logits(), logs[0]) < 2e-3
+    ctx.device_status()
+    dec.free()
+
+
 # More tiles of the prompt attention than SMs: two to a CTA, an odd number of them, ten tiles of keys through a ring of three, and
 # scores spread so far that rows are rescaled on the way.  Against the teacher the operands of the matmuls, rounded to bf16 (2^-9
 # each, of scores of some tens), leave 1e-2 (as much with any attention); against the same prompt in two calls, one tile a CTA,

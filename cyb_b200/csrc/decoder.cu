@@ -397,15 +397,23 @@ int32_t run_layer_many(qeng_ctx* ctx, qeng_decoder* d, int l, int64_t rows, int6
 }
 
 // Whether a layer's decode batch (or short prompt) of this many rows takes run_layer_batch: one rank (the fused
-// tensor-parallel exchange lives in the streaming matmul), rows that the kernel takes for every matrix.
-bool batch_fits(const qeng_ctx* ctx, const qeng_decoder* d, const Layer& L, int64_t rows) {
-  if (d->cfg.tp_world != 1 || rows >= kManyRows) return false;
-  for (const qeng_weight* w : {L.wqkv, L.wo, L.wgu, L.wdown})
-    if (!qeng_gemm_rows_fits(ctx, w, rows, 2)) return false;
+// tensor-parallel exchange lives in the streaming matmul), rows that the kernel takes for every matrix.  Four rows of 4-bit blocks go
+// with their down projection, if it is tall enough for the kernel: the others' 3 us at the most are less than a layer's
+// activations cost the integer kernel to stage in every CTA (a step of 4 sequences, 32 layers of 4096 / 11008: 2141 us there, 2028
+// here; of 3: 2023, 2030).  They went without working memory before, and still go where there is none.
+bool batch_fits(qeng_ctx* ctx, const qeng_decoder* d, const Layer& L, int64_t rows, cudaStream_t st) {
+  if (d->cfg.tp_world != 1 || rows < 4 || rows >= kManyRows) return false;
+  const qeng_weight* all[4] = {L.wqkv, L.wo, L.wgu, L.wdown};
+  for (const qeng_weight* w : all)
+    if (!qeng_gemm_rows_planned(ctx, w, rows, 2)) return false;
+  if (rows > 4) return true;
+  if (!qeng_gemm_rows_fits(ctx, L.wdown, rows, 2)) return false;
+  for (const qeng_weight* w : all)
+    if (w->fmt != QENG_FMT_Q4 || qeng_gemm_rows_reserve(ctx, w, rows, st) != QENG_OK) return false;
   return true;
 }
 
-// One layer over a decode batch (5 to 16 rows): the activations of a matmul become two bf16 planes in a small kernel
+// One layer over a decode batch (4 or 5 to 16 rows): the activations of a matmul become two bf16 planes in a small kernel
 // (with the norm, where there is one), the matmul's second kernel runs the epilogue.
 int32_t run_layer_batch(qeng_ctx* ctx, qeng_decoder* d, int l, int64_t rows, const int32_t* table, cudaStream_t st) {
   Layer& L = d->layers[l];
@@ -462,7 +470,7 @@ int32_t run_layer(qeng_ctx* ctx, qeng_decoder* d, int l, int64_t rows, int64_t T
   if ((L.qnorm == nullptr) != (L.knorm == nullptr))
     return qeng_fail(ctx, QENG_ERR_STATE, "decoder: layer %d has only one of the q / k head gains", l);
   if (rows >= kManyRows) return run_layer_many(ctx, d, l, rows, T, st);
-  if (px == nullptr && batch_fits(ctx, d, L, rows)) return run_layer_batch(ctx, d, l, rows, table, st);
+  if (px == nullptr && batch_fits(ctx, d, L, rows, st)) return run_layer_batch(ctx, d, l, rows, table, st);
   const int64_t dm = d->cfg.d_model;
   const bool fused = px != nullptr;
   float* x = fused ? *px : d->x;

@@ -25,9 +25,13 @@ using namespace qeng_tc;
 
 constexpr int kGroups = 4, kGroupWarps = 4, kWarps = kGroups * kGroupWarps, kThreadsR = (kWarps + 1) * 32;
 constexpr int kMaxRing = 16;
-// Fewer rows: the integer kernel is faster (11008 x 4096, f32: 4 rows 11.0 against 13.2 us, 8 rows 15.2 against 14; bf16: 3 rows
-// 4096 x 4096 7.1 against 5.4).
-constexpr int kLeastF32 = 5, kLeastBf16 = 3;
+// Fewer rows: the integer kernel is faster (11008 x 4096: 4 rows f32 10.8 against 11.9 us, bf16: 3 rows 4096 x 4096 7.1 against 5.4),
+// except where it has to stage so much that its ring shrinks to a few chunks a stage: 40000 values of f32 or f16 and more, over fewer
+// rows of weights than K (its stages are then short and many).  There / here, 4-bit: 4 x 11008 over 4096 16.5 / 12.6, 3 x 13824 over
+// 5120 20.6 / 15.9; 8-bit: 18.0 / 15.2, 26.5 / 21.6.  At 36864 values it is 12.8 / 11.5 and 17.2 / 13.7, at 33024 12.5 / 12.3 and
+// 16.2 / 15.1, but over more rows of weights than K 21.4 / 25.5 (3 x 11008 over 11008).
+constexpr int kLeastF32 = 5, kLeastBf16 = 3, kLeastTall = 3;
+constexpr int64_t kTallValues = 40000;
 // Beyond this many columns the tensor-memory kernel (gemm_tc.cu) takes over.  Here / there, 11008 x 4096, 4-bit: 16 rows bf16 14.2 /
 // 21.9 us, 32 rows 21.4 / 22.3, 16 rows f32 (32 columns) 19.7 / 24.6; 8-bit, 32 rows bf16 27.1 / 26.3, 16 rows f32 24.0 / 28.3;
 // K-quant, 17 rows bf16 29.7 / 28.6, 32 rows 32.5 / 28.8, 16 rows f32 22.4 / 30.8.  (Over 4096 x 4096 all are faster here.)
@@ -535,8 +539,11 @@ int32_t launch_xp(qeng_ctx* ctx, const RowsParams& p, const RowsPlan& pl, int xp
 
 }  // namespace
 
+bool qeng_gemm_rows_planned(const qeng_ctx* ctx, const qeng_weight* w, int64_t M, int planes) { return rows_plan(ctx, w, M, planes).ok; }
+
 bool qeng_gemm_rows_fits(const qeng_ctx* ctx, const qeng_weight* w, int64_t M, int planes) {
-  return M >= (planes == 1 ? kLeastBf16 : kLeastF32) && rows_plan(ctx, w, M, planes).ok;
+  const bool tall = w->fmt != QENG_FMT_K4 && w->K > w->N && M * w->K >= kTallValues;
+  return M >= (planes == 1 ? kLeastBf16 : tall ? kLeastTall : kLeastF32) && rows_plan(ctx, w, M, planes).ok;
 }
 
 static size_t planes_bytes(const qeng_weight* w, int64_t M, int planes) { return ((size_t)planes * M * w->K * 2 + 15) & ~(size_t)15; }
@@ -559,6 +566,14 @@ int32_t qeng_gemm_rows_prep(qeng_ctx* ctx, const qeng_weight* w, const float* x,
   float* sums = w->fmt == QENG_FMT_K4 ? reinterpret_cast<float*>(reinterpret_cast<char*>(sc->planes.ptr) + planes_bytes(w, M, 2)) : nullptr;
   rc = qeng_tc_prep(ctx, x, QENG_F32, M, w->K, ldx, gamma, eps, 2, sc->planes.ptr, sums, stream);
   return rc == QENG_OK ? rows_call(ctx, w, xx, QENG_BF16, true, sums, M, epi, stream, sc) : rc;
+}
+
+// the working memory of qeng_gemm_rows_prep and qeng_gemm_rows
+int32_t qeng_gemm_rows_reserve(qeng_ctx* ctx, const qeng_weight* w, int64_t M, cudaStream_t stream) {
+  const RowsPlan pl = rows_plan(ctx, w, M, 2);
+  qeng_scratch* sc = qeng_scratch_for(ctx, stream);
+  const int32_t rc = qeng_scratch_grow(ctx, sc, &sc->planes, planes_bytes(w, M, 2));
+  return rc == QENG_OK ? qeng_scratch_grow(ctx, sc, &sc->part, (size_t)pl.nsl * M * w->N * 4) : rc;
 }
 
 // made: x holds bf16 planes, with their block sums in xsum; otherwise rows of any type

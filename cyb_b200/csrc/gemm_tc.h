@@ -39,6 +39,9 @@ int32_t qeng_tc_prep(qeng_ctx* ctx, const void* x, int32_t dtype, int64_t M, int
 
 // gemm_rows.cu: a few rows (all formats) at the precision of wp = 2; planes: 1 for bf16 rows, else 2
 bool qeng_gemm_rows_fits(const qeng_ctx* ctx, const qeng_weight* w, int64_t M, int planes);
+// whether the kernel can take them at all, faster or not
+bool qeng_gemm_rows_planned(const qeng_ctx* ctx, const qeng_weight* w, int64_t M, int planes);
+int32_t qeng_gemm_rows_reserve(qeng_ctx* ctx, const qeng_weight* w, int64_t M, cudaStream_t stream);
 // rows of any type, converted by the matmul itself
 int32_t qeng_gemm_rows_raw(qeng_ctx* ctx, const qeng_weight* w, const void* x, int32_t dtype, int64_t M, int64_t ldx, const qeng_tc_epi& epi, cudaStream_t stream);
 // f32 rows, converted (and normalised, if gamma is given) by a kernel of its own: what the layers of a decoder take, where that kernel

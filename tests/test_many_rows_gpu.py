@@ -62,6 +62,47 @@ def test_few_rows_of_any_alignment(ctx, fmt, m, n, k, off, pad):
     ctx.device_status()
 
 
+# Three and four f32 / f16 rows around the line from which tall matrices leave the integer kernel (whose 15-bit activations give
+# 2e-4): 40000 values of activations, K above N.  Above it the bound of the planes.
+@pytest.mark.parametrize("fmt", ["q4", "q8"])
+@pytest.mark.parametrize("m,n,k,planes", [(4, 4096, 10016, True), (4, 272, 9984, False), (3, 1040, 13344, True), (4, 10016, 10016, False)])
+def test_few_rows_of_tall_matrices(ctx, fmt, m, n, k, planes):
+    import torch
+    w = _weight(ctx, fmt, n, k)
+    wd = w.dequant().double()
+    for dt in ("float32", "float16"):
+        x = torch.randn(m, k, device="cuda").to(getattr(torch, dt))
+        want = x.double() @ wd.T
+        err = float((ctx.gemm_q4(w, x).double() - want).abs().max() / want.abs().max())
+        assert err < (3e-5 if planes else 2e-4), (fmt, m, n, k, dt, err)
+    ctx.device_status()
+
+
+# Four sequences whose down projection is tall enough for the batch kernel take it for the whole layer.  Against the teacher; an
+# operand of 17 bits keeps far below 2e-3.
+def test_four_sequences_with_a_tall_down_projection(ctx):
+    from cyb_b200 import qeng
+    cfg = ref.DecoderConfig(layers=2, d=256, ffn=10240, heads=4, kv_heads=2, vocab=320)
+    W = ref.make_decoder_weights(cfg, seed=8)
+    dec = ctx.decoder(layers=2, d_model=256, ffn=10240, heads=4, kv_heads=2, vocab=320, max_batch=4, max_seq=32)
+    qeng.load_decoder_weights(dec, W, cfg)
+    prompt = ref.rng_of(4).integers(0, 320, (4, 3)).astype(np.int32)
+    dec.reset(4)
+    dec.prefill(prompt)
+    want, logs = ref.Decoder(cfg, W).generate(prompt, 6)
+    assert ref.err_inf(dec.logits(), logs[0]) < 2e-3
+    toks = dec.decode(6)
+    # a token may differ only where the teacher's two best logits are closer than the gate; what follows it is then free
+    for b in range(4):
+        for s in range(6):
+            if toks[b, s] != want[b, s]:
+                top = np.sort(logs[s][b])[-2:]
+                assert top[1] - top[0] < 2e-3 * np.abs(logs[s][b]).max(), (b, s)
+                break
+    ctx.device_status()
+    dec.free()
+
+
 def _plan(ctx, w, m, wp, xp, epilogue):
     """What the planner of the many-row matmul chose, for the tests below to know what they ran."""
     import ctypes

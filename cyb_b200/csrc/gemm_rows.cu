@@ -8,8 +8,9 @@
 // column tile and one fma per output value.  The contraction order inside a block is the packed one (lane t of a quad
 // holds k = 8t .. 8t+7), so A comes from one 128-bit shared load per 64 k and lane, B from one per 32 k and column tile,
 // both without conflicts.  With 32 columns the B loads are 32 of 38 shared wavefronts per chunk and bound the kernel
-// together with the MMAs (16 rows f32: shared memory busy 63 % of the cycles, the tensor pipe 41 %; 32 rows bf16: 58 and 30).  16 rows f32 over 22016 x 4096 30.7 us; 32 rows bf16 over 4096 x 11008 21.9; 8 rows bf16 over 11008 x 4096
-// 11.2 (62, 62 and 15 with the integer kernel).
+// together with the MMAs (16 rows f32: shared memory busy 63 % of the cycles, the tensor pipe 41 %; 32 rows bf16: 58 and 30).
+// 16 rows f32 over 22016 x 4096 30.7 us; 32 rows bf16 over 4096 x 11008 22.0; 8 rows bf16 over 11008 x 4096 11.3 (62, 62 and 15
+// with the integer kernel).
 //
 // Work split: K is cut into `nsl` slices so that a slice of the activations (all columns) stays in shared memory for
 // the whole kernel; a CTA owns one slice and every cps-th row tile.  A producer warp streams (tile, slice) units, which

@@ -622,18 +622,19 @@ __global__ void __launch_bounds__(128) tc_reduce_kernel(const TcParams p) {
 // the sum of its squares, stores) times the rounds of CTAs on an SM: 256 threads with four loads of 16 bytes on their way each take
 // 4096 values at once and leave room for 5 or 6 rows on an SM at 48 or 40 registers, where 512 threads had half of their registers
 // idle and room for 4 (a norm of 1800 rows 2 us less, prompts of 1800 tokens 18.36 -> 18.19 ms; 777 f32 rows over 11008 x 4096
-// 75.4 -> 74.8 us, of which the conversion is 7).
-constexpr int kPrepThreads = 256;
+// 75.4 -> 74.8 us, of which the conversion is 7).  Up to two rows to an SM, 512 threads are the shorter chain (45-token prompts and 24
+// tokens of 16 sequences: 71.6 ms, with 256 threads 72.7).
+constexpr int kPrepMany = 256, kPrepFew = 512;
 constexpr int kPrepKeep = 4;  // loads of a thread in flight
-template <bool NORM>
-__global__ void __launch_bounds__(kPrepThreads, NORM ? 5 : 6) tc_prep_kernel(const void* __restrict__ x, int dtype, long long ldx, int K,
+template <bool NORM, int THREADS>
+__global__ void __launch_bounds__(THREADS, THREADS == kPrepFew ? 2 : NORM ? 5 : 6) tc_prep_kernel(const void* __restrict__ x, int dtype, long long ldx, int K,
                                                       const float* __restrict__ gamma, float eps,
                                                       __nv_bfloat16* __restrict__ out, long long plane, int planes,
                                                       float* __restrict__ sums, int sum_blocks) {
-  __shared__ float sh[kPrepThreads / 32];
+  __shared__ float sh[THREADS / 32];
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   if (NORM)  // the weights of a layer pass through L2 between two uses of its gains
-    for (int k = threadIdx.x * 8; k < K; k += 8 * kPrepThreads) asm volatile("prefetch.global.L1 [%0];\n" ::"l"(gamma + k));
+    for (int k = threadIdx.x * 8; k < K; k += 8 * THREADS) asm volatile("prefetch.global.L1 [%0];\n" ::"l"(gamma + k));
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
   const int tid = threadIdx.x;
   const long long row = blockIdx.x;
@@ -692,37 +693,38 @@ __global__ void __launch_bounds__(kPrepThreads, NORM ? 5 : 6) tc_prep_kernel(con
       }
     }
   };
-  float v[kPrepKeep][4];
+  constexpr int kKeep = NORM || THREADS == kPrepMany ? kPrepKeep : 1;  // few rows: a thread has one load, see `parts`
+  float v[kKeep][4];
   if (!NORM) {
-    const int step = 4 * kPrepThreads * (int)gridDim.y;
-    for (int k0 = ((int)blockIdx.y * kPrepThreads + tid) * 4; (k0 & ~127) < K; k0 += kPrepKeep * step) {
+    const int step = 4 * THREADS * (int)gridDim.y;
+    for (int k0 = ((int)blockIdx.y * THREADS + tid) * 4; (k0 & ~127) < K; k0 += kKeep * step) {
 #pragma unroll
-      for (int j = 0; j < kPrepKeep; ++j) {
+      for (int j = 0; j < kKeep; ++j) {
         const int k = k0 + j * step;
         v[j][0] = v[j][1] = v[j][2] = v[j][3] = 0.f;
         if (k < K) load4(k, v[j]);
       }
 #pragma unroll
-      for (int j = 0; j < kPrepKeep; ++j) {
+      for (int j = 0; j < kKeep; ++j) {
         const int k = k0 + j * step;
         if ((k & ~127) < K) emit(k, v[j]);
       }
     }
     return;
   }
-  // the first kPrepKeep * 1024 values of the row stay in registers across the reduction
+  // the first kKeep * 4 * THREADS values of the row stay in registers across the reduction
   float ss = 0.f;
 #pragma unroll
-  for (int j = 0; j < kPrepKeep; ++j) {
-    const int k = (j * kPrepThreads + tid) * 4;
+  for (int j = 0; j < kKeep; ++j) {
+    const int k = (j * THREADS + tid) * 4;
     v[j][0] = v[j][1] = v[j][2] = v[j][3] = 0.f;
     if (k < K) load4(k, v[j]);
   }
 #pragma unroll
-  for (int j = 0; j < kPrepKeep; ++j)
+  for (int j = 0; j < kKeep; ++j)
 #pragma unroll
     for (int i = 0; i < 4; ++i) ss = fmaf(v[j][i], v[j][i], ss);
-  for (int k = (kPrepKeep * kPrepThreads + tid) * 4; k < K; k += 4 * kPrepThreads) {
+  for (int k = (kKeep * THREADS + tid) * 4; k < K; k += 4 * THREADS) {
     float w[4];
     load4(k, w);
 #pragma unroll
@@ -734,14 +736,14 @@ __global__ void __launch_bounds__(kPrepThreads, NORM ? 5 : 6) tc_prep_kernel(con
   __syncthreads();
   float tot = 0.f;
 #pragma unroll
-  for (int w = 0; w < kPrepThreads / 32; ++w) tot += sh[w];
+  for (int w = 0; w < THREADS / 32; ++w) tot += sh[w];
   rs = rsqrtf(tot / (float)K + eps);
 #pragma unroll
-  for (int j = 0; j < kPrepKeep; ++j) {
-    const int k = (j * kPrepThreads + tid) * 4;
+  for (int j = 0; j < kKeep; ++j) {
+    const int k = (j * THREADS + tid) * 4;
     if ((k & ~127) < K) emit(k, v[j]);
   }
-  for (int k = (kPrepKeep * kPrepThreads + tid) * 4; (k & ~127) < K; k += 4 * kPrepThreads) {
+  for (int k = (kKeep * THREADS + tid) * 4; (k & ~127) < K; k += 4 * THREADS) {
     float w[4] = {};
     if (k < K) load4(k, w);
     emit(k, w);
@@ -931,16 +933,20 @@ void* qeng_tensor_map_encoder() { return reinterpret_cast<void*>(encode_fn()); }
 int32_t qeng_tc_prep(qeng_ctx* ctx, const void* x, int32_t dtype, int64_t M, int64_t K, int64_t ldx, const float* gamma, float eps,
                      int planes, void* out, float* sums, cudaStream_t stream) {
   cudaLaunchConfig_t cfg = {};
-  const int64_t parts = gamma == nullptr && M < 2 * ctx->sm_count ? (K + 4 * kPrepThreads - 1) / (4 * kPrepThreads) : 1;
+  const bool few = M < 2 * ctx->sm_count;
+  const int threads = few ? kPrepFew : kPrepMany;
+  const int64_t parts = gamma == nullptr && few ? (K + 4 * threads - 1) / (4 * threads) : 1;
   cfg.gridDim = dim3((unsigned)M, (unsigned)parts);
-  cfg.blockDim = dim3(kPrepThreads);
+  cfg.blockDim = dim3((unsigned)threads);
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = ctx->pdl ? 1 : 0;
-  QENG_CUDA(ctx, cudaLaunchKernelEx(&cfg, gamma != nullptr ? tc_prep_kernel<true> : tc_prep_kernel<false>, x, (int)dtype, (long long)ldx, (int)K, gamma, eps,
+  auto* kernel = gamma != nullptr ? (few ? tc_prep_kernel<true, kPrepFew> : tc_prep_kernel<true, kPrepMany>)
+                                  : (few ? tc_prep_kernel<false, kPrepFew> : tc_prep_kernel<false, kPrepMany>);
+  QENG_CUDA(ctx, cudaLaunchKernelEx(&cfg, kernel, x, (int)dtype, (long long)ldx, (int)K, gamma, eps,
                                     reinterpret_cast<__nv_bfloat16*>(out), (long long)(M * K), planes, sums,
                                     (int)((K / 32 + 1) / 2 * 2)));
   return QENG_OK;

@@ -230,16 +230,17 @@ def test_prompt_attention_groups(ctx, heads, kv_heads):
     dec.free()
 
 
-# Norms of prompt rows wider than the 4096 values that a thread block keeps in registers: the rest is read twice, here all of
-# one warp's loads and two blocks of 1024 with a remainder.  20 rows: operands of 17 bits, so rounding stays far below 2e-3.
-@pytest.mark.parametrize("d", [4224, 6528])
-def test_norm_of_wide_prompt_rows(ctx, d):
+# Norms of prompt rows wider than what a thread block keeps in registers (4096 values from two rows to an SM on, 8192 below): the rest
+# is read twice, here one warp's loads, or two blocks of 1024 with a remainder.  Operands of 17 bits (8-bit blocks, or fewer than 256
+# rows), so rounding stays far below 2e-3.
+@pytest.mark.parametrize("d,rows,fmt", [(4224, 300, "q8"), (6528, 300, "q8"), (8256, 20, "q4")])
+def test_norm_of_wide_prompt_rows(ctx, d, rows, fmt):
     from cyb_b200 import qeng
     cfg = ref.DecoderConfig(layers=1, d=d, ffn=512, heads=2, kv_heads=1, vocab=320)
-    W = ref.make_decoder_weights(cfg, seed=7)
-    dec = ctx.decoder(layers=1, d_model=d, ffn=512, heads=2, kv_heads=1, vocab=320, max_batch=1, max_seq=32)
+    W = ref.make_decoder_weights(cfg, seed=7, fmt=fmt)
+    dec = ctx.decoder(layers=1, d_model=d, ffn=512, heads=2, kv_heads=1, vocab=320, max_batch=1, max_seq=304)
     qeng.load_decoder_weights(dec, W, cfg)
-    prompt = ref.rng_of(d).integers(0, 320, (1, 20)).astype(np.int32)
+    prompt = ref.rng_of(d).integers(0, 320, (1, rows)).astype(np.int32)
     dec.reset(1)
     dec.prefill(prompt)
     _, logs = ref.Decoder(cfg, W).generate(prompt, 1)

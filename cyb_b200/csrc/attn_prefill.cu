@@ -455,7 +455,9 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_kernel(const qeng_pr
     met[n & 1][mine][half][row] = l_run;
     meet();
     l_run += met[n & 1][mine][half ^ 1][row];
-    const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
+    // a row that attends nothing gives zeros (where no key is anybody's, O was never written); scores that are not finite give NaN
+    const bool none = l_run == 0.f;
+    const float inv = 1.f / l_run;
     __nv_bfloat16* const dst = p.out + token * p.ldo + (size_t)head * kHD + half * 64;
 #pragma unroll 1
     for (int c = 0; c < 2; ++c) {
@@ -466,7 +468,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_kernel(const qeng_pr
         uint32_t hw[4], lw[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          const float x = l_run > 0.f ? __uint_as_float(o[i + 2 * q]) * inv : 0.f, y = l_run > 0.f ? __uint_as_float(o[i + 2 * q + 1]) * inv : 0.f;
+          const float x = none ? 0.f : __uint_as_float(o[i + 2 * q]) * inv, y = none ? 0.f : __uint_as_float(o[i + 2 * q + 1]) * inv;
           hw[q] = pack_b2(x, y);
           const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&hw[q]));
           lw[q] = pack_b2(x - f.x, y - f.y);

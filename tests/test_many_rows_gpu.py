@@ -377,6 +377,37 @@ def test_prompt_rows_do_not_see_infinite_values_they_do_not_attend(ctx, window):
     dec.free()
 
 
+# The same for keys that overflow f16 (scores of both infinities, which sum to NaN): rows that attend them have no finite result, all
+# others the same bits as without.  617 rows of 32 heads make two tiles of 16 tokens a CTA; token 260 lies in the fifth stage of 64
+# keys, with a window of 116 in the second one of the tiles that it leaves.
+@pytest.mark.parametrize("rows,at,window", [(40, 20, 0), (40, 20, 8), (617, 260, 0), (617, 260, 116)])
+def test_prompt_rows_that_attend_infinite_keys(ctx, rows, at, window):
+    import torch
+    from cyb_b200 import qeng
+    heads, kv = (32, 4) if rows > 300 else (4, 2)
+    cfg = ref.DecoderConfig(layers=1, d=256, ffn=512, heads=heads, kv_heads=kv, vocab=320, sliding_window=window)
+    W = ref.make_decoder_weights(cfg, seed=5, fmt="q8")
+    q, s = W["layers"][0]["wk"]
+    q, s = q.copy(), s.copy()
+    q[:, :32], s[:, 0] = 0, 60000.0  # the first block only acts through column 0
+    q[:, 0] = 7
+    W["layers"][0]["wk"] = (q, s)
+    dec = ctx.decoder(layers=1, d_model=256, ffn=512, heads=heads, kv_heads=kv, vocab=320, max_batch=1, max_seq=640, sliding_window=window)
+    qeng.load_decoder_weights(dec, W, cfg)
+    x = torch.randn(rows, 256, device="cuda", generator=torch.Generator(device="cuda").manual_seed(3))
+    x[:, 0] = 0.0
+    plain = dec.layer(0, x, np.arange(rows))
+    assert bool(torch.isfinite(plain).all())
+    x[at, 0] = 8.0
+    got = dec.layer(0, x, np.arange(rows))
+    end = min(rows, at + window) if window else rows
+    assert not bool(torch.isfinite(got[at:end]).any())
+    rest = [r for r in range(rows) if r < at or r >= end]
+    assert torch.equal(got[rest], plain[rest])
+    ctx.device_status()
+    dec.free()
+
+
 def test_lm_head_of_infinite_activations(ctx):
     """An infinite activation makes infinite logits (of the sign of the table's entry), NaN only where infinities meet."""
     import torch

@@ -403,7 +403,7 @@ __device__ __forceinline__ void attn_decode_body(const AttnParams& p, const CUte
         L = fmaf(lr[r], f, L);
         O = fmaf(orr[r], f, O);
       }
-      p.out[((size_t)b * p.Hq + (size_t)h * p.grp + hh) * kHD + d] = L > 0.f ? O / L : 0.f;
+      p.out[((size_t)b * p.Hq + (size_t)h * p.grp + hh) * kHD + d] = L == 0.f ? 0.f : O / L;  // (an empty sequence; NaN passes)
     }
     if (cs > 1) cluster_sync();  // nobody leaves while a peer may still read its shared memory
     return;

@@ -103,6 +103,22 @@ def test_garbage_beyond_length_is_ignored(ctx):
     assert ref.err_inf(out, ref_out) < 1e-4
 
 
+# one sequence: clusters, merged through distributed shared memory; 64: splits merged in device memory, or a single one
+@pytest.mark.parametrize("B,n", [(1, 600), (1, 5), (64, 600), (64, 90)])
+def test_scores_that_are_not_finite_give_no_finite_result(ctx, B, n):
+    rng = ref.rng_of(26)
+    lens = np.full(B, n, np.int32)
+    q = rng.standard_normal((B, 8, 128), dtype=np.float32).astype(np.float16)
+    ks, vs, pool, table = ref.paged_kv(rng, lens, Hkv=2)
+    want = ref.attn_decode(q, ks, vs)
+    at = n // 2
+    pool[table[0, at // 16], 0, 0, at % 16, :] = np.float16(np.inf)  # a key of sequence 0, kv head 0
+    out = _run(ctx, q, pool, table, lens)
+    assert not np.isfinite(out[0, :4]).any()
+    out[0, :4] = want[0, :4]
+    assert ref.err_inf(out, want) < 1e-4
+
+
 def test_bad_page_id_is_reported_not_dereferenced(ctx):
     from cyb_b200 import qeng
     rng = ref.rng_of(24)

@@ -226,6 +226,7 @@ __device__ __forceinline__ void drain_pairs(const TcParams& p, int tile, uint32_
     const int at = ps;
     if (!swiglu && m + 16 < mcnt && live) ps = q.pos[m0 + m + 16];
     uint32_t v[16];
+    __syncwarp();  // lanes without a token (of the group before) or with a malformed one come from `continue`
     tmem_ld16(tacc + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, v);
 #pragma unroll
     for (int i = 0; i < 16; ++i) asm volatile("st.shared.u32 [%0], %1;\n" ::"r"(buf + (uint32_t)i * kTurnRow + (uint32_t)lane * 4u), "r"(v[i]) : "memory");
@@ -297,6 +298,7 @@ __device__ __forceinline__ void drain(const TcParams& p, int tile, bool whole, i
 #pragma unroll 1
   for (; c0 < mcnt; c0 += step) {
     uint32_t v[16];
+    __syncwarp();  // lanes of rows beyond N, or without a token, leave finish() early
     tmem_ld16(tacc + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, v);
     float f[16];
 #pragma unroll
@@ -540,6 +542,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
       const bool whole = sg.k0 == 0 && sg.k1 == p.nk;
       if (!__any_sync(0xffffffffu, failed) && whole)
         drain<true>(p, sg.tile, whole, pair, rank, tmem, warp & 3, lane, 16 * (1 + ((warp - 8) >> 2)), 16 * (1 + kHelpers / 4));
+      __syncwarp();
       asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(map_leader(smem_u32(acc_empty)));
@@ -562,6 +565,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         if (MODE == kPairs && whole) drain_pairs(p, sg.tile, rank, tmem + (uint32_t)(buf * p.acc_cols), quad, lane, ring + (uint32_t)p.nslots * kSlot);
         else drain<HELP || MODE == kPairs>(p, sg.tile, whole, pair, rank, tmem + (uint32_t)(buf * p.acc_cols), quad, lane, 0, HELP && whole ? 16 * (1 + kHelpers / 4) : 16);
       }
+      __syncwarp();
       asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(map_leader(smem_u32(acc_empty + buf)));

@@ -1,5 +1,5 @@
-"""What the kernel sources have to say for the hardware to keep it: the scope of barriers between CTAs (a missing one
-shows in no run that happens to go well)."""
+"""What the kernel sources have to say for the hardware to keep it: the scope of barriers between CTAs, converged warps (a missing
+one shows in no run that happens to go well)."""
 import glob
 import os
 import re
@@ -31,3 +31,18 @@ def test_waits_for_another_ctas_arrivals_acquire_from_the_cluster():
     fences = relay.index("fence::after_thread_sync"), relay.index("fence::before_thread_sync")
     assert relay.index("mbar_wait(") < fences[0] < fences[1] < relay.index("mbar_arrive_cluster(")
     assert "try_wait.parity.acquire.cluster" in _sources()["gemm_tc.cuh"]
+
+
+def test_lanes_that_leave_early_converge_before_tensor_memory_is_read():
+    """tcgen05.ld needs a whole warp.  Where lanes go on to the next tokens on their own (`continue`, or a return from the inlined
+    epilogue, under a condition of the lane), nothing but __syncwarp() brings them together before the next read, and before the
+    fence behind the loop."""
+    text = _sources()["gemm_tc.cu"]
+    loops = text[text.index("void drain_pairs("):text.index("// What empties an accumulator:")]
+    assert "continue;" in loops and "finish<16>(" in loops
+    assert loops.count("tmem_ld16(") == 2 == len(re.findall(r"__syncwarp\(\);[^\n]*\n *tmem_ld16\(", loops))
+    calls = list(re.finditer(r" drain(_pairs)?(<[^>]*>)?\(p, sg.tile", text))
+    assert len(calls) == 3
+    for c in calls:
+        rest = text[c.end():]
+        assert rest.index("__syncwarp();") < rest.index("tcgen05.fence::before_thread_sync")

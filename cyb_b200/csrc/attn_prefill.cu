@@ -297,7 +297,13 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_kernel(const qeng_pr
     const size_t token = (size_t)b * p.T + tt0 + at;
     const int head = h * grp + row - tok * grp;
     const uint32_t mem = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)mine * kTileCols;
-    auto meet = [&] { asm volatile("bar.sync %0, %1;\n" ::"r"(1 + mine), "n"(kSoftWarps / 2 * 32) : "memory"); };  // the tile's warps
+    // the tile's warps.  What a warp writes to tensor memory behind it (probabilities over scores) another has read before it.
+    auto meet = [&] {
+      __syncwarp();
+      fence_before();
+      asm volatile("bar.sync %0, %1;\n" ::"r"(1 + mine), "n"(kSoftWarps / 2 * 32) : "memory");
+      fence_after();
+    };
     {
       uint32_t q[32];
 #pragma unroll
@@ -306,6 +312,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_kernel(const qeng_pr
         if (live) v = *reinterpret_cast<const uint4*>(p.q16 + (token * p.Hq + head) * kHD + half * 64 + i * 8);
         q[4 * i] = v.x; q[4 * i + 1] = v.y; q[4 * i + 2] = v.z; q[4 * i + 3] = v.w;
       }
+      __syncwarp();
       tmem_st32(mem + 32 * half, q);
       st_wait();
       fence_before();
@@ -438,6 +445,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_kernel(const qeng_pr
               }
             }
           }
+          __syncwarp();
           tmem_st32(mem + kO + 32 * c, o);
         }
       }
@@ -462,6 +470,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_kernel(const qeng_pr
 #pragma unroll 1
     for (int c = 0; c < 2; ++c) {
       uint32_t o[32];
+      __syncwarp();
       tmem_ld32(mem + kO + 64 * half + 32 * c, o);
 #pragma unroll
       for (int i = 0; i < 32; i += 8) {

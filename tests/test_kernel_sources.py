@@ -46,3 +46,16 @@ def test_lanes_that_leave_early_converge_before_tensor_memory_is_read():
     for c in calls:
         rest = text[c.end():]
         assert rest.index("__syncwarp();") < rest.index("tcgen05.fence::before_thread_sync")
+
+
+def test_prompt_attention_fences_what_halves_of_a_tile_hand_over_in_tensor_memory():
+    """The probabilities of one half of a tile's warps overwrite scores that the other half has read: the barrier between stands
+    between the fences that order tensor memory, behind the reads' wait, with whole warps."""
+    text = _sources()["attn_prefill.cu"]
+    meet = text[text.index("auto meet = [&]"):]
+    meet = meet[:meet.index("};")]
+    order = [meet.index(x) for x in ("__syncwarp();", "fence_before();", "bar.sync", "fence_after();")]
+    assert order == sorted(order)
+    loop = text[text.index("tmem_ld32(mem + kS"):text.index("tmem_st16(mem + kS")]
+    assert "meet();" in loop
+    assert text[text.index("void tmem_ld32("):].index("tcgen05.wait::ld") < text[text.index("void tmem_ld32("):].index("void tmem_st32(")

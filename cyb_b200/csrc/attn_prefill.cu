@@ -156,7 +156,6 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_kernel(const qeng_pr
   const int tt0 = (int)((gridDim.x - 1 - blockIdx.x) / (unsigned)(p.Hkv * p.B)) * tpt * per_cta;
   const int ntok = min(tpt * per_cta, p.T - tt0), tiles = (ntok + tpt - 1) / tpt;
 
-  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   if (tid == 0) {
     for (int s = 0; s < kStages; ++s) {
       mbar_init(smem_u32(kfull + s), 1);
@@ -175,12 +174,16 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_kernel(const qeng_pr
   if (warp == kMmaWarp) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;\n" ::"r"(smem_u32(&tmem_slot)));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
+    // Only now, with all of the SM's tensor memory in hand: the next kernel (the output projection) takes all of it, too, before it
+    // waits for this one.  Where both fit on an SM (as compiled they do not, for registers and shared memory), one that came first
+    // would hold what this CTA waits for.
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   }
   fence_before();
-  asm volatile("griddepcontrol.wait;\n" ::: "memory");
   __syncthreads();
   fence_after();
   const uint32_t tmem = tmem_slot;
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
 
   // keys any row of the CTA attends to: [kv0, kv1); of this warp's own tile: what all its rows attend ends at len_min, begins at win_max
   const int32_t* lens = p.lens + (size_t)b * p.T + tt0;

@@ -336,7 +336,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   const uint32_t stage_bytes = KST * XP * b_plane;                 // activations: [KST][XP] planes
   const uint32_t ring = smem + (uint32_t)p.nstages * stage_bytes;  // packed-weight slots
 
-  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   if (tid == 0) {
     for (int s = 0; s < p.nstages; ++s) {
       // the CTA's own set of dequant warps; in the leader also the peer, once its set has arrived there, and the expect_tx
@@ -357,6 +356,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   if (warp == 3) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;\n" ::"r"(smem_u32(&tmem_slot)));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;\n");
+    // after the allocation: the next kernel may take all of an SM's tensor memory, too, and holds it while it waits for this one
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();

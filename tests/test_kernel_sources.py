@@ -59,3 +59,18 @@ def test_prompt_attention_fences_what_halves_of_a_tile_hand_over_in_tensor_memor
     loop = text[text.index("tmem_ld32(mem + kS"):text.index("tmem_st16(mem + kS")]
     assert "meet();" in loop
     assert text[text.index("void tmem_ld32("):].index("tcgen05.wait::ld") < text[text.index("void tmem_ld32("):].index("void tmem_st32(")
+
+
+def test_kernels_hold_their_tensor_memory_before_the_next_one_may_start():
+    """A kernel launched early takes tensor memory and keeps it while it waits for the one in front; that one must not still be
+    waiting for its own on the same SM."""
+    found = 0
+    for name, text in _sources().items():
+        for kernel in re.split(r"\n__global__ |\n *__global__ ", text)[1:]:
+            if "tcgen05.alloc" not in kernel or "griddepcontrol.launch_dependents" not in kernel:
+                continue
+            found += 1
+            # by the warp that allocates, behind it
+            assert re.search(r"tcgen05\.alloc[^}]*griddepcontrol\.launch_dependents", kernel), name
+            assert kernel.count("griddepcontrol.launch_dependents") == 1, name
+    assert found == 2

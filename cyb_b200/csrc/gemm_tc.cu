@@ -790,8 +790,12 @@ bool fit_rings(Plan* pl, int fmt, int wp, int xp) {
 //   all 106 and 163 (one waits for the other's refill).
 // Emptying an accumulator takes 17 cycles a token (store), 27 (accumulate), 12 with the dequantising warps' help, 100 (SWIGLU row by
 // row) and 250 (QKV row by row), 60 of both by drain_pairs (fitted to K of 4096: 40, 60, 80, 90 and 100 for either, prompts of 45 to
-// 1800 tokens; below 2048 the former two are kept); the next tile hides it where there are two of them (a last store then takes
-// 11).  Every tile of the first round costs 29 (the pairs' first loads meet).  Tiles cut along K pay for their parts (64 a token,
+// 1800 tokens); the next tile hides it where there are two of them (a last store then takes 11).  Two terms over K below 2048 count
+// the former two although drain_pairs empties their whole tiles as well: with 60 the plans of layers 1024 to 1920 wide come out up to
+// 6 % slower (101 and 128 tokens, 4000 of 8-bit blocks: cut tiles are then worth more than the model has them), those of 256 and 512
+// up to 15 % faster.  One term takes 60 at every K: 300 to 4000 tokens through layers 256 to 1920 wide take 2 to 23 % less than with
+// 100 and 250 (1024 wide, 1400 tokens 175 -> 147 us a layer; 1920 wide, 1000 tokens 195 -> 191), none more.
+// Every tile of the first round costs 29 (the pairs' first loads meet).  Tiles cut along K pay for their parts (64 a token,
 // 0.6 of it where another segment hides one), their sums (700 a part) and the second launch (9400).
 Plan make_plan(const qeng_ctx* ctx, const qeng_weight* w, int64_t M, int wp, int xp, int epi, bool pairs_ok, bool may_split) {
   Plan best = {};
@@ -816,7 +820,7 @@ Plan make_plan(const qeng_ctx* ctx, const qeng_weight* w, int64_t M, int wp, int
       const double mma = 2.0 * c.kst * std::max(bn, 32) * products + (one ? 34 : 0) + (two ? 106 : 0);
       const double convert = c.kst * deq + (one ? 76 : 0) + (two ? 163 : 0);
       const double stage = std::max(mma, convert);
-      const bool turned = pairs_ok && w->nchunks >= 32;
+      const bool turned = pairs_ok && (wp == 1 || w->nchunks >= 32);
       const double per_token = epi == QENG_EPI_QKV ? (turned ? 60 : 250) : epi == QENG_EPI_SWIGLU ? (turned ? 60 : 100) : epi == QENG_EPI_STORE ? (c.nacc == 1 ? 17 : 11) : c.nacc == 1 ? 12 : 27;
       const double ep = per_token * bn, body = nk * stage, tile = c.nacc == 1 ? body + ep : std::max(body, ep);
       const double dp = waves * tile + (c.nacc == 1 ? 0.0 : ep) + 29.0 * std::min(T, pairs);

@@ -151,19 +151,23 @@ def test_every_kind_of_plan(ctx, fmt, m, n, k, plan):
     ctx.device_status()
 
 
-def test_prompt_epilogues_over_several_tiles(ctx):
-    """Rotary embedding with KV append, SwiGLU and the residual adds where CTA pairs run several tiles through one
-    accumulator, then cut ones: a layer over 895 rows against the float64 teacher (operands rounded to bf16: 5e-3)."""
+# Layers narrower than 2048: 4-bit blocks (one term), several tiles a pair through two accumulators; 8-bit (two), several through
+# one, then cut ones.
+@pytest.mark.parametrize("fmt,d,plan", [("q4", 512, (2, "rounds")), ("q8", 256, (1, "mixed"))])
+def test_prompt_epilogues_over_several_tiles(ctx, fmt, d, plan):
+    """Rotary embedding with KV append, SwiGLU and the residual adds where CTA pairs run several tiles: a layer over 895 rows against
+    the float64 teacher (operands rounded to bf16: 5e-3)."""
     import torch
     from cyb_b200 import qeng
     T = 895
-    cfg = ref.DecoderConfig(layers=1, d=512, ffn=4096, heads=32, kv_heads=8, vocab=320)
-    W = ref.make_decoder_weights(cfg, seed=5)
-    dec = ctx.decoder(layers=1, d_model=512, ffn=4096, heads=32, kv_heads=8, vocab=320, max_batch=1, max_seq=896)
+    cfg = ref.DecoderConfig(layers=1, d=d, ffn=4096, heads=32, kv_heads=8, vocab=320)
+    W = ref.make_decoder_weights(cfg, seed=5, fmt=fmt)
+    dec = ctx.decoder(layers=1, d_model=d, ffn=4096, heads=32, kv_heads=8, vocab=320, max_batch=1, max_seq=896)
     qeng.load_decoder_weights(dec, W, cfg)
     SWIGLU, QKV = 3, 4
-    assert _plan(ctx, dec.weight(0, 0), T, 1, 1, QKV)[2:] == (1, "mixed")
-    assert _plan(ctx, dec.weight(0, 2), T, 1, 1, SWIGLU)[2:] == (1, "mixed")
+    terms = 1 if fmt == "q4" else 2
+    assert _plan(ctx, dec.weight(0, 0), T, terms, terms, QKV)[2:] == plan
+    assert _plan(ctx, dec.weight(0, 2), T, terms, terms, SWIGLU)[2:] == plan
     teacher = ref.Decoder(cfg, W)
     teacher.reset(1)
     x = ref.rng_of(41).standard_normal((1, T, cfg.d), dtype=np.float32)
@@ -175,11 +179,10 @@ def test_prompt_epilogues_over_several_tiles(ctx):
 
 
 def test_prompt_epilogues_of_whole_tiles(ctx):
-    """The same where the planner's constants are the ones fitted to values turned in shared memory (K of 2048 and more): whole
-    tiles of more tokens than a multiple of 16.  Against the teacher the operands rounded to bf16 leave 1e-2 here (the second
-    matrix sees products of two of them); against the same rows in two calls, in other tiles, only
-    the roundings tipped by sums in another order differ (2^-9 of single operands: 1e-3).  Three sequences give the same in another
-    order."""
+    """The same over a wider matrix (K of 2048), with whole tiles of more tokens than a multiple of 16.  Against the teacher the
+    operands rounded to bf16 leave 1e-2 here (the second matrix sees products of two of them); against the same rows in two calls,
+    in other tiles, only the roundings tipped by sums in another order differ (2^-9 of single operands: 1e-3).  Three sequences
+    give the same in another order."""
     import torch
     from cyb_b200 import qeng
     T = 601

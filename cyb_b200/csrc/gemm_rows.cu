@@ -26,11 +26,16 @@ using namespace qeng_tc;
 
 constexpr int kGroups = 4, kGroupWarps = 4, kWarps = kGroups * kGroupWarps, kThreadsR = (kWarps + 1) * 32;
 constexpr int kMaxRing = 16;
-// Fewer rows: the integer kernel is faster (11008 x 4096: 4 rows f32 10.8 against 11.9 us, bf16: 3 rows 4096 x 4096 7.1 against 5.4),
-// except where it has to stage so much that its ring shrinks to a few chunks a stage: 40000 values of f32 or f16 and more, over fewer
-// rows of weights than K (its stages are then short and many).  There / here, 4-bit: 4 x 11008 over 4096 16.5 / 12.6, 3 x 13824 over
-// 5120 20.6 / 15.9; 8-bit: 18.0 / 15.2, 26.5 / 21.6.  At 36864 values it is 12.8 / 11.5 and 17.2 / 13.7, at 33024 12.5 / 12.3 and
-// 16.2 / 15.1, but over more rows of weights than K 21.4 / 25.5 (3 x 11008 over 11008).
+// Fewer rows: the integer kernel is faster (11008 x 4096: 4 rows f32 10.8 against 11.9 us, bf16: 3 rows 4096 x 4096 7.1 against
+// 5.4), except where its shared memory does not hold the activations of all of K, so that it goes over its tiles once per slice
+// of K: from 33000 values of f32 or f16 over 8-bit blocks, from 40100 (or a K of 12300) over 4-bit ones.  From 40000 values on,
+// over fewer rows of weights than K, the calls come here.  There / here, microseconds, 4-bit and 8-bit: 4 x 11008 over 1024 14.0
+// / 7.0, 13.6 / 7.9; over 4096 16.5 / 12.5, 17.9 / 15.1; 3 x 13344 over 4096 18.7 / 13.6, 20.8 / 18.5; 4 x 10016 over 8192 18.6
+// / 17.4, 25.7 / 24.4, over 9984 21.4 / 20.4, 30.0 / 27.8.  Below the line 4-bit blocks gain nothing that every shape keeps
+// (39936 values over 4096 13.0 / 12.8, 33024 over 4096 12.3 / 11.3, over 8192 17.5 / 18.4, 29952 over 4096 11.7 / 12.5); 8-bit
+// ones would gain from 33024 values on (over 4096 16.9 / 13.1, 3 rows 16.2 / 15.0; over 8192 23.6 / 21.0), but over as many rows
+// of weights as K neither is ahead (4-bit and 8-bit, 3 x 11008 over 11008 21.2 / 25.3, 29.0 / 31.2, 3 x 13824 over 13824 35.1 /
+// 33.0, 43.2 / 50.2).
 constexpr int kLeastF32 = 5, kLeastBf16 = 3, kLeastTall = 3;
 constexpr int64_t kTallValues = 40000;
 // Beyond this many columns the tensor-memory kernel (gemm_tc.cu) takes over.  Here / there, 11008 x 4096, 4-bit: 16 rows bf16 14.2 /

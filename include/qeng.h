@@ -180,13 +180,14 @@ int32_t qeng_weight_set_next(qeng_ctx* ctx, qeng_weight* w, const qeng_weight* n
  * . dequant(W)^T, f32 accumulation.
  *   1 row, 2 to 4 (f32, f16) or 2 (bf16): integer tensor-core contraction on the codes, activations in block
  *     fixed point (22 bits for one row, 15 bits otherwise), per-block f32 scaling;
- *   to 16 (f32, f16) or 32 (bf16): the codes as exact bf16 operands, f32 / f16 activations in two bf16 terms
- *     (17 bits), per-block f32 scaling;
+ *   to 16 (f32, f16) or 32 (bf16), and 3 or 4 f32 / f16 rows over 4- and 8-bit blocks where K > N and M * K >= 40000:
+ *     the codes as exact bf16 operands, f32 / f16 activations in two bf16 terms (17 bits), per-block f32 scaling;
  *   more, and any of these that do not fit that: dequantised to two bf16 terms (17 bits), activations likewise;
  *   M >= 256 over 4-bit blocks: activations and dequantised weights rounded to bf16 (tolerance 5e-3 instead
  *     of 2e-3; f16 activations are refused).
- * The last three use working memory of the context; without room for it, rows below 256 and 8-bit or K-quant
- * blocks go through the first form in passes of 16 (K-quant: 4) rows. */
+ * The last three use working memory of the context, 3 and 4 rows over such tall matrices too (4 * M * N bytes a slice
+ * of K, at most one slice per multiprocessor); without room for it, rows below 256 and 8-bit or K-quant blocks go
+ * through the first form in passes of 16 (K-quant: 4) rows. */
 int32_t qeng_gemm_q4(qeng_ctx* ctx, const qeng_weight* w, const void* x, int32_t x_dtype,
                      int64_t M, int64_t ldx, float* y, int64_t ldy, int32_t flags, void* stream);
 /* M = 1, f32 activations: the decode GEMV. */

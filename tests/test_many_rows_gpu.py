@@ -63,18 +63,28 @@ def test_few_rows_of_any_alignment(ctx, fmt, m, n, k, off, pad):
 
 
 # Three and four f32 / f16 rows around the line from which tall matrices leave the integer kernel (whose 15-bit activations give
-# 2e-4): 40000 values of activations, K above N.  Above it the bound of the planes.
+# 2e-4): 40000 values of activations, K above N.  Above it the bound of the planes.  Which kernel it was shows where one value of
+# every block of 32 (its weights are zero) is 2^16 times the largest of the others: nothing is left of those in fixed point per block.
 @pytest.mark.parametrize("fmt", ["q4", "q8"])
 @pytest.mark.parametrize("m,n,k,planes", [(4, 4096, 10016, True), (4, 272, 9984, False), (3, 1040, 13344, True), (4, 10016, 10016, False)])
 def test_few_rows_of_tall_matrices(ctx, fmt, m, n, k, planes):
     import torch
-    w = _weight(ctx, fmt, n, k)
+    w = torch.randn(n, k, device="cuda") * 0.05
+    w[:, ::32] = 0.0
+    w = ctx.quantize_q4(w) if fmt == "q4" else ctx.quantize_q8(w)
     wd = w.dequant().double()
     for dt in ("float32", "float16"):
         x = torch.randn(m, k, device="cuda").to(getattr(torch, dt))
         want = x.double() @ wd.T
         err = float((ctx.gemm_q4(w, x).double() - want).abs().max() / want.abs().max())
         assert err < (3e-5 if planes else 2e-4), (fmt, m, n, k, dt, err)
+        x = (torch.rand(m, k, device="cuda") * 2.0 ** -16).to(getattr(torch, dt))
+        x[:, ::32] = 1.0
+        want, y = x.double() @ wd.T, ctx.gemm_q4(w, x).double()
+        if planes:
+            assert float((y - want).abs().max() / want.abs().max()) < 3e-5, (fmt, m, n, k, dt)
+        else:
+            assert not bool(y.any()), (fmt, m, n, k, dt)
     ctx.device_status()
 
 

@@ -33,17 +33,18 @@ SHAPES = [("q4", 3, "bfloat16"), ("q4", 4, "bfloat16"), ("q8", 8, "float32"), ("
 N, K = 2064, 1280
 
 
-@pytest.mark.parametrize("fmt,m,dt", SHAPES)
-def test_captured_matmul_has_a_workspace_of_its_own(ctx, fresh, fmt, m, dt):
+# three and four rows over tall matrices (40000 values of activations and more) need slices, too
+@pytest.mark.parametrize("fmt,m,dt,n,k", [s + (N, K) for s in SHAPES] + [("q4", 4, "float32", 1040, 10016), ("q8", 3, "float16", 272, 13344)])
+def test_captured_matmul_has_a_workspace_of_its_own(ctx, fresh, fmt, m, dt, n, k):
     """The first call of the context is captured; its graph is replayed beside calls on the stream that did not capture,
     and after calls that outgrow and displace every stream's buffers."""
     import torch
-    w0 = _weight(ctx, fmt, N, K)
-    w = _weight(fresh, fmt, N, K)
-    x = torch.randn(m, K, device="cuda").to(getattr(torch, dt))
-    x2 = torch.randn(m, K, device="cuda").to(getattr(torch, dt))
+    w0 = _weight(ctx, fmt, n, k)
+    w = _weight(fresh, fmt, n, k)
+    x = torch.randn(m, k, device="cuda").to(getattr(torch, dt))
+    x2 = torch.randn(m, k, device="cuda").to(getattr(torch, dt))
     want, want2 = ctx.gemm_q4(w0, x), ctx.gemm_q4(w0, x2)  # loads the kernels, too
-    y = torch.zeros(m, N, device="cuda")
+    y = torch.zeros(m, n, device="cuda")
     torch.cuda.synchronize()
     g = torch.cuda.CUDAGraph()
     with torch.cuda.graph(g):
@@ -60,7 +61,7 @@ def test_captured_matmul_has_a_workspace_of_its_own(ctx, fresh, fmt, m, dt):
         y2 = fresh.gemm_q4(w, x2)
     torch.cuda.synchronize()
     assert torch.equal(y, want) and torch.equal(y2, want2)
-    big = torch.randn(4 * m, K, device="cuda").to(getattr(torch, dt))
+    big = torch.randn(4 * m, k, device="cuda").to(getattr(torch, dt))
     for s in [torch.cuda.Stream() for _ in range(10)]:
         with torch.cuda.stream(s):
             fresh.gemm_q4(w, big)
@@ -288,3 +289,63 @@ def test_calls_that_find_no_memory_for_their_workspace(ctx, fresh):
         assert float((out - y).norm() / y.norm()) < 3e-4, w.fmt
     assert ref.err_inf(held.cpu().numpy(), want) < 1e-4
     args[0].free()
+
+
+def _fill_device():
+    """Blocks of device memory that leave none of 512 bytes (past torch's cache, which keeps to whole megabytes)."""
+    import ctypes
+    rt = ctypes.CDLL("libcudart.so.12")
+    held, size = [], 1 << 36
+    while size >= 512:
+        p = ctypes.c_void_p()
+        if rt.cudaMalloc(ctypes.byref(p), ctypes.c_size_t(size)) == 0:
+            held.append(p)
+        else:
+            rt.cudaGetLastError()
+            size >>= 1
+    return lambda: [rt.cudaFree(p) for p in held]
+
+
+def test_few_rows_of_tall_matrices_that_find_no_memory(ctx, fresh):
+    """Three and four rows over a tall matrix, and the layers of four sequences with such a down projection, go through the integer
+    kernel (15 bits per block) where there is no room for the slices of the other one (17 bits), and through that one again
+    afterwards."""
+    import torch
+    from cyb_b200 import qeng
+    calls = []
+    for fmt, m, n, k in (("q4", 4, 1040, 10016), ("q8", 3, 1040, 13344)):
+        w, small = _weight(fresh, fmt, n, k), _weight(ctx, fmt, n, 9984)
+        x = torch.randn(m, k, device="cuda")
+        calls.append((w, x, ctx.gemm_q4(w, x), torch.empty(m, n, device="cuda")))
+        ctx.gemm_q4(small, x[:, :9984])  # loads the integer kernel
+    cfgs = [ref.DecoderConfig(layers=1, d=256, ffn=f, heads=4, kv_heads=2, vocab=320) for f in (9984, 10240)]
+    prompt = ref.rng_of(4).integers(0, 320, (4, 1)).astype(np.int32)
+    decs = []
+    for c, cfg in zip((ctx, fresh), cfgs):
+        decs.append(c.decoder(layers=1, d_model=256, ffn=cfg.ffn, heads=4, kv_heads=2, vocab=320, max_batch=4, max_seq=32))
+        W = ref.make_decoder_weights(cfg, seed=8)
+        qeng.load_decoder_weights(decs[-1], W, cfg)
+        decs[-1].reset(4)
+    decs[0].prefill(prompt)
+    decs[0].logits()
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    release = _fill_device()
+    try:
+        for w, x, y, out in calls:
+            fresh.gemm_q4(w, x, out=out)
+        decs[1].prefill(prompt)
+        torch.cuda.synchronize()
+        without = decs[1].logits()
+    finally:
+        release()
+    for w, x, y, out in calls:
+        assert 0.0 < float((out - y).norm() / y.norm()) < 3e-4, w.fmt
+        assert torch.equal(fresh.gemm_q4(w, x), y)
+    decs[1].reset(4)
+    decs[1].prefill(prompt)
+    _, logs = ref.Decoder(cfgs[1], W).generate(prompt, 1)
+    assert ref.err_inf(without, logs[0]) < 2e-3 and ref.err_inf(decs[1].logits(), logs[0]) < 2e-3
+    assert not np.array_equal(decs[1].logits(), without)
+    for d in decs:
+        d.free()

@@ -399,8 +399,8 @@ int32_t run_layer_many(qeng_ctx* ctx, qeng_decoder* d, int l, int64_t rows, int6
 // Whether a layer's decode batch (or short prompt) of this many rows takes run_layer_batch: one rank (the fused
 // tensor-parallel exchange lives in the streaming matmul), rows that the kernel takes for every matrix.  Four rows of 4-bit blocks go
 // with their down projection, if it is tall enough for the kernel: the others' 3 us at the most are less than a layer's
-// activations cost the integer kernel to stage in every CTA (a step of 4 sequences, 32 layers of 4096 / 11008: 2141 us there, 2028
-// here, 1998 in another run; of 3: 2023, 2030).  They went without working memory before, and still go where there is none.
+// activations cost the integer kernel to stage in every CTA (a step of 4 sequences, 32 layers of 4096 / 11008: 2133 us there, 2005
+// here; of 3: 2023, 2030).  They went without working memory before, and still go where there is none.
 bool batch_fits(qeng_ctx* ctx, const qeng_decoder* d, const Layer& L, int64_t rows, cudaStream_t st) {
   if (d->cfg.tp_world != 1 || rows < 4 || rows >= kManyRows) return false;
   const qeng_weight* all[4] = {L.wqkv, L.wo, L.wgu, L.wdown};

@@ -181,21 +181,17 @@ struct BlkScales {
   float2 me, mo;  // minima (KQ only)
 };
 template <bool KQ>
-__device__ __forceinline__ uint32_t scale_chunk_bytes() { return KQ ? 256u : 64u; }
-template <bool KQ>
-__device__ __forceinline__ BlkScales<KQ> load_scales(uint32_t sbase, int ch, int g, bool live = true) {
+__device__ __forceinline__ BlkScales<KQ> load_scales(uint32_t sbase, int ch, int g) {
   BlkScales<KQ> r;
   if (KQ) {
-    uint4 a = lds128(sbase + (uint32_t)ch * 256u + (uint32_t)g * 32u);
-    uint4 b = lds128(sbase + (uint32_t)ch * 256u + (uint32_t)g * 32u + 16u);
-    if (!live) a = b = make_uint4(0u, 0u, 0u, 0u);
+    const uint4 a = lds128(sbase + (uint32_t)ch * 256u + (uint32_t)g * 32u);
+    const uint4 b = lds128(sbase + (uint32_t)ch * 256u + (uint32_t)g * 32u + 16u);
     r.se = make_float2(__uint_as_float(a.x), __uint_as_float(a.y));
     r.so = make_float2(__uint_as_float(a.z), __uint_as_float(a.w));
     r.me = make_float2(__uint_as_float(b.x), __uint_as_float(b.y));
     r.mo = make_float2(__uint_as_float(b.z), __uint_as_float(b.w));
   } else {
-    uint2 s2 = lds64(sbase + (uint32_t)ch * 64u + (uint32_t)g * 8u);
-    if (!live) s2 = make_uint2(0u, 0u);
+    const uint2 s2 = lds64(sbase + (uint32_t)ch * 64u + (uint32_t)g * 8u);
     r.se = __half22float2(*reinterpret_cast<const __half2*>(&s2.x));
     r.so = __half22float2(*reinterpret_cast<const __half2*>(&s2.y));
     r.me = r.mo = make_float2(0.f, 0.f);

@@ -191,9 +191,9 @@ struct Words<QENG_FMT_Q8> {
 // 16 tokens of the warp's 32 rows are turned in shared memory, so that a lane has the 16 rows of one row tile for one token: its
 // angles are four loads of 16 bytes, its results one or two stores of 16.  With a lane's row of every token the exchange between
 // lanes, the addresses and the 2-byte stores were some 30 instructions a token, which the epilogue's four warps issue between
-// those of sixteen dequantising ones: 160 tokens of q|k|v took longer than the tile's MMAs.  1800 tokens (ncu): q|k|v 6144 x 4096
-// 118 us and 9 for the sums of its cut tiles -> 86 with none cut, gate|up 290 and 8 -> 274; a prompt of 16 x 45 tokens through 32
-// layers 9.46 -> 8.07 ms, of 1800 20.1 -> 18.2.  (Asking for positions, angles and pages ahead, row by row, gave nothing: 130 us.)
+// those of sixteen dequantising ones: 160 tokens of q|k|v took longer than the tile's MMAs.  1800 tokens (ncu, both in one run):
+// q|k|v 6144 x 4096 112 us and 9 for the sums of its cut tiles -> 82 with none cut, gate|up 272 and 7 -> 258; a prompt of 16 x 45
+// tokens through 32 layers 9.46 -> 8.07 ms.  (Asking for positions, angles and pages ahead, row by row, gave nothing: 130 us.)
 constexpr uint32_t kTurnRow = 36 * 4, kTurnBytes = 4 * 16 * kTurnRow;  // 16 bytes between rows: no bank conflicts either way
 __device__ __forceinline__ void drain_pairs(const TcParams& p, int tile, uint32_t rank, uint32_t tacc, int quad, int lane, uint32_t turn) {
   int mt, nt;
@@ -626,9 +626,9 @@ __global__ void __launch_bounds__(128) tc_reduce_kernel(const TcParams p) {
 // one CTA is the time (16 rows x 11008: 6 us with a row to a CTA, 2 us split).  With many rows the time is the chain of a row (loads,
 // the sum of its squares, stores) times the rounds of CTAs on an SM: 256 threads with four loads of 16 bytes on their way each take
 // 4096 values at once and leave room for 5 or 6 rows on an SM at 48 or 40 registers, where 512 threads had half of their registers
-// idle and room for 4 (a norm of 1800 rows 2 us less, prompts of 1800 tokens 18.36 -> 18.19 ms; 777 f32 rows over 11008 x 4096
-// 75.4 -> 74.8 us, of which the conversion is 7).  Up to two rows to an SM, 512 threads are the shorter chain (45-token prompts and 24
-// tokens of 16 sequences: 71.6 ms, with 256 threads 72.7).
+// idle and room for 4 (ncu: a norm of 1800 rows 15.4 -> 13.3 us; the call of a prompt of 1800 tokens 21.20 -> 21.08 ms; the
+// conversion of 777 f32 rows is no faster for it).  Up to two rows to an SM, 512 threads are the shorter chain (45-token prompts and
+// 24 tokens of 16 sequences: 71.6 ms, with 256 threads 72.7).
 constexpr int kPrepMany = 256, kPrepFew = 512;
 constexpr int kPrepKeep = 4;  // loads of a thread in flight
 template <bool NORM, int THREADS>

@@ -184,9 +184,10 @@ __global__ void __launch_bounds__(kCT + 32 * (kTG == 0 ? 1 : kTG), 1) gemv_q4_st
   // kDeferTiles tiles), where the warps sum the partials and run the epilogues of the tiles in parallel
   constexpr bool kDefer = kTG == 0;
   // 4-bit blocks, items of one chunk (one row in three limbs, or two rows): a matrix whose tiles are one stage has a loop of its own
-  // (22016 x 4096, 22 bits 11.4 -> 9.9 us, 11008 x 4096 7.1 -> 6.5, 4096 x 4096 4.5 -> 4.4; decode steps +-0).  One row in two
-  // limbs has not: alone it gains as much (10.4 -> 9.6), but a decode step runs that kernel over both kinds of matrix in turn, and
-  // with both loops in it the step takes 1328 us where it takes 1270 with one.
+  // (kernels alone, 22 bits: 22016 x 4096 11.4 -> 9.9 us, 11008 x 4096 7.1 -> 6.5, 4096 x 4096 4.5 -> 4.3, where a call takes 6.6
+  // either way; decode steps of one sequence 1274 -> 1272 us, of two 1418 -> 1405).  One row in two limbs has not: alone it gains as
+  // much (10.4 -> 9.6), but a decode step runs that kernel over both kinds of matrix in turn, and with both loops in it the step takes
+  // 1328 us where it takes 1270 with one.
   constexpr bool kHold = !Q8 && !KQ && (MODE == kM1L3 || MODE == kM2L2);
   constexpr int kTGe = kDefer ? 1 : kTG;  // tile groups (rings, producer warps)
   constexpr int kGW = kCW / kTGe;         // warps per tile group

@@ -11,7 +11,7 @@
 // than 2^8 since it was last (the probabilities stay below 256, exact in two f16 terms as before).
 //
 // Least time: 64 keys of a tile are 32 MMAs of 16 columns (9.4 cycles each) and 8 of 128 (64): 815 cycles a tile, 37 K cycles
-// for the 450 tiles of 1800 tokens, 32 query and 8 kv heads, on 148 SMs.  There a layer takes 68 us (ncu; 152 with mma.sync,
+// for the 456 tiles of 1800 tokens, 32 query and 8 kv heads, on 148 SMs.  There a layer takes 68 us (ncu; 152 with mma.sync,
 // whose pipe alone needs 73): what is left is the chain of a tile (scores, softmax, values, the hops between them), which two
 // tiles a CTA hide by half.  128 tokens behind nothing 13.7 us (15.5), 16 x 45 tokens 13-16 (14.8): launch, first page, one
 // chain.  A softmax of four warps a tile, a lane all 64 keys: 77 us.

@@ -12,6 +12,7 @@ int32_t qeng_fail(qeng_ctx* ctx, int32_t code, const char* fmt, ...) {
   vsnprintf(buf, sizeof buf, fmt, ap);
   va_end(ap);
   if (ctx) ctx->err = buf;
+  if (code == QENG_ERR_CUDA) (void)cudaGetLastError();  // the caller has it: it is not the next launch's
   return code;
 }
 

@@ -67,3 +67,13 @@ def test_embed_rejects_bad_token(ctx):
     ctx.embed(tb, _t(np.array([3, 11], np.int32)))
     with pytest.raises(qeng.QengError):
         ctx.device_status()
+
+
+def test_a_failed_allocation_is_not_the_next_launchs_error(ctx):
+    from cyb_b200 import qeng
+    with pytest.raises(qeng.QengError):
+        ctx.kv_pool(1 << 30, 8)  # 64 TB
+    test_rmsnorm(ctx)
+    with pytest.raises(qeng.QengError):
+        ctx.decoder(layers=1, d_model=128, ffn=128, heads=8, kv_heads=8, vocab=32, max_batch=16, max_seq=1 << 26)  # a cache of 4 TB
+    test_rmsnorm(ctx)

@@ -292,24 +292,50 @@ __device__ __forceinline__ void drain(const TcParams& p, int tile, bool whole, i
   int mt, nt;
   tile_pos(p, tile, mt, nt);
   const int m0 = mt * p.bn, mcnt = min(p.bn, p.M - m0), row = quad * 32 + lane;
-  float* const mine = whole ? nullptr : partial(p, pair, tile - p.dp_tiles, rank, row);
+  const int n = nt * 256 + (int)rank * 128 + row;
   qeng_tc_epi e = p.e;
   if (FIXED) e.kind = QENG_EPI_ACCUM;
-#pragma unroll 1
-  for (; c0 < mcnt; c0 += step) {
+  auto load = [&](int c, float (&f)[16]) {
     uint32_t v[16];
-    // Lanes leave finish() apart where rows of the warp lie beyond N (a multiple of 16), or where the epilogue gives them tokens of
-    // their own.  (Asked for everywhere, 777 f32 rows over 11008 x 4096 take 0.4 us of 74 longer, so 0.1.)
-    if (e.kind > QENG_EPI_ACCUM || (p.N & 16) != 0) __syncwarp();
-    tmem_ld16(tacc + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, v);
-    float f[16];
+    tmem_ld16(tacc + ((uint32_t)(quad * 32) << 16) + (uint32_t)c, v);
 #pragma unroll
     for (int i = 0; i < 16; ++i) f[i] = __uint_as_float(v[i]);
-    if (whole) {
-      finish<16>(e, p.N, p.status, nt * 256 + (int)rank * 128 + row, m0 + c0, mcnt - c0, f, lane);
-    } else {
+  };
+  // Loops without a condition of a lane's own stay whole.  In the last one lanes part where rows lie beyond N (a multiple of 16), or
+  // where the epilogue gives them tokens of their own, and are brought together before the next load.  (One loop for all, with
+  // that in it: 777 f32 rows over 11008 x 4096 70.1 us, 900 over 22016 x 4096 154.0, 8192 bf16 over 4096 x 11008 590; so 67.7, 145.1,
+  // 568.  Rows added to y are no faster in a loop of their own.)
+  if (!whole) {
+    float* const mine = partial(p, pair, tile - p.dp_tiles, rank, row);
+#pragma unroll 1
+    for (; c0 < mcnt; c0 += step) {
+      float f[16];
+      load(c0, f);
 #pragma unroll
       for (int i = 0; i < 16; i += 4) __stcg(reinterpret_cast<float4*>(mine + (size_t)(c0 + i) * 128), make_float4(f[i], f[i + 1], f[i + 2], f[i + 3]));
+    }
+  } else if (!FIXED && e.kind == QENG_EPI_STORE && n - lane + 32 <= p.N) {
+#pragma unroll 1
+    for (; c0 < mcnt; c0 += step) {
+      float f[16];
+      load(c0, f);
+      float* const dst = e.y + (size_t)(m0 + c0) * e.ldy + n;
+      if (mcnt - c0 >= 16) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) dst[(size_t)i * e.ldy] = f[i];
+      } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+          if (i < mcnt - c0) dst[(size_t)i * e.ldy] = f[i];
+      }
+    }
+  } else {
+#pragma unroll 1
+    for (; c0 < mcnt; c0 += step) {
+      float f[16];
+      if (e.kind > QENG_EPI_ACCUM || (p.N & 16) != 0) __syncwarp();
+      load(c0, f);
+      finish<16>(e, p.N, p.status, n, m0 + c0, mcnt - c0, f, lane);
     }
   }
 }

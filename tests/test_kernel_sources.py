@@ -38,9 +38,12 @@ def test_lanes_that_leave_early_converge_before_tensor_memory_is_read():
     epilogue, under a condition of the lane), nothing but __syncwarp() brings them together before the next read, and before the
     fence behind the loop."""
     text = _sources()["gemm_tc.cu"]
-    loops = text[text.index("void drain_pairs("):text.index("// What empties an accumulator:")]
-    assert "continue;" in loops and "finish<16>(" in loops
-    assert loops.count("tmem_ld16(") == 2 == len(re.findall(r"__syncwarp\(\);[^\n]*\n *tmem_ld16\(", loops))
+    pairs = text[text.index("void drain_pairs("):text.index("// ---- one warp's part of a finished accumulator")]
+    assert "continue;" in pairs and pairs.count("tmem_ld16(") == 1 and re.search(r"__syncwarp\(\);[^\n]*\n *tmem_ld16\(", pairs)
+    rows = text[text.index("// ---- one warp's part of a finished accumulator"):text.index("// What empties an accumulator:")]
+    assert rows.count("tmem_ld16(") == 1 and rows.count(" load(c0, f);") == 3
+    assert rows.count("finish<16>(") == 1 and re.search(r"__syncwarp\(\);\n *load\(c0, f\);\n *finish<16>\(", rows)
+    assert "lane" not in rows[rows.index("if (!whole) {"):rows.index("} else if (!FIXED")]  # the other loops ask lanes for nothing
     calls = list(re.finditer(r" drain(_pairs)?(<[^>]*>)?\(p, sg.tile", text))
     assert len(calls) == 3
     for c in calls:
